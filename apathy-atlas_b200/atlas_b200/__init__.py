@@ -195,10 +195,26 @@ def _ptr(t) -> Optional[int]:
     return t.data_ptr()
 
 
+_current_stream = None
+
+
+def _bind_current_stream():
+    """A function returning the address of torch's current stream: the raw accessor where torch has it (0.1 us instead of the
+    1 us that building a Stream object costs on every call), else the public one."""
+    global _current_stream
+    import torch
+    torch.cuda.current_stream()                       # initialises CUDA
+    raw, device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+    if raw is not None and device is not None:
+        _current_stream = lambda: raw(device())
+    else:
+        _current_stream = lambda: torch.cuda.current_stream().cuda_stream
+    return _current_stream
+
+
 def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        return (_current_stream or _bind_current_stream())()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
