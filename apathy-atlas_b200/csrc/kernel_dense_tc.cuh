@@ -83,22 +83,27 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
             tma_load_2d(st + D_W_BYTES, &map_x, int32_t((kb_lo + it) * KB), int32_t(m0), BAR_FULL + 8 * s);
             if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
+        // (the whole warp, converged; one elected lane issues: see elect_one)
         constexpr uint32_t idesc = make_idesc_bf16(MT, 128u);
         uint32_t s = 0, ph = 0;
         bool ok = true;
         for (uint32_t it = 0; it < num_kb; ++it) {
-            ok = mbar_wait(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, 20);
+            ok = mbar_wait_warp(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, 20);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t st = smem_base + s * C::STAGE_BYTES;
             const uint64_t wd = make_kmajor_sw128_desc(st), xd = make_kmajor_sw128_desc(st + D_W_BYTES);
+            if (elect_one()) {
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) umma_bf16_ss<false>(tmem_acc, wd + 2 * j, xd + 2 * j, idesc, (it | j) ? 1u : 0u);
-            umma_commit<false>(BAR_EMPTY + 8 * s);
+                for (uint32_t j = 0; j < 4; ++j) umma_bf16_ss<false>(tmem_acc, wd + 2 * j, xd + 2 * j, idesc, (it | j) ? 1u : 0u);
+                umma_commit<false>(BAR_EMPTY + 8 * s);
+            }
+            __syncwarp();
             if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit<false>(BAR_ACC);
+        if (ok && elect_one()) umma_commit<false>(BAR_ACC);
+        __syncwarp();
     } else if (warp >= 2) {
         // ---- epilogue: lane = feature, TMEM column = token ----
         const uint32_t q = warp & 3u;

@@ -265,7 +265,8 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     tc::tma_load_3d(st + SHT_X_BYTES + ci * rank_pad * 128u, &map_a, k0, 0, int32_t(cslot[ci]), BAR_FULL + 8 * s);
                 if (prof) t_a += clock64() - i0;
             }
-        } else if (have_acc && warp == 4 && lane == 0) {
+        } else if (have_acc && warp == 4) {
+            // (the whole warp, converged; one elected lane issues: see tc::elect_one)
             // ================================ MMA issue ================================
             // The adapters' A tiles lie one after the other in a stage and their accumulators side by side in tensor memory,
             // so one MMA covers as many adapters as fit into 256 columns.
@@ -273,7 +274,7 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
             for (uint32_t i = 0; ok && i < n_ks; ++i) {
                 const uint32_t s = i % n_stages;
                 const long long w0 = prof ? clock64() : 0;
-                ok = tc::mbar_wait(BAR_FULL + 8 * s, (full_par >> s) & 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, 20);
+                ok = tc::mbar_wait_warp(BAR_FULL + 8 * s, (full_par >> s) & 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, 20);
                 if (prof) t_wait += clock64() - w0;
                 if (!ok) break;
                 full_par ^= 1u << s;
@@ -284,15 +285,19 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                 for (uint32_t c0 = 0; c0 < n_cs; c0 += per_mma) {
                     const uint32_t idesc = tc::make_idesc_bf16(min(per_mma, n_cs - c0) * rank_pad, 128u);
                     const uint64_t ad = tc::make_kmajor_sw128_desc(st + SHT_X_BYTES + c0 * rank_pad * 128u);
+                    if (tc::elect_one()) {
 #pragma unroll
-                    for (uint32_t j = 0; j < 4; ++j)     // 16 k = 32 bytes along the swizzled 128-byte rows
-                        tc::umma_bf16_ss<false>(tmem_acc + c0 * rank_pad, xd + 2 * j, ad + 2 * j, idesc, (i | j) ? 1u : 0u);
+                        for (uint32_t j = 0; j < 4; ++j)     // 16 k = 32 bytes along the swizzled 128-byte rows
+                            tc::umma_bf16_ss<false>(tmem_acc + c0 * rank_pad, xd + 2 * j, ad + 2 * j, idesc, (i | j) ? 1u : 0u);
+                    }
+                    __syncwarp();
                 }
                 const long long i1 = prof ? clock64() : 0;
-                tc::umma_commit<false>(BAR_EMPTY + 8 * s);
+                if (tc::elect_one()) tc::umma_commit<false>(BAR_EMPTY + 8 * s);
+                __syncwarp();
                 if (prof) { t_a += i1 - i0; t_b += clock64() - i1; }
             }
-            if (ok) tc::umma_commit<false>(BAR_ACC);
+            if (ok && tc::elect_one()) tc::umma_commit<false>(BAR_ACC);
         }
         __syncwarp();
 

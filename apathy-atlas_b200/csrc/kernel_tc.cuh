@@ -31,7 +31,7 @@
 // Warp roles (14 warps, 448 threads):
 //   warp 0        TMA producer: activation tiles, raw weight stages (packed codes + scale bytes),
 //                 LoRA operand tiles, each through its own mbarrier ring
-//   warp 1        TMEM allocation, tcgen05.mma issue, tcgen05.commit (in a pair: the first CTA's thread
+//   warp 1        TMEM allocation, tcgen05.mma issue, tcgen05.commit (in a pair: the first CTA's warp
 //                 issues for both)
 //   warps 2-5     build the tile's granule list while the main loop runs; then the epilogue
 //   warps 6-13    A16: expand raw NVFP4 into the BF16 weight operand (TMEM); A4: scale bytes -> TMEM;
@@ -218,6 +218,47 @@ __device__ __forceinline__ bool mbar_wait_timed(uint32_t bar, uint32_t parity, v
     if (!timed) return mbar_wait(bar, parity, abort_flag, code, backoff_ns);
     const long long t0 = clock64();
     const bool ok = mbar_wait(bar, parity, abort_flag, code, backoff_ns);
+    acc += (unsigned long long)(clock64() - t0);
+    return ok;
+}
+
+// One lane of a converged warp (the same one every time): the issuer of a tcgen05.mma / commit group.
+//
+// The MMA role is run by its WHOLE warp, converged, and only the instructions themselves are under elect_one().  Run by a
+// single lane inside a divergent branch, every operand (descriptors, tensor-memory addresses) has to be moved to a uniform
+// register for every instruction: about 67 cycles per MMA plus 380 per K block, measured on a pair of CTAs with nothing
+// else in the loop, however many columns the MMA has — 655 cycles per K block of four 256-column MMAs that take 512, 920
+// per block of eight 192-column ones that take 768.  Converged: 513 and 769.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0u;
+}
+
+// mbar_wait by a whole converged warp: every lane polls, every decision is a vote, so the lanes stay together.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t code,
+                                               uint32_t backoff_ns = 0) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    const uint64_t t0 = global_timer_ns();
+    uint32_t spins = 0;
+    while (true) {
+        if (backoff_ns) __nanosleep(backoff_ns);
+        if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+        if ((++spins & 63u) == 0u) {
+            const bool aborted = *abort_flag != 0u, late = global_timer_ns() - t0 > WAIT_LIMIT_NS;
+            if (__any_sync(0xFFFFFFFFu, aborted || late)) {
+                if (late && !aborted) record_status(code);
+                *abort_flag = 1u;
+                return false;
+            }
+        }
+    }
+}
+__device__ __forceinline__ bool mbar_wait_warp_timed(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t code,
+                                                     bool timed, unsigned long long& acc, uint32_t backoff_ns = 0) {
+    if (!timed) return mbar_wait_warp(bar, parity, abort_flag, code, backoff_ns);
+    const long long t0 = clock64();
+    const bool ok = mbar_wait_warp(bar, parity, abort_flag, code, backoff_ns);
     acc += (unsigned long long)(clock64() - t0);
     return ok;
 }
@@ -840,87 +881,84 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
     } else if (warp == 1) {
         // ===================================== MMA issuer =======================================
-        // One thread runs this role.  tcgen05.mma issue blocks once a couple of instructions are
-        // queued, so whatever this thread executes between the last MMA of one K block and the
-        // first of the next must fit inside that short queue or the tensor pipe drains: the loop
-        // carries its stage/phase/operand addresses incrementally and waits on ONE barrier per block.
-        if (lane == 0 && leader) {
+        // The whole warp runs this role, converged; one elected lane issues (see elect_one).
+        if (leader) {
             constexpr uint32_t idesc = make_idesc_bf16(MT, 128u * CTAS);
             unsigned long long w_full = 0;
             const long long t_begin = prof ? clock64() : 0;
             bool ok = true;
             uint32_t s = 0, ph = 0, acc = 0;
-            uint32_t bar_full = BAR_FULL, bar_empty = BAR_EMPTY, a_tmem = tmem_a0;
-            uint64_t b_desc = make_kmajor_sw128_desc(x_tile0);
-            constexpr uint64_t b_desc_step = uint64_t(C::X_TILE_BYTES >> 4);
-            bool ready = false;                              // result of an early look at this block's barrier
+            uint32_t bar_full = BAR_FULL, bar_empty = BAR_EMPTY;
             if constexpr (A4) {
                 // four K=64 block-scaled instructions per stage; both operands are the packed tiles, the
                 // scales sit in this stage's TMEM columns
                 constexpr uint32_t idesc4 = make_idesc_nvfp4(MT, 128u * CTAS);
                 uint32_t st = smem_base, sf = tmem_a0;
                 for (uint32_t it = 0; it < num_kb; ++it) {
-                    ok = mbar_wait_timed(bar_full, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+                    ok = mbar_wait_warp_timed(bar_full, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
                     tcgen05_fence_after();
                     const uint64_t wa = make_kmajor_sw128_desc(st + C::S4_W);
                     const uint64_t xb = make_kmajor_sw128_desc(st + C::S4_X);
+                    if (elect_one()) {
 #pragma unroll
-                    for (uint32_t i = 0; i < 4; ++i)   // 64 k = 32 bytes along the swizzled 128-byte row
-                        umma_nvfp4_ss<PAIR>(tmem_acc, wa + 2 * i, xb + 2 * i, idesc4, sf + 4 * i, sf + 16 + 4 * C::XSF_BLOCKS * i, acc | i);
-                    umma_commit<PAIR>(bar_empty, pair_mask);
+                        for (uint32_t i = 0; i < 4; ++i)   // 64 k = 32 bytes along the swizzled 128-byte row
+                            umma_nvfp4_ss<PAIR>(tmem_acc, wa + 2 * i, xb + 2 * i, idesc4, sf + 4 * i, sf + 16 + 4 * C::XSF_BLOCKS * i, acc | i);
+                        umma_commit<PAIR>(bar_empty, pair_mask);
+                    }
+                    __syncwarp();
                     acc = 1u;
                     bar_full += 8; bar_empty += 8; st += C::S4_BYTES; sf += C::SF_COLS;
                     if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; bar_full = BAR_FULL; bar_empty = BAR_EMPTY; st = smem_base; sf = tmem_a0; }
                 }
-            } else
-            for (uint32_t it = 0; it < num_kb; ++it) {
-                if (!ready) {
-                    ok = mbar_wait_timed(bar_full, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+            } else {
+                uint32_t a_tmem = tmem_a0;
+                uint64_t b_desc = make_kmajor_sw128_desc(x_tile0);
+                constexpr uint64_t b_desc_step = uint64_t(C::X_TILE_BYTES >> 4);
+                for (uint32_t it = 0; it < num_kb; ++it) {
+                    ok = mbar_wait_warp_timed(bar_full, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
+                    tcgen05_fence_after();
+                    if (elect_one()) {
+                        // 16 k per instruction: 8 TMEM columns of A, 32 bytes along the swizzled row of B
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; ++i) umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 8 * i, b_desc + 2 * i, idesc, acc | i);
+                        umma_commit<PAIR>(bar_empty, pair_mask);
+                    }
+                    __syncwarp();
+                    acc = 1u;
+                    bar_full += 8; bar_empty += 8; a_tmem += C::A_COLS; b_desc += b_desc_step;
+                    if (++s == uint32_t(C::STAGES)) {
+                        s = 0; ph ^= 1u;
+                        bar_full = BAR_FULL; bar_empty = BAR_EMPTY; a_tmem = tmem_a0; b_desc -= b_desc_step * C::STAGES;
+                    }
                 }
-                tcgen05_fence_after();
-                // next block's stage / phase / operands
-                uint32_t n_full = bar_full + 8, n_empty = bar_empty + 8, n_a = a_tmem + C::A_COLS, n_ph = ph;
-                uint64_t n_b = b_desc + b_desc_step;
-                if (++s == uint32_t(C::STAGES)) {
-                    s = 0; n_ph ^= 1u;
-                    n_full = BAR_FULL; n_empty = BAR_EMPTY; n_a = tmem_a0; n_b = b_desc - b_desc_step * (C::STAGES - 1);
-                }
-                // 16 k per instruction: 8 TMEM columns of A, 32 bytes along the swizzled row of B
-                umma_bf16_ts<PAIR>(tmem_acc, a_tmem, b_desc, idesc, acc);
-                umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 8, b_desc + 2, idesc, 1u);
-                // look at the next block's barrier while the tensor pipe still holds queued work
-                ready = mbar_try_wait(n_full, n_ph);
-                umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 16, b_desc + 4, idesc, 1u);
-                umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 24, b_desc + 6, idesc, 1u);
-                umma_commit<PAIR>(bar_empty, pair_mask);
-                acc = 1u;
-                bar_full = n_full; bar_empty = n_empty; a_tmem = n_a; b_desc = n_b; ph = n_ph;
             }
-            ready = false;
-            if (prof) { prof_row[14] = (unsigned long long)(clock64() - t_begin); prof_row[15] = w_full; }
+            if (prof && lane == 0) { prof_row[14] = (unsigned long long)(clock64() - t_begin); prof_row[15] = w_full; }
             // base K blocks issued; the LoRA K blocks follow once the granule list is known
-            if (ok) ok = mbar_wait(BAR_LIST, 0, abort_flag, STATUS_WAIT_EXPIRED_MMA, 32);
+            if (ok) ok = mbar_wait_warp(BAR_LIST, 0, abort_flag, STATUS_WAIT_EXPIRED_MMA, 32);
             if (ok) {
                 // LoRA K blocks: both operands are shared-memory tiles in their own ring
                 const uint32_t n_gran = misc[1];
                 uint32_t ls = 0, lph = 0;
                 for (uint32_t g0 = 4 * kz; g0 < n_gran; g0 += 4 * ks) {
-                    ok = mbar_wait_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+                    ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
                     tcgen05_fence_after();
                     const uint32_t ksteps = min(4u, n_gran - g0);
                     const uint64_t la = make_kmajor_sw32_desc(x_tile0 + ls * C::L_BLOCK);
                     const uint64_t lb_ = make_kmajor_sw32_desc(x_tile0 + ls * C::L_BLOCK + C::L_TILE_A);
-                    for (uint32_t k = 0; k < ksteps; ++k)   // one granule = one 16-wide K step with its own pair of tiles
-                        umma_bf16_ss<PAIR>(tmem_acc, la + k * (C::L_GRAN_A >> 4), lb_ + k * (C::L_GRAN_T >> 4), idesc, 1u);
-                    umma_commit<PAIR>(BAR_LEMPTY + 8 * ls, pair_mask);
+                    if (elect_one()) {
+                        for (uint32_t k = 0; k < ksteps; ++k)   // one granule = one 16-wide K step with its own pair of tiles
+                            umma_bf16_ss<PAIR>(tmem_acc, la + k * (C::L_GRAN_A >> 4), lb_ + k * (C::L_GRAN_T >> 4), idesc, 1u);
+                        umma_commit<PAIR>(BAR_LEMPTY + 8 * ls, pair_mask);
+                    }
+                    __syncwarp();
                     if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
                 }
             }
-            if (ok) umma_commit<PAIR>(BAR_ACC, pair_mask);
-            if (prof) { prof_row[0] = w_full + ((unsigned long long)(t_begin - t_entry) << 32); prof_row[2] = (unsigned long long)(clock64() - t_begin); }
+            if (ok && elect_one()) umma_commit<PAIR>(BAR_ACC, pair_mask);
+            if (prof && lane == 0) { prof_row[0] = w_full + ((unsigned long long)(t_begin - t_entry) << 32); prof_row[2] = (unsigned long long)(clock64() - t_begin); }
         }
         __syncwarp();
     } else if (warp < DEQ_WARP0) {

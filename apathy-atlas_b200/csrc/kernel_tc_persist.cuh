@@ -317,7 +317,8 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
         }
     } else if (warp == 1) {
         // ===================================== MMA issuer ====================================================
-        if (lane == 0 && leader) {
+        // (the whole warp, converged; one elected lane issues: see elect_one)
+        if (leader) {
             constexpr uint32_t idesc = make_idesc_bf16(MT, 256u);
             unsigned long long w_full = 0, w_acc = 0, w_lora = 0, w_head = 0;
             const long long t_begin = prof ? clock64() : 0;
@@ -326,7 +327,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             for (uint32_t i = 0; ok && i < my_tiles; ++i) {
                 // the accumulators of the previous pass must have been drained
                 for (uint32_t g = 0; ok && g < uint32_t(G); ++g)
-                    ok = mbar_wait_timed(BAR_ACC_EMPTY + 8 * g, (i & 1u) ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_acc, MMA_BACKOFF_NS);
+                    ok = mbar_wait_warp_timed(BAR_ACC_EMPTY + 8 * g, (i & 1u) ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_acc, MMA_BACKOFF_NS);
                 if (!ok) break;
                 tcgen05_fence_after();
                 const unsigned long long w_full_at_pass = w_full;
@@ -334,34 +335,39 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 if constexpr (A4) {
                     constexpr uint32_t idesc4 = make_idesc_nvfp4(MT, 256u);
                     for (uint32_t it = 0; it < num_kb; ++it) {
-                        ok = mbar_wait_timed(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+                        ok = mbar_wait_warp_timed(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
                         const uint32_t st = smem_base + s * C::S4_BYTES, sf = tmem_a0 + s * C::SF_COLS;
                         const uint64_t wa = make_kmajor_sw128_desc(st + C::S4_W);
                         const uint64_t xb = make_kmajor_sw128_desc(st + C::S4_X);
+                        if (elect_one()) {
 #pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j)
-                            umma_nvfp4_ss<true>(tmem_acc, wa + 2 * j, xb + 2 * j, idesc4, sf + 4 * j, sf + 16 + 4 * C::XSF_BLOCKS * j, acc | j);
-                        umma_commit<true>(BAR_EMPTY + 8 * s, pair_mask);
+                            for (uint32_t j = 0; j < 4; ++j)
+                                umma_nvfp4_ss<true>(tmem_acc, wa + 2 * j, xb + 2 * j, idesc4, sf + 4 * j, sf + 16 + 4 * C::XSF_BLOCKS * j, acc | j);
+                            umma_commit<true>(BAR_EMPTY + 8 * s, pair_mask);
+                        }
+                        __syncwarp();
                         acc = 1u;
                         if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                     }
                 } else {
                     for (uint32_t it = 0; it < num_kb; ++it) {
                         if (prof && it == 4) w_head += w_full - w_full_at_pass;
-                        ok = mbar_wait_timed(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+                        ok = mbar_wait_warp_timed(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
                         const uint32_t a_tmem = tmem_a0 + s * C::A_COLS;
+                        const uint64_t b_desc = make_kmajor_sw128_desc(x_tile0 + s * C::X_STAGE_BYTES);
+                        if (elect_one()) {
 #pragma unroll
-                        for (uint32_t g = 0; g < uint32_t(G); ++g) {
-                            const uint64_t b_desc = make_kmajor_sw128_desc(x_tile0 + s * C::X_STAGE_BYTES + g * C::X_TILE_BYTES);
+                            for (uint32_t g = 0; g < uint32_t(G); ++g)
 #pragma unroll
-                            for (uint32_t j = 0; j < 4; ++j)
-                                umma_bf16_ts<true>(tmem_acc + g * MT, a_tmem + 8 * j, b_desc + 2 * j, idesc, acc | j);
+                                for (uint32_t j = 0; j < 4; ++j)
+                                    umma_bf16_ts<true>(tmem_acc + g * MT, a_tmem + 8 * j, b_desc + g * uint64_t(C::X_TILE_BYTES >> 4) + 2 * j, idesc, acc | j);
+                            umma_commit<true>(BAR_EMPTY + 8 * s, pair_mask);
                         }
-                        umma_commit<true>(BAR_EMPTY + 8 * s, pair_mask);
+                        __syncwarp();
                         acc = 1u;
                         if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                     }
@@ -369,25 +375,29 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 if (!ok) break;
                 // LoRA K-steps: one 16-wide kind::f16 step per granule, operands from their own ring
                 if (p.seq_slot) {
-                    ok = mbar_wait_timed(BAR_LIST, i & 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
+                    ok = mbar_wait_warp_timed(BAR_LIST, i & 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
                     if (!ok) break;
                 }
                 for (uint32_t g = 0; ok && g < uint32_t(G); ++g) {
                     const uint32_t n_gran = p.seq_slot ? misc[4 + g] : 0u;
                     for (uint32_t q = 0; q < n_gran; ++q) {
-                        ok = mbar_wait_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
+                        ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
                         const uint64_t la = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE);
                         const uint64_t lb = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE + C::L_GRAN_A);
-                        umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
-                        umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                        if (elect_one()) {
+                            umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
+                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                        }
+                        __syncwarp();
                         if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
                     }
-                    if (ok) umma_commit<true>(BAR_ACC_FULL + 8 * g, pair_mask);
+                    if (ok && elect_one()) umma_commit<true>(BAR_ACC_FULL + 8 * g, pair_mask);
+                    __syncwarp();
                 }
             }
-            if (prof) {
+            if (prof && lane == 0) {
                 prof_row[0] = w_full; prof_row[2] = (unsigned long long)(clock64() - t_begin);
                 prof_row[10] = w_acc; prof_row[11] = w_lora; prof_row[9] = w_head;
             }
