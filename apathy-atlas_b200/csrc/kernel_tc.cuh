@@ -28,9 +28,9 @@
 // with half of the activation tile each (Cfg::PAIR); and, times that, k_split CTAs along z sharing one
 // tile's contraction and exchanging partial sums over distributed shared memory.
 //
-// Warp roles (14 warps, 448 threads):
-//   warp 0        TMA producer: activation tiles, raw weight stages (packed codes + scale bytes),
-//                 LoRA operand tiles, each through its own mbarrier ring
+// Warp roles (15 warps, 480 threads):
+//   warp 0        TMA producer: activation tiles (A4: packed weights and scale bytes too), LoRA operand tiles
+//   warp 14       TMA producer, A16: raw weight stages (packed codes + scale bytes)
 //   warp 1        TMEM allocation, tcgen05.mma issue, tcgen05.commit (in a pair: the first CTA's warp
 //                 issues for both)
 //   warps 2-5     build the tile's granule list while the main loop runs; then the epilogue
@@ -61,7 +61,8 @@ constexpr int RAW_SCALE_BYTES = FT * (KRAW / 16);    // 2 KiB
 // issue rate below) and takes issue slots from the MMA thread.
 constexpr int DEQ_GROUPS = 1;
 constexpr int DEQ_WARP0 = 6, DEQ_GROUP_WARPS = 8, DEQ_WARPS = 8 * DEQ_GROUPS, DEQ_THREADS = 32 * DEQ_WARPS;
-constexpr int NUM_THREADS = 32 * (DEQ_WARP0 + DEQ_WARPS);
+constexpr int RAW_WARP = DEQ_WARP0 + DEQ_WARPS;      // TMA producer of the raw weight stages
+constexpr int NUM_THREADS = 32 * (RAW_WARP + 1);
 constexpr int EPI_WARP0 = 2, EPI_THREADS = 128;
 constexpr int EPI_WARPS = 4 + DEQ_WARPS;   // warps that take part in the epilogue: the list warps and the expansion warps
 constexpr int MAX_LORAS_TC = 4096;
@@ -716,6 +717,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     const uint32_t raw_lo = kz * total_raw / ks, raw_hi = (kz + 1u) * total_raw / ks;
     const uint32_t kb_lo = A4 ? raw_lo : 4u * raw_lo;
     const uint32_t num_kb = (A4 ? raw_hi : min(4u * raw_hi, total_kb)) - kb_lo;      // pipeline steps of the base K loop
+    const uint32_t num_raw_kb = (num_kb + 3u) / 4u;                                  // A16: raw stages of the base K loop
+    const uint32_t rot_raw = (!A4 && num_kb % 4u == 0u && num_raw_kb) ? (blockIdx.x / CTAS) % num_raw_kb : 0u;   // (same for both CTAs of a pair)
     const bool prof = p.profile != nullptr;
     const long long t_entry = clock64();
     const uint64_t t_entry_ns = prof ? global_timer_ns() : 0;
@@ -796,54 +799,17 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             }
         }
         if (lane == 0 && !A4) {
-            // One thread feeds two rings without blocking on either: activation tiles (one per K
-            // block) and raw weight stages (codes + scale bytes, one per four K blocks), so the
-            // weight stream runs ahead of the activation stream.
+            // Activation tiles, one per K block (the raw weight stages have a producer of their own).
             // CTAs start their K loop at different K offsets (a rotation in units of one raw stage),
             // so concurrently running CTAs do not all pull the same activation lines at one moment.
-            const uint32_t num_raw = (num_kb + 3u) / 4u;
-            const uint32_t rot_raw = (num_kb % 4u == 0u) ? ((blockIdx.x / CTAS) % num_raw) : 0u;   // (same for both CTAs of a pair)
-            uint32_t it = 0, ri = 0, spins = 0;
-            uint64_t t0 = 0;
-            while (it < num_kb || ri < num_raw) {
-                bool progressed = false;
-                if (ri < num_raw) {
-                    const uint32_t rs = ri % C::RAW_STAGES, rph = (ri / C::RAW_STAGES) & 1u;
-                    if (mbar_try_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u)) {
-                        mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + RAW_SCALE_BYTES);
-                        const uint32_t rk = raw_lo + (ri + rot_raw) % num_raw;
-                        tma_load_2d(rawp0 + rs * RAW_PACKED_BYTES, &map_w, int32_t(rk * (KRAW / 2)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
-                        tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
-                        ++ri;
-                        progressed = true;
-                    }
-                }
-                if (it < num_kb) {
-                    const uint32_t s = it % C::STAGES, ph = (it / C::STAGES) & 1u;
-                    if (mbar_try_wait(BAR_EMPTY + 8 * s, ph ^ 1u)) {
-                        if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, CTAS * C::X_TILE_BYTES);
-                        const uint32_t kb = kb_lo + (it + 4u * rot_raw) % num_kb;
-                        if constexpr (PAIR) tma_load_2d_pair(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(mx0), full_at_leader + 8 * s);
-                        else tma_load_2d(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(m0), BAR_FULL + 8 * s);
-                        ++it;
-                        progressed = true;
-                    }
-                }
-                if (progressed) {
-                    spins = 0;
-                    t0 = 0;
-                } else {
-                    __nanosleep(64);
-                    if ((++spins & 63u) != 0u) continue;
-                    if (*abort_flag) break;
-                    const uint64_t now = global_timer_ns();
-                    if (t0 == 0) t0 = now;
-                    else if (now - t0 > WAIT_LIMIT_NS) {
-                        record_status(STATUS_WAIT_EXPIRED_PRODUCER);
-                        *abort_flag = 1u;
-                        break;
-                    }
-                }
+            uint32_t s = 0, ph = 0;
+            for (uint32_t it = 0; it < num_kb; ++it) {
+                if (!mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
+                if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, CTAS * C::X_TILE_BYTES);
+                const uint32_t kb = kb_lo + (it + 4u * rot_raw) % num_kb;
+                if constexpr (PAIR) tma_load_2d_pair(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(mx0), full_at_leader + 8 * s);
+                else tma_load_2d(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(m0), BAR_FULL + 8 * s);
+                if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
             }
         }
         if (lane == 0) {
@@ -1046,6 +1012,21 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, te);
             else epilogue_columns<MT>(p, tmem_acc, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4);
             if (prof && te == 0) prof_row[7] = (unsigned long long)(clock64() - t_epi);
+        }
+    } else if (warp == RAW_WARP) {
+        // ===================================== TMA producer, raw weight stages ===================
+        // A thread of its own: try_wait may suspend its caller for a while, so one thread polling both rings' barriers in
+        // turn keeps a free slot of one ring waiting behind the other's.
+        if (lane == 0 && !A4) {
+            uint32_t rs = 0, rph = 0;
+            for (uint32_t ri = 0; ri < num_raw_kb; ++ri) {
+                if (!mbar_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
+                mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + RAW_SCALE_BYTES);
+                const uint32_t rk = raw_lo + (ri + rot_raw) % num_raw_kb;
+                tma_load_2d(rawp0 + rs * RAW_PACKED_BYTES, &map_w, int32_t(rk * (KRAW / 2)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
+            }
         }
     } else {
         // ========================== NVFP4 -> BF16 weight operand, into TMEM ======================

@@ -29,8 +29,9 @@
 // (strided adapter pool + masked-t tiles written by the shrink).  The launcher falls back to the one-tile-per-CTA
 // kernel otherwise.
 //
-// Warp roles (19 warps, 608 threads):
-//   warp 0        TMA producer of the base K loop
+// Warp roles (20 warps, 640 threads):
+//   warp 0        TMA producer of the base K loop's activation tiles (A4: weights and scales too)
+//   warp 19       TMA producer of the raw weight stages (A16)
 //   warp 1        TMEM allocation, tcgen05.mma issue (first CTA of the pair issues for both)
 //   warps 2-5     accumulator drain; row stores; granule list of the next tile
 //   warps 6-13    A16: NVFP4 -> BF16 weight operand into tensor memory; A4: block scales into tensor memory
@@ -44,8 +45,9 @@
 namespace atlas {
 namespace tc {
 
-constexpr int P_NUM_THREADS = 32 * 19;
+constexpr int P_NUM_THREADS = 32 * 20;
 constexpr int P_LORA_WARP = 14;
+constexpr int P_RAW_WARP = 19;
 constexpr int P_EPI_WARP1 = 15;         // second group of four drain / store warps (the first is warps 2-5)
 constexpr int P_EPI_WARPS = 8;
 constexpr int P_EPI_THREADS = 32 * P_EPI_WARPS;
@@ -235,53 +237,42 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             }
         }
         if (lane == 0 && !A4) {
-            // two rings fed by one thread without blocking on either: activation tiles (one stage per K block, G
-            // tiles each) and raw weight stages (codes + scale bytes, one per four K blocks)
-            uint32_t xs = 0, xph = 0, rs = 0, rph = 0, spins = 0;
-            uint64_t t0 = 0;
-            bool dead = false;
-            for (uint32_t i = 0; i < my_tiles && !dead; ++i) {
-                const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * (MT * G);
+            // activation tiles: one stage per K block, G tiles each (the raw weight stages have a producer of their own)
+            uint32_t xs = 0, xph = 0;
+            bool ok = true;
+            for (uint32_t i = 0; ok && i < my_tiles; ++i) {
+                const uint32_t m0 = tile_pass(i) * (MT * G);
                 const uint32_t rot_raw = tile_fpair(i) % num_raw;
-                uint32_t it = 0, ri = 0;
-                while (it < num_kb || ri < num_raw) {
-                    bool progressed = false;
-                    if (ri < num_raw && mbar_try_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u)) {
-                        mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + RAW_SCALE_BYTES);
-                        const uint32_t rk = (ri + rot_raw) % num_raw;
-                        tma_load_2d(rawp0 + rs * RAW_PACKED_BYTES, &map_w, int32_t(rk * (KRAW / 2)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
-                        tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
-                        ++ri;
-                        if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
-                        progressed = true;
-                    }
-                    if (it < num_kb && mbar_try_wait(BAR_EMPTY + 8 * xs, xph ^ 1u)) {
-                        if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * xs, 2 * C::X_STAGE_BYTES);
-                        const uint32_t kb = (it + 4u * rot_raw) % num_kb;
+                for (uint32_t it = 0; it < num_kb; ++it) {
+                    ok = mbar_wait(BAR_EMPTY + 8 * xs, xph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER);
+                    if (!ok) break;
+                    if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * xs, 2 * C::X_STAGE_BYTES);
+                    const uint32_t kb = (it + 4u * rot_raw) % num_kb;
 #pragma unroll
-                        for (uint32_t g = 0; g < uint32_t(G); ++g)
-                            tma_load_2d_pair(x_tile0 + xs * C::X_STAGE_BYTES + g * C::X_TILE_BYTES, &map_x, int32_t(kb * KB),
-                                             int32_t(m0 + g * MT + cta_rank * C::XROWS), full_at_leader + 8 * xs);
-                        ++it;
-                        if (++xs == uint32_t(C::STAGES)) { xs = 0; xph ^= 1u; }
-                        progressed = true;
-                    }
-                    if (progressed) {
-                        spins = 0;
-                        t0 = 0;
-                    } else {
-                        __nanosleep(64);
-                        if ((++spins & 63u) != 0u) continue;
-                        if (*abort_flag) { dead = true; break; }
-                        const uint64_t now = global_timer_ns();
-                        if (t0 == 0) t0 = now;
-                        else if (now - t0 > WAIT_LIMIT_NS) {
-                            record_status(STATUS_WAIT_EXPIRED_PRODUCER);
-                            *abort_flag = 1u;
-                            dead = true;
-                            break;
-                        }
-                    }
+                    for (uint32_t g = 0; g < uint32_t(G); ++g)
+                        tma_load_2d_pair(x_tile0 + xs * C::X_STAGE_BYTES + g * C::X_TILE_BYTES, &map_x, int32_t(kb * KB),
+                                         int32_t(m0 + g * MT + cta_rank * C::XROWS), full_at_leader + 8 * xs);
+                    if (++xs == uint32_t(C::STAGES)) { xs = 0; xph ^= 1u; }
+                }
+            }
+        }
+    } else if (warp == P_RAW_WARP) {
+        // ===================================== TMA producer, raw weight stages ===============================
+        // (one per four K blocks; a thread of its own, see nvfp4_lora_linear_tc_kernel)
+        if (lane == 0 && !A4) {
+            uint32_t rs = 0, rph = 0;
+            bool ok = true;
+            for (uint32_t i = 0; ok && i < my_tiles; ++i) {
+                const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT;
+                const uint32_t rot_raw = tile_fpair(i) % num_raw;
+                for (uint32_t ri = 0; ri < num_raw; ++ri) {
+                    ok = mbar_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER);
+                    if (!ok) break;
+                    mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + RAW_SCALE_BYTES);
+                    const uint32_t rk = (ri + rot_raw) % num_raw;
+                    tma_load_2d(rawp0 + rs * RAW_PACKED_BYTES, &map_w, int32_t(rk * (KRAW / 2)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                    tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                    if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
                 }
             }
         }
@@ -403,7 +394,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             }
         }
         __syncwarp();
-    } else if (warp < DEQ_WARP0 || warp >= P_EPI_WARP1) {
+    } else if (warp < DEQ_WARP0 || (warp >= P_EPI_WARP1 && warp < P_EPI_WARP1 + 4)) {
         // ============================ accumulator drain, row stores, granule lists ===========================
         const uint32_t grp = warp < DEQ_WARP0 ? 0u : 1u;                            // which of the two groups of four warps
         const uint32_t te = ((warp < DEQ_WARP0 ? warp - EPI_WARP0 : warp - P_EPI_WARP1 + 4u) << 5) + lane;   // 0..255
