@@ -61,7 +61,7 @@ struct DeviceState {
     std::atomic<bool> ready{false};
     bool sm100 = false;
     int sm_count = 148;
-    bool tc_attr_set[20] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair}
+    bool tc_attr_set[40] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair}
     int known_clusters[20][9] = {};   // resident clusters per kernel instance and K split; 0 = not asked yet
     bool persist_attr_set[kPersistKernels] = {};
     int persist_clusters[kPersistKernels] = {};
@@ -354,15 +354,20 @@ static int launch_simt_linear(const atlas_b200_linear_desc& d, cudaStream_t st) 
 }
 
 // Shapes the tcgen05 path takes.  Everything here is a property of host-visible arguments.
-static bool tc_eligible(const atlas_b200_linear_desc& d) {
+// `wide`: also those for which it is only the faster of two paths — K a multiple of 32 (of 256 otherwise: the row strides of
+// codes AND scales are then the 16-byte multiples TMA wants; with K = 32 n only the codes are, and the expansion warps read
+// the scales themselves) and ranks up to 128 (64 otherwise).  What exists on this path alone (FP4 activations, placement,
+// a forced path, the shrink by itself) keeps the narrow rule.
+constexpr uint32_t TC_NARROW_RANK = 64;
+static bool tc_eligible(const atlas_b200_linear_desc& d, bool wide) {
     DeviceState* dst = device_state();
     if (!dst || !dst->sm100 || !g_encode) return false;
-    if (d.w_bf16) return false;                                   // dense base: CUDA-core path
-    if (d.k % tc::KRAW != 0) return false;                        // TMA row strides of codes and scales: 16-byte multiples
+    if (d.w_bf16) return false;                                   // dense base: a kernel of its own
+    if (d.k % tc::KRAW != 0 && (!wide || d.k % 32 != 0 || d.k < uint32_t(tc::KRAW))) return false;
     if (d.x_row_stride % 8 != 0) return false;
     if (!aligned(d.x, 16) || !aligned(d.w_packed, 16) || !aligned(d.w_scale, 16)) return false;
     if (d.seq_slot) {
-        if (d.max_rank > tc::MAX_RANK_TC || d.max_rank % 8 != 0) return false;
+        if (d.max_rank > (wide ? uint32_t(tc::MAX_RANK_TC) : TC_NARROW_RANK) || d.max_rank % 8 != 0) return false;
         if (d.max_loras > tc::MAX_LORAS_TC) return false;
         if (!aligned(d.lora_t, 16)) return false;
     }
@@ -409,8 +414,9 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
     if (!encode_2d(&m.w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_packed, d.k / 2, d.n, d.k / 2, tc::KRAW / 2, tc::FT,
                    CU_TENSOR_MAP_SWIZZLE_128B))
         return ATLAS_B200_ERR_DIMS;
-    if (!encode_2d(&m.s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, tc::KRAW / 16, tc::FT,
-                   CU_TENSOR_MAP_SWIZZLE_NONE))
+    if (d.k % tc::KRAW != 0) m.s = m.w;      // scale rows of K/16 bytes: read by the expansion warps (Params::w_scale_rows)
+    else if (!encode_2d(&m.s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, tc::KRAW / 16, tc::FT,
+                        CU_TENSOR_MAP_SWIZZLE_NONE))
         return ATLAS_B200_ERR_DIMS;
 
     // B side of the adapter pool as one 3-D tensor [max_loras][n][max_rank]: box = one granule of one slot
@@ -439,6 +445,8 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
 // the launch constants both tcgen05 kernels share
 static int fill_tc_params(const atlas_b200_linear_desc& d, bool a4, bool b_strided, const TTiles& tt, tc::Params& p) {
     p.b_pool_strided = b_strided ? 1u : 0u;
+    p.b_pool_base = reinterpret_cast<unsigned long long>(d.b_pool_base);
+    p.b_slot_stride = d.b_slot_stride;
     p.t_tile_cap = tt.tiles ? tt.cap : 0u;
     p.seq_slot = d.seq_slot;
     p.a_table = d.a_table;
@@ -458,6 +466,7 @@ static int fill_tc_params(const atlas_b200_linear_desc& d, bool a4, bool b_strid
     p.M = d.m; p.N = d.n; p.K = d.k; p.out_row_stride = d.out_row_stride;
     p.max_loras = d.max_loras; p.max_rank = d.max_rank;
     p.out_scale = a4 ? d.scale2 : d.scale2 * kWeightPreScale;
+    p.w_scale_rows = d.k % tc::KRAW != 0 ? static_cast<const uint8_t*>(d.w_scale) : nullptr;
     p.k_split = 1;
     return ATLAS_B200_OK;
 }
@@ -510,16 +519,16 @@ static int tc_active_clusters_of(uint32_t mt, bool a4, bool pair, uint32_t k_spl
     return -1;
 }
 
-template <int MT, bool A4, bool PAIR>
-static int launch_tc(const atlas_b200_linear_desc& d, int slot_idx, const ShrinkParams* shrink, const TTiles& tt,
+template <int MT, bool A4, bool PAIR, bool SROWS>
+static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const ShrinkParams* shrink, const TTiles& tt,
                      uint32_t k_split, cudaStream_t st) {
     const bool after_shrink = shrink != nullptr;     // the shrink is launched from here, once the launch shape is final
     using C = tc::Cfg<MT, A4, PAIR>;
     DeviceState* dst = device_state();
     if (!dst) return ATLAS_B200_ERR_ARCH;
-    slot_idx += (A4 ? 5 : 0) + (PAIR ? 10 : 0);
+    slot_idx += (A4 ? 5 : 0) + (PAIR ? 10 : 0) + (SROWS ? 20 : 0);
     if (!dst->tc_attr_set[slot_idx]) {
-        cudaError_t e = cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR>,
+        cudaError_t e = cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e != cudaSuccess) return cuda_status(e);
         dst->tc_attr_set[slot_idx] = true;
@@ -582,7 +591,15 @@ static int launch_tc(const atlas_b200_linear_desc& d, int slot_idx, const Shrink
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     p.wait_for_shrink = after_shrink ? 1u : 0u;
-    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR>, map_x, map_w, map_s, map_b, map_xs, map_t, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS>, map_x, map_w, map_s, map_b, map_xs, map_t, p));
+}
+
+template <int MT, bool A4, bool PAIR>
+static int launch_tc(const atlas_b200_linear_desc& d, int slot_idx, const ShrinkParams* shrink, const TTiles& tt,
+                     uint32_t k_split, cudaStream_t st) {
+    if constexpr (!A4)
+        if (d.k % tc::KRAW != 0) return launch_tc_as<MT, false, PAIR, true>(d, slot_idx, shrink, tt, k_split, st);
+    return launch_tc_as<MT, A4, PAIR, false>(d, slot_idx, shrink, tt, k_split, st);
 }
 
 // ---- the persistent form (kernel_tc_persist.cuh): one cluster of two CTAs per pair of SMs, a static tile loop ----
@@ -766,7 +783,15 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
     if (d.m == 0) return ATLAS_B200_OK;
 
     const bool staged = (d.flags & ATLAS_B200_FLAG_STAGED_LORA) != 0;
-    bool use_tc = !(d.flags & ATLAS_B200_FLAG_FORCE_SIMT) && !staged && tc_eligible(d);
+    bool use_tc = !(d.flags & ATLAS_B200_FLAG_FORCE_SIMT) && !staged && tc_eligible(d, false);
+    bool reuse_shrink = (d.flags & ATLAS_B200_FLAG_REUSE_SHRINK) != 0;
+    if (!use_tc && !staged && !shrink_only && !d.n_dest && !(d.flags & (ATLAS_B200_FLAG_FORCE_SIMT | ATLAS_B200_FLAG_FORCE_TCGEN05 | ATLAS_B200_FLAG_ACT_FP4)) &&
+        tc_eligible(d, true)) {
+        // These shapes ran on the CUDA cores (64 x 64 tiles of scalar FMAs, then the two-stage LoRA) at a few per cent of this
+        // path's rate.  That path computes its shrink on every call, so this one does too.
+        use_tc = true;
+        reuse_shrink = false;
+    }
     if (!use_tc && shrink_only) return ATLAS_B200_ERR_DIMS;
     if (!use_tc && (d.flags & ATLAS_B200_FLAG_FORCE_TCGEN05) && !(d.w_bf16 && !staged && dense_tc_eligible(d))) return ATLAS_B200_ERR_DIMS;
     if (!use_tc && d.n_dest) return ATLAS_B200_ERR_DIMS;          // placement into several buffers is the tcgen05 epilogue's
@@ -854,7 +879,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         // Many tiles per SM pair (a prefill batch): the persistent form, whose operand rings run across tile
         // boundaries and whose row stores overlap the next tile's K loop.  It takes 256-token tiles of CTA pairs
         // without a K split, 16-byte aligned destination rows, and LoRA operands that both come by TMA.
-        bool persistent = mt == 256 && pair && k_split == 1 && !(d.flags & ATLAS_B200_FLAG_NO_PERSISTENT) &&
+        bool persistent = mt == 256 && pair && k_split == 1 && !(d.flags & ATLAS_B200_FLAG_NO_PERSISTENT) && d.k % tc::KRAW == 0 &&
                           (!d.seq_slot || b_pool_is_strided(d)) && d.out_row_stride % 8 == 0 &&
                           (d.n_dest ? d.y_col_offset % 8 == 0 : aligned(d.y, 16));
         for (uint32_t r = 0; persistent && r < d.n_dest; ++r) persistent = aligned(d.y_dest[r], 16);
@@ -917,7 +942,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
             if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
             return rc;
         }
-        const ShrinkParams* shrink = (d.seq_slot && !(d.flags & ATLAS_B200_FLAG_REUSE_SHRINK)) ? &sp : nullptr;
+        const ShrinkParams* shrink = (d.seq_slot && !reuse_shrink) ? &sp : nullptr;
         if (persistent) {
             if (act_fp4) rc = launch_tc_persist<256, 1, true>(d, 1, shrink, tt, st);
             else if (two_tiles) rc = launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);

@@ -66,7 +66,10 @@ constexpr int NUM_THREADS = 32 * (RAW_WARP + 1);
 constexpr int EPI_WARP0 = 2, EPI_THREADS = 128;
 constexpr int EPI_WARPS = 4 + DEQ_WARPS;   // warps that take part in the epilogue: the list warps and the expansion warps
 constexpr int MAX_LORAS_TC = 4096;
-constexpr int MAX_RANK_TC = 64;
+constexpr int MAX_RANK_TC = 128;
+// a granule list entry: slot << GRAN_SHIFT | which 16 ranks of the slot (4096 slots of up to eight granules in 16 bits)
+constexpr uint32_t GRAN_SHIFT = 3, GRAN_MASK = 7;
+static_assert(MAX_RANK_TC / 16 <= int(GRAN_MASK) + 1 && (MAX_LORAS_TC << GRAN_SHIFT) <= 65536, "granule list entries are 16 bits");
 constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;    // 1 s
 constexpr int PROFILE_WORDS = 16;
 constexpr int MAX_DEST = 8;            // tensor-parallel ranks whose output buffers one launch can store into
@@ -124,8 +127,7 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int STAGING_BYTES = STAGING_BASE > L_STAGES * L_BLOCK ? STAGING_BASE : L_STAGES * L_BLOCK;
     static constexpr int OFF_SLOT = STAGING_BYTES;                               // int32[MT]
     static constexpr int OFF_GRAN = OFF_SLOT + MT * 4;                           // uint16[MAX_GRANULES]
-    static constexpr int OFF_GRANB = OFF_GRAN + MAX_GRANULES * 2;                // uint64[MAX_GRANULES]: B_s address of the granule
-    static constexpr int OFF_BITMAP = OFF_GRANB + MAX_GRANULES * 8;              // uint32[128]
+    static constexpr int OFF_BITMAP = OFF_GRAN + MAX_GRANULES * 2;               // uint32[128]
     static constexpr int OFF_SCAN = OFF_BITMAP + (MAX_LORAS_TC / 32) * 4;        // uint32[8]
     static constexpr int OFF_BAR = OFF_SCAN + 64;                                // mbarriers
     static constexpr int NUM_BARS = 2 * STAGES + 2 * RAW_STAGES + 4 + 2 * L_STAGES;
@@ -156,8 +158,11 @@ struct Params {
     uint32_t staged_epilogue;      // destination rows allow 16-byte stores: write the tile out through shared memory
     uint32_t t_tile_cap;           // != 0: the shrink wrote masked-t tiles (ShrinkParams::tile_out) with this many blocks
                                    //       reserved per token tile; they are fetched by TMA (map_t) and `t` is not read
-    uint32_t b_pool_strided;       // B_s tiles can be fetched by TMA from a [max_loras][N][max_rank] strided pool
+    uint32_t b_pool_strided;       // B_s tiles can be fetched by TMA from a [max_loras][N][max_rank] strided pool ...
+    unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
+    const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
+                                   //       expansion warps, because TMA wants row strides of whole 16 bytes
     unsigned long long* profile;   // nullable: per-CTA wait/busy cycle counters (PROFILE_WORDS per CTA)
 };
 
@@ -659,8 +664,12 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
     }
 }
 
-template <int MT, bool A4, bool PAIR>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
+// SROWS (A16, K not a multiple of 256): the scale rows come by the expansion warps' own loads (Params::w_scale_rows).
+// (The bound is wider than the launch so that a thread gets at most 96 registers: the shrink of a decode batch runs beside
+//  this kernel, and with 107 registers only one of its CTAs found room on an SM instead of two: 140 -> 160 us for the fused
+//  QKV projections of 64 tokens with 64 adapters.)
+template <int MT, bool A4, bool PAIR, bool SROWS = false>
+__global__ void __launch_bounds__(672, 1)
 nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                             const __grid_constant__ CUtensorMap map_w,
                             const __grid_constant__ CUtensorMap map_s,
@@ -678,7 +687,6 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     const uint32_t raws0 = smem_base + C::OFF_RAWS;
     int32_t* slot_arr = reinterpret_cast<int32_t*>(smem_gen + C::OFF_SLOT);
     uint16_t* gran = reinterpret_cast<uint16_t*>(smem_gen + C::OFF_GRAN);
-    unsigned long long* gran_b = reinterpret_cast<unsigned long long*>(smem_gen + C::OFF_GRANB);
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem_gen + C::OFF_BITMAP);
     uint32_t* scan = reinterpret_cast<uint32_t*>(smem_gen + C::OFF_SCAN);
     const uint32_t bar0 = smem_base + C::OFF_BAR;
@@ -832,8 +840,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                         if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, CTAS * ng * (C::L_GRAN_A + (p.t_tile_cap ? C::L_GRAN_T : 0)));
                         for (uint32_t g = 0; g < ng; ++g) {
                             const uint32_t e = gran[g0 + g];
-                            if constexpr (PAIR) tma_load_3d_pair(base + g * C::L_GRAN_A, &map_b, int32_t((e & 3u) * 16u), int32_t(f0), int32_t(e >> 2), lfull_at_leader + 8 * ls);
-                            else tma_load_3d(base + g * C::L_GRAN_A, &map_b, int32_t((e & 3u) * 16u), int32_t(f0), int32_t(e >> 2), BAR_LFULL + 8 * ls);
+                            if constexpr (PAIR) tma_load_3d_pair(base + g * C::L_GRAN_A, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
+                            else tma_load_3d(base + g * C::L_GRAN_A, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), BAR_LFULL + 8 * ls);
                             if (p.t_tile_cap) {
                                 const int32_t row = int32_t(t_row0 + (g0 + g) * uint32_t(C::L_GRAN_T / 256));
                                 if constexpr (PAIR) tma_load_2d_pair(base + C::L_TILE_A + g * C::L_GRAN_T, &map_t, 0, row, lfull_at_leader + 8 * ls);
@@ -967,24 +975,23 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             for (uint32_t w = word; w; w &= w - 1) {
                 const uint32_t s = te * 32 + (__ffs(w) - 1);
                 const uint32_t r = p.rank_table ? min(p.rank_table[s], p.max_rank) : p.max_rank;
-                const unsigned long long b_addr = p.b_table[s];
-                for (uint32_t g = 0; g < (r + 15u) / 16u; ++g) { gran_b[pos] = b_addr; gran[pos++] = uint16_t((s << 2) | g); }
+                for (uint32_t g = 0; g < (r + 15u) / 16u; ++g) gran[pos++] = uint16_t((s << GRAN_SHIFT) | g);
             }
             if (te == 0) misc[1] = n_gran;
             named_bar_sync(1, EPI_THREADS);
             // For every token row: where its slot's granules sit in the list (they are consecutive) and
-            // how many there are, packed (pos << 3 | count); 0xFFFF = the row takes no LoRA term.  The
+            // how many there are, packed (pos << 4 | count); 0xFFFF = the row takes no LoRA term.  The
             // slot bitmap is dead by now and its space is re-used.
             uint16_t* row_pg = reinterpret_cast<uint16_t*>(bitmap);
             for (uint32_t r = te; r < uint32_t(MT); r += EPI_THREADS) {
                 const int32_t sl = slot_arr[r];
                 uint16_t pg = 0xFFFFu;
                 if (sl >= 0) {
-                    const uint32_t key = uint32_t(sl) << 2;       // first entry >= key is (sl, granule 0)
+                    const uint32_t key = uint32_t(sl) << GRAN_SHIFT;       // first entry >= key is (sl, granule 0)
                     uint32_t lo = 0, hi = n_gran;
                     while (lo < hi) { const uint32_t mid = (lo + hi) >> 1; if (gran[mid] < key) lo = mid + 1; else hi = mid; }
                     const uint32_t rk = p.rank_table ? min(p.rank_table[sl], p.max_rank) : p.max_rank;
-                    pg = uint16_t((lo << 3) | ((rk + 15u) / 16u));
+                    pg = uint16_t((lo << 4) | ((rk + 15u) / 16u));
                 }
                 row_pg[r] = pg;
             }
@@ -998,7 +1005,9 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             if (f < p.N) {
                 for (uint32_t g = 0; g < n_gran; ++g) {
                     const uint32_t e = gran[g];
-                    const uint16_t* src = reinterpret_cast<const uint16_t*>(gran_b[g]) + size_t(f) * p.max_rank + (e & 3u) * 16u;
+                    // (a strided pool's addresses are arithmetic: a table read per granule made this loop a chain of loads)
+                    const unsigned long long b_s = p.b_pool_strided ? p.b_pool_base + (e >> GRAN_SHIFT) * p.b_slot_stride : p.b_table[e >> GRAN_SHIFT];
+                    const uint16_t* src = reinterpret_cast<const uint16_t*>(b_s) + size_t(f) * p.max_rank + (e & GRAN_MASK) * 16u;
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
                 }
             }
@@ -1021,10 +1030,10 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             uint32_t rs = 0, rph = 0;
             for (uint32_t ri = 0; ri < num_raw_kb; ++ri) {
                 if (!mbar_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
-                mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + RAW_SCALE_BYTES);
+                mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, RAW_PACKED_BYTES + (SROWS ? 0 : RAW_SCALE_BYTES));
                 const uint32_t rk = raw_lo + (ri + rot_raw) % num_raw_kb;
                 tma_load_2d(rawp0 + rs * RAW_PACKED_BYTES, &map_w, int32_t(rk * (KRAW / 2)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
-                tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                if (!SROWS) tma_load_2d(raws0 + rs * RAW_SCALE_BYTES, &map_s, int32_t(rk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * rs);
                 if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
             }
         }
@@ -1112,12 +1121,32 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 if (lane == 0) arrive_at_leader(full_at_leader + 8 * s);
                 if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
             }
-        } else
+        } else {
+        // Scale bytes of rows that TMA cannot fetch (K/16 bytes, a multiple of two): a thread needs two neighbouring bytes per
+        // K block, one 16-bit load each (the four of a raw stage lie in one or two sectors), read two raw stages ahead.
+        // Where K ends, codes and activations are zero-filled by TMA and the scales read as zero here.
+        const uint8_t* sc_row = SROWS && f0 + row < p.N ? p.w_scale_rows + size_t(f0 + row) * (p.K / 16u) : nullptr;
+        uint32_t sc_next[2][4] = {};
+        auto fetch_scales = [&](uint32_t ri, uint32_t (&dst)[4]) {
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                const uint32_t at = ((raw_lo + (ri + rot_raw) % num_raw) * 4u + j) * 4u + 2u * half;
+                dst[j] = sc_row && ri < num_raw && at < p.K / 16u ? uint32_t(__ldg(reinterpret_cast<const uint16_t*>(sc_row + at))) << (16u * half) : 0u;
+            }
+        };
+        if constexpr (SROWS) { fetch_scales(0, sc_next[0]); fetch_scales(1, sc_next[1]); }
         for (uint32_t ri = 0; ok && ri < num_raw; ++ri) {
             ok = mbar_wait_timed(BAR_FULL_RAW + 8 * rs, rph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_raw);
             if (!ok) break;
-            const uint4 sc4 = lds128(raws0 + rs * RAW_SCALE_BYTES + row * 16);
-            const uint32_t scw[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
+            uint32_t scw[4];
+            if constexpr (!SROWS) {
+                const uint4 sc4 = lds128(raws0 + rs * RAW_SCALE_BYTES + row * 16);
+                scw[0] = sc4.x; scw[1] = sc4.y; scw[2] = sc4.z; scw[3] = sc4.w;
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < 4; ++j) { scw[j] = sc_next[0][j]; sc_next[0][j] = sc_next[1][j]; }
+                fetch_scales(ri + 2, sc_next[1]);
+            }
 #pragma unroll
             for (uint32_t jr = 0; jr < 4; jr += 2 * DEQ_GROUPS) {
                 if (ri * 4 + jr + grp >= num_kb) break;
@@ -1168,6 +1197,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             __syncwarp();
             if (lane == 0) mbar_arrive(BAR_EMPTY_RAW + 8 * rs);
             if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
+        }
         }
         if (prof && td == 0) {
             prof_row[3] = w_raw; prof_row[4] = w_empty; prof_row[5] = (unsigned long long)(clock64() - t_begin);
@@ -1222,8 +1252,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 const uint32_t r = task & (XR - 1u), hh = task / XR;
                 const uint32_t tile_row = cta_rank * XR + r;
                 const uint32_t pg = (task < XR * 2 && p.seq_slot) ? row_pg[tile_row] : 0xFFFFu;
-                t_ng[u] = pg == 0xFFFFu ? 0u : (pg & 7u);
-                t_pos[u] = int32_t(pg >> 3);
+                t_ng[u] = pg == 0xFFFFu ? 0u : (pg & 15u);
+                t_pos[u] = int32_t(pg >> 4);
                 t_src[u] = p.t + size_t(m0 + tile_row) * p.max_rank + 8 * hh;
                 t_dst[u] = C::L_TILE_A + r * 32u + ((hh ^ ((r >> 2) & 1u)) << 4);
                 // granule columns beyond max_rank do not exist in t: treat as not routed
@@ -1251,10 +1281,10 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 #pragma unroll
                 for (uint32_t g = 0; g < 4; ++g) {
                     if (g < ng) {
-                        const uint32_t j0 = (gran[lb * 4 + g] & 3u) * 16u;
+                        const uint32_t e = gran[lb * 4 + g], j0 = (e & GRAN_MASK) * 16u;
                         if (td < 256u) {
                             const bool live = f < p.N && j0 + 8 * a_h < p.max_rank;
-                            const uint16_t* src = live ? reinterpret_cast<const uint16_t*>(gran_b[lb * 4 + g]) + a_src_off + j0 : p.t;
+                            const uint16_t* src = live ? reinterpret_cast<const uint16_t*>(p.b_table[e >> GRAN_SHIFT]) + a_src_off + j0 : p.t;
                             cp_async_16_zfill(base + g * C::L_GRAN_A + a_dst, src, live ? 16u : 0u);
                         }
                     }

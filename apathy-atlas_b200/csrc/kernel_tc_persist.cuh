@@ -299,7 +299,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         const uint32_t base = epi0 + ls * C::L_STAGE;
                         const uint32_t e = gran[g * C::MAX_GRANULES + q];
                         if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * C::L_STAGE);
-                        tma_load_3d_pair(base, &map_b, int32_t((e & 3u) * 16u), int32_t(f0), int32_t(e >> 2), lfull_at_leader + 8 * ls);
+                        tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
                         tma_load_2d_pair(base + C::L_GRAN_A, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
                         if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
                     }
@@ -450,7 +450,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     uint32_t pos = base + incl - cnt;
                     for (uint32_t w = word; w; w &= w - 1) {
                         const uint32_t s2 = te * 32 + (__ffs(w) - 1);
-                        for (uint32_t k = 0; k < gcount[s2]; ++k) gran[g * C::MAX_GRANULES + pos++] = uint16_t((s2 << 2) | k);
+                        for (uint32_t k = 0; k < gcount[s2]; ++k) gran[g * C::MAX_GRANULES + pos++] = uint16_t((s2 << GRAN_SHIFT) | k);
                     }
                     if (te == 0) misc[4 + g] = scan[0] + scan[1] + scan[2] + scan[3];
                 }

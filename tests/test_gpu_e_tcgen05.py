@@ -77,6 +77,46 @@ def test_fused_lora(cuda, atlas, oracle, M, K, N, ranks, max_rank, with_ranks):
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,ranks,max_rank", [
+    (1, 288, 128, [8], 8),                               # one 256-wide stage and a 32-wide rest
+    (16, 320, 200, [16] * 4, 16),                        # scale rows of 20 bytes: no K block of the rest is whole
+    (77, 2880, 520, [16] * 8, 16),                       # split K over an odd number of K blocks
+    (300, 544, 264, [8, 64], 64),                        # CTA pairs, a half K block at the end, partial second token tile
+    (40, 512, 256, [128, 16, 65], 128),                  # eight granules of one slot
+    (300, 1056, 384, [128] * 16, 128),                   # both at once, 128 granules per tile
+    (1100, 512, 2304, [128, 72], 128),                   # two-tile persistent form, ranks above 64
+    (8, 8480, 256, [104], 104),                          # max_rank not a multiple of 16, long K
+])
+def test_shapes_beyond_the_forced_path(cuda, atlas, oracle, M, K, N, ranks, max_rank):
+    """K a multiple of 32 only, ranks above 64: the default path takes them to the tensor cores, in every form a call can have,
+    while what is refused there (a forced path, FP4 activations) stays refused."""
+    from atlas_b200 import synth
+    case = synth.make_case("wide", M=M, K=K, N=N, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 3, none_frac=0.15,
+                           scale2=0.02, b_std=0.1, seed=M + K)
+    dc = DeviceCase(cuda, atlas, case, x_row_stride=K + 8, out_row_stride=N + 8)
+    want = ideal(oracle, case)
+    y, variant = dc.run(lora_ws=True)
+    assert variant == atlas.VARIANT_TCGEN05
+    assert_close(oracle, y[:, :N], want, "default path")
+    assert (y[:, N:] == 0x7FC0).all()
+    if K < 8192:                                         # tiles from the shrink, tiles built in the kernel, B_s by address
+        for form in (dict(), dict(strided=False), dict(lora_ws=True, flags=atlas.FLAG_REUSE_SHRINK)):
+            assert_close(oracle, dc.run(**form)[0][:, :N], want, f"form {form}")
+    yb, variant = dc.run(lora=False)
+    assert variant == atlas.VARIANT_TCGEN05
+    none = case.seq_slot < 0
+    assert np.array_equal(y[none][:, :N], yb[none][:, :N])      # routing is exact
+    y_simt, variant = dc.run(flags=atlas.FLAG_FORCE_SIMT)
+    assert variant == atlas.VARIANT_SIMT
+    # no further from the FP32 result than the path that took these shapes, which rounds base and delta to BF16 before it adds
+    err = [np.linalg.norm(oracle.bf16_to_f32(b[:, :N].copy()) - want) for b in (y, y_simt)]
+    assert err[0] <= err[1]
+    for flags in (atlas.FLAG_FORCE_TCGEN05, atlas.FLAG_ACT_FP4):
+        with pytest.raises(atlas.AtlasError):
+            dc.run(flags=flags, lora_ws=True)
+    assert atlas.device_status() == 0
+
+
 def test_token_permutation_is_bit_exact(cuda, atlas, oracle):
     from atlas_b200 import synth
     import copy
