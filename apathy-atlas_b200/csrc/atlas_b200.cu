@@ -28,6 +28,7 @@
 #include "kernel_dense_tc.cuh"
 #include "kernels_simt.cuh"
 #include "kernel_shrink_mma.cuh"
+#include "kernel_expand_mma.cuh"
 #include "kernel_shrink_tc.cuh"
 #include "kernels_mlp_glue.cuh"
 #include "kernel_push.cuh"
@@ -267,6 +268,22 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
 static int launch_expand(const ExpandParams& p, cudaStream_t st) {
     if (p.M == 0 || p.n_out == 0) return ATLAS_B200_OK;
     if (p.max_rank > EXPAND_MAX_RANK) return ATLAS_B200_ERR_LIMIT;
+    if (p.max_rank % 8 == 0 && p.max_rank <= uint32_t(EXM_MAX_RANK) && aligned(p.xa, 8)) {
+        // tensor cores (kernel_expand_mma.cuh) wherever xa rows can be read four ranks at a time and B_s fits in registers
+        const uint32_t chunk = EXM_ROWS, chunks = (p.M + chunk - 1) / chunk, cols = (p.n_out + EXM_OUTS - 1) / EXM_OUTS;
+        // CTAs sharing a chunk's runs: at most as many as it can have runs (one per slot that occurs, one more per sixteen
+        // rows), and no more than eight CTAs per SM in all
+        const uint32_t rows = std::min(p.M, chunk), most = (p.seq_slot ? std::min(rows, p.max_loras) : 0u) + (rows + 15) / 16;
+        uint32_t splits = 1;
+        while (splits * 2 <= most && uint64_t(cols) * chunks * splits * 2 <= uint64_t(rt_sm_count()) * 8) splits *= 2;
+        const dim3 grid(cols, chunks * splits);
+        if (grid.y > 65535) return ATLAS_B200_ERR_LIMIT;
+        if (p.max_rank <= 16) lora_expand_mma_kernel<1><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
+        else if (p.max_rank <= 32) lora_expand_mma_kernel<2><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
+        else if (p.max_rank <= 64) lora_expand_mma_kernel<4><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
+        else lora_expand_mma_kernel<8><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
+        return launch_status();
+    }
     // rows per CTA: 32 for large batches (a CTA re-uses its B rows out of L1 while neighbouring rows share an adapter),
     // fewer while the grid would otherwise leave SMs without a CTA (a decode batch)
     ExpandParams q = p;

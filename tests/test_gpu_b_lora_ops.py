@@ -48,6 +48,37 @@ def test_bgmv_matches_staged_oracle(cuda, atlas, oracle, M, K, N, ranks, max_ran
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,ranks,max_rank,xs,os_", [
+    (1, 256, 16, [8], 8, None, None),                     # half a K step, fewer features than a warp holds
+    (16, 256, 136, [24, 8], 24, None, None),              # K step and a half
+    (129, 256, 264, [16] * 40, 16, None, None),           # a second chunk of one row, more runs than sixteens
+    (40, 256, 130, [72, 128], 128, None, 131),            # features past a multiple of eight, odd row stride
+    (300, 256, 256, [64], 64, None, 264),                 # one slot throughout
+    (33, 256, 128, [136, 8], 136, None, None),            # ranks beyond the tensor-core form
+])
+def test_bgmv_expand_forms(cuda, atlas, oracle, M, K, N, ranks, max_rank, xs, os_):
+    from atlas_b200 import synth
+    case = synth.make_case("bgmv", M=M, K=K, N=N, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 2,
+                           none_frac=0.2 if M > 1 else 0.0, b_std=0.1, seed=M)
+    # an infinity and a NaN in one adapter's B are its own rows' business
+    bad = 0 if len(ranks) > 1 else None
+    if bad is not None:
+        case.adapters[bad].b[0, 0], case.adapters[bad].b[N - 1, 0] = 0x7F80, 0x7FC0
+    got, _, want, _, base = _run_bgmv(cuda, atlas, oracle, case, xs, os_)
+    ok = (case.seq_slot >= 0) & (case.seq_slot != (bad if bad is not None else -1))
+    none = case.seq_slot < 0
+    assert np.array_equal(got[none], base[none]) and np.array_equal(got[:, N:], base[:, N:])
+    f = oracle.bf16_to_f32
+    # both sides round delta and the sum to BF16, each up to one unit (2^-8) apart from an xa that may differ by one
+    g, w, b = f(got[ok][:, :N].copy()), f(want[ok][:, :N].copy()), f(base[ok][:, :N].copy())
+    assert (np.abs(g - w) <= ATOL + RTOL * np.abs(w) + 2.0 ** -8 * (np.abs(b) + np.abs(w - b))).all()
+    hit = case.seq_slot == bad
+    if bad is not None and hit.any():
+        assert not np.isfinite(f(got[hit][:, [0, N - 1]].copy())).any()
+        assert np.isfinite(f(got[hit][:, 1:N - 1].copy())).all()
+    assert atlas.device_status() == 0
+
+
 def test_bgmv_null_table_entries_and_out_of_range_slot(cuda, atlas, oracle):
     torch = cuda
     from atlas_b200 import synth
