@@ -1055,9 +1055,11 @@ int atlas_b200_dequant_nvfp4_to_bf16(const void* packed, const void* scales, voi
     if (!packed || !scales || !out_bf16) return ATLAS_B200_ERR_NULL;
     if (k % 16 != 0) return ATLAS_B200_ERR_DIMS;
     if (!aligned(out_bf16, 4)) return ATLAS_B200_ERR_ALIGN;
-    dequant_nvfp4_kernel<<<n, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const size_t groups = size_t(n) * (k / 16);
+    const unsigned blocks = unsigned(std::min<size_t>((groups + 255) / 256, size_t(rt_sm_count()) * 16));
+    dequant_nvfp4_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const uint8_t*>(packed), static_cast<const uint8_t*>(scales), static_cast<uint16_t*>(out_bf16),
-        combined_global, n, k);
+        combined_global, groups, aligned(packed, 8) && aligned(out_bf16, 16) ? 1u : 0u);
     return launch_status();
 }
 

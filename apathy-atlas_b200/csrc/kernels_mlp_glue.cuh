@@ -48,13 +48,18 @@ __device__ __forceinline__ float swiglu(float g, float u, float limit) {
     return g * (1.0f / (1.0f + __expf(-g))) * u;
 }
 
+// i / per_row, by a 32-bit division wherever the count allows (a 64-bit one takes more instructions than the rest of such a loop)
+__device__ __forceinline__ size_t row_of(size_t i, size_t per_row, size_t total) {
+    return total <= 0xFFFFFFFFu ? size_t(uint32_t(i) / uint32_t(per_row)) : i / per_row;
+}
+
 // rows of gate / up / out may be spaced wider than K (column segments of wider buffers); strides in elements, multiples of 8
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const uint16_t* __restrict__ gate, const uint16_t* __restrict__ up, uint16_t* __restrict__ out, float gate_scale,
                 float up_scale, float limit, uint32_t M, uint32_t K, uint32_t in_stride, uint32_t out_stride) {
     const size_t per_row = K / 8, total = size_t(M) * per_row;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const size_t row = i / per_row, c = (i % per_row) * 8;
+        const size_t row = row_of(i, per_row, total), c = (i - row * per_row) * 8;
         const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gate + row * in_stride + c));
         const uint4 uv = __ldg(reinterpret_cast<const uint4*>(up + row * in_stride + c));
         const uint32_t g[4] = {gv.x, gv.y, gv.z, gv.w}, u[4] = {uv.x, uv.y, uv.z, uv.w};
@@ -74,7 +79,7 @@ silu_mul_quant_nvfp4_kernel(const uint16_t* __restrict__ gate, const uint16_t* _
                             uint32_t in_stride) {
     const size_t groups = K / 16, total = size_t(M) * groups;
     for (size_t gi = size_t(blockIdx.x) * blockDim.x + threadIdx.x; gi < total; gi += size_t(gridDim.x) * blockDim.x) {
-        const size_t row = gi / groups, c = (gi % groups) * 16;
+        const size_t row = row_of(gi, groups, total), c = (gi - row * groups) * 16;
         const uint4* gp = reinterpret_cast<const uint4*>(gate + row * in_stride + c);
         const uint4* up4 = reinterpret_cast<const uint4*>(up + row * in_stride + c);
         const uint4 g0 = __ldg(gp), g1 = __ldg(gp + 1), u0 = __ldg(up4), u1 = __ldg(up4 + 1);
@@ -89,15 +94,9 @@ silu_mul_quant_nvfp4_kernel(const uint16_t* __restrict__ gate, const uint16_t* _
             gmax = fmaxf(gmax, fmaxf(fabsf(v[2 * k]), fabsf(v[2 * k + 1])));
         }
         // the activation quantiser of the FP4-activation mode: tensor scale 1, scale byte = E4M3(group max / 6)
-        const float f8 = gmax > 0.0f ? __fdiv_rn(gmax, 6.0f) : 0.0f;
-        const uint32_t byte = e4m3_encode_sw(f8);
-        scales[gi] = uint8_t(byte);
-        const float eff = e4m3_decode(byte);
-        const float inv_eff = eff > 0.0f ? __fdiv_rn(1.0f, eff) : 0.0f;
-        uint32_t q[2] = {0u, 0u};
-#pragma unroll
-        for (int k = 0; k < 16; ++k) q[k / 8] |= e2m1_quantize(__fmul_rn(v[k], inv_eff)) << (4 * (k % 8));
-        *reinterpret_cast<uint2*>(packed + gi * 8) = make_uint2(q[0], q[1]);
+        uint2 q;
+        scales[gi] = uint8_t(nvfp4_group(v, gmax, 1.0f, 1.0f, q));        // (multiplying by one changes no bit)
+        *reinterpret_cast<uint2*>(packed + gi * 8) = q;
     }
 }
 

@@ -8,24 +8,37 @@
 namespace atlas {
 
 // =============================================================================================
-// NVFP4 -> BF16 decode.  One block per row, threads stride over 8-element groups.
+// NVFP4 -> BF16 decode, one thread per group of 16 (rows are dense, so a group's place follows from its number).
 // out = bf16(E2M1[nib] * (e4m3(scale) * g)), the operation order of
 // kernels/gb10/common/dequant_nvfp4_bf16.cu:64-72, so results are bit-identical to it.
+// `vec` != 0: codes and output are 8- / 16-byte aligned, so that a group is one 64-bit load and two 128-bit stores.
 // =============================================================================================
 __global__ void __launch_bounds__(256)
 dequant_nvfp4_kernel(const uint8_t* __restrict__ packed, const uint8_t* __restrict__ scales,
-                     uint16_t* __restrict__ out, float g, uint32_t N, uint32_t K) {
-    const uint32_t row = blockIdx.x;
-    if (row >= N) return;
-    const uint8_t* rp = packed + size_t(row) * (K / 2);
-    const uint8_t* rs = scales + size_t(row) * (K / 16);
-    uint16_t* ro = out + size_t(row) * K;
-    for (uint32_t b = threadIdx.x; b < K / 2; b += blockDim.x) {
-        const float s = e4m3_decode(rs[b >> 3]) * g;
-        const uint32_t byte = rp[b];
-        const uint32_t w = uint32_t(f32_to_bf16_bits(e2m1_decode(byte & 0xFu) * s)) |
-                           (uint32_t(f32_to_bf16_bits(e2m1_decode(byte >> 4) * s)) << 16);
-        reinterpret_cast<uint32_t*>(ro)[b] = w;
+                     uint16_t* __restrict__ out, float g, size_t total, uint32_t vec) {
+    for (size_t gi = size_t(blockIdx.x) * blockDim.x + threadIdx.x; gi < total; gi += size_t(gridDim.x) * blockDim.x) {
+        const float s = e4m3_decode(scales[gi]) * g;
+        uint32_t p[2] = {0u, 0u}, w[8];
+        if (vec) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(packed) + gi);
+            p[0] = v.x; p[1] = v.y;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) p[i / 4] |= uint32_t(packed[gi * 8 + i]) << (8 * (i % 4));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t byte = p[i / 4] >> (8 * (i % 4));
+            w[i] = pack_bf16x2(e2m1_decode(byte & 0xFu) * s, e2m1_decode((byte >> 4) & 0xFu) * s);
+        }
+        uint32_t* o = reinterpret_cast<uint32_t*>(out + gi * 16);
+        if (vec) {
+            reinterpret_cast<uint4*>(o)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+            reinterpret_cast<uint4*>(o)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) o[i] = w[i];
+        }
     }
 }
 
@@ -60,22 +73,43 @@ __device__ __forceinline__ uint32_t e4m3_encode_sw(float v) {
     return (sign << 7) | (uint32_t(e) << 3) | man;
 }
 
-// E2M1 code of v with the reference's bins (|v| <= .25 -> 0, <= .75 -> .5, <= 1.25 -> 1, <= 1.75 -> 1.5, <= 2.5 -> 2,
-// <= 3.5 -> 3, <= 5 -> 4, else 6: ties go to the smaller magnitude, kernels/gb10/common/quantize_bf16_to_nvfp4.cu:109-124).
-// From 1 upward E2M1 is "one mantissa bit": adding just under half an ulp of that bit to the FP32 pattern and truncating
-// rounds half DOWN, which is exactly the `<=` of the bins (and carries into the exponent at 1.75 and 3.5); the code is
-// then twice the unbiased exponent plus the mantissa bit plus 2, clamped to 6.0's code.  Below 1 the two bins are compared
-// directly.  Same results as the chain of compares, in half the instructions (the quantiser is bound by instruction issue).
-__device__ __forceinline__ uint32_t e2m1_quantize(float v) {
-    const uint32_t bits = __float_as_uint(v);
-    const uint32_t mag = bits & 0x7FFFFFFFu;
-    const float a = __uint_as_float(mag);
-    // (mag + 0x1FFFFF) >> 22 = (biased exponent << 1) | mantissa bit, after rounding half down
-    int32_t code = int32_t((mag + 0x1FFFFFu) >> 22) - (127 * 2 - 2);
-    code = min(max(code, 2), 7);
-    uint32_t idx = a <= 0.75f ? (a <= 0.25f ? 0u : 1u) : uint32_t(code);
-    if (mag > 0x7F800000u) idx = 7u;                 // NaN compares false everywhere in the chain of bins: the last one
-    return (v < 0.0f ? 8u : 0u) | idx;
+// E2M1 codes of eight values with the reference's bins (|v| <= .25 -> 0, <= .75 -> .5, <= 1.25 -> 1, <= 1.75 -> 1.5, <= 2.5 -> 2,
+// <= 3.5 -> 3, <= 5 -> 4, else 6: ties go to the smaller magnitude, NaN to 6; the sign bit is v < 0;
+// kernels/gb10/common/quantize_bf16_to_nvfp4.cu:109-124), value i in bits [4i, 4i+4).
+// The conversion instruction rounds to nearest even and saturates (NaN to +6), which is the same except for the three ties
+// whose even neighbour is the larger one — .75, 1.75 and 3.5, the values whose FP32 mantissa is 1.1x with nothing below: those
+// are moved one ulp towards zero first — and for -0, whose sign the bins drop: adding +0 does.
+__device__ __forceinline__ float e2m1_below_tie(float v) {
+    const uint32_t bits = __float_as_uint(__fadd_rn(v, 0.0f));
+    return __uint_as_float(bits - ((bits & 0x005FFFFFu) == 0x00400000u ? 1u : 0u));
+}
+__device__ __forceinline__ uint32_t e2m1_quantize8(const float (&v)[8]) {
+    float t[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = e2m1_below_tie(v[i]);
+    uint32_t codes;
+    asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\t"
+        "cvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+        "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+        : "=r"(codes)
+        : "f"(t[0]), "f"(t[1]), "f"(t[2]), "f"(t[3]), "f"(t[4]), "f"(t[5]), "f"(t[6]), "f"(t[7]));
+    return codes;
+}
+
+// Sixteen values -> scale byte and codes: scale = E4M3(max / scale2 / 6) through the software encoder, codes of v / (scale * scale2).
+__device__ __forceinline__ uint32_t nvfp4_group(const float (&v)[16], float gmax, float scale2, float inv_scale2, uint2& codes) {
+    const float f8 = gmax > 0.0f ? __fdiv_rn(__fmul_rn(gmax, inv_scale2), 6.0f) : 0.0f;
+    const uint32_t byte = e4m3_encode_sw(f8);
+    const float eff = __fmul_rn(e4m3_decode(byte), scale2);
+    const float inv_eff = eff > 0.0f ? __fdiv_rn(1.0f, eff) : 0.0f;
+    float lo[8], hi[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { lo[i] = __fmul_rn(v[i], inv_eff); hi[i] = __fmul_rn(v[8 + i], inv_eff); }
+    codes = make_uint2(e2m1_quantize8(lo), e2m1_quantize8(hi));
+    return byte;
 }
 
 // `in_row_stride` (elements) lets the rows of `in` be spaced wider than K (activations); the outputs
@@ -89,7 +123,12 @@ quantize_nvfp4_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ pac
     const size_t total = size_t(N) * groups;
     const float inv_scale2 = scale2 > 0.0f ? __fdiv_rn(1.0f, scale2) : 0.0f;
     for (size_t gi = size_t(blockIdx.x) * blockDim.x + threadIdx.x; gi < total; gi += size_t(gridDim.x) * blockDim.x) {
-        const uint16_t* p = in + (gi / groups) * in_row_stride + (gi % groups) * 16;
+        // (dense rows need no division, and a 64-bit one is the longest piece of this loop)
+        const uint16_t* p = in + gi * 16;
+        if (in_row_stride != K) {
+            const size_t row = total <= 0xFFFFFFFFu ? uint32_t(gi) / groups : gi / groups;
+            p = in + row * in_row_stride + (gi - row * groups) * 16;
+        }
         float v[16];
         float gmax = 0.0f;
         if (vec) {
@@ -103,19 +142,13 @@ quantize_nvfp4_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ pac
         }
 #pragma unroll
         for (int i = 0; i < 16; ++i) gmax = fmaxf(gmax, fabsf(v[i]));
-        const float f8 = gmax > 0.0f ? __fdiv_rn(__fmul_rn(gmax, inv_scale2), 6.0f) : 0.0f;
-        const uint32_t byte = e4m3_encode_sw(f8);
-        scales[gi] = uint8_t(byte);
-        const float eff = __fmul_rn(e4m3_decode(byte), scale2);
-        const float inv_eff = eff > 0.0f ? __fdiv_rn(1.0f, eff) : 0.0f;
-        uint32_t q[2] = {0u, 0u};
-#pragma unroll
-        for (int i = 0; i < 16; ++i) q[i / 8] |= e2m1_quantize(__fmul_rn(v[i], inv_eff)) << (4 * (i % 8));
+        uint2 q;
+        scales[gi] = uint8_t(nvfp4_group(v, gmax, scale2, inv_scale2, q));
         if (vec) {
-            *reinterpret_cast<uint2*>(packed + gi * 8) = make_uint2(q[0], q[1]);
+            *reinterpret_cast<uint2*>(packed + gi * 8) = q;
         } else {
 #pragma unroll
-            for (int i = 0; i < 8; ++i) packed[gi * 8 + i] = uint8_t(q[i / 4] >> (8 * (i % 4)));
+            for (int i = 0; i < 8; ++i) packed[gi * 8 + i] = uint8_t((i < 4 ? q.x : q.y) >> (8 * (i % 4)));
         }
     }
 }
