@@ -715,9 +715,12 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
 }
 
 // ---- dense-BF16 base on the tensor cores (kernel_dense_tc.cuh) ----
+// K: rows of 16-byte multiples, which is what TMA wants (it fills a last, partial K block with zeros); a forced tcgen05 path
+// keeps to whole blocks
 static bool dense_tc_eligible(const atlas_b200_linear_desc& d) {
     DeviceState* dst = device_state();
-    return dst && dst->sm100 && g_encode && d.w_bf16 && d.k % tc::KB == 0 && d.x_row_stride % 8 == 0 && aligned(d.x, 16) &&
+    const uint32_t k_unit = (d.flags & ATLAS_B200_FLAG_FORCE_TCGEN05) ? uint32_t(tc::KB) : 8u;
+    return dst && dst->sm100 && g_encode && d.w_bf16 && d.k % k_unit == 0 && d.k >= uint32_t(tc::KB) && d.x_row_stride % 8 == 0 && aligned(d.x, 16) &&
            aligned(d.w_bf16, 16) && !d.n_dest;
 }
 

@@ -54,7 +54,7 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t f0 = blockIdx.x * FT, m0 = blockIdx.y * MT;
     const uint32_t ks = p.k_split, kz = blockIdx.z;
-    const uint32_t total_kb = p.K / KB;
+    const uint32_t total_kb = (p.K + KB - 1) / KB;       // (a partial last block is filled with zeros by TMA)
     const uint32_t kb_lo = kz * total_kb / ks, kb_hi = (kz + 1u) * total_kb / ks;
     const uint32_t num_kb = kb_hi - kb_lo;
 

@@ -71,3 +71,17 @@ def test_dense_bf16_tensor_core_base_shapes(cuda, atlas, oracle, M, K, N):
     none = case.seq_slot < 0
     assert np.array_equal(y[none], yb[none])
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 72, 136), (16, 5728, 264), (40, 1000, 200), (130, 96, 128)])
+def test_dense_bf16_partial_k_block(cuda, atlas, oracle, M, K, N):
+    """K a multiple of eight: the last K block is partly, or all but eight elements, filled in."""
+    from atlas_b200 import synth
+    case = synth.make_case("dense", M=M, K=K, N=N, ranks=[8], max_rank=8, base="bf16", seed=M + N)
+    dc = DeviceCase(cuda, atlas, case, x_row_stride=(K + 15) // 8 * 8)
+    y, variant = dc.run(lora=False)
+    assert variant == atlas.VARIANT_TCGEN05
+    assert_close(oracle, y, ideal(oracle, case, lora=False), "dense base")
+    with pytest.raises(atlas.AtlasError):
+        dc.run(lora=False, flags=atlas.FLAG_FORCE_TCGEN05)
+    assert atlas.device_status() == 0
