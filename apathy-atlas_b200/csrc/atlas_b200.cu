@@ -25,6 +25,7 @@
 #include "common.cuh"
 #include "kernel_tc.cuh"
 #include "kernel_tc_persist.cuh"
+#include "kernel_decode_mma.cuh"
 #include "kernel_dense_tc.cuh"
 #include "kernels_simt.cuh"
 #include "kernel_shrink_mma.cuh"
@@ -62,7 +63,7 @@ struct DeviceState {
     std::atomic<bool> ready{false};
     bool sm100 = false;
     int sm_count = 148;
-    bool tc_attr_set[40] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair}
+    bool tc_attr_set[40] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair} x {K of whole raw stages, not}
     int known_clusters[20][9] = {};   // resident clusters per kernel instance and K split; 0 = not asked yet
     bool persist_attr_set[kPersistKernels] = {};
     int persist_clusters[kPersistKernels] = {};
@@ -714,6 +715,41 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
                                           maps.xs, maps.t, p, pp));
 }
 
+// ---- the smallest batches (kernel_decode_mma.cuh) ----
+template <int TILES, int NT>
+static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+    tc::Params p{};
+    int rc = fill_tc_params(d, false, false, TTiles{}, p);
+    if (rc) return rc;
+    DecodeParams w{};
+    w.x = static_cast<const uint16_t*>(d.x);
+    w.w_packed = static_cast<const uint8_t*>(d.w_packed);
+    w.w_scale = static_cast<const uint8_t*>(d.w_scale);
+    w.x_row_stride = d.x_row_stride;
+    const uint32_t ctas = (d.n + 16 * TILES - 1) / (16 * TILES);
+    t_last_shape[0] = 8 * NT; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
+    if (shrink) {
+        rc = launch_shrink(*shrink, d.max_loras, st, true, ctas * 3 <= uint32_t(rt_sm_count()) * 2);
+        if (rc) return rc;
+    }
+    p.wait_for_shrink = shrink ? 1u : 0u;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(DCM_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = shrink ? 1 : 0;
+    return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT>, w, p));
+}
+
+static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+    // sixteen features per CTA instead of 32 while those would not give every other SM one
+    return d.n <= 32u * uint32_t(rt_sm_count()) / 2u ? launch_decode_as<1, 1>(d, shrink, st) : launch_decode_as<2, 1>(d, shrink, st);
+}
+
 // ---- dense-BF16 base on the tensor cores (kernel_dense_tc.cuh) ----
 // K: rows of 16-byte multiples, which is what TMA wants (it fills a last, partial K block with zeros); a forced tcgen05 path
 // keeps to whole blocks
@@ -877,6 +913,16 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         sp.a_pool_base = d.a_pool_base; sp.a_slot_stride = d.a_slot_stride;
         // t = scale_s / (scale2 * 2^8) * (A_s x), the unit of the MMA accumulator (no 2^8 with FP4 activations)
         sp.post = act_fp4 ? 1.0f / d.scale2 : 1.0f / (d.scale2 * kWeightPreScale);
+
+        // The smallest batches, unless a form of the tcgen05 path is asked for by a flag.
+        constexpr uint32_t tc_forms = ATLAS_B200_FLAG_FORCE_TCGEN05 | ATLAS_B200_FLAG_ACT_FP4 | ATLAS_B200_FLAG_NO_CTA_PAIR |
+                                      ATLAS_B200_FLAG_NO_K_SPLIT | ATLAS_B200_FLAG_NO_PERSISTENT | ATLAS_B200_FLAG_ONE_TILE_PASS;
+        if (d.m <= uint32_t(DCM_MAX_TOKENS) && !(d.flags & tc_forms) && !shrink_only) {
+            // (t rows in lora_t are written by every call: the tiles a tcgen05 call leaves in `ws` are not what this kernel reads)
+            rc = launch_decode(d, d.seq_slot ? &sp : nullptr, st);
+            if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
+            return rc;
+        }
 
         // Masked-t tiles: with scratch to put them in, the shrink writes the activation operand of every LoRA
         // K-step once, in the layout the MMA reads, and the fused kernel's CTAs fetch it by TMA — instead of

@@ -1,0 +1,190 @@
+// The fused NVFP4 + multi-LoRA linear for the smallest batches: weights expanded in registers, mma.sync.
+//
+//   y[m, f] = bf16( out_scale * ( sum_k W'[f,k] x[m,k] + sum_j B_s[f,j] t[m,j] ) ),   s = seq_slot[m], t pre-scaled by the shrink
+//
+// A decode batch is bound by streaming the weights once.  The tcgen05 form cannot keep up with that stream: its weight operand
+// goes through tensor memory, which fixes the order of the K elements (four byte permutes per eight codes), and its
+// eight expansion warps need 585 cycles per 128 x 64 block whatever the batch: one token x 14336 features x 4096 took 30 us
+// for 33 MB.  Here every warp of the SM expands, the operand stays in the registers the codes were expanded in, and since
+// BOTH operands of mma.sync come from registers the K elements may take any order as long as they meet their partners:
+// the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired the same way (four permutes
+// per eight elements of x, shared by all features of the warp).
+//
+// A CTA owns 16 * TILES features and all of K; its eight warps take interleaved 128-wide K steps (per thread and feature
+// row one 128-bit load of 32 codes and their two scale bytes, the next step's loads in flight while one is multiplied),
+// and the partial sums are added in warp order through shared memory.  No cluster, no tensor memory, no barriers but two.
+// The MMA's M is 16 features, its N 8 tokens (NT of them side by side).
+//
+// LoRA: granule j (16 ranks) of slot s is one more K step, done by warp (s + 3 j) % 8, so that the order in which a token's terms
+// are added depends on its own slot alone.  t rows come from the shrink this kernel may overtake (programmatic dependent
+// launch): they are first read behind griddepcontrol.wait, after the base loop.
+#pragma once
+
+#include "kernel_shrink_mma.cuh"
+#include "kernel_tc.cuh"
+
+namespace atlas {
+
+constexpr int DCM_WARPS = 8, DCM_THREADS = 32 * DCM_WARPS;
+constexpr int DCM_KSTEP = 128;
+constexpr int DCM_MAX_TOKENS = 8;
+
+struct DecodeParams {
+    const uint16_t* x;
+    const uint8_t* w_packed;
+    const uint8_t* w_scale;
+    uint32_t x_row_stride;
+};
+
+// Eight codes -> four BF16x2 words holding the pairs (i, i + 4), times the multiplier: e2m1x8_to_bf16x8 without its permutes.
+__device__ __forceinline__ void e2m1x8_to_pairs(uint32_t p, uint32_t mul, uint32_t (&h)[4]) {
+    const uint32_t q = p >> 8;
+    h[0] = bf16x2_mul(((p << 12) & 0x80008000u) | ((p << 6) & 0x01C001C0u), mul);
+    h[1] = bf16x2_mul(((p << 8) & 0x80008000u) | ((p << 2) & 0x01C001C0u), mul);
+    h[2] = bf16x2_mul(((p << 4) & 0x80008000u) | ((q << 6) & 0x01C001C0u), mul);
+    h[3] = bf16x2_mul((p & 0x80008000u) | ((q << 2) & 0x01C001C0u), mul);
+}
+
+template <int TILES, int NT>
+__global__ void __launch_bounds__(DCM_THREADS, 2)
+nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
+    __shared__ float part[DCM_WARPS][NT * 8][TILES * 16 + 1];          // [warp][token][feature]
+    __shared__ int32_t slot_s[DCM_MAX_TOKENS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t f0 = blockIdx.x * (TILES * 16);
+
+    if (tid < DCM_MAX_TOKENS) {
+        int32_t s = -1;
+        if (p.seq_slot && tid < p.M) {
+            s = p.seq_slot[tid];
+            if (s >= 0) {
+                if (uint32_t(s) >= p.max_loras) { record_status(STATUS_SLOT_OUT_OF_RANGE); s = -1; }
+                else if (p.a_table[s] == 0ull || p.b_table[s] == 0ull) s = -1;
+            }
+        }
+        slot_s[tid] = s;
+    }
+
+    // ---- base: this thread's 32 codes per step of feature rows g and g + 8 of every tile, and of x rows g (+ 8 per n-tile) ----
+    const uint32_t n_steps = (p.K + DCM_KSTEP - 1) / DCM_KSTEP;
+    const uint8_t* code_row[TILES][2];
+    const uint8_t* scale_row[TILES][2];
+#pragma unroll
+    for (int i = 0; i < TILES; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t f = min(f0 + 16 * i + 8 * h + g, p.N - 1u);          // (rows past N repeat the last one and are not stored)
+            code_row[i][h] = w.w_packed + size_t(f) * (p.K / 2u) + 16 * t;
+            scale_row[i][h] = w.w_scale + size_t(f) * (p.K / 16u) + 2 * t;
+        }
+    const uint16_t* x_row[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) x_row[n] = w.x + size_t(min(8 * n + g, p.M - 1u)) * w.x_row_stride + 32 * t;
+
+    float acc[TILES][NT][4] = {};
+    uint4 code[2][TILES][2];
+    uint32_t sc[2][TILES][2];
+    auto load = [&](uint32_t step, uint4 (&c)[TILES][2], uint32_t (&s)[TILES][2]) {
+        const bool in = step * DCM_KSTEP + 32 * t < p.K;                        // (K is a multiple of 32)
+#pragma unroll
+        for (int i = 0; i < TILES; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                c[i][h] = in ? __ldcs(reinterpret_cast<const uint4*>(code_row[i][h] + step * (DCM_KSTEP / 2))) : make_uint4(0u, 0u, 0u, 0u);
+                s[i][h] = in ? uint32_t(__ldg(reinterpret_cast<const uint16_t*>(scale_row[i][h] + step * (DCM_KSTEP / 16)))) : 0u;
+            }
+    };
+    auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2]) {
+        const bool in = step * DCM_KSTEP + 32 * t < p.K;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {                                           // eight K elements per thread at a time
+            uint32_t xb[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                const uint4 v = in && 8 * n + g < p.M ? __ldg(reinterpret_cast<const uint4*>(x_row[n] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
+                xb[n][0] = __byte_perm(v.x, v.z, 0x5410); xb[n][1] = __byte_perm(v.x, v.z, 0x7632);
+                xb[n][2] = __byte_perm(v.y, v.w, 0x5410); xb[n][3] = __byte_perm(v.y, v.w, 0x7632);
+            }
+#pragma unroll
+            for (int i = 0; i < TILES; ++i) {
+                uint32_t a[2][4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t word = u == 0 ? c[i][h].x : (u == 1 ? c[i][h].y : (u == 2 ? c[i][h].z : c[i][h].w));
+                    e2m1x8_to_pairs(word, e4m3_to_bf16x2_shifted((s[i][h] >> (u < 2 ? 0 : 8)) & 0xFFu), a[h]);
+                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n) {
+                    mma_bf16_16816(acc[i][n], a[0][0], a[1][0], a[0][1], a[1][1], xb[n][0], xb[n][1]);
+                    mma_bf16_16816(acc[i][n], a[0][2], a[1][2], a[0][3], a[1][3], xb[n][2], xb[n][3]);
+                }
+            }
+        }
+    };
+    load(warp, code[0], sc[0]);
+    for (uint32_t step = warp; step < n_steps; step += 2 * DCM_WARPS) {
+        load(step + DCM_WARPS, code[1], sc[1]);
+        multiply(step, code[0], sc[0]);
+        load(step + 2 * DCM_WARPS, code[0], sc[0]);
+        if (step + DCM_WARPS < n_steps) multiply(step + DCM_WARPS, code[1], sc[1]);
+    }
+
+    // ---- LoRA granules of this warp ----
+    if (p.seq_slot) {
+        __syncthreads();                                                        // slot_s
+        if (p.wait_for_shrink) asm volatile("griddepcontrol.wait;" ::: "memory");
+        int32_t own[NT];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) own[n] = slot_s[8 * n + g];
+        const int32_t lane_slot = lane < DCM_MAX_TOKENS ? slot_s[lane] : -1;
+        for (uint32_t left = __ballot_sync(0xFFFFFFFFu, lane_slot >= 0); left;) {
+            const int32_t s = __shfl_sync(0xFFFFFFFFu, lane_slot, __ffs(left) - 1);
+            left &= ~__ballot_sync(0xFFFFFFFFu, lane_slot == s);
+            const uint32_t rank = p.rank_table ? min(p.rank_table[s], p.max_rank) : p.max_rank;
+            const uint16_t* B = reinterpret_cast<const uint16_t*>(p.b_table[s]);
+            const bool b_vec = (reinterpret_cast<uintptr_t>(B) & 7u) == 0u;
+            for (uint32_t j = 0; 16 * j < rank; ++j) {
+                if ((uint32_t(s) + 3u * j) % DCM_WARPS != warp) continue;
+                const uint32_t j0 = 16 * j + 4 * t;
+                const bool in = j0 < p.max_rank;                                // (max_rank is a multiple of 8)
+                uint2 tv[NT];
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+                    tv[n] = in && own[n] == s ? *reinterpret_cast<const uint2*>(p.t + size_t(8 * n + g) * p.max_rank + j0) : make_uint2(0u, 0u);
+#pragma unroll
+                for (int i = 0; i < TILES; ++i) {
+                    uint2 bv[2];
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const uint16_t* q = B + size_t(min(f0 + 16 * i + 8 * h + g, p.N - 1u)) * p.max_rank + j0;
+                        if (!in) bv[h] = make_uint2(0u, 0u);
+                        else if (b_vec) bv[h] = __ldg(reinterpret_cast<const uint2*>(q));
+                        else bv[h] = make_uint2(uint32_t(q[0]) | uint32_t(q[1]) << 16, uint32_t(q[2]) | uint32_t(q[3]) << 16);
+                    }
+#pragma unroll
+                    for (int n = 0; n < NT; ++n) mma_bf16_16816(acc[i][n], bv[0].x, bv[1].x, bv[0].y, bv[1].y, tv[n].x, tv[n].y);
+                }
+            }
+        }
+    }
+
+    // ---- the warps' partial sums, added in warp order ----
+#pragma unroll
+    for (int i = 0; i < TILES; ++i)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) part[warp][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[i][n][e];
+    __syncthreads();
+    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += DCM_THREADS) {
+        const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
+        if (m >= p.M || f >= p.N) continue;
+        float sum = part[0][m][fi];
+#pragma unroll
+        for (int k = 1; k < DCM_WARPS; ++k) sum += part[k][m][fi];
+        const uint16_t bits = f32_to_bf16_bits(sum * p.out_scale);
+        for (uint32_t r = 0; r < p.n_dest; ++r) p.y_dest[r][size_t(m) * p.out_row_stride + p.y_col0 + f] = bits;
+    }
+}
+
+}  // namespace atlas
