@@ -44,6 +44,20 @@ static size_t g_profile_words = 0;
 
 static inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? ATLAS_B200_OK : ATLAS_B200_ERR_CUDA_BASE - int(e); }
 static inline int launch_status() { return cuda_status(cudaGetLastError()); }
+// A launch of a kernel that begins with pdl_wait(): it may start while its predecessor in the stream finishes.
+template <typename... P, typename... A>
+static int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
 static inline bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // ---------------------------------------------------------------------------------------------
@@ -226,13 +240,15 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         cfg.blockDim = dim3(SHT_THREADS);
         cfg.dynamicSmemBytes = SHT_SMEM_BYTES;
         cfg.stream = st;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = p.ksplit;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         return cuda_status(cudaLaunchKernelEx(&cfg, lora_shrink_tc_kernel, map_x, map_a, p));
     }
     if (p.m_begin || p.m_count || p.n_tile_dest > 1) return ATLAS_B200_ERR_DIMS;      // a row range / several destinations: that kernel only
@@ -251,13 +267,15 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         cfg.gridDim = grid;
         cfg.blockDim = dim3(SHM_THREADS);
         cfg.stream = st;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributeClusterDimension;      // SHM_KSPLIT CTAs along x share one (slot, ranks, chunk)
         attr[0].val.clusterDim.x = ksplit;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         return cuda_status(cudaLaunchKernelEx(&cfg, lora_shrink_mma_kernel, p));
     }
     dim3 grid(n_slots, (p.max_rank + SHRINK_RT - 1) / SHRINK_RT, (p.M + SHRINK_TC - 1) / SHRINK_TC);
@@ -279,11 +297,10 @@ static int launch_expand(const ExpandParams& p, cudaStream_t st) {
         while (splits * 2 <= most && uint64_t(cols) * chunks * splits * 2 <= uint64_t(rt_sm_count()) * 8) splits *= 2;
         const dim3 grid(cols, chunks * splits);
         if (grid.y > 65535) return ATLAS_B200_ERR_LIMIT;
-        if (p.max_rank <= 16) lora_expand_mma_kernel<1><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
-        else if (p.max_rank <= 32) lora_expand_mma_kernel<2><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
-        else if (p.max_rank <= 64) lora_expand_mma_kernel<4><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
-        else lora_expand_mma_kernel<8><<<grid, EXM_THREADS, 0, st>>>(p, chunk, splits);
-        return launch_status();
+        if (p.max_rank <= 16) return launch_chained(lora_expand_mma_kernel<1>, grid, EXM_THREADS, st, p, chunk, splits);
+        if (p.max_rank <= 32) return launch_chained(lora_expand_mma_kernel<2>, grid, EXM_THREADS, st, p, chunk, splits);
+        if (p.max_rank <= 64) return launch_chained(lora_expand_mma_kernel<4>, grid, EXM_THREADS, st, p, chunk, splits);
+        return launch_chained(lora_expand_mma_kernel<8>, grid, EXM_THREADS, st, p, chunk, splits);
     }
     // rows per CTA: 32 for large batches (a CTA re-uses its B rows out of L1 while neighbouring rows share an adapter),
     // fewer while the grid would otherwise leave SMs without a CTA (a decode batch)
@@ -745,9 +762,23 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT>, w, p));
 }
 
+// Where it is the faster one, both sides measured at cold L2 (8 adapters of rank 16; us, this kernel / tcgen05):
+//   1 token    1024 x 4096 13/17   4096 x 4096 15/20   14336 x 4096 28/34   4096 x 14336 24/34   28672 x 8192 63/104
+//   8 tokens   1024 x 4096 15/20   4096 x 4096 20/22   14336 x 4096 32/36   4096 x 14336 40/34   28672 x 8192 77/106
+//   16 tokens  1024 x 4096 15/20   4096 x 4096 24/21   14336 x 4096 34/36   4096 x 14336 52/34   28672 x 8192 89/105
+//              8192 x 8192 42/36; without adapters 28/34, and the faster one at all of these
+// With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does.
+static bool decode_pays(const atlas_b200_linear_desc& d) {
+    if (d.m > uint32_t(DCM_MAX_TOKENS)) return false;
+    if (!d.seq_slot || uint64_t(d.n) >= 2ull * d.k) return true;
+    return d.m <= 8 && uint64_t(d.m) * d.k <= 8ull * 14000;
+}
+
 static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
-    // sixteen features per CTA instead of 32 while those would not give every other SM one
-    return d.n <= 32u * uint32_t(rt_sm_count()) / 2u ? launch_decode_as<1, 1>(d, shrink, st) : launch_decode_as<2, 1>(d, shrink, st);
+    // sixteen features per CTA instead of 32 where the two CTAs that fit on an SM then still cover them in one wave
+    const bool narrow = d.n <= 16u * 2u * uint32_t(rt_sm_count());
+    if (d.m <= 8) return narrow ? launch_decode_as<1, 1>(d, shrink, st) : launch_decode_as<2, 1>(d, shrink, st);
+    return narrow ? launch_decode_as<1, 2>(d, shrink, st) : launch_decode_as<2, 2>(d, shrink, st);
 }
 
 // ---- dense-BF16 base on the tensor cores (kernel_dense_tc.cuh) ----
@@ -782,13 +813,15 @@ static int launch_dense_tc_mt(const atlas_b200_linear_desc& d, int idx, uint32_t
     cfg.blockDim = dim3(tc::D_THREADS);
     cfg.dynamicSmemBytes = C::SMEM_BYTES;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = k_split;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = k_split;
     cfg.attrs = attr;
-    cfg.numAttrs = k_split > 1 ? 1 : 0;
+    cfg.numAttrs = k_split > 1 ? 2 : 1;
     return cuda_status(cudaLaunchKernelEx(&cfg, tc::dense_bf16_linear_tc_kernel<MT>, map_x, map_w, p));
 }
 
@@ -864,9 +897,8 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         if (!(d.flags & ATLAS_B200_FLAG_ACT_FP4_READY) && !shrink_only) {
         const size_t groups = size_t(d.m) * (d.k / 16);
         const unsigned blocks = unsigned(std::min<size_t>((groups + 255) / 256, size_t(rt_sm_count()) * 16));
-        quantize_nvfp4_kernel<<<blocks, 256, 0, st>>>(static_cast<const uint16_t*>(d.x), codes, codes + act_fp4_codes_bytes(d),
-                                                      1.0f, d.m, d.k, d.x_row_stride, 1u);
-        rc = launch_status();
+        rc = launch_chained(quantize_nvfp4_kernel, blocks, 256, st, static_cast<const uint16_t*>(d.x), codes, codes + act_fp4_codes_bytes(d),
+                            1.0f, d.m, d.k, d.x_row_stride, 1u);
         if (rc) return rc;
         }
     }
@@ -917,7 +949,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         // The smallest batches, unless a form of the tcgen05 path is asked for by a flag.
         constexpr uint32_t tc_forms = ATLAS_B200_FLAG_FORCE_TCGEN05 | ATLAS_B200_FLAG_ACT_FP4 | ATLAS_B200_FLAG_NO_CTA_PAIR |
                                       ATLAS_B200_FLAG_NO_K_SPLIT | ATLAS_B200_FLAG_NO_PERSISTENT | ATLAS_B200_FLAG_ONE_TILE_PASS;
-        if (d.m <= uint32_t(DCM_MAX_TOKENS) && !(d.flags & tc_forms) && !shrink_only) {
+        if (decode_pays(d) && !(d.flags & tc_forms) && !shrink_only) {
             // (t rows in lora_t are written by every call: the tiles a tcgen05 call leaves in `ws` are not what this kernel reads)
             rc = launch_decode(d, d.seq_slot ? &sp : nullptr, st);
             if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
@@ -1120,9 +1152,8 @@ int atlas_b200_quantize_bf16_to_nvfp4(const void* in_bf16, void* packed, void* s
     const size_t groups = size_t(n) * (k / 16);
     const unsigned blocks = unsigned(std::min<size_t>((groups + 255) / 256, size_t(rt_sm_count()) * 16));
     const uint32_t vec = aligned(in_bf16, 16) && aligned(packed, 8) && k % 16 == 0;
-    quantize_nvfp4_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    return launch_chained(quantize_nvfp4_kernel, blocks, 256, static_cast<cudaStream_t>(stream),
         static_cast<const uint16_t*>(in_bf16), static_cast<uint8_t*>(packed), static_cast<uint8_t*>(scales), scale2, n, k, k, vec);
-    return launch_status();
 }
 
 int atlas_b200_nvfp4_global_absmax(const void* in_bf16, float* global_max_dev, size_t total, void* stream) {
@@ -1198,10 +1229,9 @@ static int kv_norm_rope_cache_write(const void* k_in, const void* v_in, uint32_t
     const dim3 grid((tokens + KVE_TOKENS - 1) / KVE_TOKENS), block(KVE_WARPS * 32);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool exact = rotary_dim == 64 && fp8_inv_scale == 0.0f && (head_dim == 64 || head_dim == 128 || head_dim == 256);
-    if (head_dim <= 64) exact ? kv_norm_rope_cache_kernel<2, true><<<grid, block, 0, st>>>(p) : kv_norm_rope_cache_kernel<2, false><<<grid, block, 0, st>>>(p);
-    else if (head_dim <= 128) exact ? kv_norm_rope_cache_kernel<4, true><<<grid, block, 0, st>>>(p) : kv_norm_rope_cache_kernel<4, false><<<grid, block, 0, st>>>(p);
-    else exact ? kv_norm_rope_cache_kernel<8, true><<<grid, block, 0, st>>>(p) : kv_norm_rope_cache_kernel<8, false><<<grid, block, 0, st>>>(p);
-    return launch_status();
+    if (head_dim <= 64) return exact ? launch_chained(kv_norm_rope_cache_kernel<2, true>, grid, block, st, p) : launch_chained(kv_norm_rope_cache_kernel<2, false>, grid, block, st, p);
+    if (head_dim <= 128) return exact ? launch_chained(kv_norm_rope_cache_kernel<4, true>, grid, block, st, p) : launch_chained(kv_norm_rope_cache_kernel<4, false>, grid, block, st, p);
+    return exact ? launch_chained(kv_norm_rope_cache_kernel<8, true>, grid, block, st, p) : launch_chained(kv_norm_rope_cache_kernel<8, false>, grid, block, st, p);
 }
 
 int atlas_b200_kv_norm_rope_cache_write(const void* k_in, const void* v_in, uint32_t in_row_stride, const void* k_norm_weight,
@@ -1260,13 +1290,12 @@ int atlas_b200_qkv_norm_rope_cache_write(void* q, const void* k_in, const void* 
     p.rms_eps = rms_eps; p.attention_factor = attention_factor; p.norm_offset_one = norm_offset_one ? 1u : 0u;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const bool exact = rotary_dim == 64 && (head_dim == 64 || head_dim == 128 || head_dim == 256);
-    if (head_dim <= 64) exact ? qkv_norm_rope_cache_kernel<1, true><<<tokens, KVE_WARPS * 32, 0, st>>>(p)
-                              : qkv_norm_rope_cache_kernel<1, false><<<tokens, KVE_WARPS * 32, 0, st>>>(p);
-    else if (head_dim <= 128) exact ? qkv_norm_rope_cache_kernel<2, true><<<tokens, KVE_WARPS * 32, 0, st>>>(p)
-                                    : qkv_norm_rope_cache_kernel<2, false><<<tokens, KVE_WARPS * 32, 0, st>>>(p);
-    else exact ? qkv_norm_rope_cache_kernel<4, true><<<tokens, KVE_WARPS * 32, 0, st>>>(p)
-               : qkv_norm_rope_cache_kernel<4, false><<<tokens, KVE_WARPS * 32, 0, st>>>(p);
-    return launch_status();
+    if (head_dim <= 64) return exact ? launch_chained(qkv_norm_rope_cache_kernel<1, true>, tokens, KVE_WARPS * 32, st, p)
+                              : launch_chained(qkv_norm_rope_cache_kernel<1, false>, tokens, KVE_WARPS * 32, st, p);
+    if (head_dim <= 128) return exact ? launch_chained(qkv_norm_rope_cache_kernel<2, true>, tokens, KVE_WARPS * 32, st, p)
+                                    : launch_chained(qkv_norm_rope_cache_kernel<2, false>, tokens, KVE_WARPS * 32, st, p);
+    return exact ? launch_chained(qkv_norm_rope_cache_kernel<4, true>, tokens, KVE_WARPS * 32, st, p)
+               : launch_chained(qkv_norm_rope_cache_kernel<4, false>, tokens, KVE_WARPS * 32, st, p);
 }
 
 int atlas_b200_copy_columns(const void* src, uint32_t src_row_stride, void* const* dest, uint32_t n_dest, uint32_t dst_row_stride,
@@ -1293,10 +1322,9 @@ int atlas_b200_silu_mul(const void* gate_bf16, const void* up_bf16, void* out_bf
         return ATLAS_B200_ERR_ALIGN;
     const size_t vecs = size_t(m) * (k / 8);
     const unsigned blocks = unsigned(std::min<size_t>((vecs + 255) / 256, size_t(rt_sm_count()) * 16));
-    silu_mul_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    return launch_chained(silu_mul_kernel, blocks, 256, static_cast<cudaStream_t>(stream), 
         static_cast<const uint16_t*>(gate_bf16), static_cast<const uint16_t*>(up_bf16), static_cast<uint16_t*>(out_bf16), gate_scale,
         up_scale, swiglu_limit, m, k, in_row_stride, out_row_stride);
-    return launch_status();
 }
 
 int atlas_b200_silu_mul_quant_nvfp4(const void* gate_bf16, const void* up_bf16, void* ws, size_t ws_bytes, float gate_scale, float up_scale,
@@ -1310,10 +1338,9 @@ int atlas_b200_silu_mul_quant_nvfp4(const void* gate_bf16, const void* up_bf16, 
     const size_t groups = size_t(m) * (k / 16);
     const unsigned blocks = unsigned(std::min<size_t>((groups + 255) / 256, size_t(rt_sm_count()) * 16));
     uint8_t* codes = static_cast<uint8_t*>(ws);
-    silu_mul_quant_nvfp4_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    return launch_chained(silu_mul_quant_nvfp4_kernel, blocks, 256, static_cast<cudaStream_t>(stream), 
         static_cast<const uint16_t*>(gate_bf16), static_cast<const uint16_t*>(up_bf16), codes, codes + codes_bytes, gate_scale, up_scale,
         swiglu_limit, m, k, in_row_stride);
-    return launch_status();
 }
 
 int atlas_b200_nvfp4_lora_linear(const atlas_b200_linear_desc* desc, void* stream) {

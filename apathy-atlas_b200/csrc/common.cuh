@@ -26,6 +26,19 @@ __device__ uint32_t g_status_word = 0;
 
 __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_status_word, 0u, code); }
 
+// ---- programmatic dependent launch ------------------------------------------------------------
+// A decode step is a chain of short kernels, and between two of them an ordinary launch leaves the machine idle for a few
+// microseconds.  Kernels of this library therefore (a) let the next launch start as soon as all their own CTAs run, and (b) when
+// launched that way, begin by waiting until everything before them in the stream has completed and is visible.  Only the main
+// kernel of a linear call reads anything ahead of that wait, and it follows a shrink that has waited before releasing it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// The pointer as a value that does not exist before this point: keeps read-only loads through it behind pdl_wait().
+template <typename T> __device__ __forceinline__ T* pdl_after(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
+
 // ---- BF16 <-> FP32 ---------------------------------------------------------------------------
 __device__ __forceinline__ float bf16_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w & 0xFFFF0000u); }

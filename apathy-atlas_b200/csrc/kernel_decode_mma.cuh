@@ -27,7 +27,7 @@ namespace atlas {
 
 constexpr int DCM_WARPS = 8, DCM_THREADS = 32 * DCM_WARPS;
 constexpr int DCM_KSTEP = 128;
-constexpr int DCM_MAX_TOKENS = 8;
+constexpr int DCM_MAX_TOKENS = 16;
 
 struct DecodeParams {
     const uint16_t* x;
@@ -50,8 +50,11 @@ __global__ void __launch_bounds__(DCM_THREADS, 2)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     __shared__ float part[DCM_WARPS][NT * 8][TILES * 16 + 1];          // [warp][token][feature]
     __shared__ int32_t slot_s[DCM_MAX_TOKENS];
+    __shared__ uint32_t rank_s[DCM_MAX_TOKENS];                        // of the slot in slot_s: its rank
+    __shared__ uint64_t b_s[DCM_MAX_TOKENS];                           // and its B (read once, not granule by granule behind the shrink)
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t f0 = blockIdx.x * (TILES * 16);
+    pdl_release();
 
     if (tid < DCM_MAX_TOKENS) {
         int32_t s = -1;
@@ -59,7 +62,11 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             s = p.seq_slot[tid];
             if (s >= 0) {
                 if (uint32_t(s) >= p.max_loras) { record_status(STATUS_SLOT_OUT_OF_RANGE); s = -1; }
-                else if (p.a_table[s] == 0ull || p.b_table[s] == 0ull) s = -1;
+                else {
+                    b_s[tid] = p.b_table[s];
+                    rank_s[tid] = p.rank_table ? min(p.rank_table[s], p.max_rank) : p.max_rank;
+                    if (p.a_table[s] == 0ull || b_s[tid] == 0ull) s = -1;
+                }
             }
         }
         slot_s[tid] = s;
@@ -82,9 +89,12 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     for (int n = 0; n < NT; ++n) x_row[n] = w.x + size_t(min(8 * n + g, p.M - 1u)) * w.x_row_stride + 32 * t;
 
     float acc[TILES][NT][4] = {};
+    // (one n-tile: x travels with the codes; more of them would not fit in registers and are read where they are used)
+    constexpr bool X_AHEAD = NT == 1;
+    uint4 xv[2][X_AHEAD ? 4 : 1];
     uint4 code[2][TILES][2];
     uint32_t sc[2][TILES][2];
-    auto load = [&](uint32_t step, uint4 (&c)[TILES][2], uint32_t (&s)[TILES][2]) {
+    auto load = [&](uint32_t step, uint4 (&c)[TILES][2], uint32_t (&s)[TILES][2], uint4 (&xs)[X_AHEAD ? 4 : 1]) {
         const bool in = step * DCM_KSTEP + 32 * t < p.K;                        // (K is a multiple of 32)
 #pragma unroll
         for (int i = 0; i < TILES; ++i)
@@ -93,15 +103,21 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
                 c[i][h] = in ? __ldcs(reinterpret_cast<const uint4*>(code_row[i][h] + step * (DCM_KSTEP / 2))) : make_uint4(0u, 0u, 0u, 0u);
                 s[i][h] = in ? uint32_t(__ldg(reinterpret_cast<const uint16_t*>(scale_row[i][h] + step * (DCM_KSTEP / 16)))) : 0u;
             }
+        if constexpr (X_AHEAD)
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                xs[u] = in && g < p.M ? __ldg(reinterpret_cast<const uint4*>(x_row[0] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
     };
-    auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2]) {
+    auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2], const uint4 (&xs)[X_AHEAD ? 4 : 1]) {
         const bool in = step * DCM_KSTEP + 32 * t < p.K;
 #pragma unroll
         for (int u = 0; u < 4; ++u) {                                           // eight K elements per thread at a time
             uint32_t xb[NT][4];
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                const uint4 v = in && 8 * n + g < p.M ? __ldg(reinterpret_cast<const uint4*>(x_row[n] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
+                uint4 v;
+                if constexpr (X_AHEAD) v = xs[u];
+                else v = in && 8 * n + g < p.M ? __ldg(reinterpret_cast<const uint4*>(x_row[n] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
                 xb[n][0] = __byte_perm(v.x, v.z, 0x5410); xb[n][1] = __byte_perm(v.x, v.z, 0x7632);
                 xb[n][2] = __byte_perm(v.y, v.w, 0x5410); xb[n][3] = __byte_perm(v.y, v.w, 0x7632);
             }
@@ -121,27 +137,34 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             }
         }
     };
-    load(warp, code[0], sc[0]);
+    load(warp, code[0], sc[0], xv[0]);
     for (uint32_t step = warp; step < n_steps; step += 2 * DCM_WARPS) {
-        load(step + DCM_WARPS, code[1], sc[1]);
-        multiply(step, code[0], sc[0]);
-        load(step + 2 * DCM_WARPS, code[0], sc[0]);
-        if (step + DCM_WARPS < n_steps) multiply(step + DCM_WARPS, code[1], sc[1]);
+        load(step + DCM_WARPS, code[1], sc[1], xv[1]);
+        multiply(step, code[0], sc[0], xv[0]);
+        load(step + 2 * DCM_WARPS, code[0], sc[0], xv[0]);
+        if (step + DCM_WARPS < n_steps) multiply(step + DCM_WARPS, code[1], sc[1], xv[1]);
     }
 
     // ---- LoRA granules of this warp ----
     if (p.seq_slot) {
-        __syncthreads();                                                        // slot_s
-        if (p.wait_for_shrink) asm volatile("griddepcontrol.wait;" ::: "memory");
+        __syncthreads();                                                        // slot_s, rank_s, b_s
+        // this CTA's rows of B into L2 while the shrink may still run
+        for (uint32_t m = warp; m < p.M; m += DCM_WARPS) {
+            if (slot_s[m] < 0 || lane >= TILES * 16u || f0 + lane >= p.N) continue;
+            const uint16_t* B = reinterpret_cast<const uint16_t*>(b_s[m]) + size_t(f0 + lane) * p.max_rank;
+            for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(B + j));
+        }
+        if (p.wait_for_shrink) pdl_wait();
         int32_t own[NT];
 #pragma unroll
         for (int n = 0; n < NT; ++n) own[n] = slot_s[8 * n + g];
         const int32_t lane_slot = lane < DCM_MAX_TOKENS ? slot_s[lane] : -1;
         for (uint32_t left = __ballot_sync(0xFFFFFFFFu, lane_slot >= 0); left;) {
-            const int32_t s = __shfl_sync(0xFFFFFFFFu, lane_slot, __ffs(left) - 1);
+            const uint32_t first = __ffs(left) - 1;                             // first token of this slot
+            const int32_t s = __shfl_sync(0xFFFFFFFFu, lane_slot, first);
             left &= ~__ballot_sync(0xFFFFFFFFu, lane_slot == s);
-            const uint32_t rank = p.rank_table ? min(p.rank_table[s], p.max_rank) : p.max_rank;
-            const uint16_t* B = reinterpret_cast<const uint16_t*>(p.b_table[s]);
+            const uint32_t rank = rank_s[first];
+            const uint16_t* B = reinterpret_cast<const uint16_t*>(b_s[first]);
             const bool b_vec = (reinterpret_cast<uintptr_t>(B) & 7u) == 0u;
             for (uint32_t j = 0; 16 * j < rank; ++j) {
                 if ((uint32_t(s) + 3u * j) % DCM_WARPS != warp) continue;

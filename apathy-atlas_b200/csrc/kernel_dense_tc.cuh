@@ -70,6 +70,8 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     tcgen05_fence_before();
     __syncthreads();
     tcgen05_fence_after();
+    pdl_release();
+    pdl_wait();                                          // (x and w come by TMA, issued below)
     const uint32_t tmem_acc = misc[0];
     bool acc_ready = false;
 

@@ -29,13 +29,16 @@ constexpr int EXM_MAX_RANK = 128;    // B_s fragments of 32 features are held in
 // KS: 16-wide K steps held in registers, >= ceil(max_rank / 16)
 template <int KS>
 __global__ void __launch_bounds__(EXM_THREADS, KS >= 8 ? 3 : (KS >= 4 ? 4 : 6))
-lora_expand_mma_kernel(const ExpandParams p, uint32_t chunk, uint32_t splits) {
+lora_expand_mma_kernel(ExpandParams p, uint32_t chunk, uint32_t splits) {
     __shared__ __align__(16) uint32_t slot_in[EXM_ROWS];     // slot, ~0 for a row without a term
     __shared__ int32_t slot_s[EXM_ROWS];
     __shared__ uint64_t b_s[EXM_ROWS];
     __shared__ float scale_s[EXM_ROWS];
     __shared__ uint16_t row_s[EXM_ROWS];
     __shared__ uint32_t n_s;
+    pdl_release();
+    pdl_wait();
+    p.b_uniform = pdl_after(p.b_uniform); p.b_table = pdl_after(p.b_table); p.scale_table = pdl_after(p.scale_table); p.xa = pdl_after(p.xa);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t m0 = (blockIdx.y / splits) * chunk, split = blockIdx.y % splits;
     const uint32_t n_in = min(chunk, p.M - m0);

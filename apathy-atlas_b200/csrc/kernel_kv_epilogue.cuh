@@ -103,6 +103,9 @@ template <uint32_t NG, bool EXACT>
 __global__ void __launch_bounds__(KVE_WARPS * 32)
 kv_norm_rope_cache_kernel(KvEpilogueParams p) {
     static_assert(KVE_TOKENS == KVE_WARPS, "one warp per token of the CTA");
+    pdl_release();
+    pdl_wait();
+    p.k_in = pdl_after(p.k_in); p.v_in = pdl_after(p.v_in); p.positions = pdl_after(p.positions); p.slot_mapping = pdl_after(p.slot_mapping);
     if constexpr (EXACT) { p.head_dim = 32u * NG; p.rotary_dim = 64u; p.fp8_inv_scale = 0.0f; }
     // One CTA per KVE_TOKENS tokens.  The rotation's frequency depends on the pair only and its cosine and sine on
     // (token, pair) only, so the FP64 power is evaluated once per CTA and pair, the two transcendental calls once per
@@ -247,6 +250,10 @@ struct QkvEpilogueParams {
 template <uint32_t MAX_GRP, bool EXACT>
 __global__ void __launch_bounds__(KVE_WARPS * 32, MAX_GRP == 4 ? 4 : 6)     // (occupancy matters more here than a few held values)
 qkv_norm_rope_cache_kernel(QkvEpilogueParams p) {
+    pdl_release();
+    pdl_wait();
+    p.q = pdl_after(p.q); p.k_in = pdl_after(p.k_in); p.v_in = pdl_after(p.v_in); p.positions = pdl_after(p.positions);
+    p.slot_mapping = pdl_after(p.slot_mapping);
     if constexpr (EXACT) { p.head_dim = 64u * MAX_GRP; p.rotary_dim = 64u; }
     // one CTA per token; cosine and sine of the token's angles evaluated once for all its heads (see above)
     __shared__ uint16_t normed_s[EXACT ? 1 : KVE_WARPS][EXACT ? 2 : KVE_MAX_HEAD_DIM];

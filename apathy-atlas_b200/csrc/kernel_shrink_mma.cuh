@@ -46,11 +46,14 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 }
 
 __global__ void __launch_bounds__(SHM_THREADS, 8)
-lora_shrink_mma_kernel(const ShrinkParams p) {
+lora_shrink_mma_kernel(ShrinkParams p) {
     __shared__ uint16_t rows[SHM_CHUNK];
     __shared__ float part[SHM_TOKENS][SHM_RANKS];          // this CTA's tile, read by the cluster's first CTA
 
-    if (p.release_dependents) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (in this order: the kernel released here reads x and the weights without a wait of its own)
+    pdl_wait();
+    if (p.release_dependents) pdl_release();
+    p.x = pdl_after(p.x); p.a_uniform = pdl_after(p.a_uniform); p.a_table = pdl_after(p.a_table);
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t krank = cluster.block_rank();            // this CTA's share of K
     const uint32_t ksplit = p.ksplit;                       // = the cluster's size
@@ -63,29 +66,37 @@ lora_shrink_mma_kernel(const ShrinkParams p) {
     const uint16_t* A;
     float f = 1.0f;
     uint32_t rank = p.max_rank;
+    bool hit[2];
     if (p.seq_slot) {
-        const uint64_t a_addr = p.a_table[s];
-        if (a_addr == 0ull) return;
-        if (p.b_table && p.b_table[s] == 0ull) return;
+        // everything the routing decides on is requested before the first of it is looked at: one memory latency, not five
+        int32_t routed[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t m = m_base + h * SHM_THREADS + tid;
+            routed[h] = (h * SHM_THREADS + tid < chunk && m < p.M) ? p.seq_slot[m] : -1;
+        }
+        const uint64_t a_addr = p.a_table[s], b_addr = p.b_table ? p.b_table[s] : 1ull;
+        const uint32_t own_rank = p.rank_table ? p.rank_table[s] : p.max_rank;
+        const float scale = p.post != 0.0f ? p.scale_table[s] : 1.0f;
+        if (a_addr == 0ull || b_addr == 0ull) return;
         A = reinterpret_cast<const uint16_t*>(a_addr);
-        if (p.rank_table) rank = min(p.rank_table[s], p.max_rank);
+        rank = min(own_rank, p.max_rank);
         if (p.tile_out && j0 >= rank) return;               // no such granule in any tile's list (whole cluster leaves)
-        if (p.post != 0.0f) f = p.scale_table[s] * p.post;
+        if (p.post != 0.0f) f = scale * p.post;
+        hit[0] = routed[0] == int32_t(s);
+        hit[1] = routed[1] == int32_t(s);
     } else {
         A = p.a_uniform;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) hit[h] = h * SHM_THREADS + tid < chunk && m_base + h * SHM_THREADS + tid < p.M;
     }
 
     // ---- ordered list of this chunk's rows routed to slot s (two candidates per thread) ----
     uint32_t n_rows;
-    bool hit[2];
     {
         uint32_t ballot[2];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t m = m_base + h * SHM_THREADS + tid;
-            hit[h] = (h * SHM_THREADS + tid < chunk) && (m < p.M) && (p.seq_slot ? (p.seq_slot[m] == int32_t(s)) : true);
-            ballot[h] = __ballot_sync(0xFFFFFFFFu, hit[h]);
-        }
+        for (int h = 0; h < 2; ++h) ballot[h] = __ballot_sync(0xFFFFFFFFu, hit[h]);
         __shared__ uint32_t cnt[2][SHM_THREADS / 32];
         if (lane == 0) { cnt[0][warp] = __popc(ballot[0]); cnt[1][warp] = __popc(ballot[1]); }
         __syncthreads();
@@ -188,6 +199,28 @@ lora_shrink_mma_kernel(const ShrinkParams p) {
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) ar[nt] = A + size_t(min(j0 + nt * 8 + g, p.max_rank - 1)) * p.k_in + 8 * t;
 
+            if (n_rows - r0 <= 8) {
+                // at most eight rows (a slot of a decode batch): rows 8 to 31 of the pass are neither read nor multiplied, and
+                // the registers hold four chunks in flight instead of two
+#pragma unroll 4
+                for (uint32_t c = krank + ksplit * warp; c < n_chunks; c += ksplit * (SHM_THREADS / 32)) {
+                    const uint4 xv = *reinterpret_cast<const uint4*>(xr[0][0] + c * 32);
+                    uint4 av[2];
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) {
+                        if (a_aligned) av[nt] = __ldg(reinterpret_cast<const uint4*>(ar[nt] + c * 32));
+                        else {
+                            const uint32_t* q = reinterpret_cast<const uint32_t*>(ar[nt] + c * 32);   // 4-byte aligned at least
+                            av[nt] = make_uint4(__ldg(q), __ldg(q + 1), __ldg(q + 2), __ldg(q + 3));
+                        }
+                    }
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) {
+                        mma_bf16_16816(acc[0][nt], xv.x, 0u, xv.y, 0u, av[nt].x, av[nt].y);
+                        mma_bf16_16816(acc[0][nt], xv.z, 0u, xv.w, 0u, av[nt].z, av[nt].w);
+                    }
+                }
+            } else
 #pragma unroll 2
             for (uint32_t c = krank + ksplit * warp; c < n_chunks; c += ksplit * (SHM_THREADS / 32)) {
                 uint4 xv[2][2], av[2];

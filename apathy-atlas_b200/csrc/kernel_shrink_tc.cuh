@@ -70,6 +70,7 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
     __shared__ uint64_t bars[2 * SHT_MAX_STAGES + 1];
     __shared__ uint32_t tmem_base_s, abort_s;
 
+    pdl_wait();
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t ksn = p.ksplit ? p.ksplit : 1u;       // CTAs per cluster (consecutive blockIdx.x)
     const uint32_t kz = ksn > 1u ? tc::cluster_cta_rank() : 0u;

@@ -777,6 +777,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     auto arrive_at_leader = [&](uint32_t bar_at_leader) {
         if constexpr (PAIR) mbar_arrive_cluster(bar_at_leader); else mbar_arrive(bar_at_leader);
     };
+    pdl_release();
     const uint32_t tmem_acc = misc[0];
     const uint32_t tmem_a0 = tmem_acc + C::TMEM_A_BASE;   // A16: weight-operand stages [tmem_a0 + s * A_COLS, + A_COLS);
                                                           // A4: scale-factor stages [tmem_a0 + s * SF_COLS, + SF_COLS)

@@ -202,6 +202,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     __syncwarp();
     cluster_sync_all();
     tcgen05_fence_after();
+    pdl_release();
     const uint32_t full_at_leader = map_to_cta(BAR_FULL, 0);
     const uint32_t lfull_at_leader = map_to_cta(BAR_LFULL, 0);
     const uint32_t acc_empty_at_leader = map_to_cta(BAR_ACC_EMPTY, 0);

@@ -57,6 +57,9 @@ __device__ __forceinline__ size_t row_of(size_t i, size_t per_row, size_t total)
 __global__ void __launch_bounds__(256)
 silu_mul_kernel(const uint16_t* __restrict__ gate, const uint16_t* __restrict__ up, uint16_t* __restrict__ out, float gate_scale,
                 float up_scale, float limit, uint32_t M, uint32_t K, uint32_t in_stride, uint32_t out_stride) {
+    pdl_release();
+    pdl_wait();
+    gate = pdl_after(gate); up = pdl_after(up);
     const size_t per_row = K / 8, total = size_t(M) * per_row;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
         const size_t row = row_of(i, per_row, total), c = (i - row * per_row) * 8;
@@ -77,6 +80,9 @@ __global__ void __launch_bounds__(256)
 silu_mul_quant_nvfp4_kernel(const uint16_t* __restrict__ gate, const uint16_t* __restrict__ up, uint8_t* __restrict__ packed,
                             uint8_t* __restrict__ scales, float gate_scale, float up_scale, float limit, uint32_t M, uint32_t K,
                             uint32_t in_stride) {
+    pdl_release();
+    pdl_wait();
+    gate = pdl_after(gate); up = pdl_after(up);
     const size_t groups = K / 16, total = size_t(M) * groups;
     for (size_t gi = size_t(blockIdx.x) * blockDim.x + threadIdx.x; gi < total; gi += size_t(gridDim.x) * blockDim.x) {
         const size_t row = row_of(gi, groups, total), c = (gi - row * groups) * 16;

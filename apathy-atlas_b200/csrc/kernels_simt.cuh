@@ -119,6 +119,9 @@ __global__ void __launch_bounds__(256)
 quantize_nvfp4_kernel(const uint16_t* __restrict__ in, uint8_t* __restrict__ packed,
                       uint8_t* __restrict__ scales, float scale2, uint32_t N, uint32_t K, uint32_t in_row_stride,
                       uint32_t vec) {
+    pdl_release();
+    pdl_wait();
+    in = pdl_after(in);
     const uint32_t groups = K / 16;
     const size_t total = size_t(N) * groups;
     const float inv_scale2 = scale2 > 0.0f ? __fdiv_rn(1.0f, scale2) : 0.0f;

@@ -117,6 +117,38 @@ def test_shapes_beyond_the_forced_path(cuda, atlas, oracle, M, K, N, ranks, max_
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,ranks,max_rank", [
+    (1, 256, 16, [8], 8),                                # two K steps for eight warps, one feature tile
+    (5, 288, 40, [16, 8], 16),                           # K step of one thread's 32 codes, features past a tile
+    (8, 1056, 5000, [24, 128, 64], 128),                 # 32 features per CTA, granule and a half
+    (9, 512, 1040, [16] * 9, 16),                        # second n-tile with one token
+    (16, 2304, 5008, [8, 64], 64),                       # full second n-tile, an odd number of K steps per warp
+])
+def test_small_batches(cuda, atlas, oracle, M, K, N, ranks, max_rank):
+    """The form for up to sixteen tokens: against the oracle, with and without adapters, and a token's bits do not depend on
+    the tokens beside it."""
+    from atlas_b200 import synth
+    case = synth.make_case("small", M=M, K=K, N=N, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 1, none_frac=0.2 if M > 1 else 0.0,
+                           scale2=0.02, b_std=0.1, seed=M + K)
+    dc = DeviceCase(cuda, atlas, case, x_row_stride=K + 8, out_row_stride=N + 3)
+    y, variant = dc.run()
+    assert variant == atlas.VARIANT_TCGEN05
+    assert_close(oracle, y[:, :N], ideal(oracle, case), "fused")
+    assert (y[:, N:] == 0x7FC0).all()
+    y_tab, _ = dc.run(strided=False)
+    assert np.array_equal(y_tab, y)
+    yb, _ = dc.run(lora=False)
+    assert_close(oracle, yb[:, :N], ideal(oracle, case, lora=False), "base")
+    none = case.seq_slot < 0
+    assert np.array_equal(y[none], yb[none])             # (N >= 2 K where there are more than eight: both calls take this form)
+    import copy
+    c2 = copy.copy(case)
+    c2.x, c2.seq_slot = case.x[::-1].copy(), case.seq_slot[::-1].copy()
+    y2, _ = DeviceCase(cuda, atlas, c2, x_row_stride=K + 8, out_row_stride=N + 3).run()
+    assert np.array_equal(y2, y[::-1])
+    assert atlas.device_status() == 0
+
+
 def test_token_permutation_is_bit_exact(cuda, atlas, oracle):
     from atlas_b200 import synth
     import copy
