@@ -380,6 +380,8 @@ lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_co
                     w[u] = pack_bf16x2(a, b);
                 }
                 if (p.tile_out) {
+                    // (the CTA's rows may lie in two token tiles: an adapter of the other one has no block in this row's tile)
+                    if (!((present_t[tl][sl >> 5] >> (sl & 31u)) & 1u)) continue;
                     const uint32_t q = uint32_t(cq0[tl][ci]) + j0 / 16;
                     if (q >= p.tile_cap) { record_status(STATUS_TILE_CAPACITY); continue; }
                     store_block_row(row_at + q * q_step, swap, make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]));

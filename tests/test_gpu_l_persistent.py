@@ -108,3 +108,23 @@ def test_placement_into_several_buffers(cuda, atlas, oracle, fp4):
         assert np.array_equal(got[:, :N], want)
         assert (got[:, N:] == 0x7FC0).all()
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("low_first", [False, True])
+def test_adapters_that_change_inside_a_shrink_clusters_rows(cuda, atlas, oracle, low_first):
+    """128 rows of the shrink cross a border of the 192-token tiles (row 576) at which the adapter changes as well: an adapter
+    of the next tile has no block in this one, and its zero rows must not land in another adapter's."""
+    from atlas_b200 import synth
+    M, N, K = 1152, 9472, 512
+    # t is rounded to BF16: |t_j| about 1.2, so a sum over 48 ranks is off by about sqrt(48) 1.2 b_std 2^-9 / sqrt(3), that is 0.001
+    # at b_std 0.1 (0.003 at 0.3, where one of 50,000 values passes the absolute tolerance of 0.01); a lost term is 0.5
+    case = synth.make_case("border", M=M, K=K, N=N, ranks=[16, 48, 16], max_rank=48, max_loras=3, scale2=0.02, b_std=0.1, seed=9)
+    before, after = (0, 2) if low_first else (2, 0)
+    case.seq_slot = np.where(np.arange(M) < 576, before, after).astype(np.int32)
+    case.seq_slot[700:] = 1
+    y, _ = DeviceCase(cuda, atlas, case).run(lora_ws=True)
+    shape = atlas.last_launch_shape()
+    assert shape["token_tile"] == 192 and shape["lora_tiles_from_shrink"]
+    rows, cols = np.arange(500, 720, dtype=np.uint32), np.arange(0, N, 37, dtype=np.uint32)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "rows around the border")
+    assert atlas.device_status() == 0
