@@ -447,8 +447,8 @@ lora_expand_fold_kernel(const ExpandParams p) {
 // =============================================================================================
 // Shape-agnostic tiled linear on CUDA cores:  y[m,f] = bf16(scale2 * sum_k x[m,k] * w[f,k]),
 // w decoded to FP32 exactly (E2M1 * E4M3), FP32 accumulation.  64 x 64 output tile, K step 32,
-// 256 threads with 4 x 4 outputs each.  Serves shapes the tcgen05 path rejects (K not a
-// multiple of 256, unaligned strides) and the dense-BF16 base.
+// 256 threads with 4 x 4 outputs each.  Serves shapes the tensor-core paths reject
+// (K not a multiple of 32, or of eight with a dense base; ranks above 128; unaligned strides).
 // =============================================================================================
 constexpr int SIMT_TM = 64, SIMT_TF = 64, SIMT_TK = 32;
 
