@@ -230,9 +230,12 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         if (p.m_begin % 64 != 0 || p.m_begin >= p.M) return ATLAS_B200_ERR_DIMS;
         if (p.tile_out && p.chunk && p.chunk < uint32_t(SHT_ROWS)) return ATLAS_B200_ERR_DIMS;   // a cluster's rows lie in at most two token tiles
         const uint32_t rows = p.m_count ? std::min(p.m_count, p.M - p.m_begin) : p.M - p.m_begin;
-        // two CTAs per 128 rows, each contracting half of K: fixed by K alone, so that a row's result does not depend on
-        // how the batch is cut into launches
-        p.ksplit = (p.k_in / SHT_KSTAGE >= 2) ? 2u : 1u;
+        // CTAs per 128 rows, each contracting a share of K: two, or four where the batch (the whole of it, not this launch's
+        // range: a row's result must not depend on how the batch is cut into launches) leaves room for them in one wave.  The
+        // K loop is a serial chain of two thirds of the launch: 1237 tokens, eight adapters, K = 4096 38 -> 30 us, K = 14336
+        // 91 -> 58 us; 2048 tokens of one adapter 23 -> 17 us.
+        const uint32_t k_blocks = p.k_in / SHT_KSTAGE, row_groups = (p.M + SHT_ROWS - 1) / SHT_ROWS;
+        p.ksplit = k_blocks >= 8 && row_groups * SHT_MAX_KSPLIT <= uint32_t(rt_sm_count()) ? uint32_t(SHT_MAX_KSPLIT) : (k_blocks >= 2 ? 2u : 1u);
         const uint32_t n_ctas = p.ksplit * ((rows + SHT_ROWS - 1) / SHT_ROWS);
         p.profile = (g_profile_buf && size_t(n_ctas) * 16 <= g_profile_words) ? g_profile_buf : nullptr;
         cudaLaunchConfig_t cfg = {};
