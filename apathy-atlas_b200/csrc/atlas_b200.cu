@@ -868,6 +868,114 @@ struct ShrinkOnly {
     void* const* ws_dest;
 };
 
+// The launch shape of a call on the tensor-core path: a function of the descriptor's sizes and addresses and of `flags`
+// (d.flags, or those of another call that shares its scratch).
+struct TcPlan {
+    bool decode = false;           // kernel_decode_mma.cuh; of the rest only `tt` (none) is meant
+    uint32_t mt = 16, k_split = 1; // token tile; CTAs sharing one tile's contraction
+    bool pair = false, persistent = false, two_tiles = false;
+    uint32_t mt_tiles = 16;        // token tile of the shrink's masked-t blocks
+    TTiles tt;
+};
+
+// flags that pick a form of the tcgen05 kernels (the smallest batches then run on them too)
+constexpr uint32_t kTcForms = ATLAS_B200_FLAG_FORCE_TCGEN05 | ATLAS_B200_FLAG_NO_CTA_PAIR | ATLAS_B200_FLAG_NO_K_SPLIT |
+                              ATLAS_B200_FLAG_NO_PERSISTENT | ATLAS_B200_FLAG_ONE_TILE_PASS;
+
+// `shrink_tiles`: the shrink of this call can write masked-t tiles
+static TcPlan plan_tc(const atlas_b200_linear_desc& d, uint32_t flags, bool shrink_tiles) {
+    TcPlan p;
+    const bool act_fp4 = (flags & ATLAS_B200_FLAG_ACT_FP4) != 0;
+    if (decode_pays(d) && !(flags & (kTcForms | ATLAS_B200_FLAG_ACT_FP4))) {
+        p.decode = true;
+        return p;
+    }
+    // Token tile: the smallest power of two that covers m, at most 256 — then halved (down to 64)
+    // while the grid would leave more than a quarter of the SMs without a CTA, e.g. for a
+    // column shard of a wide layer: more, lighter CTAs finish sooner than few heavy ones.
+    p.mt = 16;
+    while (p.mt < 256 && p.mt < d.m) p.mt <<= 1;
+    const uint32_t f_tiles = (d.n + tc::FT - 1) / tc::FT;
+    // Fewer tiles than half the SMs (a decode batch, a column shard): several CTAs share a tile, each
+    // contracting a share of K, rather than leaving SMs idle — a CTA's time is set by the weights it has
+    // to expand, which only a K split divides.  Clusters of at most 8 CTAs; whole 256-element stages.
+    p.k_split = 1;
+    p.pair = p.mt >= 128 && !(flags & ATLAS_B200_FLAG_NO_CTA_PAIR);    // pairs of CTAs issue their MMAs together (see tc::Cfg)
+    if (!(flags & ATLAS_B200_FLAG_NO_K_SPLIT)) {
+        const uint32_t m_tiles = (d.m + p.mt - 1) / p.mt;
+        const uint32_t fit = uint32_t(rt_sm_count()) / (f_tiles * m_tiles);
+        p.k_split = std::max(1u, std::min(std::min(fit, 8u), d.k / uint32_t(tc::KRAW)));
+        // ... but only as many as still lets every cluster be resident at once (a second wave would cost more than the
+        // split saves), preferring the shape with pairs, then the one without, then a smaller split
+        const bool may_pair = p.pair;
+        for (; p.k_split > 1; --p.k_split) {
+            if (may_pair && p.k_split <= 4 &&
+                tc_active_clusters_of(p.mt, act_fp4, true, p.k_split) >= int(((f_tiles + 1) / 2) * m_tiles)) { p.pair = true; break; }
+            if (tc_active_clusters_of(p.mt, act_fp4, false, p.k_split) >= int(f_tiles * m_tiles)) { p.pair = false; break; }
+        }
+        if (p.k_split == 1) p.pair = may_pair;
+    }
+    if (p.k_split == 1) {
+        while (p.mt > 64 && f_tiles * ((d.m + p.mt - 1) / p.mt) * 4 < uint32_t(rt_sm_count()) * 3) p.mt >>= 1;
+        p.pair = p.mt >= 128 && !(flags & ATLAS_B200_FLAG_NO_CTA_PAIR);
+    }
+
+    // Masked-t tiles: with scratch to put them in, the shrink writes the activation operand of every LoRA
+    // K-step once, in the layout the MMA reads, and the fused kernel's CTAs fetch it by TMA — instead of
+    // each CTA rebuilding the same tiles from lora_t.  Needs the strided pool (the TMA producer then feeds
+    // both LoRA operands) and the tensor-core shrink; otherwise the in-kernel build stays in use.
+    auto tiles_in_ws = [&](uint32_t tile, uint32_t part_rows) {
+        TTiles t;
+        if (!d.seq_slot || !d.ws || !shrink_tiles) return t;
+        const size_t off = act_fp4 ? (act_fp4_ws_bytes(d) + 255) / 256 * 256 : 0;
+        const uint32_t cap = std::min(tile, d.max_loras) * ((d.max_rank + 15u) / 16u);
+        const size_t rows = size_t((d.m + tile - 1) / tile) * cap * tile;
+        if (aligned(d.ws, 256) && d.ws_bytes >= off + rows * 32 && rows < (1ull << 31)) {
+            t.tiles = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(d.ws) + off);
+            t.cap = cap;
+            t.part_rows = part_rows;
+        }
+        return t;
+    };
+    p.mt_tiles = p.mt;
+    if (b_pool_is_strided(d)) p.tt = tiles_in_ws(p.mt, p.pair ? p.mt / 2 : p.mt);
+    // Many tiles per SM pair (a prefill batch): the persistent form, whose operand rings run across tile
+    // boundaries and whose row stores overlap the next tile's K loop.  It takes 256-token tiles of CTA pairs
+    // without a K split, 16-byte aligned destination rows, and LoRA operands that both come by TMA.
+    p.persistent = p.mt == 256 && p.pair && p.k_split == 1 && !(flags & ATLAS_B200_FLAG_NO_PERSISTENT) && d.k % tc::KRAW == 0 &&
+                      (!d.seq_slot || b_pool_is_strided(d)) && d.out_row_stride % 8 == 0 &&
+                      (d.n_dest ? d.y_col_offset % 8 == 0 : aligned(d.y, 16));
+    for (uint32_t r = 0; p.persistent && r < d.n_dest; ++r) p.persistent = aligned(d.y_dest[r], 16);
+    // two token tiles of 192 per pass (the expanded weight operand is used twice) where the batch has several passes
+    p.two_tiles = p.persistent && !act_fp4 && !(flags & ATLAS_B200_FLAG_ONE_TILE_PASS) && d.m >= 768;
+    if (p.two_tiles) {
+        // ... unless whole waves say otherwise: a pass of two 192-token tiles takes about 977 cycles per K block, a pass
+        // of one 256-token tile about 725 (measured), and the last wave costs a full pass however few CTA pairs it holds
+        // (a 1024-feature projection over 8192 tokens: 88 two-tile passes or 128 one-tile passes on 74 pairs, two waves each)
+        const int c2 = persist_resident_clusters<192, 2, false>(2), c1 = persist_resident_clusters<256, 1, false>(0);
+        if (c1 > 0 && c2 > 0) {
+            const uint64_t w2 = (persist_tiles<192, 2>(d) + uint32_t(c2) - 1) / uint32_t(c2);
+            const uint64_t w1 = (persist_tiles<256, 1>(d) + uint32_t(c1) - 1) / uint32_t(c1);
+            if (w1 * 725 < w2 * 977) p.two_tiles = false;
+        }
+    }
+    if (p.persistent) {
+        const int clusters = act_fp4 ? persist_resident_clusters<256, 1, true>(1)
+                                     : (p.two_tiles ? persist_resident_clusters<192, 2, false>(2) : persist_resident_clusters<256, 1, false>(0));
+        const uint32_t tiles = p.two_tiles ? persist_tiles<192, 2>(d) : persist_tiles<256, 1>(d);
+        // (two-tile passes that fit one wave were chosen above because 256-token tiles would take two: 1237 tokens x 4096
+        //  features are 64 two-tile passes or 80 tiles on 74 pairs, q_proj 74 -> 38 us)
+        p.persistent = clusters > 0 && (p.two_tiles || tiles > uint32_t(clusters));
+    }
+    if (p.persistent && d.seq_slot) {
+        const uint32_t tile = p.two_tiles ? 192u : p.mt;
+        const TTiles t = tiles_in_ws(tile, tile / 2);
+        p.persistent = t.tiles != nullptr;
+        if (t.tiles) { p.tt = t; p.mt_tiles = tile; }
+    }
+    return p;
+}
+
 int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const ShrinkOnly* shrink_only = nullptr) {
     int rc = validate_linear(d);
     if (rc) return rc;
@@ -906,36 +1014,6 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         }
     }
     if (use_tc) {
-        // Token tile: the smallest power of two that covers m, at most 256 — then halved (down to 64)
-        // while the grid would leave more than a quarter of the SMs without a CTA, e.g. for a
-        // column shard of a wide layer: more, lighter CTAs finish sooner than few heavy ones.
-        uint32_t mt = 16;
-        while (mt < 256 && mt < d.m) mt <<= 1;
-        const uint32_t f_tiles = (d.n + tc::FT - 1) / tc::FT;
-        // Fewer tiles than half the SMs (a decode batch, a column shard): several CTAs share a tile, each
-        // contracting a share of K, rather than leaving SMs idle — a CTA's time is set by the weights it has
-        // to expand, which only a K split divides.  Clusters of at most 8 CTAs; whole 256-element stages.
-        uint32_t k_split = 1;
-        bool pair = mt >= 128 && !(d.flags & ATLAS_B200_FLAG_NO_CTA_PAIR);    // pairs of CTAs issue their MMAs together (see tc::Cfg)
-        if (!(d.flags & ATLAS_B200_FLAG_NO_K_SPLIT)) {
-            const uint32_t m_tiles = (d.m + mt - 1) / mt;
-            const uint32_t fit = uint32_t(rt_sm_count()) / (f_tiles * m_tiles);
-            k_split = std::max(1u, std::min(std::min(fit, 8u), d.k / uint32_t(tc::KRAW)));
-            // ... but only as many as still lets every cluster be resident at once (a second wave would cost more than the
-            // split saves), preferring the shape with pairs, then the one without, then a smaller split
-            const bool may_pair = pair;
-            for (; k_split > 1; --k_split) {
-                if (may_pair && k_split <= 4 &&
-                    tc_active_clusters_of(mt, act_fp4, true, k_split) >= int(((f_tiles + 1) / 2) * m_tiles)) { pair = true; break; }
-                if (tc_active_clusters_of(mt, act_fp4, false, k_split) >= int(f_tiles * m_tiles)) { pair = false; break; }
-            }
-            if (k_split == 1) pair = may_pair;
-        }
-        if (k_split == 1) {
-            while (mt > 64 && f_tiles * ((d.m + mt - 1) / mt) * 4 < uint32_t(rt_sm_count()) * 3) mt >>= 1;
-            pair = mt >= 128 && !(d.flags & ATLAS_B200_FLAG_NO_CTA_PAIR);
-        }
-
         ShrinkParams sp{};
         sp.x = static_cast<const uint16_t*>(d.x);
         sp.seq_slot = d.seq_slot;
@@ -949,82 +1027,27 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         // t = scale_s / (scale2 * 2^8) * (A_s x), the unit of the MMA accumulator (no 2^8 with FP4 activations)
         sp.post = act_fp4 ? 1.0f / d.scale2 : 1.0f / (d.scale2 * kWeightPreScale);
 
-        // The smallest batches, unless a form of the tcgen05 path is asked for by a flag.
-        constexpr uint32_t tc_forms = ATLAS_B200_FLAG_FORCE_TCGEN05 | ATLAS_B200_FLAG_ACT_FP4 | ATLAS_B200_FLAG_NO_CTA_PAIR |
-                                      ATLAS_B200_FLAG_NO_K_SPLIT | ATLAS_B200_FLAG_NO_PERSISTENT | ATLAS_B200_FLAG_ONE_TILE_PASS;
-        if (decode_pays(d) && !(d.flags & tc_forms) && !shrink_only) {
+        // (the shrink alone writes tiles, which the decode form does not read: it is planned as a call of the tcgen05 form)
+        const TcPlan plan = plan_tc(d, shrink_only ? d.flags | ATLAS_B200_FLAG_FORCE_TCGEN05 : d.flags, shrink_takes_mma_path(sp));
+        if (plan.decode) {
             // (t rows in lora_t are written by every call: the tiles a tcgen05 call leaves in `ws` are not what this kernel reads)
             rc = launch_decode(d, d.seq_slot ? &sp : nullptr, st);
             if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
             return rc;
         }
-
-        // Masked-t tiles: with scratch to put them in, the shrink writes the activation operand of every LoRA
-        // K-step once, in the layout the MMA reads, and the fused kernel's CTAs fetch it by TMA — instead of
-        // each CTA rebuilding the same tiles from lora_t.  Needs the strided pool (the TMA producer then feeds
-        // both LoRA operands) and the tensor-core shrink; otherwise the in-kernel build stays in use.
-        TTiles tt;
-        if (d.seq_slot && d.ws && b_pool_is_strided(d) && shrink_takes_mma_path(sp)) {
-            const size_t off = act_fp4 ? (act_fp4_ws_bytes(d) + 255) / 256 * 256 : 0;
-            const uint32_t cap = std::min(mt, d.max_loras) * ((d.max_rank + 15u) / 16u);
-            const size_t bytes = size_t((d.m + mt - 1) / mt) * cap * mt * 32;
-            if (aligned(d.ws, 256) && d.ws_bytes >= off + bytes && size_t((d.m + mt - 1) / mt) * cap * mt < (1ull << 31)) {
-                tt.tiles = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(d.ws) + off);
-                tt.cap = cap;
-                sp.tile_out = tt.tiles;
-                sp.tile_cap = cap;
-                sp.chunk = mt;
-                sp.part_rows = tt.part_rows = pair ? mt / 2 : mt;
-            }
+        const TTiles tt = plan.tt;
+        if (tt.tiles) {
+            sp.tile_out = tt.tiles;
+            sp.tile_cap = tt.cap;
+            sp.chunk = plan.mt_tiles;
+            sp.part_rows = tt.part_rows;
         }
-        // Many tiles per SM pair (a prefill batch): the persistent form, whose operand rings run across tile
-        // boundaries and whose row stores overlap the next tile's K loop.  It takes 256-token tiles of CTA pairs
-        // without a K split, 16-byte aligned destination rows, and LoRA operands that both come by TMA.
-        bool persistent = mt == 256 && pair && k_split == 1 && !(d.flags & ATLAS_B200_FLAG_NO_PERSISTENT) && d.k % tc::KRAW == 0 &&
-                          (!d.seq_slot || b_pool_is_strided(d)) && d.out_row_stride % 8 == 0 &&
-                          (d.n_dest ? d.y_col_offset % 8 == 0 : aligned(d.y, 16));
-        for (uint32_t r = 0; persistent && r < d.n_dest; ++r) persistent = aligned(d.y_dest[r], 16);
-        // two token tiles of 192 per pass (the expanded weight operand is used twice) where the batch has several passes
-        bool two_tiles = persistent && !act_fp4 && !(d.flags & ATLAS_B200_FLAG_ONE_TILE_PASS) && d.m >= 768;
-        if (two_tiles) {
-            // ... unless whole waves say otherwise: a pass of two 192-token tiles takes about 977 cycles per K block, a pass
-            // of one 256-token tile about 725 (measured), and the last wave costs a full pass however few CTA pairs it holds
-            // (a 1024-feature projection over 8192 tokens: 88 two-tile passes or 128 one-tile passes on 74 pairs, two waves each)
-            const int c2 = persist_resident_clusters<192, 2, false>(2), c1 = persist_resident_clusters<256, 1, false>(0);
-            if (c1 > 0 && c2 > 0) {
-                const uint64_t w2 = (persist_tiles<192, 2>(d) + uint32_t(c2) - 1) / uint32_t(c2);
-                const uint64_t w1 = (persist_tiles<256, 1>(d) + uint32_t(c1) - 1) / uint32_t(c1);
-                if (w1 * 725 < w2 * 977) two_tiles = false;
-            }
-        }
-        if (persistent) {
-            const int clusters = act_fp4 ? persist_resident_clusters<256, 1, true>(1)
-                                         : (two_tiles ? persist_resident_clusters<192, 2, false>(2) : persist_resident_clusters<256, 1, false>(0));
-            const uint32_t tiles = two_tiles ? persist_tiles<192, 2>(d) : persist_tiles<256, 1>(d);
-            // (two-tile passes that fit one wave were chosen above because 256-token tiles would take two: 1237 tokens x 4096
-            //  features are 64 two-tile passes or 80 tiles on 74 pairs, q_proj 74 -> 38 us)
-            persistent = clusters > 0 && (two_tiles || tiles > uint32_t(clusters));
-        }
-        const uint32_t mt_tiles = (persistent && two_tiles) ? 192u : mt;     // token tile of the shrink's masked-t blocks
-        if (persistent && d.seq_slot) {
-            TTiles t2;
-            ShrinkParams sp2 = sp;
-            sp2.tile_out = nullptr;
-            if (d.ws && shrink_takes_mma_path(sp)) {
-                const size_t off = act_fp4 ? (act_fp4_ws_bytes(d) + 255) / 256 * 256 : 0;
-                const uint32_t cap = std::min(mt_tiles, d.max_loras) * ((d.max_rank + 15u) / 16u);
-                const size_t n_t = (d.m + mt_tiles - 1) / mt_tiles;
-                const size_t bytes = n_t * cap * mt_tiles * 32;
-                if (aligned(d.ws, 256) && d.ws_bytes >= off + bytes && n_t * cap * mt_tiles < (1ull << 31)) {
-                    t2.tiles = reinterpret_cast<uint16_t*>(static_cast<uint8_t*>(d.ws) + off);
-                    t2.cap = cap;
-                    sp2.tile_out = t2.tiles;
-                    sp2.tile_cap = cap;
-                    sp2.chunk = mt_tiles;
-                    sp2.part_rows = t2.part_rows = mt_tiles / 2;
-                }
-            }
-            if (t2.tiles) { tt = t2; sp = sp2; } else persistent = false;
+        if (reuse_shrink && (d.flags & kTcForms)) {
+            // The call whose result this one is to reuse was made without the form flags: what it left is read only where this
+            // form would have left the same.  (It may be rows of lora_t where this one reads tiles — the smallest batches — or
+            // tiles of another height.)
+            const TcPlan left = plan_tc(d, d.flags & ~kTcForms, shrink_takes_mma_path(sp));
+            reuse_shrink = left.tt.tiles == tt.tiles && (!tt.tiles || (left.mt_tiles == plan.mt_tiles && left.tt.part_rows == tt.part_rows));
         }
         if (shrink_only) {
             // the shrink alone, for a row range, into several copies of the scratch: the launch shape decided above fixes
@@ -1044,24 +1067,24 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
             return rc;
         }
         const ShrinkParams* shrink = (d.seq_slot && !reuse_shrink) ? &sp : nullptr;
-        if (persistent) {
+        if (plan.persistent) {
             if (act_fp4) rc = launch_tc_persist<256, 1, true>(d, 1, shrink, tt, st);
-            else if (two_tiles) rc = launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);
+            else if (plan.two_tiles) rc = launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);
             else rc = launch_tc_persist<256, 1, false>(d, 0, shrink, tt, st);
             if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
             return rc;
         }
         if (act_fp4) {
-            if (mt == 16) rc = launch_tc<16, true, false>(d, 0, shrink, tt, k_split, st);
-            else if (mt == 32) rc = launch_tc<32, true, false>(d, 1, shrink, tt, k_split, st);
-            else if (mt == 64) rc = launch_tc<64, true, false>(d, 2, shrink, tt, k_split, st);
-            else if (mt == 128) rc = pair ? launch_tc<128, true, true>(d, 3, shrink, tt, k_split, st) : launch_tc<128, true, false>(d, 3, shrink, tt, k_split, st);
-            else rc = pair ? launch_tc<256, true, true>(d, 4, shrink, tt, k_split, st) : launch_tc<256, true, false>(d, 4, shrink, tt, k_split, st);
-        } else if (mt == 16) rc = launch_tc<16, false, false>(d, 0, shrink, tt, k_split, st);
-        else if (mt == 32) rc = launch_tc<32, false, false>(d, 1, shrink, tt, k_split, st);
-        else if (mt == 64) rc = launch_tc<64, false, false>(d, 2, shrink, tt, k_split, st);
-        else if (mt == 128) rc = pair ? launch_tc<128, false, true>(d, 3, shrink, tt, k_split, st) : launch_tc<128, false, false>(d, 3, shrink, tt, k_split, st);
-        else rc = pair ? launch_tc<256, false, true>(d, 4, shrink, tt, k_split, st) : launch_tc<256, false, false>(d, 4, shrink, tt, k_split, st);
+            if (plan.mt == 16) rc = launch_tc<16, true, false>(d, 0, shrink, tt, plan.k_split, st);
+            else if (plan.mt == 32) rc = launch_tc<32, true, false>(d, 1, shrink, tt, plan.k_split, st);
+            else if (plan.mt == 64) rc = launch_tc<64, true, false>(d, 2, shrink, tt, plan.k_split, st);
+            else if (plan.mt == 128) rc = plan.pair ? launch_tc<128, true, true>(d, 3, shrink, tt, plan.k_split, st) : launch_tc<128, true, false>(d, 3, shrink, tt, plan.k_split, st);
+            else rc = plan.pair ? launch_tc<256, true, true>(d, 4, shrink, tt, plan.k_split, st) : launch_tc<256, true, false>(d, 4, shrink, tt, plan.k_split, st);
+        } else if (plan.mt == 16) rc = launch_tc<16, false, false>(d, 0, shrink, tt, plan.k_split, st);
+        else if (plan.mt == 32) rc = launch_tc<32, false, false>(d, 1, shrink, tt, plan.k_split, st);
+        else if (plan.mt == 64) rc = launch_tc<64, false, false>(d, 2, shrink, tt, plan.k_split, st);
+        else if (plan.mt == 128) rc = plan.pair ? launch_tc<128, false, true>(d, 3, shrink, tt, plan.k_split, st) : launch_tc<128, false, false>(d, 3, shrink, tt, plan.k_split, st);
+        else rc = plan.pair ? launch_tc<256, false, true>(d, 4, shrink, tt, plan.k_split, st) : launch_tc<256, false, false>(d, 4, shrink, tt, plan.k_split, st);
         if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
         return rc;
     }

@@ -58,9 +58,12 @@ extern "C" {
 #define ATLAS_B200_FLAG_FORCE_SIMT     1u   /* always take the CUDA-core path */
 #define ATLAS_B200_FLAG_FORCE_TCGEN05  2u   /* fail with -1 instead of falling back */
 #define ATLAS_B200_FLAG_STAGED_LORA    4u   /* reference rounding: base->bf16, then shrink/expand/fold in place */
-#define ATLAS_B200_FLAG_REUSE_SHRINK   8u   /* tcgen05 path only: lora_t already holds this call's shrink result (same x,
-                                               seq_slot, tables and scale2 as the call that wrote it); skip the shrink launch.
-                                               Small batches, K not a multiple of 256 and ranks above 64 compute it anyway */
+#define ATLAS_B200_FLAG_REUSE_SHRINK   8u   /* tcgen05 path only: lora_t and ws still hold this call's shrink result (same x,
+                                               seq_slot, tables, scale2, scratch and ACT_FP4 as the call that wrote it, which had
+                                               none of the flags for comparison runs); skip the shrink launch.  Computed all the
+                                               same where that call left it in another form than this one reads: for the smallest
+                                               batches, K not a multiple of 256, ranks above 64, and calls with a comparison
+                                               flag that lay their LoRA activations out differently */
 #define ATLAS_B200_FLAG_ACT_FP4       16u   /* W4A4: the base product sees x quantised to NVFP4 (group of 16, E4M3 scale =
                                                group max / 6, tensor scale 1) and runs as a block-scaled FP4 x FP4 MMA; the
                                                LoRA term still sees exact x.  The opt-in W4A4 arm of the reference:

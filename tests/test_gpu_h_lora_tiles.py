@@ -53,3 +53,27 @@ def test_scratch_too_small_falls_back_to_the_build(cuda, atlas, oracle):
     assert np.array_equal(y.cpu().numpy().view(np.uint16), y0)
     assert (ws == 0).all()
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,strided_ws", [
+    (8, 512, 1040, True),              # the plain call takes the form for the smallest batches and leaves no tiles
+    (8, 512, 1040, False),             # ... without scratch both read rows of lora_t
+    (1237, 512, 4096, True),           # the plain call's passes of two 192-token tiles fit one wave
+])
+def test_reuse_after_a_plain_call(cuda, atlas, oracle, M, K, N, strided_ws):
+    """FLAG_REUSE_SHRINK together with a flag for comparison runs, after a call without: the bits of a call that computes its
+    own shrink, whatever form the plain call left its result in."""
+    from atlas_b200 import synth
+    case = synth.make_case("reuse", M=M, K=K, N=N, ranks=[16] * 5, max_rank=16, max_loras=6, none_frac=0.1, scale2=0.02,
+                           b_std=0.1, seed=M)
+    dc = DeviceCase(cuda, atlas, case)
+    y_plain, _ = dc.run(lora_ws=strided_ws)
+    ws = dc.ws if strided_ws else None
+    left, t_left = ws.clone() if strided_ws else None, dc.lora_t.clone()
+    assert_close(oracle, y_plain, ideal(oracle, case), "plain")
+    for flag in (0, atlas.FLAG_FORCE_TCGEN05, atlas.FLAG_NO_K_SPLIT, atlas.FLAG_NO_CTA_PAIR, atlas.FLAG_NO_PERSISTENT, atlas.FLAG_ONE_TILE_PASS):
+        want, _ = dc.run(flags=flag, lora_ws=strided_ws)
+        dc.lora_t.copy_(t_left)
+        y, _ = dc.run(flags=flag | atlas.FLAG_REUSE_SHRINK, ws=left.clone() if strided_ws else None)
+        assert np.array_equal(y, want), f"flag {flag}"
+    assert atlas.device_status() == 0
