@@ -155,9 +155,14 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(B + j));
         }
         if (p.wait_for_shrink) pdl_wait();
-        int32_t own[NT];
+        // slots of the token this thread loads t for, and of the two tokens (columns) whose sums it holds
+        int32_t own[NT], col[NT][2];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) own[n] = slot_s[8 * n + g];
+        for (int n = 0; n < NT; ++n) {
+            own[n] = slot_s[8 * n + g];
+            col[n][0] = slot_s[8 * n + 2 * t];
+            col[n][1] = slot_s[8 * n + 2 * t + 1];
+        }
         const int32_t lane_slot = lane < DCM_MAX_TOKENS ? slot_s[lane] : -1;
         for (uint32_t left = __ballot_sync(0xFFFFFFFFu, lane_slot >= 0); left;) {
             const uint32_t first = __ffs(left) - 1;                             // first token of this slot
@@ -185,7 +190,14 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
                         else bv[h] = make_uint2(uint32_t(q[0]) | uint32_t(q[1]) << 16, uint32_t(q[2]) | uint32_t(q[3]) << 16);
                     }
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) mma_bf16_16816(acc[i][n], bv[0].x, bv[1].x, bv[0].y, bv[1].y, tv[n].x, tv[n].y);
+                    for (int n = 0; n < NT; ++n) {
+                        // into the columns of this slot alone: an infinity in one adapter's B, times the zeros that stand for
+                        // the other tokens, must not reach them
+                        float d[4] = {acc[i][n][0], acc[i][n][1], acc[i][n][2], acc[i][n][3]};
+                        mma_bf16_16816(d, bv[0].x, bv[1].x, bv[0].y, bv[1].y, tv[n].x, tv[n].y);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[i][n][e] = col[n][e & 1] == s ? d[e] : acc[i][n][e];
+                    }
                 }
             }
         }

@@ -149,6 +149,31 @@ def test_small_batches(cuda, atlas, oracle, M, K, N, ranks, max_rank):
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,ranks,max_rank", [
+    (8, 512, 72, [16, 8, 24], 24),                       # 16 features per CTA, one n-tile
+    (7, 288, 5000, [128, 16], 128),                      # 32 features per CTA, eight granules
+    (16, 512, 1040, [16] * 5, 16),                       # two n-tiles
+    (13, 1056, 5008, [40, 72], 72),
+])
+def test_small_batches_keep_adapters_apart(cuda, atlas, oracle, M, K, N, ranks, max_rank):
+    """An infinity and a NaN in one adapter's B are its own rows' business."""
+    from atlas_b200 import synth
+    import copy
+    case = synth.make_case("apart", M=M, K=K, N=N, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 1, none_frac=0.2,
+                           scale2=0.02, b_std=0.1, seed=M + N)
+    case.seq_slot[:3] = [0, 1, -1]
+    y_clean, _ = DeviceCase(cuda, atlas, case).run()
+    bad = copy.deepcopy(case)
+    bad.adapters[0].b[0, 0], bad.adapters[0].b[N - 1, ranks[0] - 1] = 0x7F80, 0x7FC0
+    y, variant = DeviceCase(cuda, atlas, bad).run()
+    assert variant == atlas.VARIANT_TCGEN05
+    hit = case.seq_slot == 0
+    assert np.array_equal(y[~hit], y_clean[~hit])
+    assert np.array_equal(y[hit][:, 1:N - 1], y_clean[hit][:, 1:N - 1])
+    assert not np.isfinite(oracle.bf16_to_f32(y[hit][:, [0, N - 1]].copy())).any()
+    assert atlas.device_status() == 0
+
+
 def test_token_permutation_is_bit_exact(cuda, atlas, oracle):
     from atlas_b200 import synth
     import copy
