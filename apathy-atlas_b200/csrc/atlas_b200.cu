@@ -480,6 +480,9 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
     return ATLAS_B200_OK;
 }
 
+// What the shrink multiplies A_s x by, beside scale_s: t is in the unit of the MMA accumulator (no 2^8 with FP4 activations)
+static float lora_post(const atlas_b200_linear_desc& d, bool act_fp4) { return act_fp4 ? 1.0f / d.scale2 : 1.0f / (d.scale2 * kWeightPreScale); }
+
 // the launch constants both tcgen05 kernels share
 static int fill_tc_params(const atlas_b200_linear_desc& d, bool a4, bool b_strided, const TTiles& tt, tc::Params& p) {
     p.b_pool_strided = b_strided ? 1u : 0u;
@@ -506,6 +509,14 @@ static int fill_tc_params(const atlas_b200_linear_desc& d, bool a4, bool b_strid
     p.out_scale = a4 ? d.scale2 : d.scale2 * kWeightPreScale;
     p.w_scale_rows = d.k % tc::KRAW != 0 ? static_cast<const uint8_t*>(d.w_scale) : nullptr;
     p.k_split = 1;
+    // the shapes of the wide rule alone: their LoRA term was added row by row before they came to this path
+    p.isolate = d.seq_slot && !tc_eligible(d, false) ? 1u : 0u;
+    p.x = static_cast<const uint16_t*>(d.x);
+    p.w_packed = static_cast<const uint8_t*>(d.w_packed);
+    p.w_scale = static_cast<const uint8_t*>(d.w_scale);
+    p.scale_table = d.scale_table;
+    p.x_row_stride = d.x_row_stride;
+    p.post = lora_post(d, a4);
     return ATLAS_B200_OK;
 }
 
@@ -1024,8 +1035,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         sp.out = static_cast<uint16_t*>(d.lora_t);
         sp.M = d.m; sp.k_in = d.k; sp.max_rank = d.max_rank; sp.x_row_stride = d.x_row_stride; sp.max_loras = d.max_loras;
         sp.a_pool_base = d.a_pool_base; sp.a_slot_stride = d.a_slot_stride;
-        // t = scale_s / (scale2 * 2^8) * (A_s x), the unit of the MMA accumulator (no 2^8 with FP4 activations)
-        sp.post = act_fp4 ? 1.0f / d.scale2 : 1.0f / (d.scale2 * kWeightPreScale);
+        sp.post = lora_post(d, act_fp4);
 
         // (the shrink alone writes tiles, which the decode form does not read: it is planned as a call of the tcgen05 form)
         const TcPlan plan = plan_tc(d, shrink_only ? d.flags | ATLAS_B200_FLAG_FORCE_TCGEN05 : d.flags, shrink_takes_mma_path(sp));
@@ -1071,10 +1081,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
             if (act_fp4) rc = launch_tc_persist<256, 1, true>(d, 1, shrink, tt, st);
             else if (plan.two_tiles) rc = launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);
             else rc = launch_tc_persist<256, 1, false>(d, 0, shrink, tt, st);
-            if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
-            return rc;
-        }
-        if (act_fp4) {
+        } else if (act_fp4) {
             if (plan.mt == 16) rc = launch_tc<16, true, false>(d, 0, shrink, tt, plan.k_split, st);
             else if (plan.mt == 32) rc = launch_tc<32, true, false>(d, 1, shrink, tt, plan.k_split, st);
             else if (plan.mt == 64) rc = launch_tc<64, true, false>(d, 2, shrink, tt, plan.k_split, st);

@@ -46,6 +46,7 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "isolate.cuh"
 
 namespace atlas {
 namespace tc {
@@ -163,6 +164,13 @@ struct Params {
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
+    // isolate != 0: outputs that another adapter's infinity or NaN has made a NaN are computed again (isolate.cuh), from:
+    uint32_t isolate, x_row_stride;
+    const uint16_t* x;
+    const uint8_t* w_packed;
+    const uint8_t* w_scale;
+    const float* scale_table;
+    float post;                    // t = scale_s * post * (A_s x)
     unsigned long long* profile;   // nullable: per-CTA wait/busy cycle counters (PROFILE_WORDS per CTA)
 };
 
@@ -518,7 +526,7 @@ __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return r
 // features (4 bytes) of one token.
 template <int MT>
 __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_acc, uint32_t q, uint32_t lane,
-                                                 uint32_t f0, uint32_t m0, uint32_t part, uint32_t nparts) {
+                                                 uint32_t f0, uint32_t m0, uint32_t part, uint32_t nparts, uint32_t& nan_seen) {
     const uint32_t f = f0 + q * 32 + lane;
     const float osc = p.out_scale;
     const bool pair_ok = (p.out_row_stride % 2u == 0u) && ((reinterpret_cast<uintptr_t>(p.y) & 3u) == 0u);
@@ -537,6 +545,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
                 const uint32_t m = m0 + c0 + 2 * i + (odd ? 1u : 0u);
                 const uint32_t fe = f & ~1u;
                 const uint32_t w = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);
+                nan_seen |= bf16x2_nan_bits(w);
                 if (m < p.M) {
                     if (fe + 1 < p.N) *reinterpret_cast<uint32_t*>(p.y + size_t(m) * p.out_row_stride + fe) = w;
                     else if (fe < p.N) p.y[size_t(m) * p.out_row_stride + fe] = uint16_t(w & 0xFFFFu);
@@ -546,7 +555,9 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const uint32_t m = m0 + c0 + i;
-                if (m < p.M) p.y[size_t(m) * p.out_row_stride + f] = f32_to_bf16_bits(__uint_as_float(v[i]) * osc);
+                const uint16_t bits = f32_to_bf16_bits(__uint_as_float(v[i]) * osc);
+                nan_seen |= bf16x2_nan_bits(bits);
+                if (m < p.M) p.y[size_t(m) * p.out_row_stride + f] = bits;
             }
         }
     }
@@ -563,7 +574,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
 template <int MT>
 __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_acc, uint32_t tile, uint32_t bar_epi,
                                                 volatile uint32_t* abort_flag, uint32_t q, uint32_t lane, uint32_t f0,
-                                                uint32_t m0, uint32_t part, uint32_t nparts, uint32_t e_tid) {
+                                                uint32_t m0, uint32_t part, uint32_t nparts, uint32_t e_tid, uint32_t& nan_seen) {
     const float osc = p.out_scale;
     const bool odd = lane & 1u;
     const uint32_t fe = (q * 32u + lane) & ~1u;                  // even feature of this lane pair, within the tile
@@ -595,6 +606,7 @@ __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_a
         const uint32_t m = m0 + row;
         if (m >= p.M) break;
         const uint4 val = lds128(tile + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
+        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         for (uint32_t r = 0; r < p.n_dest; ++r) {
             uint16_t* dst = p.y_dest[r] + at;
@@ -631,7 +643,7 @@ __device__ __forceinline__ void split_send(uint32_t tmem_acc, uint32_t recv0, ui
 // Second half: the owner adds the ks partial tiles of its columns in source order, scales, converts and stores.
 template <int MT>
 __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t recv0, uint32_t ks, uint32_t kz, uint32_t f0,
-                                                   uint32_t m0, uint32_t e_tid) {
+                                                   uint32_t m0, uint32_t e_tid, uint32_t& nan_seen) {
     const uint32_t lc_n = (uint32_t(MT) / 16u + ks - 1u) / ks;
     const uint32_t n_chunks = uint32_t(MT) / 16u;
     const uint32_t mine = n_chunks > kz ? (n_chunks - kz + ks - 1u) / ks : 0u;      // chunks kz, kz + ks, ...
@@ -650,6 +662,7 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
         uint4 val;
         val.x = pack_bf16x2(acc[0] * osc, acc[1] * osc); val.y = pack_bf16x2(acc[2] * osc, acc[3] * osc);
         val.z = pack_bf16x2(acc[4] * osc, acc[5] * osc); val.w = pack_bf16x2(acc[6] * osc, acc[7] * osc);
+        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         const bool whole = p.staged_epilogue && f + 8u <= p.N;
         for (uint32_t r = 0; r < p.n_dest; ++r) {
@@ -676,7 +689,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                             const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_xs,
                             const __grid_constant__ CUtensorMap map_t,
-                            const Params p) {
+                            const __grid_constant__ Params p) {
     using C = Cfg<MT, A4, PAIR>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -709,6 +722,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     bool acc_ready = false;                              // split K: this warp saw the accumulator complete
+    uint32_t nan_seen = 0;                               // (kNanBits) this thread stored a NaN
     const uint32_t f0 = blockIdx.x * FT;
     const uint32_t m0 = blockIdx.y * MT;
     constexpr uint32_t CTAS = PAIR ? 2u : 1u;
@@ -1019,8 +1033,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const long long t_epi = clock64();
             tcgen05_fence_after();
             if (ks > 1) acc_ready = true;                   // split K: the tile is finished by the whole cluster, below
-            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, te);
-            else epilogue_columns<MT>(p, tmem_acc, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4);
+            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, te, nan_seen);
+            else epilogue_columns<MT>(p, tmem_acc, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, nan_seen);
             if (prof && te == 0) prof_row[7] = (unsigned long long)(clock64() - t_epi);
         }
     } else if (warp == RAW_WARP) {
@@ -1334,8 +1348,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (ok && mbar_wait(BAR_ACC, 0, abort_flag, STATUS_WAIT_EXPIRED_EPILOGUE, 64)) {
             tcgen05_fence_after();
             if (ks > 1) acc_ready = true;
-            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, EPI_THREADS + td);
-            else epilogue_columns<MT>(p, tmem_acc, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4);
+            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, EPI_THREADS + td, nan_seen);
+            else epilogue_columns<MT>(p, tmem_acc, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, nan_seen);
         }
     }
 
@@ -1351,8 +1365,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
         __syncwarp();
         cluster_sync_all();                                  // all partial tiles have arrived
-        if (warp >= EPI_WARP0 && acc_ready) split_reduce_store<MT>(p, x_tile0, ks, kz, f0, m0, tid - EPI_WARP0 * 32);
+        if (warp >= EPI_WARP0 && acc_ready) split_reduce_store<MT>(p, x_tile0, ks, kz, f0, m0, tid - EPI_WARP0 * 32, nan_seen);
     }
+
+    // (tiles in shared memory have been read by now: its first bytes serve as scratch)
+    if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
+        isolate_tile(p, m0, min(m0 + uint32_t(MT), p.M), f0, min(f0 + uint32_t(FT), p.N), ks, kz, reinterpret_cast<uint16_t*>(smem_gen));
 
     // ========================================= teardown ==========================================
     if (*abort_flag) {

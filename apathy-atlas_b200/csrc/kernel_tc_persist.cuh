@@ -114,7 +114,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                                        const __grid_constant__ CUtensorMap map_b,
                                        const __grid_constant__ CUtensorMap map_xs,
                                        const __grid_constant__ CUtensorMap map_t,
-                                       const Params p, const PParams pp) {
+                                       const __grid_constant__ Params p, const __grid_constant__ PParams pp) {
     using C = PCfg<MT, G, A4>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -153,6 +153,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     const uint32_t num_raw = A4 ? num_kb : num_kb / 4u;
     const uint32_t my_tiles = pp.n_tiles > pair ? (pp.n_tiles - pair + n_pairs - 1u) / n_pairs : 0u;
     const bool prof = p.profile != nullptr;
+    uint32_t nan_seen = 0;                                              // (kNanBits) this thread stored a NaN
     const long long t_entry = clock64();
     unsigned long long* prof_row = prof ? p.profile + size_t(blockIdx.x) * PROFILE_WORDS : nullptr;
 
@@ -534,6 +535,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         const uint32_t m = m_base + row;
                         if (m >= p.M) break;
                         const uint4 val = lds128(epi0 + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
+                        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
                         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
                         for (uint32_t r = 0; r < p.n_dest; ++r) {
                             uint16_t* dst = p.y_dest[r] + at;
@@ -689,6 +691,13 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             prof_row[3] = w_raw; prof_row[4] = w_empty; prof_row[5] = (unsigned long long)(clock64() - t_begin);
         }
     }
+
+    // (every stage and tile in shared memory has been read by now: its first bytes serve as scratch)
+    if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
+        for (uint32_t i = 0; i < my_tiles; ++i) {
+            const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * (MT * G);
+            isolate_tile(p, m0, min(m0 + uint32_t(MT * G), p.M), f0, min(f0 + uint32_t(FT), p.N), 1, 0, reinterpret_cast<uint16_t*>(smem_gen));
+        }
 
     // ========================================= teardown ==========================================
     if (*abort_flag) {

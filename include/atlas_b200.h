@@ -236,6 +236,9 @@ typedef struct atlas_b200_linear_desc {
     const float*    scale_table;    /* [max_loras] */
     const uint32_t* rank_table;     /* [max_loras] true ranks, or NULL (= max_rank everywhere) */
     uint32_t        max_loras, max_rank;
+    /* Adapters are meant to be finite.  An infinity or a NaN in row f of one B_s stays in the rows routed to s on the staged
+     * paths, in the smallest batches, and where K is not a multiple of 256 or max_rank is above 64; elsewhere it makes a NaN
+     * of feature f for all tokens that share a token tile (16 to 256 consecutive rows) with one of s. */
     /* output */
     void*           y;              /* [m, out_row_stride] bf16 */
     uint32_t        out_row_stride;

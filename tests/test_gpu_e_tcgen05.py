@@ -174,6 +174,42 @@ def test_small_batches_keep_adapters_apart(cuda, atlas, oracle, M, K, N, ranks, 
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,ranks,max_rank", [
+    (17, 288, 130, [16, 8, 24], 24),                     # odd row stride: no row but the first on a 16-byte boundary
+    (77, 2880, 520, [16] * 8, 16),                       # split K
+    (40, 512, 256, [128, 16, 65], 128),                  # ranks above 64
+    (300, 1056, 384, [128] * 6, 128),                    # CTA pairs
+    (1100, 512, 4096, [128, 72], 128),                   # persistent form
+])
+def test_shapes_beyond_the_forced_path_keep_adapters_apart(cuda, atlas, oracle, M, K, N, ranks, max_rank):
+    """An infinity and a NaN in one adapter's B and a NaN in one token's x are the business of their own rows."""
+    from atlas_b200 import synth
+    import copy
+    case = synth.make_case("apart", M=M, K=K, N=N, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 1, none_frac=0.2,
+                           scale2=0.02, b_std=0.1, seed=M + N)
+    case.seq_slot[:4] = [0, 1, -1, 1]
+    stride = N + 1 if M == 17 else N
+    bad = copy.deepcopy(case)
+    bad.adapters[0].b[1, 0], bad.adapters[0].b[N - 1, ranks[0] - 1] = 0x7F80, 0x7FC0
+    bad.x[3, 5] = 0x7FC0
+    for form in (dict(lora_ws=True), dict(strided=False)):
+        y_clean, _ = DeviceCase(cuda, atlas, case, out_row_stride=stride).run(**form)
+        y, variant = DeviceCase(cuda, atlas, bad, out_row_stride=stride).run(**form)
+        assert (atlas.last_launch_shape()["persistent_cta_pairs"] > 0) == (M == 1100 and "lora_ws" in form)
+        assert variant == atlas.VARIANT_TCGEN05
+        hit = case.seq_slot == 0
+        clean = ~hit
+        clean[3] = False
+        at = np.array([1, N - 1])
+        rest = np.setdiff1d(np.arange(N), at)
+        assert np.array_equal(y[clean][:, rest], y_clean[clean][:, rest])
+        assert np.array_equal(y[hit][:, rest], y_clean[hit][:, rest])
+        assert_close(oracle, y[clean][:, at], ideal(oracle, case)[clean][:, at], "computed again")
+        assert not np.isfinite(oracle.bf16_to_f32(y[hit][:, at].copy())).any()
+        assert not np.isfinite(oracle.bf16_to_f32(y[3:4, :N].copy())).any()
+    assert atlas.device_status() == 0
+
+
 def test_token_permutation_is_bit_exact(cuda, atlas, oracle):
     from atlas_b200 import synth
     import copy
