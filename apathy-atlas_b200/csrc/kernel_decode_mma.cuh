@@ -151,8 +151,8 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
         // this CTA's rows of B into L2 while the shrink may still run
         for (uint32_t m = warp; m < p.M; m += DCM_WARPS) {
             if (slot_s[m] < 0 || lane >= TILES * 16u || f0 + lane >= p.N) continue;
-            const uint16_t* B = reinterpret_cast<const uint16_t*>(b_s[m]) + size_t(f0 + lane) * p.max_rank;
-            for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(B + j));
+            const uint64_t row = b_s[m] + size_t(f0 + lane) * p.max_rank * 2u;
+            for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"((row + 2u * j) & ~15ull));
         }
         if (p.wait_for_shrink) pdl_wait();
         // slots of the token this thread loads t for, and of the two tokens (columns) whose sums it holds

@@ -1022,8 +1022,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     const uint32_t e = gran[g];
                     // (a strided pool's addresses are arithmetic: a table read per granule made this loop a chain of loads)
                     const unsigned long long b_s = p.b_pool_strided ? p.b_pool_base + (e >> GRAN_SHIFT) * p.b_slot_stride : p.b_table[e >> GRAN_SHIFT];
-                    const uint16_t* src = reinterpret_cast<const uint16_t*>(b_s) + size_t(f) * p.max_rank + (e & GRAN_MASK) * 16u;
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(src));
+                    const unsigned long long src = b_s + (size_t(f) * p.max_rank + (e & GRAN_MASK) * 16u) * 2u;
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(src & ~15ull));
                 }
             }
         }
@@ -1300,7 +1300,10 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                         if (td < 256u) {
                             const bool live = f < p.N && j0 + 8 * a_h < p.max_rank;
                             const uint16_t* src = live ? reinterpret_cast<const uint16_t*>(p.b_table[e >> GRAN_SHIFT]) + a_src_off + j0 : p.t;
-                            cp_async_16_zfill(base + g * C::L_GRAN_A + a_dst, src, live ? 16u : 0u);
+                            const uint32_t dst = base + g * C::L_GRAN_A + a_dst;
+                            if ((reinterpret_cast<uintptr_t>(src) & 15u) == 0u) cp_async_16_zfill(dst, src, live ? 16u : 0u);
+                            else sts128(dst, src[0] | uint32_t(src[1]) << 16, src[2] | uint32_t(src[3]) << 16,     // (B_s at any address)
+                                        src[4] | uint32_t(src[5]) << 16, src[6] | uint32_t(src[7]) << 16);
                         }
                     }
                 }

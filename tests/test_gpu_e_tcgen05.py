@@ -210,6 +210,31 @@ def test_shapes_beyond_the_forced_path_keep_adapters_apart(cuda, atlas, oracle, 
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N,max_rank", [
+    (8, 512, 136, 24),                                   # the smallest batches
+    (40, 512, 136, 24),
+    (77, 288, 200, 16),                                  # K not a multiple of 256
+    (300, 512, 264, 72),                                 # CTA pairs, ranks above 64
+])
+def test_b_at_any_address(cuda, atlas, oracle, M, K, N, max_rank):
+    """Without a strided pool B_s is read wherever its table entry says, two bytes past a 16-byte boundary too."""
+    from atlas_b200 import synth
+    case = synth.make_case("anywhere", M=M, K=K, N=N, ranks=[8, 16, max_rank], max_rank=max_rank, none_frac=0.1, scale2=0.02,
+                           b_std=0.1, seed=M + K)
+    dc = DeviceCase(cuda, atlas, case)
+    want, _ = dc.run(strided=False)
+    assert_close(oracle, want, ideal(oracle, case), "aligned")
+    pool = dc.pool.b_pool
+    moved = cuda.empty(pool.numel() + 8, dtype=pool.dtype, device="cuda")
+    moved[1:1 + pool.numel()].copy_(pool.reshape(-1))
+    dc.pool._b_host = [a and a - pool.data_ptr() + moved.data_ptr() + 2 for a in dc.pool._b_host]
+    dc.pool.refresh_tables()
+    y, variant = dc.run(strided=False)
+    assert variant == atlas.VARIANT_TCGEN05
+    assert np.array_equal(y, want)
+    assert atlas.device_status() == 0
+
+
 def test_token_permutation_is_bit_exact(cuda, atlas, oracle):
     from atlas_b200 import synth
     import copy
