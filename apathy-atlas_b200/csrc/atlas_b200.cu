@@ -162,9 +162,17 @@ static bool encode_tiled(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank
     cuuint32_t bx[3], es[3] = {1, 1, 1};
     for (uint32_t i = 0; i < rank; ++i) { gd[i] = dims[i]; bx[i] = box[i]; }
     for (uint32_t i = 0; i + 1 < rank; ++i) gs[i] = strides[i];
-    if (g_encode(map, dt, rank, const_cast<void*>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                 promo, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    auto encode = [&] {
+        return g_encode(map, dt, rank, const_cast<void*>(base), gd, gs, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, promo,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult rc = encode();
+    int dev = -1;
+    // a thread whose first call of CUDA this is has no context yet, and unlike the runtime's calls this one does not make one current
+    if ((rc == CUDA_ERROR_INVALID_CONTEXT || rc == CUDA_ERROR_NOT_INITIALIZED) && cudaGetDevice(&dev) == cudaSuccess &&
+        cudaSetDevice(dev) == cudaSuccess)
+        rc = encode();
+    if (rc != CUDA_SUCCESS) return false;
     e.key = key; e.map = *map; e.valid = true;
     return true;
 }

@@ -275,6 +275,32 @@ def test_auto_dispatch_and_fallback(cuda, atlas, oracle):
         dc.run(flags=atlas.FLAG_FORCE_TCGEN05)
 
 
+def test_first_cuda_call_of_a_thread(cuda, atlas, oracle):
+    """A thread that has made no call of CUDA yet: tensor maps are encoded there too."""
+    import threading
+    from atlas_b200 import synth
+    case = synth.make_case("thread", M=40, K=512, N=136, ranks=[8], max_rank=8, scale2=0.02, seed=5)
+    dc = DeviceCase(cuda, atlas, case)
+    want, _ = dc.run(lora=False)
+    y = cuda.zeros((40, 136), dtype=cuda.int16, device="cuda")
+    d = atlas.make_linear_desc(x=dc.x, m=40, k=512, n=136, y=y, w_packed=dc.packed, w_scale=dc.scales, scale2=case.scale2)
+    said = []
+
+    def call():
+        try:
+            said.append(atlas.nvfp4_lora_linear(d, 0))
+        except atlas.AtlasError as e:
+            said.append(e)
+
+    cuda.cuda.synchronize()
+    thread = threading.Thread(target=call)
+    thread.start()
+    thread.join()
+    cuda.cuda.synchronize()
+    assert said == [atlas.VARIANT_TCGEN05]
+    assert np.array_equal(y.cpu().numpy().view(np.uint16), want)
+
+
 def test_config1_full_size_sampled(cuda, atlas, oracle):
     """Benchmark configuration 1 at full size (M=256, K=5120, N=17408, 16 adapters of rank 32):
     a random sample of outputs against the oracle, and exact routing on the adapter-less rows."""
