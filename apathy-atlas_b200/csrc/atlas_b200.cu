@@ -20,7 +20,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
-#include <utility>
+#include <new>
 
 #include "common.cuh"
 #include "kernel_tc.cuh"
@@ -118,11 +118,11 @@ static DeviceState* device_state() {
 static int rt_sm_count() { DeviceState* st = device_state(); return st ? st->sm_count : 148; }
 
 // Encoded tensor maps are a pure function of (address, shape, strides, box, type, swizzle): a serving loop calls with the
-// same tensors step after step, so the most recent encodings are kept per host thread (direct-mapped, 64 entries) and a
-// repeated call costs a compare instead of a driver call per map.  A 32-layer model has some 1300 maps per batch shape, so
-// the cache holds 4096 in sets of four, the most recently used first (0.9 MB per calling thread, allocated at its first
-// call and given back when it ends); with 64 direct-mapped entries a decode step of one layer evicted its own maps and
-// spent about half of its host time (145 us) in the driver's encoder.
+// same tensors step after step, so recent encodings are kept per host thread and a repeated call costs a compare instead of a
+// driver call per map.  A 32-layer model has some 1300 maps per batch shape: 4096 are held, in sets of four of which the least
+// recently used one is replaced (1 MiB per calling thread, allocated at its first call and given back when the thread ends; with
+// no memory for it every map is encoded anew).  With 64 entries a decode step of one layer evicted its own maps and spent about
+// half of its host time (145 us) in the driver's encoder.
 struct MapKey {
     const void* base;
     uint64_t dims[3], strides[2];
@@ -131,11 +131,13 @@ struct MapKey {
 };
 struct MapEntry {
     MapKey key;
+    uint64_t used;           // t_map_tick at its last use; 0 = empty
     CUtensorMap map;
-    bool valid;
 };
+static_assert(sizeof(MapEntry) == 256, "4096 entries are 1 MiB");
 constexpr uint32_t kMapSets = 1024, kMapWays = 4;
 static thread_local std::unique_ptr<MapEntry[]> t_map_cache;
+static thread_local uint64_t t_map_tick = 0;
 
 static bool encode_tiled(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank, const void* base, const uint64_t* dims,
                          const uint64_t* strides, const uint32_t* box, CUtensorMapSwizzle swz,
@@ -149,15 +151,19 @@ static bool encode_tiled(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank
     h ^= (key.dims[0] * 31 + key.dims[1]) * 0xBF58476D1CE4E5B9ull + key.box[0] * 131 + key.box[1] * 17 + uint64_t(key.swizzle);
     h ^= uint64_t(key.rank) * 0x94D049BB133111EBull + key.dims[2] + key.strides[0] * 0x2545F4914F6CDD1Dull;
     h *= 0x9E3779B97F4A7C15ull;
-    if (!t_map_cache) t_map_cache.reset(new MapEntry[size_t(kMapSets) * kMapWays]());
-    MapEntry* set = &t_map_cache[size_t((h >> 32) % kMapSets) * kMapWays];
-    for (uint32_t w = 0; w < kMapWays; ++w)
-        if (set[w].valid && std::memcmp(&set[w].key, &key, sizeof(key)) == 0) {
-            *map = set[w].map;
-            if (w) std::swap(set[w], set[w - 1]);
-            return true;
+    if (!t_map_cache) t_map_cache.reset(new (std::nothrow) MapEntry[size_t(kMapSets) * kMapWays]());
+    MapEntry* e = nullptr;                                   // the set's least recently used entry
+    if (t_map_cache) {
+        MapEntry* set = e = &t_map_cache[size_t((h >> 32) % kMapSets) * kMapWays];
+        for (uint32_t w = 0; w < kMapWays; ++w) {
+            if (set[w].used && std::memcmp(&set[w].key, &key, sizeof(key)) == 0) {
+                set[w].used = ++t_map_tick;
+                *map = set[w].map;
+                return true;
+            }
+            if (set[w].used < e->used) e = &set[w];
         }
-    MapEntry& e = set[kMapWays - 1];
+    }
     cuuint64_t gd[3], gs[2];
     cuuint32_t bx[3], es[3] = {1, 1, 1};
     for (uint32_t i = 0; i < rank; ++i) { gd[i] = dims[i]; bx[i] = box[i]; }
@@ -173,7 +179,7 @@ static bool encode_tiled(CUtensorMap* map, CUtensorMapDataType dt, uint32_t rank
         cudaSetDevice(dev) == cudaSuccess)
         rc = encode();
     if (rc != CUDA_SUCCESS) return false;
-    e.key = key; e.map = *map; e.valid = true;
+    if (e) { e->key = key; e->map = *map; e->used = ++t_map_tick; }
     return true;
 }
 

@@ -301,6 +301,34 @@ def test_first_cuda_call_of_a_thread(cuda, atlas, oracle):
     assert np.array_equal(y.cpu().numpy().view(np.uint16), want)
 
 
+def test_more_tensor_maps_than_are_kept(cuda, atlas, oracle):
+    """Two passes over more activation addresses than a thread keeps encoded maps for, from two threads at once: the same bits."""
+    import threading
+    from atlas_b200 import synth
+    M, K, N, windows = 17, 256, 64, 4600
+    case = synth.make_case("maps", M=M + windows, K=K, N=N, ranks=[8], max_rank=8, scale2=0.02, seed=4)
+    dc = DeviceCase(cuda, atlas, case)
+    out = cuda.zeros((4, windows, M, N), dtype=cuda.int16, device="cuda")
+    cuda.cuda.synchronize()
+
+    def passes(t):
+        stream = cuda.cuda.Stream()
+        for i in range(2 * windows):
+            d = atlas.make_linear_desc(x=dc.x[i % windows:], m=M, k=K, n=N, y=out[2 * t + i // windows, i % windows], w_packed=dc.packed,
+                                       w_scale=dc.scales, scale2=case.scale2, flags=atlas.FLAG_FORCE_TCGEN05)
+            atlas.nvfp4_lora_linear(d, stream)
+        stream.synchronize()
+
+    threads = [threading.Thread(target=passes, args=(t,)) for t in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert all(cuda.equal(out[0], out[i]) for i in (1, 2, 3))
+    want = ideal(oracle, case, lora=False)
+    for i in (0, 2300, windows - 1):
+        assert_close(oracle, out[0, i].cpu().numpy().view(np.uint16), want[i:i + M], f"window {i}")
+    assert atlas.device_status() == 0
+
+
 def test_config1_full_size_sampled(cuda, atlas, oracle):
     """Benchmark configuration 1 at full size (M=256, K=5120, N=17408, 16 adapters of rank 32):
     a random sample of outputs against the oracle, and exact routing on the adapter-less rows."""
