@@ -291,7 +291,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     const uint32_t n_gran = misc[4 + g];
                     if (n_gran && !waited_for_shrink) {
                         // the masked-t tiles are the shrink grid's output: it must be complete before the first fetch
-                        if (p.wait_for_shrink) asm volatile("griddepcontrol.wait;" ::: "memory");
+                        if (p.wait_for_shrink) pdl_wait();
                         waited_for_shrink = true;
                     }
                     const uint32_t t_row0 = ((tile_pass(i) * G + g) * 2u + cta_rank) * p.t_tile_cap * uint32_t(C::L_GRAN_T / 256);
@@ -307,6 +307,8 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     }
                 }
             }
+            // (no granule in any tile: whatever waits for this grid may not overtake the shrink either)
+            if (p.wait_for_shrink && !waited_for_shrink) pdl_wait();
         }
     } else if (warp == 1) {
         // ===================================== MMA issuer ====================================================

@@ -128,3 +128,25 @@ def test_adapters_that_change_inside_a_shrink_clusters_rows(cuda, atlas, oracle,
     rows, cols = np.arange(500, 720, dtype=np.uint32), np.arange(0, N, 37, dtype=np.uint32)
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "rows around the border")
     assert atlas.device_status() == 0
+
+
+def test_a_batch_without_adapters(cuda, atlas, oracle):
+    """Every token routed nowhere: no tile has a granule, and the routing may change right behind the call."""
+    from atlas_b200 import synth
+    case = _case(synth, 1024, 512, 4864, seed=6)
+    case.seq_slot[:] = -1
+    dc = DeviceCase(cuda, atlas, case)
+    base, _ = dc.run(lora=False)
+    y, _ = dc.run(lora_ws=True)
+    assert atlas.last_launch_shape()["persistent_cta_pairs"] > 0
+    assert np.array_equal(y, base)
+    out = cuda.zeros((case.M, case.N), dtype=cuda.int16, device="cuda")
+    d = atlas.make_linear_desc(x=dc.x, m=case.M, k=case.K, n=case.N, y=out, w_packed=dc.packed, w_scale=dc.scales, scale2=case.scale2,
+                               seq_slot=dc.seq_slot, route=dc.pool.route(True, True), lora_t=dc.lora_t, ws=dc.ws, ws_bytes=dc.ws.numel())
+    for _ in range(20):
+        dc.seq_slot.fill_(-1)
+        atlas.nvfp4_lora_linear(d)
+        dc.seq_slot.fill_(0)
+    cuda.cuda.synchronize()
+    assert np.array_equal(bits_from_dev(out), base)
+    assert atlas.device_status() == 0
