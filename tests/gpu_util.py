@@ -3,6 +3,7 @@ import ctypes as C
 import os
 
 import numpy as np
+import pytest
 
 RTOL, ATOL = 2e-2, 1e-2      # the tolerance the path's specification states for BF16 outputs
 
@@ -134,3 +135,10 @@ class RefModule:
 def ref_available():
     import oracle.oracle_ctypes as oc
     return os.path.exists(os.path.join(oc.REF_DIR, "lora_bgmv.cubin"))
+
+
+def needs_reference():
+    """Skips what only a comparison with the reference's kernels can say: they are compiled from a checkout of the reference
+    (`make -C oracle REF=<checkout>`, or build() with one beside the repository) and are no part of this repository."""
+    if not ref_available():
+        pytest.skip("oracle/_ref/*.cubin are not built here (make -C oracle REF=<checkout of the reference>)")

@@ -4,18 +4,14 @@ library's replacements for them."""
 import numpy as np
 import pytest
 
-from gpu_util import ATOL, RTOL, DeviceCase, RefModule, assert_close, bits_from_dev, device_pool, host_pool, ideal, ref_available, to_dev
+from gpu_util import ATOL, RTOL, DeviceCase, RefModule, assert_close, bits_from_dev, device_pool, host_pool, ideal, needs_reference, to_dev
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.fixture(autouse=True)
 def _reference_cubins():
-    """These tests are the pin of the oracle to the reference's own kernels: without the compiled kernels they fail, they
-    do not skip.  The cubins are built by `make -C oracle REF=<checkout>` (or build() with the checkout beside the
-    repository) and travel with the working tree."""
-    if not ref_available():
-        pytest.fail("oracle/_ref/*.cubin are missing: build them from a checkout of the reference (make -C oracle REF=...)")
+    needs_reference()
 
 
 def u32(v):
