@@ -545,7 +545,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
                 const uint32_t m = m0 + c0 + 2 * i + (odd ? 1u : 0u);
                 const uint32_t fe = f & ~1u;
                 const uint32_t w = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);
-                nan_seen |= bf16x2_nan_bits(w);
+                if (p.isolate) nan_seen |= bf16x2_nan_bits(w);
                 if (m < p.M) {
                     if (fe + 1 < p.N) *reinterpret_cast<uint32_t*>(p.y + size_t(m) * p.out_row_stride + fe) = w;
                     else if (fe < p.N) p.y[size_t(m) * p.out_row_stride + fe] = uint16_t(w & 0xFFFFu);
@@ -556,7 +556,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
             for (int i = 0; i < 16; ++i) {
                 const uint32_t m = m0 + c0 + i;
                 const uint16_t bits = f32_to_bf16_bits(__uint_as_float(v[i]) * osc);
-                nan_seen |= bf16x2_nan_bits(bits);
+                if (p.isolate) nan_seen |= bf16x2_nan_bits(bits);
                 if (m < p.M) p.y[size_t(m) * p.out_row_stride + f] = bits;
             }
         }
@@ -606,7 +606,7 @@ __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_a
         const uint32_t m = m0 + row;
         if (m >= p.M) break;
         const uint4 val = lds128(tile + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
-        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         for (uint32_t r = 0; r < p.n_dest; ++r) {
             uint16_t* dst = p.y_dest[r] + at;
@@ -662,7 +662,7 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
         uint4 val;
         val.x = pack_bf16x2(acc[0] * osc, acc[1] * osc); val.y = pack_bf16x2(acc[2] * osc, acc[3] * osc);
         val.z = pack_bf16x2(acc[4] * osc, acc[5] * osc); val.w = pack_bf16x2(acc[6] * osc, acc[7] * osc);
-        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         const bool whole = p.staged_epilogue && f + 8u <= p.N;
         for (uint32_t r = 0; r < p.n_dest; ++r) {

@@ -537,7 +537,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         const uint32_t m = m_base + row;
                         if (m >= p.M) break;
                         const uint4 val = lds128(epi0 + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
-                        nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+                        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
                         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
                         for (uint32_t r = 0; r < p.n_dest; ++r) {
                             uint16_t* dst = p.y_dest[r] + at;
