@@ -83,6 +83,7 @@ struct DeviceState {
     int persist_clusters[kPersistKernels] = {};
     bool carveout_set = false;
     bool shrink_tc_attr_set = false;
+    int shrink_tc_clusters = 0;       // resident clusters of SHT_MAX_KSPLIT CTAs of the prefill shrink; 0 = not asked yet
     bool push_attr_set = false;
     bool dense_attr_set[5] = {};      // token tiles 16, 32, 64, 128, 256 of the dense-BF16 kernel
 };
@@ -202,6 +203,28 @@ static bool shrink_takes_mma_path(const ShrinkParams& p) {
     return (p.k_in % 32 == 0) && (p.x_row_stride % 8 == 0) && aligned(p.x, 16) && (p.seq_slot || aligned(p.a_uniform, 4));
 }
 
+// How many clusters of `ksplit` CTAs of the prefill shrink can be resident at once (they live inside one GPC: fewer than the SM
+// count suggests).  Asked once per device.
+static int shrink_tc_clusters(DeviceState& dst, uint32_t ksplit) {
+    if (dst.shrink_tc_clusters == 0) {
+        cudaLaunchConfig_t q{};
+        q.gridDim = dim3(ksplit);
+        q.blockDim = dim3(SHT_THREADS);
+        q.dynamicSmemBytes = SHT_SMEM_BYTES;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ksplit;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        q.attrs = attr;
+        q.numAttrs = 1;
+        int n = 0;
+        dst.shrink_tc_clusters = cudaOccupancyMaxActiveClusters(&n, lora_shrink_tc_kernel, &q) == cudaSuccess && n > 0 ? n : -1;
+        (void)cudaGetLastError();
+    }
+    return dst.shrink_tc_clusters;
+}
+
 static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool release_dependents = false,
                          bool dependent_leaves_sms_free = false) {
     p.release_dependents = release_dependents ? 1u : 0u;
@@ -244,12 +267,13 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         if (p.m_begin % 64 != 0 || p.m_begin >= p.M) return ATLAS_B200_ERR_DIMS;
         if (p.tile_out && p.chunk && p.chunk < uint32_t(SHT_ROWS)) return ATLAS_B200_ERR_DIMS;   // a cluster's rows lie in at most two token tiles
         const uint32_t rows = p.m_count ? std::min(p.m_count, p.M - p.m_begin) : p.M - p.m_begin;
-        // CTAs per 128 rows, each contracting a share of K: two, or four where the batch (the whole of it, not this launch's
-        // range: a row's result must not depend on how the batch is cut into launches) leaves room for them in one wave.  The
-        // K loop is a serial chain of two thirds of the launch: 1237 tokens, eight adapters, K = 4096 38 -> 30 us, K = 14336
-        // 91 -> 58 us; 2048 tokens of one adapter 23 -> 17 us.
+        // CTAs per 128 rows, each contracting a share of K: two, or four where the clusters of the batch (the whole of it, not this
+        // launch's range: a row's result must not depend on how the batch is cut into launches) are all resident at once — a
+        // second wave costs more than the split gains.  Two / four CTAs, eight adapters of rank 64: 1237 tokens, K = 4096 41 / 32 us,
+        // K = 14336 95 / 60 us; 4096 tokens 25 / 20 and 61 / 39 us; but 4352 tokens (34 clusters) 29 / 36 and 70 / 74 us.
         const uint32_t k_blocks = p.k_in / SHT_KSTAGE, row_groups = (p.M + SHT_ROWS - 1) / SHT_ROWS;
-        p.ksplit = k_blocks >= 8 && row_groups * SHT_MAX_KSPLIT <= uint32_t(rt_sm_count()) ? uint32_t(SHT_MAX_KSPLIT) : (k_blocks >= 2 ? 2u : 1u);
+        const bool four = k_blocks >= 8 && int(row_groups) <= shrink_tc_clusters(*dst, SHT_MAX_KSPLIT);
+        p.ksplit = four ? uint32_t(SHT_MAX_KSPLIT) : (k_blocks >= 2 ? 2u : 1u);
         const uint32_t n_ctas = p.ksplit * ((rows + SHT_ROWS - 1) / SHT_ROWS);
         p.profile = (g_profile_buf && size_t(n_ctas) * 16 <= g_profile_words) ? g_profile_buf : nullptr;
         cudaLaunchConfig_t cfg = {};
