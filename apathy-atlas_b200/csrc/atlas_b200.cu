@@ -814,16 +814,27 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT>, w, p));
 }
 
-// Where it is the faster one, both sides measured at cold L2 (8 adapters of rank 16; us, this kernel / tcgen05):
-//   1 token    1024 x 4096 13/17   4096 x 4096 15/20   14336 x 4096 28/34   4096 x 14336 24/34   28672 x 8192 63/104
-//   8 tokens   1024 x 4096 15/20   4096 x 4096 20/22   14336 x 4096 32/36   4096 x 14336 40/34   28672 x 8192 77/106
-//   16 tokens  1024 x 4096 15/20   4096 x 4096 24/21   14336 x 4096 34/36   4096 x 14336 52/34   28672 x 8192 89/105
-//              8192 x 8192 42/36; without adapters 28/34, and the faster one at all of these
-// With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does.
+// Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):
+//   no adapters          1 token     1024 x 4096 5/9    4096 x 4096 7/12   14336 x 4096 17/28   4096 x 14336 17/26   28672 x 8192 51/95
+//                        16 tokens   1024 x 4096 6/10   4096 x 4096 9/12   14336 x 4096 21/28   4096 x 14336 24/27   28672 x 8192 63/96
+//   8 of rank 16         1 token     1024 x 4096 6/11   4096 x 4096 8/14   14336 x 4096 20/30   4096 x 14336 18/29   28672 x 8192 55/101
+//                        8 tokens    1024 x 4096 7/12   4096 x 4096 10/15  14336 x 4096 23/31   8192 x 8192 21/32    28672 x 8192 64/102
+//                        16 tokens                                         14336 x 4096 27/31                        28672 x 8192 73/103
+//   8 of rank 64         8 tokens    1024 x 4096 11/13  4096 x 4096 16/17  14336 x 4096 29/33   8192 x 8192 30/34    28672 x 8192 80/107
+// With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does: up
+// to eight tokens there unless the weights (N >= 2 K) outweigh it, and a long K only as long as the shrink is short (4096 x 14336,
+// 7 tokens: eight of rank 32 25/30, of rank 64 37/32; 6 tokens of rank 64 32/31).
+// Beyond eight tokens a granule (16 ranks of a slot) costs it some 0.3 us more than the tcgen05 form, against what it gains on the
+// weights: most where those are more than one wave of tiles there.  N >= 2 K, 16 adapters, 16 tokens: 32 granules 14336 x 4096 38/36,
+// 16384 x 6144 53/47, 28672 x 8192 100/110; 64 granules 47/43, 74/59, 122/122; 96 granules (12 tokens) 28672 x 8192 135/140.
 static bool decode_pays(const atlas_b200_linear_desc& d) {
     if (d.m > uint32_t(DCM_MAX_TOKENS)) return false;
-    if (!d.seq_slot || uint64_t(d.n) >= 2ull * d.k) return true;
-    return d.m <= 8 && uint64_t(d.m) * d.k <= 8ull * 14000;
+    if (!d.seq_slot) return true;
+    if (uint64_t(d.n) >= 2ull * d.k) {
+        const uint32_t granules = std::min(d.m, d.max_loras) * ((d.max_rank + 15) / 16), waves = (d.n + tc::FT - 1) / tc::FT > uint32_t(rt_sm_count()) ? 2 : 1;
+        return d.m <= 8 || granules <= std::max(32u, d.k / (waves > 1 ? 80u : 128u));
+    }
+    return d.m <= 8 && uint64_t(d.m) * d.k <= (d.max_rank > 32 ? 86400u : 112000u);
 }
 
 static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
