@@ -211,14 +211,28 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) part[warp][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[i][n][e];
     __syncthreads();
-    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += DCM_THREADS) {
+    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += DCM_THREADS) {          // (whole warps: a multiple of 128)
         const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
-        if (m >= p.M || f >= p.N) continue;
         float sum = part[0][m][fi];
 #pragma unroll
         for (int k = 1; k < DCM_WARPS; ++k) sum += part[k][m][fi];
-        const uint16_t bits = f32_to_bf16_bits(sum * p.out_scale);
-        for (uint32_t r = 0; r < p.n_dest; ++r) p.y_dest[r][size_t(m) * p.out_row_stride + p.y_col0 + f] = bits;
+        const uint32_t bits = f32_to_bf16_bits(sum * p.out_scale);
+        const bool in = m < p.M && f < p.N;
+        const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
+        if (p.n_dest == 1) {
+            if (in) p.y_dest[0][at] = uint16_t(bits);
+            continue;
+        }
+        // several buffers, peers' among them (their rows allow 16-byte stores): eight lanes' features in one store.  (Into one
+        // buffer the shuffles cost more than the narrow stores: a decode layer 97.6 instead of 96.7 us.)
+        const uint32_t w0 = bits | __shfl_down_sync(0xFFFFFFFFu, bits, 1) << 16, w1 = __shfl_down_sync(0xFFFFFFFFu, w0, 2);
+        const uint32_t w2 = __shfl_down_sync(0xFFFFFFFFu, w0, 4), w3 = __shfl_down_sync(0xFFFFFFFFu, w1, 4);
+        if (!in) continue;
+        const bool whole = (f & ~7u) + 8u <= p.N;
+        for (uint32_t r = 0; r < p.n_dest; ++r) {
+            if (!whole) p.y_dest[r][at] = uint16_t(bits);
+            else if (lane % 8u == 0) *reinterpret_cast<uint4*>(p.y_dest[r] + at) = make_uint4(w0, w1, w2, w3);
+        }
     }
 }
 

@@ -51,6 +51,28 @@ def test_column_shards_fill_every_ranks_buffer(cuda, atlas, oracle, tp, act_fp4)
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 8, 13])
+def test_small_batches_fill_every_ranks_buffer(cuda, atlas, oracle, M):
+    """The form for the smallest batches, shards of 1048 columns (half a tile at the end), columns either side untouched; rows
+    that do not allow 16-byte stores give the same bits in one buffer."""
+    from atlas_b200 import synth, tp as tpmod
+    K, N, tp = 512, 2096, 2
+    case = synth.make_case("tp_small", M=M, K=K, N=N, ranks=[16, 8, 24], max_rank=24, none_frac=0.1, scale2=0.02, b_std=0.1, seed=M)
+    y_direct, _ = DeviceCase(cuda, atlas, case, out_row_stride=N + 3).run()
+    stride = N + 24
+    bufs = [cuda.full((M, stride), 0x7FC0, dtype=cuda.int16, device="cuda") for _ in range(tp)]
+    for r in range(tp):
+        sh = tpmod.DeviceShard(cuda, atlas, case, tp, r)
+        atlas.nvfp4_lora_linear(sh.desc(None, out_row_stride=stride, y_dest=bufs, y_col_offset=8 + r * sh.n_local))
+    cuda.cuda.synchronize()
+    for b in bufs:
+        got = bits_from_dev(b)
+        assert np.array_equal(got[:, 8:8 + N], y_direct[:, :N])
+        assert (got[:, :8] == 0x7FC0).all() and (got[:, 8 + N:] == 0x7FC0).all()
+    assert_close(oracle, y_direct[:, :N], ideal(oracle, case), "small")
+    assert atlas.device_status() == 0
+
+
 def test_placement_argument_errors(cuda, atlas, oracle):
     from atlas_b200 import synth, tp as tpmod
     case = synth.make_case("tp_err", M=32, K=256, N=256, ranks=[8], max_rank=8, seed=2)
