@@ -796,7 +796,7 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     w.w_scale = static_cast<const uint8_t*>(d.w_scale);
     w.x_row_stride = d.x_row_stride;
     const uint32_t ctas = (d.n + 16 * TILES - 1) / (16 * TILES);
-    t_last_shape[0] = 8 * NT; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
+    t_last_shape[0] = 8u; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
     if (shrink) {
         rc = launch_shrink(*shrink, d.max_loras, st, true, ctas * 3 <= uint32_t(rt_sm_count()) * 2);
         if (rc) return rc;

@@ -483,7 +483,7 @@ ATLAS_B200_API int atlas_b200_device_status(uint32_t* out_word, int clear);
 ATLAS_B200_API int atlas_b200_selftest_bounded_wait(uint64_t limit_ns, uint32_t out[3]);
 ATLAS_B200_API int atlas_b200_last_variant(void);
 /* Launch shape of the most recent tcgen05 call on this thread (launcher audit, no counterpart in the reference):
- * out[0] = token tile, out[1] = 1 if CTAs were paired for two-CTA MMAs, out[2] = CTAs per output tile (K split),
+ * out[0] = token tile (8: the mma.sync form of the smallest batches; 16 and more otherwise), out[1] = 1 if CTAs were paired for two-CTA MMAs, out[2] = CTAs per output tile (K split),
  * out[3] = 1 if the LoRA activation tiles came from the shrink through `ws`. */
 ATLAS_B200_API int atlas_b200_last_launch_shape(uint32_t out[4]);
 /* The persistent form of the most recent tcgen05 call on this thread: out[0] = token tiles per pass (0: the call ran one

@@ -84,7 +84,8 @@ def test_fused_lora(cuda, atlas, oracle, M, K, N, ranks, max_rank, with_ranks):
     (300, 544, 264, [8, 64], 64),                        # CTA pairs, a half K block at the end, partial second token tile
     (40, 512, 256, [128, 16, 65], 128),                  # eight granules of one slot
     (300, 1056, 384, [128] * 16, 128),                   # both at once, 128 granules per tile
-    (1100, 512, 2304, [128, 72], 128),                   # two-tile persistent form, ranks above 64
+    (1100, 512, 2304, [128, 72], 128),                   # token tiles of 128, ranks above 64
+    (1100, 512, 4096, [128, 72], 128),                   # two-tile persistent form, ranks above 64
     (8, 8480, 256, [104], 104),                          # max_rank not a multiple of 16, long K
 ])
 def test_shapes_beyond_the_forced_path(cuda, atlas, oracle, M, K, N, ranks, max_rank):
@@ -97,6 +98,7 @@ def test_shapes_beyond_the_forced_path(cuda, atlas, oracle, M, K, N, ranks, max_
     want = ideal(oracle, case)
     y, variant = dc.run(lora_ws=True)
     assert variant == atlas.VARIANT_TCGEN05
+    assert (atlas.last_launch_shape()["persistent_tiles_per_pass"] == 2) == (N == 4096)
     assert_close(oracle, y[:, :N], want, "default path")
     assert (y[:, N:] == 0x7FC0).all()
     if K < 8192:                                         # tiles from the shrink, tiles built in the kernel, B_s by address
@@ -132,7 +134,7 @@ def test_small_batches(cuda, atlas, oracle, M, K, N, ranks, max_rank):
                            scale2=0.02, b_std=0.1, seed=M + K)
     dc = DeviceCase(cuda, atlas, case, x_row_stride=K + 8, out_row_stride=N + 3)
     y, variant = dc.run()
-    assert variant == atlas.VARIANT_TCGEN05
+    assert variant == atlas.VARIANT_TCGEN05 and atlas.last_launch_shape()["token_tile"] == 8
     assert_close(oracle, y[:, :N], ideal(oracle, case), "fused")
     assert (y[:, N:] == 0x7FC0).all()
     y_tab, _ = dc.run(strided=False)
@@ -146,6 +148,23 @@ def test_small_batches(cuda, atlas, oracle, M, K, N, ranks, max_rank):
     c2.x, c2.seq_slot = case.x[::-1].copy(), case.seq_slot[::-1].copy()
     y2, _ = DeviceCase(cuda, atlas, c2, x_row_stride=K + 8, out_row_stride=N + 3).run()
     assert np.array_equal(y2, y[::-1])
+    assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,ads,max_rank,small", [
+    (8, 512, 264, 3, 64, True), (9, 512, 264, 3, 16, False), (9, 512, 1024, 3, 16, True),         # N >= 2 K beyond eight tokens
+    (16, 512, 1024, 16, 32, True), (16, 512, 1024, 16, 40, False), (16, 512, 1024, 2, 64, True),  # up to 32 granules there
+    (17, 512, 1024, 3, 16, False), (16, 512, 264, 0, 8, True),
+    (6, 14336, 136, 2, 64, True), (7, 14336, 136, 2, 64, False), (7, 14336, 136, 2, 32, True), (8, 14336, 136, 2, 32, False),
+])
+def test_which_batches_are_small(cuda, atlas, oracle, M, K, N, ads, max_rank, small):
+    """Either side of every line of the rule; what runs instead is the tcgen05 form, with the same values."""
+    from atlas_b200 import synth
+    case = synth.make_case("line", M=M, K=K, N=N, ranks=[max_rank] * max(ads, 1), max_rank=max_rank, scale2=0.02, b_std=0.1, seed=M + N)
+    y, variant = DeviceCase(cuda, atlas, case).run(lora=ads > 0)
+    assert variant == atlas.VARIANT_TCGEN05
+    assert (atlas.last_launch_shape()["token_tile"] == 8) == small
+    assert_close(oracle, y, ideal(oracle, case, lora=ads > 0), "either form")
     assert atlas.device_status() == 0
 
 
@@ -166,7 +185,7 @@ def test_small_batches_keep_adapters_apart(cuda, atlas, oracle, M, K, N, ranks, 
     bad = copy.deepcopy(case)
     bad.adapters[0].b[0, 0], bad.adapters[0].b[N - 1, ranks[0] - 1] = 0x7F80, 0x7FC0
     y, variant = DeviceCase(cuda, atlas, bad).run()
-    assert variant == atlas.VARIANT_TCGEN05
+    assert variant == atlas.VARIANT_TCGEN05 and atlas.last_launch_shape()["token_tile"] == 8
     hit = case.seq_slot == 0
     assert np.array_equal(y[~hit], y_clean[~hit])
     assert np.array_equal(y[hit][:, 1:N - 1], y_clean[hit][:, 1:N - 1])
