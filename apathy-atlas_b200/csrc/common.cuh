@@ -28,9 +28,16 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 
 // ---- programmatic dependent launch ------------------------------------------------------------
 // A decode step is a chain of short kernels, and between two of them an ordinary launch leaves the machine idle for a few
-// microseconds.  Kernels of this library therefore (a) let the next launch start as soon as all their own CTAs run, and (b) when
-// launched that way, begin by waiting until everything before them in the stream has completed and is visible.  Only the main
-// kernel of a linear call reads anything ahead of that wait, and it follows a shrink that has waited before releasing it.
+// microseconds.  A kernel may (a) release the next launch once all its own CTAs run, and (b) be launched as a dependent, which may
+// then start early and has to wait until everything before it in the stream has completed and is visible.
+//   launched as dependents     both tensor-core shrinks, the main kernel behind a shrink, the tensor-core expand, the dense linear,
+//                              the QKV consumers, SwiGLU in both forms, the quantiser
+//   releasing                  all of these but the shrinks: lora_shrink_tc_kernel never does, the mma.sync one and
+//                              lora_shrink_grouped_kernel only in front of a main kernel
+//   neither                    a main kernel without adapters releases but is launched in order; the NVFP4 decode, the maximum, the
+//                              CUDA-core linear and expand do neither
+// A dependent begins with the wait.  Only the main kernel reads anything ahead of it (x, weights, routing), and it follows a shrink
+// that has waited before releasing it; it waits before it reads t, on every path, so that nothing behind it overtakes the shrink.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The pointer as a value that does not exist before this point: keeps read-only loads through it behind pdl_wait().

@@ -4,8 +4,8 @@
 //
 // The fused kernels can store their tiles into the peers themselves (n_dest > 1); when a rank's share of a projection
 // is a single wave of tiles, those stores all happen at the end of the one wave and nothing is left to hide them
-// behind.  This kernel is the other way to overlap: it is small (128 threads, no shared memory), so its CTAs are
-// resident next to the CTAs of the NEXT projection's kernels, and it runs on a second stream while they compute.
+// behind.  This kernel is the other way to overlap: it is small (128 threads, no shared memory) and runs on a second stream while
+// the NEXT projection's kernels compute, on the SMs that such a share of a projection leaves free.
 // It replaces the all-gather that follows a column-parallel linear in the reference
 // (crates/spark-comm/src/nccl_backend/comm_impl.rs:130-145).
 #pragma once
@@ -27,7 +27,9 @@ struct PushParams {
     uint32_t dst_row_chunks;
 };
 
-// (at most 40 registers: a CTA must fit beside a 608-thread, 96-register CTA of the persistent kernel)
+// (At most 40 registers.  Beside a CTA of the persistent kernel, 640 threads of 96 registers, there is no room for one: launched
+//  250 us into four gate_proj calls of 8192 tokens it ran when the first of them ended, with 32 registers too, and when that kernel
+//  had one warp less.)
 __global__ void __launch_bounds__(PUSH_THREADS, 12)
 push_columns_kernel(const PushParams p) {
     const uint64_t total = uint64_t(p.m) * p.chunks_per_row;

@@ -227,7 +227,7 @@ lora_shrink_grouped_kernel(const ShrinkParams p) {
 
     // The fused layer launches its main kernel as a programmatic dependent of this grid; it reads
     // this grid's output only behind its own griddepcontrol.wait, so it may start right away.
-    if (p.release_dependents) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (p.release_dependents) pdl_release();
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t s = blockIdx.x;
     const uint32_t j0 = blockIdx.y * SHRINK_RT;
