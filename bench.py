@@ -49,11 +49,11 @@ FP4_PEAK_TFLOPS = 9000.0          # B200 dense NVFP4, nominal (no measured figur
 # summarised under profiles/ (per workload and activation mode; absent = no capture)
 NCU_TRAFFIC_BYTES = {
     # (workload, dominant projection, activations)
-    ("config3-layer", "gate", "bf16"): 432.6e6,      # persistent kernel <192, 2, A16>
-    ("config3-layer", "gate", "fp4"): 336.8e6,       # persistent kernel <256, 1, A4>
-    ("config4-mlp", "gate", "bf16"): 409.1e6,        # persistent kernel <256, 1, A16>
-    ("config1", "config1", "bf16"): 73.1e6,          # one-tile kernel <256>
-    ("config2", "config2", "bf16"): 66.1e6,          # one-tile kernel <64>
+    ("config3-layer", "gate", "bf16"): 432.7e6,      # persistent kernel <192, 2, A16>
+    ("config3-layer", "gate", "fp4"): 335.1e6,       # persistent kernel <256, 1, A4>
+    ("config4-mlp", "gate", "bf16"): 408.7e6,        # persistent kernel <256, 1, A16>
+    ("config1", "config1", "bf16"): 73.4e6,          # one-tile kernel <256>
+    ("config2", "config2", "bf16"): 66.2e6,          # one-tile kernel <64>
     ("config0", "config0", "bf16"): 33.7e6,          # dense BF16 kernel <16>
 }
 WORKLOADS = {
