@@ -72,12 +72,12 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 // (opt-in shared memory, carve-out) and occupancy answers belong to a device, so everything here is kept per
 // device ordinal and created under a lock the first time that device is current in a call.
 constexpr int kMaxDevices = 64;
-constexpr int kPersistKernels = 3;
+constexpr int kPersistKernels = 5;
 struct DeviceState {
     std::atomic<bool> ready{false};
     bool sm100 = false;
     int sm_count = 148;
-    bool tc_attr_set[40] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair} x {K of whole raw stages, not}
+    bool tc_attr_set[60] = {};        // token tiles 16..256 x {A16, A4} x {single CTA, CTA pair} x {K of whole raw stages, not, ranks above 64}
     int known_clusters[20][9] = {};   // resident clusters per kernel instance and K split; 0 = not asked yet
     bool persist_attr_set[kPersistKernels] = {};
     int persist_clusters[kPersistKernels] = {};
@@ -518,6 +518,11 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
     return ATLAS_B200_OK;
 }
 
+// The shapes of the wide rule alone: their LoRA term was added row by row before they came to the fused kernels (isolate.cuh).
+static bool isolates(const atlas_b200_linear_desc& d) {
+    return d.seq_slot && (d.k % tc::KRAW != 0 || d.max_rank > TC_NARROW_RANK);
+}
+
 // What the shrink multiplies A_s x by, beside scale_s: t is in the unit of the MMA accumulator (no 2^8 with FP4 activations)
 static float lora_post(const atlas_b200_linear_desc& d, bool act_fp4) { return act_fp4 ? 1.0f / d.scale2 : 1.0f / (d.scale2 * kWeightPreScale); }
 
@@ -547,8 +552,7 @@ static int fill_tc_params(const atlas_b200_linear_desc& d, bool a4, bool b_strid
     p.out_scale = a4 ? d.scale2 : d.scale2 * kWeightPreScale;
     p.w_scale_rows = d.k % tc::KRAW != 0 ? static_cast<const uint8_t*>(d.w_scale) : nullptr;
     p.k_split = 1;
-    // the shapes of the wide rule alone: their LoRA term was added row by row before they came to this path
-    p.isolate = d.seq_slot && !tc_eligible(d, false) ? 1u : 0u;
+    p.isolate = isolates(d) ? 1u : 0u;
     p.x = static_cast<const uint16_t*>(d.x);
     p.w_packed = static_cast<const uint8_t*>(d.w_packed);
     p.w_scale = static_cast<const uint8_t*>(d.w_scale);
@@ -606,16 +610,16 @@ static int tc_active_clusters_of(uint32_t mt, bool a4, bool pair, uint32_t k_spl
     return -1;
 }
 
-template <int MT, bool A4, bool PAIR, bool SROWS>
+template <int MT, bool A4, bool PAIR, bool SROWS, bool ISO>
 static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const ShrinkParams* shrink, const TTiles& tt,
                      uint32_t k_split, cudaStream_t st) {
     const bool after_shrink = shrink != nullptr;     // the shrink is launched from here, once the launch shape is final
     using C = tc::Cfg<MT, A4, PAIR>;
     DeviceState* dst = device_state();
     if (!dst) return ATLAS_B200_ERR_ARCH;
-    slot_idx += (A4 ? 5 : 0) + (PAIR ? 10 : 0) + (SROWS ? 20 : 0);
+    slot_idx += (A4 ? 5 : 0) + (PAIR ? 10 : 0) + (SROWS ? 20 : (ISO ? 40 : 0));
     if (!dst->tc_attr_set[slot_idx]) {
-        cudaError_t e = cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS>,
+        cudaError_t e = cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS, ISO>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
         if (e != cudaSuccess) return cuda_status(e);
         dst->tc_attr_set[slot_idx] = true;
@@ -678,27 +682,30 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     p.wait_for_shrink = after_shrink ? 1u : 0u;
-    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS>, map_x, map_w, map_s, map_b, map_xs, map_t, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS, ISO>, map_x, map_w, map_s, map_b, map_xs, map_t, p));
 }
 
 template <int MT, bool A4, bool PAIR>
 static int launch_tc(const atlas_b200_linear_desc& d, int slot_idx, const ShrinkParams* shrink, const TTiles& tt,
                      uint32_t k_split, cudaStream_t st) {
     if constexpr (!A4)
-        if (d.k % tc::KRAW != 0) return launch_tc_as<MT, false, PAIR, true>(d, slot_idx, shrink, tt, k_split, st);
-    return launch_tc_as<MT, A4, PAIR, false>(d, slot_idx, shrink, tt, k_split, st);
+    {
+        if (d.k % tc::KRAW != 0) return launch_tc_as<MT, false, PAIR, true, true>(d, slot_idx, shrink, tt, k_split, st);
+        if (isolates(d)) return launch_tc_as<MT, false, PAIR, false, true>(d, slot_idx, shrink, tt, k_split, st);
+    }
+    return launch_tc_as<MT, A4, PAIR, false, false>(d, slot_idx, shrink, tt, k_split, st);
 }
 
 // ---- the persistent form (kernel_tc_persist.cuh): one cluster of two CTAs per pair of SMs, a static tile loop ----
-// instance index: 0 = <256, 1, A16>, 1 = <256, 1, A4>, 2 = <192, 2, A16>
-template <int MT, int G, bool A4>
+// instance index: 0 = <256, 1, A16>, 1 = <256, 1, A4>, 2 = <192, 2, A16>, 3 and 4 = 0 and 2 for calls that isolate
+template <int MT, int G, bool A4, bool ISO = false>
 static int persist_resident_clusters(int idx) {
     using C = tc::PCfg<MT, G, A4>;
     DeviceState* dst = device_state();
     if (!dst) return -1;
     if (dst->persist_clusters[idx] == 0) {
         if (!dst->persist_attr_set[idx]) {
-            if (cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4>,
+            if (cudaFuncSetAttribute(tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4, ISO>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES) != cudaSuccess) {
                 (void)cudaGetLastError();
                 return -1;
@@ -718,7 +725,7 @@ static int persist_resident_clusters(int idx) {
         q.numAttrs = 1;
         int n = 0;
         dst->persist_clusters[idx] =
-            cudaOccupancyMaxActiveClusters(&n, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4>, &q) == cudaSuccess && n > 0 ? n : -1;
+            cudaOccupancyMaxActiveClusters(&n, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4, ISO>, &q) == cudaSuccess && n > 0 ? n : -1;
         (void)cudaGetLastError();
     }
     return dst->persist_clusters[idx];
@@ -732,10 +739,10 @@ static uint32_t persist_tiles(const atlas_b200_linear_desc& d) {
     return n_fpairs * n_passes;
 }
 
-template <int MT, int G, bool A4>
+template <int MT, int G, bool A4, bool ISO = false>
 static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const ShrinkParams* shrink, const TTiles& tt, cudaStream_t st) {
     using C = tc::PCfg<MT, G, A4>;
-    const int clusters = persist_resident_clusters<MT, G, A4>(idx);
+    const int clusters = persist_resident_clusters<MT, G, A4, ISO>(idx);
     if (clusters <= 0) return ATLAS_B200_ERR_DIMS;
     TcMaps maps;
     {
@@ -780,7 +787,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     p.wait_for_shrink = shrink ? 1u : 0u;
-    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4>, maps.x, maps.w, maps.s, maps.b,
+    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4, ISO>, maps.x, maps.w, maps.s, maps.b,
                                           maps.xs, maps.t, p, pp));
 }
 
@@ -1009,14 +1016,15 @@ static TcPlan plan_tc(const atlas_b200_linear_desc& d, uint32_t flags, bool shri
     // two token tiles of 192 per pass (the expanded weight operand is used twice) where the batch has several passes
     p.two_tiles = p.persistent && !act_fp4 && !(flags & ATLAS_B200_FLAG_ONE_TILE_PASS) && d.m >= 768;
     if (p.two_tiles) {
-        // ... unless whole waves say otherwise: a pass of two 192-token tiles takes about 977 cycles per K block, a pass
-        // of one 256-token tile about 725 (measured), and the last wave costs a full pass however few CTA pairs it holds
-        // (a 1024-feature projection over 8192 tokens: 88 two-tile passes or 128 one-tile passes on 74 pairs, two waves each)
+        // ... unless whole waves say otherwise: the last wave costs a full pass however few CTA pairs it holds, and a pass of two
+        // 192-token tiles takes about 1.4 times as long as one of a 256-token tile.  One-tile / two-tile calls by waves (us,
+        // K = 4096; K = 14336): 2 : 2 83 / 109; 209 / 303   5 : 4 158 / 172; 495 / 544   4 : 3 129 / 140; 374 / 414   7 : 5 206 / 207;
+        // 686 / 683   3 : 2 110 / 108; 291 / 286   6 : 4 178 / 171; 579 / 552.  The line lies between 4 : 3 and 7 : 5.
         const int c2 = persist_resident_clusters<192, 2, false>(2), c1 = persist_resident_clusters<256, 1, false>(0);
         if (c1 > 0 && c2 > 0) {
             const uint64_t w2 = (persist_tiles<192, 2>(d) + uint32_t(c2) - 1) / uint32_t(c2);
             const uint64_t w1 = (persist_tiles<256, 1>(d) + uint32_t(c1) - 1) / uint32_t(c1);
-            if (w1 * 725 < w2 * 977) p.two_tiles = false;
+            if (w1 * 100 < w2 * 135) p.two_tiles = false;
         }
     }
     if (p.persistent) {
@@ -1128,8 +1136,8 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         const ShrinkParams* shrink = (d.seq_slot && !reuse_shrink) ? &sp : nullptr;
         if (plan.persistent) {
             if (act_fp4) rc = launch_tc_persist<256, 1, true>(d, 1, shrink, tt, st);
-            else if (plan.two_tiles) rc = launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);
-            else rc = launch_tc_persist<256, 1, false>(d, 0, shrink, tt, st);
+            else if (plan.two_tiles) rc = isolates(d) ? launch_tc_persist<192, 2, false, true>(d, 4, shrink, tt, st) : launch_tc_persist<192, 2, false>(d, 2, shrink, tt, st);
+            else rc = isolates(d) ? launch_tc_persist<256, 1, false, true>(d, 3, shrink, tt, st) : launch_tc_persist<256, 1, false>(d, 0, shrink, tt, st);
         } else if (act_fp4) {
             if (plan.mt == 16) rc = launch_tc<16, true, false>(d, 0, shrink, tt, plan.k_split, st);
             else if (plan.mt == 32) rc = launch_tc<32, true, false>(d, 1, shrink, tt, plan.k_split, st);

@@ -6,10 +6,9 @@
 // NaN of feature f for the whole tile.  That NaN survives every later addition, so it is enough to look for NaNs in what is
 // stored: a CTA that has stored one computes again, behind its last store, what a row's own x, A and B leave finite.
 //
-// The look costs three integer operations per two outputs and one barrier (77 tokens x 2880 features x 2880: 17.1 us with and
-// without it; as a kernel of its own behind the main one 19.3).  Calls of other shapes skip it: looking all the same cost a
-// layer of 1237 tokens 0.5 %.  A NaN costs a dot product of length K per output concerned,
-// by one warp.
+// The look costs three integer operations per two outputs and one barrier (77 tokens x 2880 features x 2880: 17.2 us with it,
+// 17.0 without; as a kernel of its own behind the main one 19.3).  It is compiled into instances of their own (ISO): in all of them
+// it cost the calls of other shapes 0.5 to 1.3 %.  A NaN costs a dot product of length K per output concerned, by one warp.
 #pragma once
 
 #include "common.cuh"
@@ -86,9 +85,10 @@ __device__ __forceinline__ void isolate_row(const P& p, uint32_t m, uint32_t f_l
     }
 }
 
+// (Inlined: as a call it made the kernels that use it spill in their K loops, up to 3 % of a call.)
 // The tile [m_lo, m_hi) x [f_lo, f_hi) that this CTA has stored; of its 16-token chunks only every ks-th, from kz (split K).
 template <typename P>
-__device__ __noinline__ void isolate_tile(const P& p, uint32_t m_lo, uint32_t m_hi, uint32_t f_lo, uint32_t f_hi, uint32_t ks, uint32_t kz,
+__device__ __forceinline__ void isolate_tile(const P& p, uint32_t m_lo, uint32_t m_hi, uint32_t f_lo, uint32_t f_hi, uint32_t ks, uint32_t kz,
                                           uint16_t* t_s) {
     for (uint32_t m = m_lo; m < m_hi; ++m) {
         if (((m - m_lo) / 16u) % ks != kz) continue;

@@ -164,7 +164,7 @@ struct Params {
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
-    // isolate != 0: outputs that another adapter's infinity or NaN has made a NaN are computed again (isolate.cuh), from:
+    // isolate != 0 (ISO instances only): outputs that another adapter's infinity or NaN has made a NaN are computed again (isolate.cuh), from:
     uint32_t isolate, x_row_stride;
     const uint16_t* x;
     const uint8_t* w_packed;
@@ -524,7 +524,7 @@ __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return r
 // Epilogue for one participant: `q` = TMEM lane quadrant of this warp, chunks of 16 token columns
 // c = part, part + nparts, ...  Lane pairs exchange values so every thread stores two adjacent
 // features (4 bytes) of one token.
-template <int MT>
+template <int MT, bool ISO>
 __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_acc, uint32_t q, uint32_t lane,
                                                  uint32_t f0, uint32_t m0, uint32_t part, uint32_t nparts, uint32_t& nan_seen) {
     const uint32_t f = f0 + q * 32 + lane;
@@ -545,7 +545,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
                 const uint32_t m = m0 + c0 + 2 * i + (odd ? 1u : 0u);
                 const uint32_t fe = f & ~1u;
                 const uint32_t w = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);
-                if (p.isolate) nan_seen |= bf16x2_nan_bits(w);
+                if constexpr (ISO) nan_seen |= bf16x2_nan_bits(w);
                 if (m < p.M) {
                     if (fe + 1 < p.N) *reinterpret_cast<uint32_t*>(p.y + size_t(m) * p.out_row_stride + fe) = w;
                     else if (fe < p.N) p.y[size_t(m) * p.out_row_stride + fe] = uint16_t(w & 0xFFFFu);
@@ -556,7 +556,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
             for (int i = 0; i < 16; ++i) {
                 const uint32_t m = m0 + c0 + i;
                 const uint16_t bits = f32_to_bf16_bits(__uint_as_float(v[i]) * osc);
-                if (p.isolate) nan_seen |= bf16x2_nan_bits(bits);
+                if constexpr (ISO) nan_seen |= bf16x2_nan_bits(bits);
                 if (m < p.M) p.y[size_t(m) * p.out_row_stride + f] = bits;
             }
         }
@@ -571,7 +571,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
 // fall into different banks), meet on an mbarrier, then copy whole rows out with 16-byte stores — to every
 // destination buffer in turn.  `e_tid` = 0 .. 32 * EPI_WARPS - 1 numbers the participating threads.
 // Requires 16-byte aligned destination rows (checked by the caller); returns false if the wait expired.
-template <int MT>
+template <int MT, bool ISO>
 __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_acc, uint32_t tile, uint32_t bar_epi,
                                                 volatile uint32_t* abort_flag, uint32_t q, uint32_t lane, uint32_t f0,
                                                 uint32_t m0, uint32_t part, uint32_t nparts, uint32_t e_tid, uint32_t& nan_seen) {
@@ -606,7 +606,7 @@ __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_a
         const uint32_t m = m0 + row;
         if (m >= p.M) break;
         const uint4 val = lds128(tile + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
-        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+        if constexpr (ISO) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         for (uint32_t r = 0; r < p.n_dest; ++r) {
             uint16_t* dst = p.y_dest[r] + at;
@@ -641,7 +641,7 @@ __device__ __forceinline__ void split_send(uint32_t tmem_acc, uint32_t recv0, ui
 }
 
 // Second half: the owner adds the ks partial tiles of its columns in source order, scales, converts and stores.
-template <int MT>
+template <int MT, bool ISO>
 __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t recv0, uint32_t ks, uint32_t kz, uint32_t f0,
                                                    uint32_t m0, uint32_t e_tid, uint32_t& nan_seen) {
     const uint32_t lc_n = (uint32_t(MT) / 16u + ks - 1u) / ks;
@@ -662,7 +662,7 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
         uint4 val;
         val.x = pack_bf16x2(acc[0] * osc, acc[1] * osc); val.y = pack_bf16x2(acc[2] * osc, acc[3] * osc);
         val.z = pack_bf16x2(acc[4] * osc, acc[5] * osc); val.w = pack_bf16x2(acc[6] * osc, acc[7] * osc);
-        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+        if constexpr (ISO) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         const bool whole = p.staged_epilogue && f + 8u <= p.N;
         for (uint32_t r = 0; r < p.n_dest; ++r) {
@@ -678,10 +678,12 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
 }
 
 // SROWS (A16, K not a multiple of 256): the scale rows come by the expansion warps' own loads (Params::w_scale_rows).
-// (The bound is wider than the launch so that a thread gets at most 96 registers: the shrink of a decode batch runs beside
-//  this kernel, and with 107 registers only one of its CTAs found room on an SM instead of two: 140 -> 160 us for the fused
-//  QKV projections of 64 tokens with 64 adapters.)
-template <int MT, bool A4, bool PAIR, bool SROWS = false>
+// ISO: the form for calls with Params::isolate.
+// (The bound is wider than the launch: with it a thread gets 80 registers instead of 107.  The shrink runs beside this kernel, and
+//  at 107 only one of its CTAs found room on an SM instead of two: 140 -> 160 us for the fused QKV projections of 64 tokens with
+//  64 adapters.  Nothing spills but two values of the SROWS forms, outside the K loop.  Without the cap from 128 tokens on,
+//  256 tokens x 17408 x 5120 gain 1 %, but 80 to 256 tokens of 128 adapters of rank 64 over 14336 x 4096 lose 2 to 4 %.)
+template <int MT, bool A4, bool PAIR, bool SROWS = false, bool ISO = SROWS>
 __global__ void __launch_bounds__(672, 1)
 nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                             const __grid_constant__ CUtensorMap map_w,
@@ -844,7 +846,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 // the staging area may be overwritten once the expansion warps have seen every base MMA finish
                 if (n_gran && mbar_wait(BAR_DRAINED, 0, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32)) {
                     // masked-t tiles are the shrink grid's output: it must be complete before they are fetched
-                    if (p.t_tile_cap && p.wait_for_shrink) asm volatile("griddepcontrol.wait;" ::: "memory");
+                    if (p.t_tile_cap && p.wait_for_shrink) pdl_wait();
                     // this CTA's blocks: [XROWS x 16] BF16 images, C::L_GRAN_T bytes each, consecutive in list order
                     const uint32_t t_row0 = (blockIdx.y * CTAS + cta_rank) * p.t_tile_cap * uint32_t(C::L_GRAN_T / 256);
                     uint32_t ls = 0, lph = 0;
@@ -1033,8 +1035,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const long long t_epi = clock64();
             tcgen05_fence_after();
             if (ks > 1) acc_ready = true;                   // split K: the tile is finished by the whole cluster, below
-            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, te, nan_seen);
-            else epilogue_columns<MT>(p, tmem_acc, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, nan_seen);
+            else if (p.staged_epilogue) epilogue_staged<MT, ISO>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, te, nan_seen);
+            else epilogue_columns<MT, ISO>(p, tmem_acc, warp & 3u, lane, f0, m0, 0, 1 + DEQ_WARPS / 4, nan_seen);
             if (prof && te == 0) prof_row[7] = (unsigned long long)(clock64() - t_epi);
         }
     } else if (warp == RAW_WARP) {
@@ -1228,7 +1230,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (ok) ok = mbar_wait(BAR_LIST, 0, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, 32);
         // t is produced by the shrink grid this kernel may have overtaken: everything above ran
         // without it; from here on its writes must be complete and visible.
-        if (p.wait_for_shrink) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (p.wait_for_shrink) pdl_wait();
         const uint32_t n_gran = ok ? misc[1] : 0u;
         const uint32_t n_lb = (n_gran + 3u) / 4u;
         s = num_kb % uint32_t(C::STAGES);                    // stage / phase the K block after the last one would take
@@ -1351,8 +1353,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (ok && mbar_wait(BAR_ACC, 0, abort_flag, STATUS_WAIT_EXPIRED_EPILOGUE, 64)) {
             tcgen05_fence_after();
             if (ks > 1) acc_ready = true;
-            else if (p.staged_epilogue) epilogue_staged<MT>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, EPI_THREADS + td, nan_seen);
-            else epilogue_columns<MT>(p, tmem_acc, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, nan_seen);
+            else if (p.staged_epilogue) epilogue_staged<MT, ISO>(p, tmem_acc, x_tile0, BAR_EPI, abort_flag, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, EPI_THREADS + td, nan_seen);
+            else epilogue_columns<MT, ISO>(p, tmem_acc, q, lane, f0, m0, 1 + ((warp - DEQ_WARP0) >> 2), 1 + DEQ_WARPS / 4, nan_seen);
         }
     }
 
@@ -1368,12 +1370,13 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         }
         __syncwarp();
         cluster_sync_all();                                  // all partial tiles have arrived
-        if (warp >= EPI_WARP0 && acc_ready) split_reduce_store<MT>(p, x_tile0, ks, kz, f0, m0, tid - EPI_WARP0 * 32, nan_seen);
+        if (warp >= EPI_WARP0 && acc_ready) split_reduce_store<MT, ISO>(p, x_tile0, ks, kz, f0, m0, tid - EPI_WARP0 * 32, nan_seen);
     }
 
     // (tiles in shared memory have been read by now: its first bytes serve as scratch)
-    if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
-        isolate_tile(p, m0, min(m0 + uint32_t(MT), p.M), f0, min(f0 + uint32_t(FT), p.N), ks, kz, reinterpret_cast<uint16_t*>(smem_gen));
+    if constexpr (ISO)
+        if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
+            isolate_tile(p, m0, min(m0 + uint32_t(MT), p.M), f0, min(f0 + uint32_t(FT), p.N), ks, kz, reinterpret_cast<uint16_t*>(smem_gen));
 
     // ========================================= teardown ==========================================
     if (*abort_flag) {

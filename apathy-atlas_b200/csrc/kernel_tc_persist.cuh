@@ -106,7 +106,7 @@ struct PParams {
     uint32_t n_tiles;        // n_fpairs * n_passes
 };
 
-template <int MT, int G, bool A4>
+template <int MT, int G, bool A4, bool ISO = false>
 __global__ void __launch_bounds__(P_NUM_THREADS, 1)
 nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x,
                                        const __grid_constant__ CUtensorMap map_w,
@@ -537,7 +537,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         const uint32_t m = m_base + row;
                         if (m >= p.M) break;
                         const uint4 val = lds128(epi0 + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
-                        if (p.isolate) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
+                        if constexpr (ISO) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
                         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
                         for (uint32_t r = 0; r < p.n_dest; ++r) {
                             uint16_t* dst = p.y_dest[r] + at;
@@ -695,11 +695,12 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     }
 
     // (every stage and tile in shared memory has been read by now: its first bytes serve as scratch)
-    if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
-        for (uint32_t i = 0; i < my_tiles; ++i) {
-            const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * (MT * G);
-            isolate_tile(p, m0, min(m0 + uint32_t(MT * G), p.M), f0, min(f0 + uint32_t(FT), p.N), 1, 0, reinterpret_cast<uint16_t*>(smem_gen));
-        }
+    if constexpr (ISO)
+        if (p.isolate && __syncthreads_or(nan_seen & kNanBits))
+            for (uint32_t i = 0; i < my_tiles; ++i) {
+                const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * (MT * G);
+                isolate_tile(p, m0, min(m0 + uint32_t(MT * G), p.M), f0, min(f0 + uint32_t(FT), p.N), 1, 0, reinterpret_cast<uint16_t*>(smem_gen));
+            }
 
     // ========================================= teardown ==========================================
     if (*abort_flag) {
