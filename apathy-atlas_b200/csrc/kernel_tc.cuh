@@ -681,7 +681,7 @@ __device__ __forceinline__ void split_reduce_store(const Params& p, uint32_t rec
 // ISO: the form for calls with Params::isolate.
 // (The bound is wider than the launch: with it a thread gets 80 registers instead of 107.  The shrink runs beside this kernel, and
 //  at 107 only one of its CTAs found room on an SM instead of two: 140 -> 160 us for the fused QKV projections of 64 tokens with
-//  64 adapters.  Nothing spills but two values of the SROWS forms, outside the K loop.  Without the cap from 128 tokens on,
+//  64 adapters.  Only the paired FP4 form of 256 tokens spills, six words.  Without the cap from 128 tokens on,
 //  256 tokens x 17408 x 5120 gain 1 %, but 80 to 256 tokens of 128 adapters of rank 64 over 14336 x 4096 lose 2 to 4 %.)
 template <int MT, bool A4, bool PAIR, bool SROWS = false, bool ISO = SROWS>
 __global__ void __launch_bounds__(672, 1)
@@ -691,7 +691,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                             const __grid_constant__ CUtensorMap map_b,
                             const __grid_constant__ CUtensorMap map_xs,
                             const __grid_constant__ CUtensorMap map_t,
-                            const __grid_constant__ Params p) {
+                            const Params p) {
     using C = Cfg<MT, A4, PAIR>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;

@@ -114,7 +114,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                                        const __grid_constant__ CUtensorMap map_b,
                                        const __grid_constant__ CUtensorMap map_xs,
                                        const __grid_constant__ CUtensorMap map_t,
-                                       const __grid_constant__ Params p, const __grid_constant__ PParams pp) {
+                                       const Params p, const PParams pp) {
     using C = PCfg<MT, G, A4>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
