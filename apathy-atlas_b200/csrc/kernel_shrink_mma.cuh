@@ -67,9 +67,9 @@ lora_shrink_mma_kernel(ShrinkParams p) {
     float f = 1.0f;
     uint32_t rank = p.max_rank;
     bool hit[2];
+    int32_t routed[2] = {-1, -1};
     if (p.seq_slot) {
         // everything the routing decides on is requested before the first of it is looked at: one memory latency, not five
-        int32_t routed[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t m = m_base + h * SHM_THREADS + tid;
@@ -127,26 +127,21 @@ lora_shrink_mma_kernel(ShrinkParams p) {
     if (p.tile_out) {
         if (!any_live) return;                               // the pair is not in the tile's list (whole cluster leaves)
         if (krank == 0) {
-            // pairs ahead of this one: every granule of every valid slot below s that occurs in the tile
+            // pairs ahead of this one: every granule of every valid slot below s that occurs in the tile.  Each row reads its own
+            // slot's tables, all rows at once, and the first row of a slot counts it (slot by slot it was a chain of latencies)
             __shared__ uint32_t present[SHM_THREADS];        // one bit per slot, 32 * 128 = 4096 slots
             __shared__ uint32_t ahead[SHM_THREADS / 32];
             present[tid] = 0u;
             __syncthreads();
+            uint32_t cnt = 0;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t idx = h * SHM_THREADS + tid, m = m_base + idx;
-                if (idx < chunk && m < p.M) {
-                    const int32_t s2 = p.seq_slot[m];
-                    if (s2 >= 0 && uint32_t(s2) < s && p.a_table[s2] != 0ull && (!p.b_table || p.b_table[s2] != 0ull))
-                        atomicOr(&present[uint32_t(s2) >> 5], 1u << (uint32_t(s2) & 31u));
+                const int32_t s2 = routed[h];                // (-1 outside the chunk)
+                if (s2 >= 0 && uint32_t(s2) < s) {
+                    const uint64_t a2 = p.a_table[s2], b2 = p.b_table ? p.b_table[s2] : 1ull;
+                    const uint32_t r2 = p.rank_table ? min(p.rank_table[s2], p.max_rank) : p.max_rank, bit = 1u << (uint32_t(s2) & 31u);
+                    if (a2 != 0ull && b2 != 0ull && !(atomicOr(&present[uint32_t(s2) >> 5], bit) & bit)) cnt += (r2 + 15u) / 16u;
                 }
-            }
-            __syncthreads();
-            uint32_t cnt = 0;
-            for (uint32_t w = present[tid]; w; w &= w - 1) {
-                const uint32_t s2 = tid * 32 + (__ffs(w) - 1);
-                const uint32_t r2 = p.rank_table ? min(p.rank_table[s2], p.max_rank) : p.max_rank;
-                cnt += (r2 + 15u) / 16u;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xFFFFFFFFu, cnt, o);
