@@ -84,34 +84,52 @@ __device__ __forceinline__ uint32_t bf16x2_mul(uint32_t a, uint32_t b) {
     return d;
 }
 
-// E4M3 scale byte -> BF16x2 {f, f} with f = e4m3(byte) * 2^118.
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
+    return d;
+}
+
+// The expansion is bound by the integer pipe (shifts, logic and permutes issue at half rate), so positions are reached by
+// multiplications, which the FMA pipe does beside it: a nibble n in each half of a word, times 0x1040, has its sign at bit 15
+// (n << 12) and its three magnitude bits at bits 6 to 8 (n << 6), the BF16 exponent's last two and the mantissa's first:
+// value * 2^-126, subnormal included.
+constexpr uint32_t kE2m1At = 0x1040u, kE2m1Bits = 0x81C081C0u;
+
+// Four E4M3 scale bytes with NaN bytes (0x7F, 0xFF) replaced by zeros of their sign.
+__device__ __forceinline__ uint32_t e4m3x4_clear_nan(uint32_t w) {
+    const uint32_t nan = (((w & 0x7F7F7F7Fu) + 0x01010101u) & 0x80808080u) >> 7;
+    return w ^ (nan * 0x7Fu);
+}
+// Bytes i0 and i1 of `w` (no NaN), chosen by sel = i0 | 4 << 4 | i1 << 8 | 4 << 12, as BF16x2 multipliers {f, f} with f = e4m3 * 2^118.
 // (byte & 0x7F) << 4 read as BF16 is e4m3 * 2^-120 for normals and subnormals alike.
-__device__ __forceinline__ uint32_t e4m3_to_bf16x2_shifted(uint32_t byte) {
-    const uint32_t mag = byte & 0x7Fu;
-    uint32_t bits = (mag == 0x7Fu) ? 0u : (mag << 4);
-    bits |= (byte & 0x80u) << 8;
-    uint32_t v = bits | (bits << 16);
+__device__ __forceinline__ void e4m3x2_to_bf16x2_shifted(uint32_t w, uint32_t sel, uint32_t& f0, uint32_t& f1) {
+    const uint32_t b = prmt(w, 0u, sel);
+    uint32_t v = ((b * 0x10u) & 0x07F007F0u) | ((b * 0x100u) & 0x80008000u);
     v = bf16x2_mul(v, 0x7B807B80u);   // * 2^120 : exact E4M3 value
     v = bf16x2_mul(v, 0x7A807A80u);   // * 2^118
-    return v;
+    f0 = prmt(v, 0u, 0x1010u);
+    f1 = prmt(v, 0u, 0x3232u);
 }
 
 // Eight E2M1 codes (element i in bits [4i, 4i+4)) times a BF16x2 multiplier {f, f}
 // -> eight BF16 values in element order, as four BF16x2 words.
 // With f = scale * 2^118 each output is E2M1 * scale * 2^-8, exact in BF16 (<= 6 significant bits).
 __device__ __forceinline__ void e2m1x8_to_bf16x8(uint32_t p, uint32_t mul, uint32_t (&out)[4]) {
-    // pair i holds elements (i, i+4): sign to bit 15/31, 3 magnitude bits to bits 6..8 / 22..24
-    // (BF16 exponent lsbs + mantissa msb), i.e. value * 2^-126.
-    const uint32_t b0 = ((p << 12) & 0x80008000u) | ((p << 6) & 0x01C001C0u);
-    const uint32_t b1 = ((p << 8) & 0x80008000u) | ((p << 2) & 0x01C001C0u);
-    const uint32_t b2 = ((p << 4) & 0x80008000u) | ((p >> 2) & 0x01C001C0u);
-    const uint32_t b3 = (p & 0x80008000u) | ((p >> 6) & 0x01C001C0u);
-    const uint32_t h0 = bf16x2_mul(b0, mul), h1 = bf16x2_mul(b1, mul);
-    const uint32_t h2 = bf16x2_mul(b2, mul), h3 = bf16x2_mul(b3, mul);
-    out[0] = __byte_perm(h0, h1, 0x5410);   // (e0, e1)
-    out[1] = __byte_perm(h2, h3, 0x5410);   // (e2, e3)
-    out[2] = __byte_perm(h0, h1, 0x7632);   // (e4, e5)
-    out[3] = __byte_perm(h2, h3, 0x7632);   // (e6, e7)
+    const uint32_t even = p & 0x0F0F0F0Fu, odd = (p >> 4) & 0x0F0F0F0Fu;
+    // byte i of both, one to each half of a word; the bytes between are the (clear) sign bits of the same bytes
+    out[0] = bf16x2_mul((prmt(even, odd, 0xC480u) * kE2m1At) & kE2m1Bits, mul);
+    out[1] = bf16x2_mul((prmt(even, odd, 0xD591u) * kE2m1At) & kE2m1Bits, mul);
+    out[2] = bf16x2_mul((prmt(even, odd, 0xE6A2u) * kE2m1At) & kE2m1Bits, mul);
+    out[3] = bf16x2_mul((prmt(even, odd, 0xF7B3u) * kE2m1At) & kE2m1Bits, mul);
+}
+// The same without the order: words of the pairs (i, i + 4), which need no permutes.
+__device__ __forceinline__ void e2m1x8_to_pairs(uint32_t p, uint32_t mul, uint32_t (&h)[4]) {
+    const uint32_t q = p >> 8;
+    h[0] = bf16x2_mul(((p & 0x000F000Fu) * kE2m1At) & kE2m1Bits, mul);
+    h[1] = bf16x2_mul(((p & 0x00F000F0u) * (kE2m1At >> 4)) & kE2m1Bits, mul);
+    h[2] = bf16x2_mul(((q & 0x000F000Fu) * kE2m1At) & kE2m1Bits, mul);
+    h[3] = bf16x2_mul(((q & 0x00F000F0u) * (kE2m1At >> 4)) & kE2m1Bits, mul);
 }
 
 constexpr float kWeightPreScale = 256.0f;   // 2^8: weights enter the MMA as value * 2^-8

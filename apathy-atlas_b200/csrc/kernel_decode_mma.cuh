@@ -36,15 +36,6 @@ struct DecodeParams {
     uint32_t x_row_stride;
 };
 
-// Eight codes -> four BF16x2 words holding the pairs (i, i + 4), times the multiplier: e2m1x8_to_bf16x8 without its permutes.
-__device__ __forceinline__ void e2m1x8_to_pairs(uint32_t p, uint32_t mul, uint32_t (&h)[4]) {
-    const uint32_t q = p >> 8;
-    h[0] = bf16x2_mul(((p << 12) & 0x80008000u) | ((p << 6) & 0x01C001C0u), mul);
-    h[1] = bf16x2_mul(((p << 8) & 0x80008000u) | ((p << 2) & 0x01C001C0u), mul);
-    h[2] = bf16x2_mul(((p << 4) & 0x80008000u) | ((q << 6) & 0x01C001C0u), mul);
-    h[3] = bf16x2_mul((p & 0x80008000u) | ((q << 2) & 0x01C001C0u), mul);
-}
-
 template <int TILES, int NT>
 __global__ void __launch_bounds__(DCM_THREADS, 2)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
@@ -110,6 +101,11 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     };
     auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2], const uint4 (&xs)[X_AHEAD ? 4 : 1]) {
         const bool in = step * DCM_KSTEP + 32 * t < p.K;
+        uint32_t mul[TILES][2][2];
+#pragma unroll
+        for (int i = 0; i < TILES; ++i)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) e4m3x2_to_bf16x2_shifted(e4m3x4_clear_nan(s[i][h]), 0x4140u, mul[i][h][0], mul[i][h][1]);
 #pragma unroll
         for (int u = 0; u < 4; ++u) {                                           // eight K elements per thread at a time
             uint32_t xb[NT][4];
@@ -127,7 +123,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const uint32_t word = u == 0 ? c[i][h].x : (u == 1 ? c[i][h].y : (u == 2 ? c[i][h].z : c[i][h].w));
-                    e2m1x8_to_pairs(word, e4m3_to_bf16x2_shifted((s[i][h] >> (u < 2 ? 0 : 8)) & 0xFFu), a[h]);
+                    e2m1x8_to_pairs(word, mul[i][h][u < 2 ? 0 : 1], a[h]);
                 }
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {

@@ -1161,6 +1161,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 fetch_scales(ri + 2, sc_next[1]);
             }
 #pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) scw[j] = e4m3x4_clear_nan(scw[j]);
+#pragma unroll
             for (uint32_t jr = 0; jr < 4; jr += 2 * DEQ_GROUPS) {
                 if (ri * 4 + jr + grp >= num_kb) break;
                 const bool two = ri * 4 + jr + grp + DEQ_GROUPS < num_kb;
@@ -1172,9 +1174,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     const uint4 pk = lds128(rawp0 + rs * RAW_PACKED_BYTES + sw128_off(row, 2 * j + half));
                     const uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
                     const uint32_t scj = j == 0 ? scw[0] : (j == 1 ? scw[1] : (j == 2 ? scw[2] : scw[3]));
-                    const uint32_t sbytes = scj >> (16 * half);          // scale bytes 2*half, 2*half+1 of word j
-                    const uint32_t mul0 = e4m3_to_bf16x2_shifted(sbytes & 0xFFu);
-                    const uint32_t mul1 = e4m3_to_bf16x2_shifted((sbytes >> 8) & 0xFFu);
+                    uint32_t mul0, mul1;                                        // of scale bytes 2 * half, 2 * half + 1 of word j
+                    e4m3x2_to_bf16x2_shifted(scj, half ? 0x4342u : 0x4140u, mul0, mul1);
 #pragma unroll
                     for (uint32_t qd = 0; qd < 4; ++qd) {
                         uint32_t o4[4];

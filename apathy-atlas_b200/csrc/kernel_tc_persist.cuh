@@ -641,7 +641,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     ok = mbar_wait_timed(BAR_FULL_RAW + 8 * rs, rph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_raw);
                     if (!ok) break;
                     const uint4 sc4 = lds128(raws0 + rs * RAW_SCALE_BYTES + row * 16);
-                    const uint32_t scw[4] = {sc4.x, sc4.y, sc4.z, sc4.w};
+                    const uint32_t scw[4] = {e4m3x4_clear_nan(sc4.x), e4m3x4_clear_nan(sc4.y), e4m3x4_clear_nan(sc4.z), e4m3x4_clear_nan(sc4.w)};
 #pragma unroll
                     for (uint32_t jr = 0; jr < 4; jr += 2) {
                         uint32_t o[2][16];
@@ -651,9 +651,8 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                             const uint4 pk = lds128(rawp0 + rs * RAW_PACKED_BYTES + sw128_off(row, 2 * j + half));
                             const uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
                             const uint32_t scj = j == 0 ? scw[0] : (j == 1 ? scw[1] : (j == 2 ? scw[2] : scw[3]));
-                            const uint32_t sbytes = scj >> (16 * half);
-                            const uint32_t mul0 = e4m3_to_bf16x2_shifted(sbytes & 0xFFu);
-                            const uint32_t mul1 = e4m3_to_bf16x2_shifted((sbytes >> 8) & 0xFFu);
+                            uint32_t mul0, mul1;                                        // of scale bytes 2 * half, 2 * half + 1 of word j
+                            e4m3x2_to_bf16x2_shifted(scj, half ? 0x4342u : 0x4140u, mul0, mul1);
 #pragma unroll
                             for (uint32_t qd = 0; qd < 4; ++qd) {
                                 uint32_t o4[4];
