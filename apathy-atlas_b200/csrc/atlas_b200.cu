@@ -83,7 +83,7 @@ struct DeviceState {
     int persist_clusters[kPersistKernels] = {};
     bool carveout_set = false;
     bool shrink_tc_attr_set = false;
-    int shrink_tc_clusters = 0;       // resident clusters of SHT_MAX_KSPLIT CTAs of the prefill shrink; 0 = not asked yet
+    int shrink_tc_clusters[SHT_MAX_KSPLIT + 1] = {};   // resident clusters of that many CTAs of the prefill shrink; 0 = not asked yet
     bool push_attr_set = false;
     bool dense_attr_set[5] = {};      // token tiles 16, 32, 64, 128, 256 of the dense-BF16 kernel
 };
@@ -206,7 +206,7 @@ static bool shrink_takes_mma_path(const ShrinkParams& p) {
 // How many clusters of `ksplit` CTAs of the prefill shrink can be resident at once (they live inside one GPC: fewer than the SM
 // count suggests).  Asked once per device.
 static int shrink_tc_clusters(DeviceState& dst, uint32_t ksplit) {
-    if (dst.shrink_tc_clusters == 0) {
+    if (dst.shrink_tc_clusters[ksplit] == 0) {
         cudaLaunchConfig_t q{};
         q.gridDim = dim3(ksplit);
         q.blockDim = dim3(SHT_THREADS);
@@ -219,10 +219,10 @@ static int shrink_tc_clusters(DeviceState& dst, uint32_t ksplit) {
         q.attrs = attr;
         q.numAttrs = 1;
         int n = 0;
-        dst.shrink_tc_clusters = cudaOccupancyMaxActiveClusters(&n, lora_shrink_tc_kernel, &q) == cudaSuccess && n > 0 ? n : -1;
+        dst.shrink_tc_clusters[ksplit] = cudaOccupancyMaxActiveClusters(&n, lora_shrink_tc_kernel, &q) == cudaSuccess && n > 0 ? n : -1;
         (void)cudaGetLastError();
     }
-    return dst.shrink_tc_clusters;
+    return dst.shrink_tc_clusters[ksplit];
 }
 
 static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool release_dependents = false,
@@ -267,13 +267,15 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         if (p.m_begin % 64 != 0 || p.m_begin >= p.M) return ATLAS_B200_ERR_DIMS;
         if (p.tile_out && p.chunk && p.chunk < uint32_t(SHT_ROWS)) return ATLAS_B200_ERR_DIMS;   // a cluster's rows lie in at most two token tiles
         const uint32_t rows = p.m_count ? std::min(p.m_count, p.M - p.m_begin) : p.M - p.m_begin;
-        // CTAs per 128 rows, each contracting a share of K: two, or four where the clusters of the batch (the whole of it, not this
-        // launch's range: a row's result must not depend on how the batch is cut into launches) are all resident at once — a
-        // second wave costs more than the split gains.  Two / four CTAs, eight adapters of rank 64: 1237 tokens, K = 4096 41 / 32 us,
-        // K = 14336 95 / 60 us; 4096 tokens 25 / 20 and 61 / 39 us; but 4352 tokens (34 clusters) 29 / 36 and 70 / 74 us.
+        // CTAs per 128 rows, each contracting a share of K: two, or four or eight where the clusters of the batch (the whole of it, not
+        // this launch's range: a row's result must not depend on how the batch is cut into launches) are all resident at once — a
+        // second wave costs more than the split gains (4352 tokens, 34 clusters of four: 36 instead of 29 us).  Two / four / eight CTAs,
+        // eight adapters of rank 64: 1237 tokens, K = 4096 34 / 25 / 22 us, K = 14336 81 / 48 / 34 us; 4096 tokens 29 / 22 and 68 / 43 us.
         const uint32_t k_blocks = p.k_in / SHT_KSTAGE, row_groups = (p.M + SHT_ROWS - 1) / SHT_ROWS;
-        const bool four = k_blocks >= 8 && int(row_groups) <= shrink_tc_clusters(*dst, SHT_MAX_KSPLIT);
-        p.ksplit = four ? uint32_t(SHT_MAX_KSPLIT) : (k_blocks >= 2 ? 2u : 1u);
+        p.ksplit = k_blocks >= 2 ? 2u : 1u;
+        for (uint32_t ks = SHT_MAX_KSPLIT; ks > 2; ks >>= 1)
+            if (k_blocks >= 2 * ks && int(row_groups) <= shrink_tc_clusters(*dst, ks)) { p.ksplit = ks; break; }
+        p.release_dependents = 1u;
         const uint32_t n_ctas = p.ksplit * ((rows + SHT_ROWS - 1) / SHT_ROWS);
         p.profile = (g_profile_buf && size_t(n_ctas) * 16 <= g_profile_words) ? g_profile_buf : nullptr;
         cudaLaunchConfig_t cfg = {};

@@ -32,8 +32,8 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 // then start early and has to wait until everything before it in the stream has completed and is visible.
 //   launched as dependents     both tensor-core shrinks, the main kernel behind a shrink, the tensor-core expand, the dense linear,
 //                              the QKV consumers, SwiGLU in both forms, the quantiser
-//   releasing                  all of these but the shrinks: lora_shrink_tc_kernel never does, the mma.sync one and
-//                              lora_shrink_grouped_kernel only in front of a main kernel
+//   releasing                  all of these but lora_shrink_mma_kernel and lora_shrink_grouped_kernel, which do so only in front of a
+//                              main kernel
 //   neither                    a main kernel without adapters releases but is launched in order; the NVFP4 decode, the maximum, the
 //                              CUDA-core linear and expand do neither
 // A dependent begins with the wait.  Only the main kernel reads anything ahead of it (x, weights, routing), and it follows a shrink
