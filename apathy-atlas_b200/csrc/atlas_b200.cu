@@ -475,8 +475,10 @@ struct TTiles {
 // tile, `l_gran_t` = bytes of one masked-t block as the shrink writes it ([part_rows x 16] BF16).
 struct TcMaps { CUtensorMap x, w, s, b, xs, t; };
 
+// `a4_scale_row` = scale bytes per row of a stage (FP4 activations).
 static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xrows, uint32_t mt, uint32_t l_gran_t,
-                          const TTiles& tt, TcMaps& m) {
+                          const TTiles& tt, TcMaps& m, uint32_t a4_scale_row = tc::KRAW / 16) {
+    const CUtensorMapSwizzle scale_swizzle = a4_scale_row == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE;
     if (a4) {
         // the quantised activations in `ws`, in the weights' own layout
         const uint8_t* codes = static_cast<const uint8_t*>(d.ws);
@@ -484,7 +486,7 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
                        CU_TENSOR_MAP_SWIZZLE_128B))
             return ATLAS_B200_ERR_DIMS;
         if (!encode_2d(&m.xs, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes + act_fp4_codes_bytes(d), d.k / 16, d.m, d.k / 16,
-                       tc::KRAW / 16, mt, CU_TENSOR_MAP_SWIZZLE_NONE))
+                       a4_scale_row, mt, scale_swizzle))
             return ATLAS_B200_ERR_DIMS;
     } else if (!encode_2d(&m.x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, d.x, d.k, d.m, uint64_t(d.x_row_stride) * 2, tc::KB, xrows,
                           CU_TENSOR_MAP_SWIZZLE_128B))
@@ -493,8 +495,8 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
                    CU_TENSOR_MAP_SWIZZLE_128B))
         return ATLAS_B200_ERR_DIMS;
     if (d.k % tc::KRAW != 0) m.s = m.w;      // scale rows of K/16 bytes: read by the expansion warps (Params::w_scale_rows)
-    else if (!encode_2d(&m.s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, tc::KRAW / 16, tc::FT,
-                        CU_TENSOR_MAP_SWIZZLE_NONE))
+    else if (!encode_2d(&m.s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, a4 ? a4_scale_row : tc::KRAW / 16, tc::FT,
+                        a4 ? scale_swizzle : CU_TENSOR_MAP_SWIZZLE_NONE))
         return ATLAS_B200_ERR_DIMS;
 
     // B side of the adapter pool as one 3-D tensor [max_loras][n][max_rank]: box = one granule of one slot
@@ -748,7 +750,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     if (clusters <= 0) return ATLAS_B200_ERR_DIMS;
     TcMaps maps;
     {
-        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps);
+        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, tc::A4_SCALE_ROW);
         if (rc) return rc;
     }
     tc::Params p{};

@@ -517,6 +517,10 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 // byte offset of logical 16-byte chunk `c` (0..7) of row `r` in a SWIZZLE_128B tile of 128-byte rows
 __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
 
+// FP4 activations: the K block with which a pair of feature tiles starts, so that pairs running at one moment do not all pull the
+// same activation lines.  In units of four; two share a stage of scales in the persistent kernel.
+__device__ __forceinline__ uint32_t a4_rotation(uint32_t fpair, uint32_t num_kb) { return num_kb % 4u == 0u && num_kb ? 4u * (fpair % (num_kb / 4u)) : 0u; }
+
 // ---------------------------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------------------------
@@ -802,7 +806,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (lane == 0 && A4) {
             // One ring: a stage's two packed operand tiles complete FULL[s] (which the MMA thread waits
             // on), its two scale-byte tiles FULL_RAW[s] (which the warps that move them to TMEM wait on).
-            const uint32_t rot = (blockIdx.x / CTAS) % num_kb;     // (the CTAs of a pair walk K in the same order)
+            const uint32_t rot = a4_rotation(blockIdx.x / CTAS, num_kb);      // (the CTAs of a pair walk K in the same order)
             uint32_t s = 0, ph = 0;
             for (uint32_t it = 0; it < num_kb; ++it) {
                 if (!mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32)) break;

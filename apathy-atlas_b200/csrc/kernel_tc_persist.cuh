@@ -52,6 +52,12 @@ constexpr int P_EPI_WARP1 = 15;         // second group of four drain / store wa
 constexpr int P_EPI_WARPS = 8;
 constexpr int P_EPI_THREADS = 32 * P_EPI_WARPS;
 
+// FP4 activations: bytes of a row of block scales in a stage of them, which serves two K blocks.  A TMA copy costs about 1.5 cycles
+// per ROW of its box, however short: fetched K block by K block the scales (384 rows of 16 bytes) took longer than the codes (256
+// rows of 128 bytes) and both together longer than the MMAs: 8192 tokens x 14336 x 4096 took 372 thousand cycles, 333 with two blocks at
+// a time (four, with a stage of codes less for them in shared memory: 347).
+constexpr int A4_SCALE_ROW = 32, A4_SCALE_BLOCKS = A4_SCALE_ROW * 16 / KRAW;
+
 template <int MT, int G, bool A4> struct PCfg {
     static_assert(MT % 64 == 0 && MT >= 128 && MT <= 256, "token tile of a pass");
     static_assert(!A4 || G == 1, "FP4 activations: one token tile per pass");
@@ -60,9 +66,9 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int X_STAGE_BYTES = G * X_TILE_BYTES;
     static constexpr int S4_W = 0;
     static constexpr int S4_X = S4_W + RAW_PACKED_BYTES;
-    static constexpr int S4_WS = S4_X + XROWS * 128;
-    static constexpr int S4_XS = S4_WS + RAW_SCALE_BYTES;
-    static constexpr int S4_BYTES = ((S4_XS + MT * 16) + 1023) / 1024 * 1024;
+    static constexpr int S4_BYTES = S4_X + XROWS * 128;
+    // A4: the block scales of two K blocks at a time, rows of 32 bytes (SWIZZLE_32B): W [128 x 32 B] | x [MT x 32 B]
+    static constexpr int S4_SCALES = (FT + MT) * A4_SCALE_ROW;
     static constexpr int A_COLS = KB / 2;
     static constexpr int XSF_BLOCKS = MT > 128 ? MT / 128 : 1;
     static constexpr int SF_COLS = 16 + 16 * XSF_BLOCKS;
@@ -75,7 +81,7 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int L_STAGES = EPI_BYTES / L_STAGE > 16 ? 16 : EPI_BYTES / L_STAGE;
     // ring depths: what the 227 KB of shared memory and the 512 columns of tensor memory leave
     static constexpr int STAGES = A4 ? 4 : (G == 1 ? 6 : 3);
-    static constexpr int RAW_STAGES = A4 ? STAGES : (G == 1 ? 3 : 2);
+    static constexpr int RAW_STAGES = G == 1 && !A4 ? 3 : 2;             // (A4: of block scales)
     static constexpr int TMEM_A_BASE = ACC_COLS;
     static constexpr int TMEM_NEEDED = TMEM_A_BASE + (A4 ? STAGES * SF_COLS : STAGES * A_COLS);
     static constexpr int TMEM_COLS = 512;
@@ -83,7 +89,8 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int OFF_X = 0;
     static constexpr int OFF_RAWP = OFF_X + STAGES * X_STAGE_BYTES;
     static constexpr int OFF_RAWS = OFF_RAWP + RAW_STAGES * RAW_PACKED_BYTES;
-    static constexpr int OFF_EPI = A4 ? STAGES * S4_BYTES : OFF_RAWS + RAW_STAGES * RAW_SCALE_BYTES;
+    static constexpr int OFF_SCALES = STAGES * S4_BYTES;
+    static constexpr int OFF_EPI = A4 ? OFF_SCALES + RAW_STAGES * S4_SCALES : OFF_RAWS + RAW_STAGES * RAW_SCALE_BYTES;
     static constexpr int OFF_SLOT = OFF_EPI + EPI_BYTES;                          // int32[MT]  (scratch of the list build)
     static constexpr int OFF_GRAN = OFF_SLOT + MT * 4;                            // uint16[G][MAX_GRANULES]
     static constexpr int OFF_BITMAP = OFF_GRAN + G * MAX_GRANULES * 2;            // uint32[128]
@@ -220,19 +227,16 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             uint32_t s = 0, ph = 0;
             for (uint32_t i = 0; i < my_tiles; ++i) {
                 const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * MT;
-                const uint32_t rot = tile_fpair(i) % num_kb;
+                uint32_t kk = a4_rotation(tile_fpair(i), num_kb);
                 bool ok = true;
                 for (uint32_t it = 0; it < num_kb; ++it) {
                     ok = mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
                     if (!ok) break;
                     const uint32_t st = smem_base + s * C::S4_BYTES;
-                    const uint32_t kk = (it + rot) % num_kb;
-                    mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * s, RAW_SCALE_BYTES + MT * 16);
-                    tma_load_2d(st + C::S4_WS, &map_s, int32_t(kk * (KRAW / 16)), int32_t(f0), BAR_FULL_RAW + 8 * s);
-                    tma_load_2d(st + C::S4_XS, &map_xs, int32_t(kk * (KRAW / 16)), int32_t(m0), BAR_FULL_RAW + 8 * s);
                     if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, 2 * (RAW_PACKED_BYTES + C::XROWS * 128));
                     tma_load_2d_pair(st + C::S4_W, &map_w, int32_t(kk * (KRAW / 2)), int32_t(f0), full_at_leader + 8 * s);
                     tma_load_2d_pair(st + C::S4_X, &map_x, int32_t(kk * (KRAW / 2)), int32_t(m0 + cta_rank * C::XROWS), full_at_leader + 8 * s);
+                    if (++kk == num_kb) kk = 0;
                     if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
@@ -261,6 +265,26 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     } else if (warp == P_RAW_WARP) {
         // ===================================== TMA producer, raw weight stages ===============================
         // (one per four K blocks; a thread of its own, see nvfp4_lora_linear_tc_kernel)
+        if (lane == 0 && A4) {
+            // block scales of both operands, two K blocks to a stage (zero-filled past K)
+            const uint32_t n_ss = (num_kb + A4_SCALE_BLOCKS - 1u) / A4_SCALE_BLOCKS;
+            uint32_t rs = 0, rph = 0;
+            bool ok = true;
+            for (uint32_t i = 0; ok && i < my_tiles; ++i) {
+                const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT, m0 = tile_pass(i) * MT;
+                uint32_t ss = a4_rotation(tile_fpair(i), num_kb) / A4_SCALE_BLOCKS;
+                for (uint32_t si = 0; si < n_ss; ++si) {
+                    ok = mbar_wait(BAR_EMPTY_RAW + 8 * rs, rph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 64);
+                    if (!ok) break;
+                    const uint32_t st = smem_base + C::OFF_SCALES + rs * C::S4_SCALES;
+                    mbar_arrive_expect_tx(BAR_FULL_RAW + 8 * rs, C::S4_SCALES);
+                    tma_load_2d(st, &map_s, int32_t(ss * A4_SCALE_ROW), int32_t(f0), BAR_FULL_RAW + 8 * rs);
+                    tma_load_2d(st + FT * A4_SCALE_ROW, &map_xs, int32_t(ss * A4_SCALE_ROW), int32_t(m0), BAR_FULL_RAW + 8 * rs);
+                    if (++ss == n_ss) ss = 0;
+                    if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
+                }
+            }
+        }
         if (lane == 0 && !A4) {
             uint32_t rs = 0, rph = 0;
             bool ok = true;
@@ -578,22 +602,23 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
         uint32_t s = 0, ph = 0, rs = 0, rph = 0;
         if constexpr (A4) {
             uint32_t itg = 0;                                 // K blocks since kernel start: the halves take alternate ones
+            const uint32_t swz = (lane >> 2) & 1u;            // of rows lane, lane + 32, ... in a SWIZZLE_32B tile of 32-byte rows
             for (uint32_t i = 0; ok && i < my_tiles; ++i) {
                 for (uint32_t it = 0; ok && it < num_kb; ++it, ++itg) {
-                    if ((itg & 1u) != half) {
-                        if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
-                        continue;
+                    const uint32_t j = it % A4_SCALE_BLOCKS;
+                    // (every warp waits for every stage of scales, whether it takes a block of it or not: what it releases below it has seen full)
+                    if (j == 0u) {
+                        ok = mbar_wait_timed(BAR_FULL_RAW + 8 * rs, rph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_raw);
+                        if (!ok) break;
                     }
-                    ok = mbar_wait_timed(BAR_FULL_RAW + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_raw);
-                    if (!ok) break;
-                    const uint32_t st = smem_base + s * C::S4_BYTES;
-                    const uint32_t sf = tmem_a0 + lane_base + s * C::SF_COLS;
-                    {
+                    if ((itg & 1u) == half) {
+                        const uint32_t st = smem_base + C::OFF_SCALES + rs * C::S4_SCALES + lane * A4_SCALE_ROW + ((j ^ swz) << 4);
+                        const uint32_t sf = tmem_a0 + lane_base + s * C::SF_COLS;
                         uint32_t r[16];
                         uint32_t neg = 0;
 #pragma unroll
                         for (uint32_t c = 0; c < 4; ++c) {
-                            const uint4 v = lds128(st + C::S4_WS + (lane + 32 * c) * 16);
+                            const uint4 v = lds128(st + 32 * c * A4_SCALE_ROW);
                             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                             for (uint32_t u = 0; u < 4; ++u) {
@@ -603,35 +628,37 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                             }
                         }
                         if (neg & 0x80808080u) record_status(STATUS_NEGATIVE_SCALE);
+                        ok = mbar_wait_timed(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
+                        if (!ok) break;
+                        tcgen05_fence_after();
                         tmem_st16(sf, r);
-                    }
-                    if constexpr (C::XSF_BLOCKS == 1) {
-                        uint32_t r[16];
+                        const uint32_t xst = st + FT * A4_SCALE_ROW;
+                        uint32_t rx[C::XSF_BLOCKS][16];       // one block of 128 tokens: column = 4 u + c; two: 8 u + 4 blk + c
+                        static_assert(C::XSF_BLOCKS <= 2, "token tiles of at most 256");
 #pragma unroll
-                        for (uint32_t c = 0; c < 4; ++c) {
-                            const uint32_t xr = lane + 32 * c;
-                            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                            if (xr < uint32_t(MT)) v = lds128(st + C::S4_XS + xr * 16);
-                            r[c] = v.x; r[4 + c] = v.y; r[8 + c] = v.z; r[12 + c] = v.w;
-                        }
-                        tmem_st16(sf + 16, r);
-                    } else {
-                        uint32_t r0[16], r1[16];
-#pragma unroll
-                        for (uint32_t blk = 0; blk < 2; ++blk)
+                        for (uint32_t blk = 0; blk < uint32_t(C::XSF_BLOCKS); ++blk)
 #pragma unroll
                             for (uint32_t c = 0; c < 4; ++c) {
-                                const uint4 v = lds128(st + C::S4_XS + (128 * blk + 32 * c + lane) * 16);
-                                r0[4 * blk + c] = v.x; r0[8 + 4 * blk + c] = v.y;
-                                r1[4 * blk + c] = v.z; r1[8 + 4 * blk + c] = v.w;
+                                const uint4 v = lds128(xst + (128 * blk + 32 * c) * A4_SCALE_ROW);
+                                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                                for (uint32_t u = 0; u < 4; ++u) {
+                                    const uint32_t col = u * 4 * C::XSF_BLOCKS + 4 * blk + c;
+                                    rx[col / 16][col % 16] = w[u];
+                                }
                             }
-                        tmem_st16(sf + 16, r0);
-                        tmem_st16(sf + 32, r1);
+#pragma unroll
+                        for (uint32_t blk = 0; blk < uint32_t(C::XSF_BLOCKS); ++blk) tmem_st16(sf + 16 + 16 * blk, rx[blk]);
+                        tmem_st_wait();
+                        tcgen05_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(full_at_leader + 8 * s);
                     }
-                    tmem_st_wait();
-                    tcgen05_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive_cluster(full_at_leader + 8 * s);
+                    if (j == A4_SCALE_BLOCKS - 1u || it + 1u == num_kb) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(BAR_EMPTY_RAW + 8 * rs);
+                        if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
+                    }
                     if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                 }
             }
