@@ -474,6 +474,34 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
 }
+// 16 lanes x 8 N columns in the fragment layout of an 8 x 8 matrix store: registers 4 k and 4 k + 1 of lane i are columns 8 k + 2 (i % 4)
+// and the next one of TMEM lane i / 4, registers 4 k + 2 and 4 k + 3 the same of lane i / 4 + 8.
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr) : "memory");
+}
+// Four 8 x 8 matrices of 16-bit elements, transposed: lane 8 m + j gives the address of 16 bytes that receive column j of matrix m.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// Accumulator columns (tokens) into the [token][128 features] BF16 tile of an epilogue: sixteen tokens of sixteen of this warp's 32
+// features from two fragments at v.  The tile's 16-byte chunks are permuted by the token's last three bits, which keeps both these
+// stores and the row reads free of bank conflicts (tile_chunk).  Going through transposing matrix stores instead of lane exchanges
+// and 4-byte stores takes a quarter of the shared-memory instructions; the drain is what the tensor pipe waits for between passes.
+__device__ __forceinline__ uint32_t tile_chunk(uint32_t token, uint32_t chunk) { return token * 256u + ((chunk ^ (token & 7u)) << 4); }
+__device__ __forceinline__ void store_fragments(uint32_t tile, uint32_t token0, uint32_t feature_chunk0, uint32_t lane, const uint32_t* v, float osc) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = pack_bf16x2(__uint_as_float(v[2 * i]) * osc, __uint_as_float(v[2 * i + 1]) * osc);
+    stmatrix_x4_trans(tile + tile_chunk(token0 + 8u * (lane >> 4) + (lane & 7u), feature_chunk0 + ((lane >> 3) & 1u)), w[0], w[1], w[2], w[3]);
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) {
@@ -570,8 +598,7 @@ __device__ __forceinline__ void epilogue_columns(const Params& p, uint32_t tmem_
 // their scale bytes; map_b: the strided adapter pool's B side; map_xs: A4 only, activation scale bytes [M, K/16];
 // map_t: the shrink's masked-t blocks as rows of 256 bytes, when p.t_tile_cap != 0.
 // Epilogue through shared memory: the warps first lay the tile down as [token][128 features] BF16 (256-byte
-// rows; the 16-byte chunks of odd rows rotated by four so that the two rows a store instruction touches
-// fall into different banks), meet on an mbarrier, then copy whole rows out with 16-byte stores — to every
+// rows, see store_fragments), meet on an mbarrier, then copy whole rows out with 16-byte stores — to every
 // destination buffer in turn.  `e_tid` = 0 .. 32 * EPI_WARPS - 1 numbers the participating threads.
 // Requires 16-byte aligned destination rows (checked by the caller); returns false if the wait expired.
 template <int MT, bool ISO>
@@ -579,23 +606,14 @@ __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_a
                                                 volatile uint32_t* abort_flag, uint32_t q, uint32_t lane, uint32_t f0,
                                                 uint32_t m0, uint32_t part, uint32_t nparts, uint32_t e_tid, uint32_t& nan_seen) {
     const float osc = p.out_scale;
-    const bool odd = lane & 1u;
-    const uint32_t fe = (q * 32u + lane) & ~1u;                  // even feature of this lane pair, within the tile
 #pragma unroll 1
     for (uint32_t c0 = part * 16; c0 < uint32_t(MT); c0 += nparts * 16) {
-        uint32_t v[16];
-        tmem_ld16(tmem_acc + ((q * 32u) << 16) + c0, v);
+        uint32_t v[2][8];
+#pragma unroll
+        for (uint32_t h = 0; h < 2; ++h) tmem_ld_frag(tmem_acc + ((q * 32u + 16u * h) << 16) + c0, v[h]);
         tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float a = __uint_as_float(v[2 * i]) * osc, b = __uint_as_float(v[2 * i + 1]) * osc;
-            const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? a : b, 1);
-            // even lane: token 2i, features (fe, fe+1); odd lane: token 2i+1, the same two features
-            const uint32_t row = c0 + 2 * i + (odd ? 1u : 0u);
-            const uint32_t w = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);
-            const uint32_t chunk = (fe >> 3) ^ ((row & 1u) << 2);
-            asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + row * 256u + chunk * 16u + (fe & 7u) * 2u), "r"(w) : "memory");
-        }
+        for (uint32_t h = 0; h < 2; ++h) store_fragments(tile, c0, q * 4u + 2u * h, lane, v[h], osc);
     }
     __syncwarp();
     if (lane == 0) mbar_arrive(bar_epi);
@@ -608,7 +626,7 @@ __device__ __forceinline__ bool epilogue_staged(const Params& p, uint32_t tmem_a
     for (uint32_t row = e_tid >> 4; row < uint32_t(MT); row += (32u * EPI_WARPS) >> 4) {
         const uint32_t m = m0 + row;
         if (m >= p.M) break;
-        const uint4 val = lds128(tile + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
+        const uint4 val = lds128(tile + tile_chunk(row, j));
         if constexpr (ISO) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
         for (uint32_t r = 0; r < p.n_dest; ++r) {

@@ -493,8 +493,6 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             if (ok && te == 0) mbar_arrive(BAR_LIST);
         }
         const float osc = p.out_scale;
-        const bool odd = lane & 1u;
-        const uint32_t fe = (q * 32u + lane) & ~1u;
         for (uint32_t i = 0; ok && i < my_tiles; ++i) {
             const uint32_t f0 = (tile_fpair(i) * 2u + cta_rank) * FT;
             // the next pass's routing entries travel while this pass's accumulators complete
@@ -517,29 +515,22 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 // loads are issued before the current block is converted and stored, so their latency is not exposed.
                 constexpr uint32_t N_BLK = uint32_t(MT) / 64u;
                 const uint32_t t_col0 = tmem_acc + ((q * 32u) << 16) + g * MT + grp * 32u;
-                uint32_t v[2][2][16];
-                tmem_ld16(t_col0, v[0][0]);
-                tmem_ld16(t_col0 + 16, v[0][1]);
+                uint32_t v[2][2][16];                         // [buffer][features 0-15, 16-31 of the quadrant][fragments of 32 tokens]
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) tmem_ld_frag(t_col0 + ((16u * h) << 16), v[0][h]);
                 tmem_ld_wait();
 #pragma unroll
                 for (uint32_t blk = 0; blk < N_BLK; ++blk) {
                     const uint32_t cur = blk & 1u;
                     if (blk + 1 < N_BLK) {
-                        tmem_ld16(t_col0 + 64 * (blk + 1), v[cur ^ 1u][0]);
-                        tmem_ld16(t_col0 + 64 * (blk + 1) + 16, v[cur ^ 1u][1]);
+#pragma unroll
+                        for (uint32_t h = 0; h < 2; ++h) tmem_ld_frag(t_col0 + 64 * (blk + 1) + ((16u * h) << 16), v[cur ^ 1u][h]);
                     }
                     const uint32_t c0 = grp * 32 + 64 * blk;
 #pragma unroll
-                    for (int h = 0; h < 2; ++h)
+                    for (uint32_t h = 0; h < 2; ++h)
 #pragma unroll
-                        for (int u = 0; u < 8; ++u) {
-                            const float a = __uint_as_float(v[cur][h][2 * u]) * osc, b = __uint_as_float(v[cur][h][2 * u + 1]) * osc;
-                            const float got = __shfl_xor_sync(0xFFFFFFFFu, odd ? a : b, 1);
-                            const uint32_t row = c0 + 16 * h + 2 * u + (odd ? 1u : 0u);
-                            const uint32_t w = odd ? pack_bf16x2(got, b) : pack_bf16x2(a, got);
-                            const uint32_t chunk = (fe >> 3) ^ ((row & 1u) << 2);
-                            asm volatile("st.shared.b32 [%0], %1;" ::"r"(tile + row * 256u + chunk * 16u + (fe & 7u) * 2u), "r"(w) : "memory");
-                        }
+                        for (uint32_t u = 0; u < 2; ++u) store_fragments(tile, c0 + 16 * u, q * 4u + 2u * h, lane, v[cur][h] + 8 * u, osc);
                     if (blk + 1 < N_BLK) tmem_ld_wait();
                 }
                 tcgen05_fence_before();
@@ -560,7 +551,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     for (uint32_t row = te >> 4; row < uint32_t(MT * G); row += P_EPI_THREADS >> 4) {
                         const uint32_t m = m_base + row;
                         if (m >= p.M) break;
-                        const uint4 val = lds128(epi0 + row * 256u + ((j ^ ((row & 1u) << 2)) << 4));
+                        const uint4 val = lds128(epi0 + tile_chunk(row, j));
                         if constexpr (ISO) nan_seen |= bf16x2_nan_bits(val.x) | bf16x2_nan_bits(val.y) | bf16x2_nan_bits(val.z) | bf16x2_nan_bits(val.w);
                         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
                         for (uint32_t r = 0; r < p.n_dest; ++r) {
