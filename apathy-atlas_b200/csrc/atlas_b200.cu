@@ -475,9 +475,9 @@ struct TTiles {
 // tile, `l_gran_t` = bytes of one masked-t block as the shrink writes it ([part_rows x 16] BF16).
 struct TcMaps { CUtensorMap x, w, s, b, xs, t; };
 
-// `a4_scale_row` = scale bytes per row of a stage (FP4 activations).
+// `a4_scale_row` = scale bytes per row of a stage (FP4 activations), `lora_wide` = granules of B_s per copy.
 static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xrows, uint32_t mt, uint32_t l_gran_t,
-                          const TTiles& tt, TcMaps& m, uint32_t a4_scale_row = tc::KRAW / 16) {
+                          const TTiles& tt, TcMaps& m, uint32_t a4_scale_row = tc::KRAW / 16, uint32_t lora_wide = 1) {
     const CUtensorMapSwizzle scale_swizzle = a4_scale_row == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE;
     if (a4) {
         // the quantised activations in `ws`, in the weights' own layout
@@ -499,12 +499,13 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
                         a4 ? scale_swizzle : CU_TENSOR_MAP_SWIZZLE_NONE))
         return ATLAS_B200_ERR_DIMS;
 
-    // B side of the adapter pool as one 3-D tensor [max_loras][n][max_rank]: box = one granule of one slot
+    // B side of the adapter pool as one 3-D tensor [max_loras][n][max_rank]: box = some granules of one slot
     if (b_pool_is_strided(d)) {
         const uint64_t dims[3] = {d.max_rank, d.n, d.max_loras};
         const uint64_t strides[2] = {uint64_t(d.max_rank) * 2, uint64_t(d.b_slot_stride)};
-        const uint32_t box[3] = {16, tc::FT, 1};
-        if (!encode_tiled(&m.b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d.b_pool_base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_32B))
+        const uint32_t box[3] = {16 * lora_wide, tc::FT, 1};
+        if (!encode_tiled(&m.b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d.b_pool_base, dims, strides, box,
+                          lora_wide == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : (lora_wide == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B)))
             return ATLAS_B200_ERR_DIMS;
     } else {
         m.b = m.s;   // never dereferenced
@@ -748,9 +749,13 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     using C = tc::PCfg<MT, G, A4>;
     const int clusters = persist_resident_clusters<MT, G, A4, ISO>(idx);
     if (clusters <= 0) return ATLAS_B200_ERR_DIMS;
+    // Granules of B_s per copy: a copy of 128 rows takes as long for one granule as for four.  Two in the ring of a one-tile BF16
+    // pass, which holds only two stages of four, and slots of lower rank leave part of a stage unused (thousand cycles, two / four:
+    // ranks 8 to 64, 1237 tokens x 14336 x 4096 162.8 / 165.1; FP4, rank 64, 8192 tokens 376 / 362).
+    const uint32_t lora_wide = d.max_rank % 64 == 0 && (A4 || G == 2) ? 4u : (d.max_rank % 32 == 0 ? 2u : 1u);
     TcMaps maps;
     {
-        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, tc::A4_SCALE_ROW);
+        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, tc::A4_SCALE_ROW, lora_wide);
         if (rc) return rc;
     }
     tc::Params p{};
@@ -763,6 +768,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     pp.n_fpairs = ((d.n + tc::FT - 1) / tc::FT + 1) / 2;
     pp.n_passes = (d.m + MT * G - 1) / (MT * G);
     pp.n_tiles = pp.n_fpairs * pp.n_passes;
+    pp.lora_wide = d.seq_slot ? lora_wide : 1u;
     const uint32_t pairs = std::min<uint32_t>(uint32_t(clusters), pp.n_tiles);
     t_last_shape[0] = MT; t_last_shape[1] = 1u; t_last_shape[2] = 1u; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs;

@@ -519,6 +519,11 @@ __device__ __forceinline__ uint64_t make_kmajor_sw32_desc(uint32_t smem_addr) {
     return uint64_t((smem_addr & 0x3FFFFu) >> 4) | (uint64_t(1) << 16) | (uint64_t(256 >> 4) << 32) |
            (uint64_t(1) << 46) | (uint64_t(6) << 61);
 }
+// K-major operand tile of 16 n BF16 (n = 1, 2, 4: rows of 32, 64, 128 bytes, swizzled over their own width)
+__device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr, uint32_t n) {
+    return uint64_t((smem_addr & 0x3FFFFu) >> 4) | (uint64_t(1) << 16) | (uint64_t(n * 256u >> 4) << 32) | (uint64_t(1) << 46) |
+           (uint64_t(n == 4u ? 2u : (n == 2u ? 4u : 6u)) << 61);
+}
 // byte offset of 16-byte chunk `c` (0..1) of row `r` in a SWIZZLE_32B tile of 32-byte rows
 __device__ __forceinline__ uint32_t sw32_off(uint32_t r, uint32_t c) { return r * 32u + ((c ^ ((r >> 2) & 1u)) << 4); }
 // kind::f16 instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128, N = n.

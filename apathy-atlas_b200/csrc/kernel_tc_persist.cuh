@@ -9,8 +9,9 @@
 //   * the operand rings (activation tiles, raw weight stages, the expanded weight operand in tensor memory)
 //     run straight across tile boundaries: while tile i's last K blocks are multiplied, tile i+1's first
 //     stages are already fetched and expanded;
-//   * the LoRA K-steps have their own ring of (B_s tile, masked-t tile) stages, fetched by their own producer
-//     thread while the base K loop runs, so they are issued back to back after the last base block;
+//   * the LoRA K-steps have their own ring of (B_s tile, masked-t tiles) stages, fetched by their own producer
+//     thread while the base K loop runs, so they are issued back to back after the last base block.  B_s comes up to
+//     four granules of a slot at a time: a TMA copy costs cycles per row of its box, 128 here, however short the rows;
 //   * the epilogue is split: four warps first move the accumulator out of tensor memory into a shared-memory
 //     tile (BF16, [token][128 features]) and hand the accumulator back to the MMA thread, and only then write
 //     the rows to global memory (to every destination buffer), under the next tile's K loop.  The tensor pipe
@@ -101,7 +102,7 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;                       // tmem ptr, abort, n_gran[G]
     static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;
     static_assert(OFF_EPI % 1024 == 0, "drain tile / LoRA ring alignment");
-    static_assert(L_STAGE % 256 == 0, "LoRA ring stages keep the 32-byte swizzle atom aligned");
+    static_assert(L_STAGE % 256 == 0, "LoRA ring stages keep the swizzle atoms aligned: 256 bytes for one granule wide, 512 for two, 1024 for four");
     static_assert(TMEM_NEEDED <= 512, "tensor memory budget");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
@@ -111,6 +112,7 @@ struct PParams {
     uint32_t n_fpairs;       // pairs of feature tiles along N
     uint32_t n_passes;       // token passes (G tiles of MT tokens each) along M
     uint32_t n_tiles;        // n_fpairs * n_passes
+    uint32_t lora_wide;      // granules of B_s in one fetch: 1, 2 or 4
 };
 
 template <int MT, int G, bool A4, bool ISO = false>
@@ -160,6 +162,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     const uint32_t num_raw = A4 ? num_kb : num_kb / 4u;
     const uint32_t my_tiles = pp.n_tiles > pair ? (pp.n_tiles - pair + n_pairs - 1u) / n_pairs : 0u;
     const bool prof = p.profile != nullptr;
+    const uint32_t lw = pp.lora_wide, n_ls = uint32_t(C::L_STAGES) / lw;      // stages of the LoRA ring: lw granules of B_s, as many of t
     uint32_t nan_seen = 0;                                              // (kNanBits) this thread stored a NaN
     const long long t_entry = clock64();
     unsigned long long* prof_row = prof ? p.profile + size_t(blockIdx.x) * PROFILE_WORDS : nullptr;
@@ -319,15 +322,16 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         waited_for_shrink = true;
                     }
                     const uint32_t t_row0 = ((tile_pass(i) * G + g) * 2u + cta_rank) * p.t_tile_cap * uint32_t(C::L_GRAN_T / 256);
-                    for (uint32_t q = 0; q < n_gran; ++q) {
+                    for (uint32_t q = 0; q < n_gran;) {
                         ok = mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
                         if (!ok) break;
-                        const uint32_t base = epi0 + ls * C::L_STAGE;
-                        const uint32_t e = gran[g * C::MAX_GRANULES + q];
-                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * C::L_STAGE);
+                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE), e = gran[g * C::MAX_GRANULES + q];
+                        const uint32_t n = lw > 1u ? min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw) : 1u;      // of this slot, from this granule on
+                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * (lw * C::L_GRAN_A + n * C::L_GRAN_T));
                         tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
-                        tma_load_2d_pair(base + C::L_GRAN_A, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
-                        if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
+                        for (uint32_t k = 0; k < n; ++k, ++q)
+                            tma_load_2d_pair(base + lw * C::L_GRAN_A + k * C::L_GRAN_T, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
+                        if (++ls == n_ls) { ls = 0; lph ^= 1u; }
                     }
                 }
             }
@@ -399,18 +403,33 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 }
                 for (uint32_t g = 0; ok && g < uint32_t(G); ++g) {
                     const uint32_t n_gran = p.seq_slot ? misc[4 + g] : 0u;
-                    for (uint32_t q = 0; q < n_gran; ++q) {
+                    for (uint32_t q = 0; q < n_gran;) {
                         ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        const uint64_t la = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE);
-                        const uint64_t lb = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE + C::L_GRAN_A);
-                        if (elect_one()) {
-                            umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
-                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE);
+                        uint32_t n = 1u;
+                        const uint64_t lb = make_kmajor_sw32_desc(base + lw * C::L_GRAN_A);
+                        if (lw == 1u) {
+                            const uint64_t la = make_kmajor_desc(base, 1u);
+                            if (elect_one()) {
+                                umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
+                                umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                            }
+                        } else {
+                            const uint32_t e = gran[g * C::MAX_GRANULES + q];
+                            n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);
+                            const uint64_t la = make_kmajor_desc(base, lw);
+                            if (elect_one()) {
+#pragma unroll
+                                for (uint32_t k = 0; k < 4; ++k)     // 16 ranks = 32 bytes along the swizzled row of B_s; a block of masked t each
+                                    if (k < n) umma_bf16_ss<true>(tmem_acc + g * MT, la + 2 * k, lb + k * uint64_t(C::L_GRAN_T >> 4), idesc, 1u);
+                                umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                            }
                         }
                         __syncwarp();
-                        if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
+                        q += n;
+                        if (++ls == n_ls) { ls = 0; lph ^= 1u; }
                     }
                     if (ok && elect_one()) umma_commit<true>(BAR_ACC_FULL + 8 * g, pair_mask);
                     __syncwarp();
