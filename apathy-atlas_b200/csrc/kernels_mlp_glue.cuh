@@ -19,13 +19,15 @@ nvfp4_global_absmax_kernel(const uint16_t* __restrict__ in, float* __restrict__ 
     float local = 0.0f;
     const size_t stride = size_t(gridDim.x) * blockDim.x;
     const size_t vecs = ((reinterpret_cast<uintptr_t>(in) & 15u) == 0) ? total / 8 : 0;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < vecs; i += stride) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(in) + i);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) local = fmaxf(local, fmaxf(fabsf(bf16_lo(w[k])), fabsf(bf16_hi(w[k]))));
-    }
-    for (size_t i = vecs * 8 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
+    uint32_t top = 0u;                                          // maxima of the words' two halves; a NaN gives way
+    const uint4* in4 = reinterpret_cast<const uint4*>(in);
+    auto take = [&](const uint4& v) {
+        top = bf16x2_max(top, bf16x2_max(bf16x2_max(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), bf16x2_max(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu)));
+    };
+    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    for (; i < vecs; i += stride) take(__ldg(in4 + i));
+    local = fmaxf(bf16_lo(top), bf16_hi(top));
+    for (i = vecs * 8 + size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
         local = fmaxf(local, fabsf(__uint_as_float(uint32_t(in[i]) << 16)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) local = fmaxf(local, __shfl_xor_sync(0xFFFFFFFFu, local, o));
@@ -101,7 +103,7 @@ silu_mul_quant_nvfp4_kernel(const uint16_t* __restrict__ gate, const uint16_t* _
         }
         // the activation quantiser of the FP4-activation mode: tensor scale 1, scale byte = E4M3(group max / 6)
         uint2 q;
-        scales[gi] = uint8_t(nvfp4_group(v, gmax, 1.0f, 1.0f, q));        // (multiplying by one changes no bit)
+        scales[gi] = uint8_t(nvfp4_group<false>(v, gmax, 1.0f, 1.0f, q));        // (multiplying by one changes no bit)
         *reinterpret_cast<uint2*>(packed + gi * 8) = q;
     }
 }
