@@ -872,7 +872,7 @@ static bool dense_tc_eligible(const atlas_b200_linear_desc& d) {
 }
 
 template <int MT>
-static int launch_dense_tc_mt(const atlas_b200_linear_desc& d, int idx, uint32_t k_split, cudaStream_t st) {
+static int launch_dense_tc_mt(const atlas_b200_linear_desc& d, int idx, uint32_t k_split, bool after_shrink, cudaStream_t st) {
     using C = tc::DCfg<MT>;
     DeviceState* dst = device_state();
     if (!dst->dense_attr_set[idx]) {
@@ -887,6 +887,7 @@ static int launch_dense_tc_mt(const atlas_b200_linear_desc& d, int idx, uint32_t
     tc::DParams p{};
     p.y = static_cast<uint16_t*>(d.y);
     p.M = d.m; p.N = d.n; p.K = d.k; p.out_row_stride = d.out_row_stride; p.k_split = k_split;
+    p.after_shrink = after_shrink ? 1u : 0u;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((d.n + tc::FT - 1) / tc::FT, (d.m + MT - 1) / MT, k_split);
     if (cfg.gridDim.y > 65535) return ATLAS_B200_ERR_LIMIT;
@@ -905,7 +906,7 @@ static int launch_dense_tc_mt(const atlas_b200_linear_desc& d, int idx, uint32_t
     return cuda_status(cudaLaunchKernelEx(&cfg, tc::dense_bf16_linear_tc_kernel<MT>, map_x, map_w, p));
 }
 
-static int launch_dense_tc(const atlas_b200_linear_desc& d, cudaStream_t st) {
+static int launch_dense_tc(const atlas_b200_linear_desc& d, bool after_shrink, cudaStream_t st) {
     uint32_t mt = 16;
     while (mt < 128 && mt < d.m) mt <<= 1;
     // few output tiles (a decode batch): CTAs along z share a tile's K so that every SM streams weights
@@ -913,10 +914,10 @@ static int launch_dense_tc(const atlas_b200_linear_desc& d, cudaStream_t st) {
     uint32_t k_split = std::max(1u, std::min(std::min(uint32_t(rt_sm_count()) / std::max(tiles, 1u), 8u), d.k / uint32_t(tc::KB)));
     while (k_split & (k_split - 1)) --k_split;           // a power of two: clusters of 1, 2, 4 or 8
     t_last_shape[0] = mt; t_last_shape[1] = 0u; t_last_shape[2] = k_split; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
-    if (mt == 16) return launch_dense_tc_mt<16>(d, 0, k_split, st);
-    if (mt == 32) return launch_dense_tc_mt<32>(d, 1, k_split, st);
-    if (mt == 64) return launch_dense_tc_mt<64>(d, 2, k_split, st);
-    return launch_dense_tc_mt<128>(d, 3, k_split, st);
+    if (mt == 16) return launch_dense_tc_mt<16>(d, 0, k_split, after_shrink, st);
+    if (mt == 32) return launch_dense_tc_mt<32>(d, 1, k_split, after_shrink, st);
+    if (mt == 64) return launch_dense_tc_mt<64>(d, 2, k_split, after_shrink, st);
+    return launch_dense_tc_mt<128>(d, 3, k_split, after_shrink, st);
 }
 
 static int validate_linear(const atlas_b200_linear_desc& d) {
@@ -1166,8 +1167,15 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
     // Base linear — a dense BF16 weight on the tensor cores where the shape allows, everything else on CUDA cores —
     // then the reference's two-stage LoRA in place
     const bool dense_tc = !(d.flags & ATLAS_B200_FLAG_FORCE_SIMT) && !staged && dense_tc_eligible(d);
-    rc = dense_tc ? launch_dense_tc(d, st) : launch_simt_linear(d, st);
-    if (rc) return rc;
+    // The shrink goes first where the base can run beside it (a batch whose shrink leaves it room): it waits for what is before the
+    // call, and the base then starts at once.  (Behind the base, with that
+    // kernel's former reduction: 16 tokens x 4096 x 4096, 4 adapters of rank 16 23.9 instead of 14.0 us.)
+    const bool shrink_first = dense_tc && d.seq_slot && d.m <= 1024;
+    auto base = [&]() { return dense_tc ? launch_dense_tc(d, shrink_first, st) : launch_simt_linear(d, st); };
+    if (!shrink_first) {
+        rc = base();
+        if (rc) return rc;
+    }
     if (d.seq_slot) {
         ShrinkParams sp{};
         sp.x = static_cast<const uint16_t*>(d.x);
@@ -1178,8 +1186,12 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         sp.out = static_cast<uint16_t*>(d.lora_t);
         sp.M = d.m; sp.k_in = d.k; sp.max_rank = d.max_rank; sp.x_row_stride = d.x_row_stride; sp.max_loras = d.max_loras;
         sp.post = 0.0f;
-        rc = launch_shrink(sp, d.max_loras, st);
+        rc = launch_shrink(sp, d.max_loras, st, shrink_first);
         if (rc) return rc;
+        if (shrink_first) {
+            rc = base();
+            if (rc) return rc;
+        }
         ExpandParams ep{};
         ep.xa = static_cast<const uint16_t*>(d.lora_t);
         ep.seq_slot = d.seq_slot;

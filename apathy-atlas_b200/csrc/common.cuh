@@ -33,11 +33,12 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 //   launched as dependents     both tensor-core shrinks, the main kernel behind a shrink, the tensor-core expand, the dense linear,
 //                              the QKV consumers, SwiGLU in both forms, the quantiser
 //   releasing                  all of these but lora_shrink_mma_kernel and lora_shrink_grouped_kernel, which do so only in front of a
-//                              main kernel
+//                              main kernel or of the dense linear
 //   neither                    a main kernel without adapters releases but is launched in order; the NVFP4 decode, the maximum, the
 //                              CUDA-core linear and expand do neither
-// A dependent begins with the wait.  Only the main kernel reads anything ahead of it (x, weights, routing), and it follows a shrink
-// that has waited before releasing it; it waits before it reads t, on every path, so that nothing behind it overtakes the shrink.
+// A dependent begins with the wait.  Only the main kernel and the dense linear behind their shrink read anything ahead of it (x, weights,
+// routing), and that shrink has waited before releasing them; they wait before they read t, or before they end, on every path, so that
+// nothing behind them overtakes the shrink.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The pointer as a value that does not exist before this point: keeps read-only loads through it behind pdl_wait().

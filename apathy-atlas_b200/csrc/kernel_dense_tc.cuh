@@ -7,8 +7,8 @@
 // (kind::f16, both operands from shared memory); nothing is expanded, no warp touches the operands.
 //
 // A decode batch has few output tiles (N / 128) and is bound by streaming w: `ks` CTAs along grid z form a cluster and
-// each contracts a share of K, so that every SM pulls weights; their FP32 partial tiles are added by the cluster's
-// first CTA over distributed shared memory, in rank order (results do not depend on timing).
+// each contracts a share of K, so that every SM pulls weights; their FP32 partial tiles are added over distributed
+// shared memory, the tokens dealt out to the CTAs, in rank order (results do not depend on timing).
 //
 // Roles (6 warps): warp 0 TMA producer · warp 1 TMEM allocation and MMA issue · warps 2-5 epilogue (one per TMEM lane
 // quadrant).  Every wait is bounded as in kernel_tc.cuh.
@@ -37,6 +37,7 @@ template <int MT> struct DCfg {
 struct DParams {
     uint16_t* y;
     uint32_t M, N, K, out_row_stride, k_split;
+    uint32_t after_shrink;         // launched behind a shrink that has waited for everything before it: x and w are read at once
 };
 
 template <int MT>
@@ -71,7 +72,7 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
     __syncthreads();
     tcgen05_fence_after();
     pdl_release();
-    pdl_wait();                                          // (x and w come by TMA, issued below)
+    if (!p.after_shrink) pdl_wait();                     // (x and w come by TMA, issued below)
     const uint32_t tmem_acc = misc[0];
     bool acc_ready = false;
 
@@ -138,24 +139,36 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         tcgen05_fence_before();
         __syncwarp();
         cluster_sync_all();                              // every CTA's partial tile is in its shared memory
-        if (kz == 0 && warp >= 2 && acc_ready) {
+        // Tokens kz, kz + ks, ... by this CTA, four at a time, all their loads in flight before the first sum.  (All of them by
+        // the first CTA, sum by sum, were a chain of remote latencies: this kernel 11.5 -> 7.7 us for 16 tokens x 4096 x 4096.)
+        if (warp >= 2 && acc_ready) {
             const uint32_t te = tid - 64;                // 0..127 = feature within the tile
             const uint32_t f = f0 + te;
-            for (uint32_t i = 0; i < uint32_t(MT); ++i) {
-                const uint32_t m = m0 + i;
-                if (m >= p.M || f >= p.N) continue;
-                float acc = 0.0f;
-                for (uint32_t z = 0; z < ks; ++z) {
-                    uint32_t bits;
-                    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(bits) : "r"(map_to_cta(smem_base + (i * FT + te) * 4u, z)) : "memory");
-                    acc += __uint_as_float(bits);
+            constexpr uint32_t ROWS = MT < 64 ? 2 : 4;
+            for (uint32_t i0 = kz; i0 < uint32_t(MT) && m0 + i0 < p.M; i0 += ROWS * ks) {
+                uint32_t bits[ROWS][8];
+#pragma unroll
+                for (uint32_t u = 0; u < ROWS; ++u)
+#pragma unroll
+                    for (uint32_t z = 0; z < 8; ++z)
+                        if (i0 + u * ks < uint32_t(MT) && z < ks)
+                            asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(bits[u][z]) : "r"(map_to_cta(smem_base + ((i0 + u * ks) * FT + te) * 4u, z)) : "memory");
+#pragma unroll
+                for (uint32_t u = 0; u < ROWS; ++u) {
+                    const uint32_t m = m0 + i0 + u * ks;
+                    if (i0 + u * ks >= uint32_t(MT) || m >= p.M || f >= p.N) continue;
+                    float acc = 0.0f;
+#pragma unroll
+                    for (uint32_t z = 0; z < 8; ++z)
+                        if (z < ks) acc += __uint_as_float(bits[u][z]);
+                    p.y[size_t(m) * p.out_row_stride + f] = f32_to_bf16_bits(acc);
                 }
-                p.y[size_t(m) * p.out_row_stride + f] = f32_to_bf16_bits(acc);
             }
         }
         __syncwarp();
         cluster_sync_all();                              // the tiles stay alive until they have been read
     }
+    if (p.after_shrink) pdl_wait();                      // what is launched behind this kernel may not overtake the shrink
     if (*abort_flag) {
         const uint64_t t0 = global_timer_ns();
         while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
