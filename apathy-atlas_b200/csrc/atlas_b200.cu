@@ -802,7 +802,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
 }
 
 // ---- the smallest batches (kernel_decode_mma.cuh) ----
-template <int TILES, int NT>
+template <int TILES, int NT, int WARPS>
 static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
     tc::Params p{};
     int rc = fill_tc_params(d, false, false, TTiles{}, p);
@@ -821,14 +821,14 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     p.wait_for_shrink = shrink ? 1u : 0u;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(DCM_THREADS);
+    cfg.blockDim = dim3(32 * WARPS);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = shrink ? 1 : 0;
-    return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT>, w, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS>, w, p));
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):
@@ -855,10 +855,16 @@ static bool decode_pays(const atlas_b200_linear_desc& d) {
 }
 
 static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
-    // sixteen features per CTA instead of 32 where the two CTAs that fit on an SM then still cover them in one wave
-    const bool narrow = d.n <= 16u * 2u * uint32_t(rt_sm_count());
-    if (d.m <= 8) return narrow ? launch_decode_as<1, 1>(d, shrink, st) : launch_decode_as<2, 1>(d, shrink, st);
-    return narrow ? launch_decode_as<1, 2>(d, shrink, st) : launch_decode_as<2, 2>(d, shrink, st);
+    // Sixteen warps fit on an SM.  Sixteen features per CTA instead of 32 where the two CTAs of eight warps that fit on an SM then still
+    // cover them in one wave; and four warps to a CTA where even with 32 features they do not: four such CTAs on an SM are one wave up
+    // to 18944 features, and beyond, CTAs at different points of their lives fill each other's gaps.  Eight / four warps, 1 and 8
+    // tokens, 8 adapters of rank 16 (us): 11008 x 4096 15.9 / 14.0, 21.4 / 16.7; 14336 x 4096 17.9 / 16.3, 22.1 / 19.5; 28672 x 8192
+    // 48.1 / 45.4, 56.8 / 52.3; but 8192 x 8192 (256 CTAs) 17.1 / 18.6, 19.7 / 25.9.
+    const uint32_t slots = 2u * uint32_t(rt_sm_count());
+    const bool few = d.m <= 8;
+    if (d.n <= 16u * slots) return few ? launch_decode_as<1, 1, 8>(d, shrink, st) : launch_decode_as<1, 2, 8>(d, shrink, st);
+    if (d.n <= 32u * slots) return few ? launch_decode_as<2, 1, 8>(d, shrink, st) : launch_decode_as<2, 2, 8>(d, shrink, st);
+    return few ? launch_decode_as<2, 1, 4>(d, shrink, st) : launch_decode_as<2, 2, 4>(d, shrink, st);
 }
 
 // ---- dense-BF16 base on the tensor cores (kernel_dense_tc.cuh) ----

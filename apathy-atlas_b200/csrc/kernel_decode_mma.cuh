@@ -10,12 +10,12 @@
 // the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired the same way (four permutes
 // per eight elements of x, shared by all features of the warp).
 //
-// A CTA owns 16 * TILES features and all of K; its eight warps take interleaved 128-wide K steps (per thread and feature
+// A CTA owns 16 * TILES features and all of K; its WARPS warps (eight, or four with as many more CTAs on an SM) take interleaved 128-wide K steps (per thread and feature
 // row one 128-bit load of 32 codes and their two scale bytes, the next step's loads in flight while one is multiplied),
 // and the partial sums are added in warp order through shared memory.  No cluster, no tensor memory, no barriers but two.
 // The MMA's M is 16 features, its N 8 tokens (NT of them side by side).
 //
-// LoRA: granule j (16 ranks) of slot s is one more K step, done by warp (s + 3 j) % 8, so that the order in which a token's terms
+// LoRA: granule j (16 ranks) of slot s is one more K step, done by warp (s + 3 j) % WARPS, so that the order in which a token's terms
 // are added depends on its own slot alone.  t rows come from the shrink this kernel may overtake (programmatic dependent
 // launch): they are first read behind griddepcontrol.wait, after the base loop.
 #pragma once
@@ -25,7 +25,6 @@
 
 namespace atlas {
 
-constexpr int DCM_WARPS = 8, DCM_THREADS = 32 * DCM_WARPS;
 constexpr int DCM_KSTEP = 128;
 constexpr int DCM_MAX_TOKENS = 16;
 
@@ -36,10 +35,10 @@ struct DecodeParams {
     uint32_t x_row_stride;
 };
 
-template <int TILES, int NT>
-__global__ void __launch_bounds__(DCM_THREADS, 2)
+template <int TILES, int NT, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
-    __shared__ float part[DCM_WARPS][NT * 8][TILES * 16 + 1];          // [warp][token][feature]
+    __shared__ float part[WARPS][NT * 8][TILES * 16 + 1];          // [warp][token][feature]
     __shared__ int32_t slot_s[DCM_MAX_TOKENS];
     __shared__ uint32_t rank_s[DCM_MAX_TOKENS];                        // of the slot in slot_s: its rank
     __shared__ uint64_t b_s[DCM_MAX_TOKENS];                           // and its B (read once, not granule by granule behind the shrink)
@@ -134,18 +133,18 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
         }
     };
     load(warp, code[0], sc[0], xv[0]);
-    for (uint32_t step = warp; step < n_steps; step += 2 * DCM_WARPS) {
-        load(step + DCM_WARPS, code[1], sc[1], xv[1]);
+    for (uint32_t step = warp; step < n_steps; step += 2 * WARPS) {
+        load(step + WARPS, code[1], sc[1], xv[1]);
         multiply(step, code[0], sc[0], xv[0]);
-        load(step + 2 * DCM_WARPS, code[0], sc[0], xv[0]);
-        if (step + DCM_WARPS < n_steps) multiply(step + DCM_WARPS, code[1], sc[1], xv[1]);
+        load(step + 2 * WARPS, code[0], sc[0], xv[0]);
+        if (step + WARPS < n_steps) multiply(step + WARPS, code[1], sc[1], xv[1]);
     }
 
     // ---- LoRA granules of this warp ----
     if (p.seq_slot) {
         __syncthreads();                                                        // slot_s, rank_s, b_s
         // this CTA's rows of B into L2 while the shrink may still run
-        for (uint32_t m = warp; m < p.M; m += DCM_WARPS) {
+        for (uint32_t m = warp; m < p.M; m += WARPS) {
             if (slot_s[m] < 0 || lane >= TILES * 16u || f0 + lane >= p.N) continue;
             const uint64_t row = b_s[m] + size_t(f0 + lane) * p.max_rank * 2u;
             for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"((row + 2u * j) & ~15ull));
@@ -168,7 +167,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             const uint16_t* B = reinterpret_cast<const uint16_t*>(b_s[first]);
             const bool b_vec = (reinterpret_cast<uintptr_t>(B) & 7u) == 0u;
             for (uint32_t j = 0; 16 * j < rank; ++j) {
-                if ((uint32_t(s) + 3u * j) % DCM_WARPS != warp) continue;
+                if ((uint32_t(s) + 3u * j) % WARPS != warp) continue;
                 const uint32_t j0 = 16 * j + 4 * t;
                 const bool in = j0 < p.max_rank;                                // (max_rank is a multiple of 8)
                 uint2 tv[NT];
@@ -207,11 +206,11 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) part[warp][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[i][n][e];
     __syncthreads();
-    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += DCM_THREADS) {          // (whole warps: a multiple of 128)
+    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
         const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
         float sum = part[0][m][fi];
 #pragma unroll
-        for (int k = 1; k < DCM_WARPS; ++k) sum += part[k][m][fi];
+        for (int k = 1; k < WARPS; ++k) sum += part[k][m][fi];
         const uint32_t bits = f32_to_bf16_bits(sum * p.out_scale);
         const bool in = m < p.M && f < p.N;
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;
