@@ -120,3 +120,20 @@ def test_dense_base_beside_its_shrink(cuda, atlas, oracle, M, K, N):
     rows, cols = _sample(case, 32, 128, M)
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 512, 9472), (1, 512, 9488), (8, 288, 9500), (7, 1024, 18960), (16, 256, 28672)])
+def test_small_batches_of_four_and_eight_warps(cuda, atlas, oracle, M, K, N):
+    """Either side of the line between the two, ragged features, K of a part of a step; a token's bits in a batch and alone."""
+    from atlas_b200 import synth
+    case = synth.make_case("warps", M=M, K=K, N=N, ranks=[16, 8], max_rank=16, scale2=0.02, b_std=0.1, seed=N)
+    dc = DeviceCase(cuda, atlas, case)
+    y, _ = dc.run()
+    assert atlas.last_launch_shape()["token_tile"] == 8
+    rows, cols = _sample(case, 16, 512, N)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
+    whole_x, whole_slot = case.x, case.seq_slot
+    case.M, case.x, case.seq_slot = 1, whole_x[M - 1:], whole_slot[M - 1:]
+    alone, _ = DeviceCase(cuda, atlas, case).run()
+    assert np.array_equal(alone[0], y[M - 1])
+    assert atlas.device_status() == 0
