@@ -16,6 +16,9 @@
 // x, and of row g of A_s.  Elements 0..3 feed one MMA, 4..7 the next; x and A_s use the same
 // assignment, so each K element meets its partner and every 32-byte sector fetched is used in full.
 //
+// A slot with many rows in its chunk (a prefill batch of few sequences) is a chain of such passes of 32 rows: 2^ShrinkParams::row_parts_log2
+// clusters share them.
+//
 // A CTA is small on purpose (128 threads, well under 64 registers): in the fused layer this grid runs
 // next to the tcgen05 kernel's CTAs on the same SMs (programmatic dependent launch), and must fit in
 // what that kernel leaves free.
@@ -57,13 +60,15 @@ lora_shrink_mma_kernel(ShrinkParams p) {
     const uint32_t s = blockIdx.x / ksplit;
     const uint32_t j0 = blockIdx.y * SHM_RANKS;
     const uint32_t chunk = p.chunk ? p.chunk : uint32_t(SHM_CHUNK);
-    const uint32_t m_base = blockIdx.z * chunk;
+    const uint32_t chunk_i = blockIdx.z >> p.row_parts_log2;
+    const uint32_t row_lo = (blockIdx.z - (chunk_i << p.row_parts_log2)) * SHM_TOKENS;        // this cluster's first pass over a slot's rows
+    const uint32_t m_base = chunk_i * chunk;
 
     // While the kernel ahead still runs: this granule of A_s into L2, the cluster's CTAs taking its lines in turn.  Nothing that
     // is read here decides anything but what is prefetched (the tables may be about to change: past the first-level cache, read
     // again below; only an address that is both in the table and in the declared pool is touched).  64 tokens, 64 adapters of
     // mixed ranks, three projections of a decode layer (16 MB of A each): 109 -> 96 us.
-    if (p.seq_slot && p.a_pool_base) {
+    if (p.seq_slot && p.a_pool_base && row_lo == 0) {
         const uint64_t a = __ldcg(p.a_table + s);
         const uint32_t rank = p.rank_table ? min(__ldcg(p.rank_table + s), p.max_rank) : p.max_rank;
         bool want = false;
@@ -139,7 +144,7 @@ lora_shrink_mma_kernel(ShrinkParams p) {
         n_rows = total;
         __syncthreads();
     }
-    if (n_rows == 0) return;
+    if (n_rows <= row_lo) return;                            // (whole cluster)
 
     // ranks at or beyond the adapter's true rank are written as zeros and never read
     const bool any_live = j0 < rank;
@@ -172,11 +177,11 @@ lora_shrink_mma_kernel(ShrinkParams p) {
             const uint32_t q = ahead[0] + ahead[1] + ahead[2] + ahead[3] + blockIdx.y;
             if (q < p.tile_cap) {
                 // part 0's block of this pair; part 1's lies tile_cap blocks further on
-                tile = p.tile_out + (size_t(blockIdx.z) * (chunk / p.part_rows) * p.tile_cap + q) * p.part_rows * 16;
+                tile = p.tile_out + (size_t(chunk_i) * (chunk / p.part_rows) * p.tile_cap + q) * p.part_rows * 16;
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const uint32_t idx = h * SHM_THREADS + tid;
-                    if (idx < chunk && !hit[h]) {
+                    if (row_lo == 0 && idx < chunk && !hit[h]) {
                         const uint32_t part = idx / p.part_rows, r = idx % p.part_rows;
                         uint4* z = reinterpret_cast<uint4*>(tile + (size_t(part) * p.tile_cap * p.part_rows + r) * 16);
                         z[0] = make_uint4(0u, 0u, 0u, 0u);
@@ -192,7 +197,7 @@ lora_shrink_mma_kernel(ShrinkParams p) {
     const uint32_t n_chunks = p.k_in / 32;
     const bool a_aligned = (reinterpret_cast<uintptr_t>(A) & 15u) == 0;
 
-    for (uint32_t r0 = 0; r0 < n_rows; r0 += SHM_TOKENS) {
+    for (uint32_t r0 = row_lo; r0 < n_rows; r0 += uint32_t(SHM_TOKENS) << p.row_parts_log2) {
         float acc[2][2][4];
 #pragma unroll
         for (int mt = 0; mt < 2; ++mt)

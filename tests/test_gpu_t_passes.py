@@ -137,3 +137,18 @@ def test_small_batches_of_four_and_eight_warps(cuda, atlas, oracle, M, K, N):
     alone, _ = DeviceCase(cuda, atlas, case).run()
     assert np.array_equal(alone[0], y[M - 1])
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,ads", [(33, 1), (64, 1), (65, 2), (130, 1), (256, 2), (257, 1), (700, 3)])
+def test_many_rows_of_a_slot(cuda, atlas, oracle, M, ads):
+    """Passes of 32 rows shared by several clusters: whole and partial last passes, masked tiles and rows of t."""
+    from atlas_b200 import synth
+    case = synth.make_case("rows", M=M, K=512, N=384, ranks=[16, 40, 8][:ads], max_rank=40, max_loras=ads, ids="segments", segments=ads,
+                           none_frac=0.05, scale2=0.02, b_std=0.1, seed=M)
+    dc = DeviceCase(cuda, atlas, case)
+    y, _ = dc.run(flags=atlas.FLAG_FORCE_TCGEN05, lora_ws=True)
+    build, _ = dc.run(flags=atlas.FLAG_FORCE_TCGEN05)
+    assert np.array_equal(y, build)
+    rows, cols = _sample(case, 64, 96, M)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
+    assert atlas.device_status() == 0
