@@ -869,10 +869,15 @@ static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* sh
     // to 18944 features, and beyond, CTAs at different points of their lives fill each other's gaps.  Eight / four warps, 1 and 8
     // tokens, 8 adapters of rank 16 (us): 11008 x 4096 15.9 / 14.0, 21.4 / 16.7; 14336 x 4096 17.9 / 16.3, 22.1 / 19.5; 28672 x 8192
     // 48.1 / 45.4, 56.8 / 52.3; but 8192 x 8192 (256 CTAs) 17.1 / 18.6, 19.7 / 25.9.
+    // Granules are shared by half as many warps then.  8 tokens, 8 adapters of rank 64: 14336 x 4096 30.8 / 29.7, x 5120 35.4 / 36.2, 14848 x
+    // 6912 44.0 / 49.8; of rank 128: 37.5 / 41.5, 43.6 / 49.8, 52.5 / 61.7.  (By what the pool may hold, not by the batch: a token's sums are
+    // the same in any batch of up to eight.)
+    const uint32_t granules = d.seq_slot ? std::min(d.max_loras, uint32_t(DCM_MAX_TOKENS)) * ((d.max_rank + 15) / 16) : 0u;
+    const bool four = granules <= (d.k <= 4096 ? 32u : 8u);
     const uint32_t slots = 2u * uint32_t(rt_sm_count());
     const bool few = d.m <= 8;
     if (d.n <= 16u * slots) return few ? launch_decode_as<1, 1, 8>(d, shrink, st) : launch_decode_as<1, 2, 8>(d, shrink, st);
-    if (d.n <= 32u * slots) return few ? launch_decode_as<2, 1, 8>(d, shrink, st) : launch_decode_as<2, 2, 8>(d, shrink, st);
+    if (d.n <= 32u * slots || !four) return few ? launch_decode_as<2, 1, 8>(d, shrink, st) : launch_decode_as<2, 2, 8>(d, shrink, st);
     return few ? launch_decode_as<2, 1, 4>(d, shrink, st) : launch_decode_as<2, 2, 4>(d, shrink, st);
 }
 
