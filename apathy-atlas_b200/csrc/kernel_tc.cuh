@@ -47,6 +47,7 @@
 
 #include "common.cuh"
 #include "isolate.cuh"
+#include "share_rules.hpp"
 
 namespace atlas {
 namespace tc {
@@ -1043,7 +1044,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (n_gran) {
             const uint32_t f = f0 + te;
             if (f < p.N) {
-                for (uint32_t i = 0, g = 4 * kz; g < n_gran; g = 4 * (kz + (++i >> 2) * ks) + (i & 3u)) {
+                for (uint32_t g = 4 * kz; g < n_gran; g = next_own_granule(g, ks)) {
                     const uint32_t e = gran[g];
                     // (a strided pool's addresses are arithmetic: a table read per granule made this loop a chain of loads)
                     const unsigned long long b_s = p.b_pool_strided ? p.b_pool_base + (e >> GRAN_SHIFT) * p.b_slot_stride : p.b_table[e >> GRAN_SHIFT];
