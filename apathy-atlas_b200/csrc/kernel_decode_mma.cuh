@@ -10,12 +10,14 @@
 // the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired the same way (four permutes
 // per eight elements of x, shared by all features of the warp).
 //
-// A CTA owns 16 * TILES features and all of K; its WARPS warps (eight, or four with as many more CTAs on an SM) take interleaved 128-wide K steps (per thread and feature
-// row one 128-bit load of 32 codes and their two scale bytes, the next step's loads in flight while one is multiplied),
-// and the partial sums are added in warp order through shared memory.  No cluster, no tensor memory, no barriers but two.
+// A CTA owns 16 * TILES features and all of K.  Interleaved 128-wide K steps make eight partial sums, one to each of eight warps or
+// two to each of four (with as many more CTAs on an SM): the same bits, so that either form may be taken for any batch and pool, and
+// a row without an adapter is the base call's.  Per thread and feature row a step is one 128-bit load of 32 codes and their two scale
+// bytes, the next step's loads in flight while one is multiplied; the partial sums are added in their order through shared
+// memory.  No cluster, no tensor memory, no barriers but two.
 // The MMA's M is 16 features, its N 8 tokens (NT of them side by side).
 //
-// LoRA: granule j (16 ranks) of slot s is one more K step, done by warp (s + 3 j) % WARPS, so that the order in which a token's terms
+// LoRA: granule j (16 ranks) of slot s is one more K step of partial sum (s + 3 j) % 8, so that the order in which a token's terms
 // are added depends on its own slot alone.  t rows come from the shrink this kernel may overtake (programmatic dependent
 // launch): they are first read behind griddepcontrol.wait, after the base loop.
 #pragma once
@@ -25,6 +27,7 @@
 
 namespace atlas {
 
+constexpr int DCM_SUMS = 8;          // partial sums of an output, whatever the number of warps
 constexpr int DCM_KSTEP = 128;
 constexpr int DCM_MAX_TOKENS = 16;
 
@@ -38,7 +41,9 @@ struct DecodeParams {
 template <int TILES, int NT, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
-    __shared__ float part[WARPS][NT * 8][TILES * 16 + 1];          // [warp][token][feature]
+    constexpr int SETS = DCM_SUMS / WARPS;                             // partial sums of a warp
+    static_assert(SETS * WARPS == DCM_SUMS && SETS <= 2, "two steps to a turn of the base loop, one for either sum");
+    __shared__ float part[DCM_SUMS][NT * 8][TILES * 16 + 1];           // [partial sum][token][feature]
     __shared__ int32_t slot_s[DCM_MAX_TOKENS];
     __shared__ uint32_t rank_s[DCM_MAX_TOKENS];                        // of the slot in slot_s: its rank
     __shared__ uint64_t b_s[DCM_MAX_TOKENS];                           // and its B (read once, not granule by granule behind the shrink)
@@ -78,7 +83,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
     for (int n = 0; n < NT; ++n) x_row[n] = w.x + size_t(min(8 * n + g, p.M - 1u)) * w.x_row_stride + 32 * t;
 
-    float acc[TILES][NT][4] = {};
+    float acc[SETS][TILES][NT][4] = {};                                // sums `warp`, `warp` + WARPS
     // (one n-tile: x travels with the codes; more of them would not fit in registers and are read where they are used)
     constexpr bool X_AHEAD = NT == 1;
     uint4 xv[2][X_AHEAD ? 4 : 1];
@@ -98,7 +103,8 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             for (int u = 0; u < 4; ++u)
                 xs[u] = in && g < p.M ? __ldg(reinterpret_cast<const uint4*>(x_row[0] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
     };
-    auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2], const uint4 (&xs)[X_AHEAD ? 4 : 1]) {
+    auto multiply = [&](uint32_t step, const uint4 (&c)[TILES][2], const uint32_t (&s)[TILES][2], const uint4 (&xs)[X_AHEAD ? 4 : 1],
+                        float (&sum)[TILES][NT][4]) {
         const bool in = step * DCM_KSTEP + 32 * t < p.K;
         uint32_t mul[TILES][2][2];
 #pragma unroll
@@ -126,8 +132,8 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
                 }
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    mma_bf16_16816(acc[i][n], a[0][0], a[1][0], a[0][1], a[1][1], xb[n][0], xb[n][1]);
-                    mma_bf16_16816(acc[i][n], a[0][2], a[1][2], a[0][3], a[1][3], xb[n][2], xb[n][3]);
+                    mma_bf16_16816(sum[i][n], a[0][0], a[1][0], a[0][1], a[1][1], xb[n][0], xb[n][1]);
+                    mma_bf16_16816(sum[i][n], a[0][2], a[1][2], a[0][3], a[1][3], xb[n][2], xb[n][3]);
                 }
             }
         }
@@ -135,9 +141,9 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     load(warp, code[0], sc[0], xv[0]);
     for (uint32_t step = warp; step < n_steps; step += 2 * WARPS) {
         load(step + WARPS, code[1], sc[1], xv[1]);
-        multiply(step, code[0], sc[0], xv[0]);
+        multiply(step, code[0], sc[0], xv[0], acc[0]);
         load(step + 2 * WARPS, code[0], sc[0], xv[0]);
-        if (step + WARPS < n_steps) multiply(step + WARPS, code[1], sc[1], xv[1]);
+        if (step + WARPS < n_steps) multiply(step + WARPS, code[1], sc[1], xv[1], acc[SETS - 1]);
     }
 
     // ---- LoRA granules of this warp ----
@@ -167,7 +173,8 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             const uint16_t* B = reinterpret_cast<const uint16_t*>(b_s[first]);
             const bool b_vec = (reinterpret_cast<uintptr_t>(B) & 7u) == 0u;
             for (uint32_t j = 0; 16 * j < rank; ++j) {
-                if ((uint32_t(s) + 3u * j) % WARPS != warp) continue;
+                const uint32_t to = (uint32_t(s) + 3u * j) % DCM_SUMS;
+                if (to % WARPS != warp) continue;
                 const uint32_t j0 = 16 * j + 4 * t;
                 const bool in = j0 < p.max_rank;                                // (max_rank is a multiple of 8)
                 uint2 tv[NT];
@@ -188,29 +195,35 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
                     for (int n = 0; n < NT; ++n) {
                         // into the columns of this slot alone: an infinity in one adapter's B, times the zeros that stand for
                         // the other tokens, must not reach them
-                        float d[4] = {acc[i][n][0], acc[i][n][1], acc[i][n][2], acc[i][n][3]};
+                        float d[4];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) d[e] = SETS > 1 && to >= WARPS ? acc[SETS - 1][i][n][e] : acc[0][i][n][e];
                         mma_bf16_16816(d, bv[0].x, bv[1].x, bv[0].y, bv[1].y, tv[n].x, tv[n].y);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) acc[i][n][e] = col[n][e & 1] == s ? d[e] : acc[i][n][e];
+                        for (int h = 0; h < SETS; ++h)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[h][i][n][e] = col[n][e & 1] == s && to / WARPS == h ? d[e] : acc[h][i][n][e];
                     }
                 }
             }
         }
     }
 
-    // ---- the warps' partial sums, added in warp order ----
+    // ---- the partial sums, added in their order ----
 #pragma unroll
-    for (int i = 0; i < TILES; ++i)
+    for (int h = 0; h < SETS; ++h)
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int i = 0; i < TILES; ++i)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) part[warp][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[i][n][e];
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) part[warp + h * WARPS][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[h][i][n][e];
     __syncthreads();
     for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
         const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
         float sum = part[0][m][fi];
 #pragma unroll
-        for (int k = 1; k < WARPS; ++k) sum += part[k][m][fi];
+        for (int k = 1; k < DCM_SUMS; ++k) sum += part[k][m][fi];
         const uint32_t bits = f32_to_bf16_bits(sum * p.out_scale);
         const bool in = m < p.M && f < p.N;
         const size_t at = size_t(m) * p.out_row_stride + p.y_col0 + f;

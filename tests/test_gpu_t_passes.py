@@ -139,6 +139,28 @@ def test_small_batches_of_four_and_eight_warps(cuda, atlas, oracle, M, K, N):
     assert atlas.device_status() == 0
 
 
+@pytest.mark.parametrize("M", [1, 7, 8, 13, 16])
+def test_small_batches_have_the_bits_of_any_pool(cuda, atlas, oracle, M):
+    """Four warps to a CTA (a pool of two slots, no pool at all) and eight (one of twenty): the same partial sums."""
+    from atlas_b200 import synth
+    case = synth.make_case("pools", M=M, K=4352, N=9488, ranks=[16, 8], max_rank=16, none_frac=0.3, scale2=0.02, b_std=0.1, seed=M)
+    if M > 2:
+        case.seq_slot[:3] = (0, 1, -1)
+    small, _ = DeviceCase(cuda, atlas, case).run()
+    assert atlas.last_launch_shape()["token_tile"] == 8
+    case.max_loras, case.adapters = 20, list(case.adapters) + [None] * 18
+    dc = DeviceCase(cuda, atlas, case)
+    large, _ = dc.run()
+    assert atlas.last_launch_shape()["token_tile"] == 8
+    assert np.array_equal(small, large)
+    base, _ = dc.run(lora=False)
+    none = case.seq_slot < 0
+    assert np.array_equal(large[none], base[none])
+    rows, cols = _sample(case, 16, 256, M)
+    assert_close(oracle, large[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
+    assert atlas.device_status() == 0
+
+
 @pytest.mark.parametrize("M,ads", [(33, 1), (64, 1), (65, 2), (130, 1), (256, 2), (257, 1), (700, 3)])
 def test_many_rows_of_a_slot(cuda, atlas, oracle, M, ads):
     """Passes of 32 rows shared by several clusters: whole and partial last passes, masked tiles and rows of t."""
