@@ -10,7 +10,8 @@ RANK, ADAPTERS, PASSES = 16, 4, 16
 
 
 class Chain:
-    """One layer's calls (fused QKV and its consumer, gate, up, SwiGLU, down), the staged operators and a dense linear."""
+    """One layer's calls (fused QKV and its consumer, gate, up, SwiGLU, down), the staged operators and a dense linear, without adapters
+    and with them (its base then starts beside the shrink)."""
 
     def __init__(self, torch, ab, m, fp4):
         self.torch, self.ab, self.m, self.fp4 = torch, ab, m, fp4
@@ -21,6 +22,7 @@ class Chain:
         width = (HEADS + 2 * KV_HEADS) * HEAD_DIM
         self.weights = {name: self.linear(n, k) for name, n, k in (("q", HEADS * HEAD_DIM, HIDDEN), ("k", KV_HEADS * HEAD_DIM, HIDDEN),
                         ("v", KV_HEADS * HEAD_DIM, HIDDEN), ("gate", INTER, HIDDEN), ("up", INTER, HIDDEN), ("down", HIDDEN, INTER))}
+        self.dense_pool = self.pool(512, HIDDEN)
         self.w_dense, self.wq, self.wk = self.normal(512, HIDDEN, std=0.03), self.normal(HEAD_DIM, std=0.1), self.normal(HEAD_DIM, std=0.1)
         self.pos = torch.randint(0, 4096, (m,), generator=g, device="cuda").to(torch.int32)
         self.cache_at = torch.randperm(m, generator=g, device="cuda")
@@ -39,10 +41,13 @@ class Chain:
     def linear(self, n, k):
         packed = self.torch.randint(0, 256, (n, k // 2), generator=self.g, device="cuda", dtype=self.torch.uint8)
         scales = self.torch.empty((n, k // 16), device="cuda").normal_(generator=self.g).abs_().to(self.torch.float8_e4m3fn).view(self.torch.uint8)
+        return n, k, packed, scales, self.pool(n, k)
+
+    def pool(self, n, k):
         pool = self.ab.LoraPool(k, n, RANK, ADAPTERS)
         for s in range(ADAPTERS):
             pool.pack(s, self.normal(RANK, k, std=k ** -0.5), self.normal(n, RANK, std=0.05), 2.0)
-        return n, k, packed, scales, pool
+        return pool
 
     def call(self, name, x, y, stride=None, flags=0):
         n, k, packed, scales, pool = self.weights[name]
@@ -53,7 +58,8 @@ class Chain:
     def outputs(self):
         pages, cache = (self.m + PAGE - 1) // PAGE, (PAGE, KV_HEADS, HEAD_DIM)
         return [dict(qkv=self.zeros(*self.qkv.shape), k_cache=self.zeros(pages, *cache), v_cache=self.zeros(pages, *cache),
-                     down=self.zeros(self.m, HIDDEN), staged=self.zeros(self.m, KV_HEADS * HEAD_DIM), dense=self.zeros(self.m, 512))
+                     down=self.zeros(self.m, HIDDEN), staged=self.zeros(self.m, KV_HEADS * HEAD_DIM), dense=self.zeros(self.m, 512),
+                     dense_lora=self.zeros(self.m, 512))
                 for _ in range(PASSES)]
 
     def run(self, out, behind):
@@ -86,11 +92,59 @@ class Chain:
             d = ab.make_linear_desc(x=x, m=m, k=HIDDEN, n=512, y=o["dense"], w_bf16=self.w_dense)
             ab.nvfp4_lora_linear(d)
             behind()
+            d = ab.make_linear_desc(x=x, m=m, k=HIDDEN, n=512, y=o["dense_lora"], w_bf16=self.w_dense, seq_slot=self.slot,
+                                    route=self.dense_pool.route(), lora_t=self.t)
+            ab.nvfp4_lora_linear(d)
+            behind()
+
+
+class RewrittenRouting(Chain):
+    """The same, with tokens routed anew and slots coming and going in the stream behind every call: what a kernel reads of the
+    routing ahead of its wait is not what it is to use."""
+
+    def __init__(self, torch, ab, m, fp4):
+        super().__init__(torch, ab, m, fp4)
+        self.pools = [w[4] for w in self.weights.values()] + [self.dense_pool]
+        self.slots = [torch.randint(-1, ADAPTERS, (m,), generator=self.g, device="cuda").to(torch.int32) for _ in range(5)]
+        self.tables = []
+        for gone in range(3):                              # slot `gone` has no adapter, the one behind it half its ranks and another scale
+            version = []
+            for p in self.pools:
+                a, b, scale, rank = p.a_table.clone(), p.b_table.clone(), p.scale_table.clone(), p.rank_table.clone()
+                a[gone] = b[gone] = 0
+                scale[gone + 1], rank[gone + 1] = 1.0 + gone, RANK // 2
+                version.append((a, b, scale, rank))
+            self.tables.append(version)
+
+    def rewrite(self):
+        self.slot.copy_(self.slots[self.calls % len(self.slots)])
+        for p, (a, b, scale, rank) in zip(self.pools, self.tables[self.calls % len(self.tables)]):
+            p.a_table.copy_(a)
+            p.b_table.copy_(b)
+            p.scale_table.copy_(scale)
+            p.rank_table.copy_(rank)
+        self.calls += 1
+
+    def run(self, out, behind):
+        def both():
+            behind()
+            self.rewrite()
+        self.calls = 0
+        self.rewrite()
+        super().run(out, both)
 
 
 @pytest.mark.parametrize("m,fp4", [(1, False), (8, False), (16, False), (40, True), (300, False), (1100, False), (1100, True)])
 def test_a_chain_without_synchronisation(cuda, atlas, m, fp4):
-    chain = Chain(cuda, atlas, m, fp4)
+    _same_bits(cuda, atlas, Chain(cuda, atlas, m, fp4))
+
+
+@pytest.mark.parametrize("m,fp4", [(1, False), (8, False), (40, True), (300, False), (1100, False)])
+def test_a_chain_over_rewritten_routing(cuda, atlas, m, fp4):
+    _same_bits(cuda, atlas, RewrittenRouting(cuda, atlas, m, fp4))
+
+
+def _same_bits(cuda, atlas, chain):
     want, got, captured = chain.outputs(), chain.outputs(), chain.outputs()
     chain.run(want, cuda.cuda.synchronize)
     chain.run(got, lambda: None)
