@@ -244,9 +244,9 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
     const size_t a_stride = p.seq_slot ? p.a_slot_stride : size_t(p.max_rank) * p.k_in * 2;
     if (mma_ok && p.M >= 1024 && !release_dependents && p.k_in % SHT_KSTAGE == 0 && p.max_rank % 16 == 0 && p.max_rank <= 256 &&
         n_slots <= 4096 && dst && dst->sm100 && g_encode && a_base && aligned(a_base, 16) && a_stride % 16 == 0 &&
-        (!p.tile_out || (p.part_rows && p.chunk % p.part_rows == 0))) {
+        (!p.tile_out || (p.part_rows && p.chunk % p.part_rows == 0 && p.chunk >= uint32_t(SHT_ROWS)))) {
         // a prefill batch: one cluster per 128 tokens and all ranks of all their adapters on the tcgen05 tensor cores,
-        // x read once (kernel_shrink_tc.cuh)
+        // x read once (kernel_shrink_tc.cuh); its rows lie in at most two token tiles
         if (!dst->shrink_tc_attr_set) {
             cudaError_t e = cudaFuncSetAttribute(lora_shrink_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SHT_SMEM_BYTES);
             if (e != cudaSuccess) return cuda_status(e);
@@ -265,7 +265,6 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
         }
         p.a_pool_base = nullptr;      // host-side fields: not part of what the kernel reads
         if (p.m_begin % 64 != 0 || p.m_begin >= p.M) return ATLAS_B200_ERR_DIMS;
-        if (p.tile_out && p.chunk && p.chunk < uint32_t(SHT_ROWS)) return ATLAS_B200_ERR_DIMS;   // a cluster's rows lie in at most two token tiles
         const uint32_t rows = p.m_count ? std::min(p.m_count, p.M - p.m_begin) : p.M - p.m_begin;
         // CTAs per 128 rows, each contracting a share of K: two, or four or eight where the clusters of the batch (the whole of it, not
         // this launch's range: a row's result must not depend on how the batch is cut into launches) are all resident at once — a

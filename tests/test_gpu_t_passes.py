@@ -174,3 +174,22 @@ def test_many_rows_of_a_slot(cuda, atlas, oracle, M, ads):
     rows, cols = _sample(case, 64, 96, M)
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,no_split", [(1100, 256, 128, False), (1025, 256, 640, False), (1500, 1024, 384, True), (2000, 512, 256, True)])
+def test_many_tokens_of_a_short_tile(cuda, atlas, oracle, M, K, N, no_split):
+    """More than 1024 tokens where few features leave token tiles of 64: masked tiles of that height, as with rows of t."""
+    from atlas_b200 import synth
+    case = synth.make_case("short", M=M, K=K, N=N, ranks=[16, 64, 8], max_rank=64, max_loras=4, ids="segments", segments=9, none_frac=0.1,
+                           scale2=0.02, b_std=0.1, seed=M)
+    dc = DeviceCase(cuda, atlas, case)
+    flags = atlas.FLAG_NO_K_SPLIT if no_split else 0
+    y, _ = dc.run(flags=flags, lora_ws=True)
+    shape = atlas.last_launch_shape()
+    assert shape["token_tile"] == 64 and shape["lora_tiles_from_shrink"]
+    build, _ = dc.run(flags=flags)
+    rows, cols = _sample(case, 200, 64, M)
+    want = ideal(oracle, case, rows=rows, cols=cols)
+    assert_close(oracle, y[np.ix_(rows, cols)], want, "tiles")
+    assert_close(oracle, build[np.ix_(rows, cols)], want, "rows of t")
+    assert atlas.device_status() == 0
