@@ -322,11 +322,23 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         waited_for_shrink = true;
                     }
                     const uint32_t t_row0 = ((tile_pass(i) * G + g) * 2u + cta_rank) * p.t_tile_cap * uint32_t(C::L_GRAN_T / 256);
-                    for (uint32_t q = 0; q < n_gran;) {
+                    // (granule by granule in a loop of its own: with many adapters of one granule the LoRA steps take as long as this thread
+                    //  and the MMA thread need to get round; 1000 tokens of 128 adapters of rank 16 x 14336 x 4096, this kernel alone, 138 us,
+                    //  153 in the loop below)
+                    for (uint32_t q = 0; lw == 1u && q < n_gran; ++q) {
+                        ok = mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
+                        if (!ok) break;
+                        const uint32_t base = epi0 + ls * C::L_STAGE, e = gran[g * C::MAX_GRANULES + q];
+                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * C::L_STAGE);
+                        tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
+                        tma_load_2d_pair(base + C::L_GRAN_A, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
+                        if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
+                    }
+                    for (uint32_t q = 0; lw > 1u && q < n_gran;) {
                         ok = mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
                         if (!ok) break;
                         const uint32_t base = epi0 + ls * (lw * C::L_STAGE), e = gran[g * C::MAX_GRANULES + q];
-                        const uint32_t n = lw > 1u ? min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw) : 1u;      // of this slot, from this granule on
+                        const uint32_t n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);      // of this slot, from this granule on
                         if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * (lw * C::L_GRAN_A + n * C::L_GRAN_T));
                         tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
                         for (uint32_t k = 0; k < n; ++k, ++q)
@@ -403,29 +415,31 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 }
                 for (uint32_t g = 0; ok && g < uint32_t(G); ++g) {
                     const uint32_t n_gran = p.seq_slot ? misc[4 + g] : 0u;
-                    for (uint32_t q = 0; q < n_gran;) {
+                    for (uint32_t q = 0; lw == 1u && q < n_gran; ++q) {
                         ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE);
-                        uint32_t n = 1u;
-                        const uint64_t lb = make_kmajor_sw32_desc(base + lw * C::L_GRAN_A);
-                        if (lw == 1u) {
-                            const uint64_t la = make_kmajor_desc(base, 1u);
-                            if (elect_one()) {
-                                umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
-                                umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
-                            }
-                        } else {
-                            const uint32_t e = gran[g * C::MAX_GRANULES + q];
-                            n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);
-                            const uint64_t la = make_kmajor_desc(base, lw);
-                            if (elect_one()) {
+                        const uint64_t la = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE);
+                        const uint64_t lb = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE + C::L_GRAN_A);
+                        if (elect_one()) {
+                            umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
+                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
+                        }
+                        __syncwarp();
+                        if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
+                    }
+                    for (uint32_t q = 0; lw > 1u && q < n_gran;) {
+                        ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
+                        if (!ok) break;
+                        tcgen05_fence_after();
+                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE), e = gran[g * C::MAX_GRANULES + q];
+                        const uint32_t n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);
+                        const uint64_t la = make_kmajor_desc(base, lw), lb = make_kmajor_sw32_desc(base + lw * C::L_GRAN_A);
+                        if (elect_one()) {
 #pragma unroll
-                                for (uint32_t k = 0; k < 4; ++k)     // 16 ranks = 32 bytes along the swizzled row of B_s; a block of masked t each
-                                    if (k < n) umma_bf16_ss<true>(tmem_acc + g * MT, la + 2 * k, lb + k * uint64_t(C::L_GRAN_T >> 4), idesc, 1u);
-                                umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
-                            }
+                            for (uint32_t k = 0; k < 4; ++k)         // 16 ranks = 32 bytes along the swizzled row of B_s; a block of masked t each
+                                if (k < n) umma_bf16_ss<true>(tmem_acc + g * MT, la + 2 * k, lb + k * uint64_t(C::L_GRAN_T >> 4), idesc, 1u);
+                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
                         }
                         __syncwarp();
                         q += n;
