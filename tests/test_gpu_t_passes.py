@@ -37,15 +37,22 @@ def test_granules_of_b_fetched_together(cuda, atlas, oracle, max_rank, ranks, fp
     assert atlas.device_status() == 0
 
 
-def test_granules_of_b_rank_128(cuda, atlas, oracle):
-    """Two copies of four granules per slot."""
+@pytest.mark.parametrize("max_rank,ranks", [(96, [96, 80, 8, 33]), (128, [128, 80, 64, 8])])
+def test_granules_of_b_above_rank_64(cuda, atlas, oracle, max_rank, ranks):
+    """Several copies to a slot: of two granules (96; one token tile per pass), of four (128, two token tiles).  (FP4 activations take
+    ranks up to 64.)"""
     from atlas_b200 import synth
-    case = synth.make_case("wide128", M=2085, K=512, N=4992, ranks=[128, 64, 80, 8], max_rank=128, none_frac=0.1, scale2=0.02, b_std=0.1, seed=4)
+    case = synth.make_case("wide128", M=2085, K=512, N=4992, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 1, none_frac=0.1, scale2=0.02,
+                           b_std=0.1, seed=4)
     dc = DeviceCase(cuda, atlas, case)
-    y, _ = dc.run(lora_ws=True)
-    assert atlas.last_launch_shape()["persistent_tiles_per_pass"] > 0
+    one, _ = dc.run(flags=atlas.FLAG_NO_PERSISTENT, lora_ws=True)
+    assert atlas.last_launch_shape()["persistent_tiles_per_pass"] == 0
+    for flags, tiles in ((0, 2), (atlas.FLAG_ONE_TILE_PASS, 1)):
+        y, _ = dc.run(flags=flags, lora_ws=True)
+        assert atlas.last_launch_shape()["persistent_tiles_per_pass"] == tiles
+        assert np.array_equal(y, one)
     rows, cols = _sample(case, 48, 64, 5)
-    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
+    assert_close(oracle, one[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "sample")
     assert atlas.device_status() == 0
 
 
