@@ -296,22 +296,12 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
     if (p.m_begin || p.m_count || p.n_tile_dest > 1) return ATLAS_B200_ERR_DIMS;      // a row range / several destinations: that kernel only
     if (mma_ok) {
         const uint32_t chunk = p.chunk ? p.chunk : uint32_t(SHM_CHUNK);
-        // CTAs per (slot, granule, chunk) sharing K: 8 for the sake of loads in flight; fewer when the dependent kernel
-        // runs beside this grid on a part of the machine only (a decode batch) and this grid would otherwise be so
-        // large that the dependent's CTAs find no room until it has drained
-        const size_t items = size_t(n_slots) * ((p.max_rank + SHM_RANKS - 1) / SHM_RANKS) * ((p.M + chunk - 1) / chunk);
-        uint32_t ksplit = SHM_KSPLIT;
-        while (release_dependents && dependent_leaves_sms_free && ksplit > 2 && items * ksplit > size_t(rt_sm_count()) * 4) ksplit >>= 1;
-        p.ksplit = ksplit;
-        // Clusters sharing the rows of each: one per 32 rows that a slot may have, as long as all of the grid is resident at once (CTAs
-        // without rows leave after their look at the routing).  One / several (us): 160 tokens, 2 adapters of rank 16 x 4096 x 4096
-        // 31.7 / 22.0, 130 tokens in sequences of 8 adapters of rank 64 32.5 / 23.4, the same tokens of mixed adapters 23.7 / 23.5.
-        const size_t resident = size_t(rt_sm_count()) * 8;
-        p.row_parts_log2 = 0;
-        while ((uint32_t(SHM_TOKENS) << p.row_parts_log2) < std::min(p.M, chunk) && (items * ksplit << (p.row_parts_log2 + 1)) <= resident) ++p.row_parts_log2;
-        // A is prefetched ahead of the wait by CTAs that are resident by then: of a larger grid most are not, and only look the routing up
-        // twice (512 tokens of 128 adapters of rank 16 x 14336 x 4096 92.3 -> 94.4 us).
-        if ((items * ksplit << p.row_parts_log2) > resident) p.a_pool_base = nullptr;
+        const MmaShrinkGrid rule = mma_shrink_grid(n_slots, (p.max_rank + SHM_RANKS - 1) / SHM_RANKS, (p.M + chunk - 1) / chunk, std::min(p.M, chunk),
+                                                   uint32_t(rt_sm_count()), !release_dependents ? MachineBeside::none
+                                                   : dependent_leaves_sms_free ? MachineBeside::part : MachineBeside::all);
+        const uint32_t ksplit = p.ksplit = rule.ksplit;
+        p.row_parts_log2 = rule.row_parts_log2;
+        p.prefetch_ctas = rule.prefetch_ctas;
         dim3 grid(n_slots * ksplit, (p.max_rank + SHM_RANKS - 1) / SHM_RANKS, ((p.M + chunk - 1) / chunk) << p.row_parts_log2);
         if (grid.y > 65535 || grid.z > 65535) return ATLAS_B200_ERR_LIMIT;
         cudaLaunchConfig_t cfg{};

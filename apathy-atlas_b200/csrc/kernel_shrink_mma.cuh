@@ -16,12 +16,13 @@
 // x, and of row g of A_s.  Elements 0..3 feed one MMA, 4..7 the next; x and A_s use the same
 // assignment, so each K element meets its partner and every 32-byte sector fetched is used in full.
 //
-// A slot with many rows in its chunk (a prefill batch of few sequences) is a chain of such passes of 32 rows: 2^ShrinkParams::row_parts_log2
-// clusters share them.
+// A slot with many rows in its chunk (a prefill batch of few sequences) is a chain of such passes of 32 rows:
+// 2^ShrinkParams::row_parts_log2 clusters share them.
 //
-// A CTA is small on purpose (128 threads, well under 64 registers): in the fused layer this grid runs
-// next to the tcgen05 kernel's CTAs on the same SMs (programmatic dependent launch), and must fit in
-// what that kernel leaves free.
+// A CTA is small on purpose (128 threads of 64 registers, 3 KB of shared memory): in the fused layer this grid runs next to
+// the tcgen05 kernel's CTAs on the same SMs (programmatic dependent launch), and must fit in what that kernel leaves free.
+// The compiler spills six words around the K loop.  Without them, the block's address kept in shared memory, it was slower
+// (160 tokens, 2 adapters of rank 16 x 4096 x 14336 38.4 us instead of 37.1, 8 of rank 16 39.1 instead of 37.3).
 //
 // Output rounding, rank handling and the uniform mode are those of lora_shrink_grouped_kernel, which
 // remains the path for shapes this kernel does not take (K not a multiple of 32, unaligned rows).
@@ -30,15 +31,16 @@
 #include <cooperative_groups.h>
 
 #include "kernels_simt.cuh"
+#include "share_rules.hpp"
 
 namespace atlas {
 namespace cg = cooperative_groups;
 
 constexpr int SHM_THREADS = 128;
 constexpr int SHM_RANKS = 16;     // ranks per CTA (two n-tiles of 8)
-constexpr int SHM_TOKENS = 32;    // tokens per pass (two m-tiles of 16)
+constexpr int SHM_TOKENS = MMA_SHRINK_PASS;    // tokens per pass (two m-tiles of 16)
 constexpr int SHM_CHUNK = 256;    // tokens scanned per CTA
-constexpr int SHM_KSPLIT = 8;     // CTAs per cluster, splitting K, at most (the launch picks 1, 2, 4 or 8: ShrinkParams::ksplit)
+constexpr int SHM_KSPLIT = MMA_SHRINK_KSPLIT;  // CTAs per cluster, splitting K, at most (the launch picks 2, 4 or 8: ShrinkParams::ksplit)
 
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
@@ -48,7 +50,7 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(SHM_THREADS, 8)
+__global__ void __launch_bounds__(SHM_THREADS, MMA_SHRINK_CTAS_PER_SM)
 lora_shrink_mma_kernel(ShrinkParams p) {
     __shared__ uint16_t rows[SHM_CHUNK];
     __shared__ float part[SHM_TOKENS][SHM_RANKS];          // this CTA's tile, read by the cluster's first CTA
@@ -67,8 +69,9 @@ lora_shrink_mma_kernel(ShrinkParams p) {
     // While the kernel ahead still runs: this granule of A_s into L2, the cluster's CTAs taking its lines in turn.  Nothing that
     // is read here decides anything but what is prefetched (the tables may be about to change: past the first-level cache, read
     // again below; only an address that is both in the table and in the declared pool is touched).  64 tokens, 64 adapters of
-    // mixed ranks, three projections of a decode layer (16 MB of A each): 109 -> 96 us.
-    if (p.seq_slot && p.a_pool_base && row_lo == 0) {
+    // mixed ranks, three projections of a decode layer (16 MB of A each): 109 -> 96 us.  Only by the CTAs that are resident by then: the
+    // others would look the routing up twice (1000 tokens of 64 adapters of rank 64 x 4096 x 4096 139.5 us, 142.7 if all do, 139.8 if none).
+    if (p.seq_slot && p.a_pool_base && row_lo == 0 && blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z) < p.prefetch_ctas) {
         const uint64_t a = __ldcg(p.a_table + s);
         const uint32_t rank = p.rank_table ? min(__ldcg(p.rank_table + s), p.max_rank) : p.max_rank;
         bool want = false;

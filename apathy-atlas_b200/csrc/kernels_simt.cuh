@@ -211,6 +211,7 @@ struct ShrinkParams {
     uint32_t part_rows;             // chunk or chunk / 2
     uint32_t ksplit;                // tensor-core shrink: CTAs per cluster sharing K (set by the launcher)
     uint32_t row_parts_log2;        // mma.sync shrink: clusters sharing the rows of a (slot, granule, chunk) (set by the launcher)
+    uint32_t prefetch_ctas;         // mma.sync shrink: the first CTAs of the grid, which prefetch A ahead of their wait (set by the launcher)
     // Token-sharded tile output (tcgen05 shrink only): the launch covers rows [m_begin, m_begin + m_count) of the batch
     // (m_count == 0: all of it) and writes every block row into n_tile_dest buffers of identical layout —
     // tile_out itself and tile_out_more[0 .. n_tile_dest - 2] (the same scratch on other GPUs, mapped into this process).

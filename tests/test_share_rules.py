@@ -11,6 +11,10 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 SOURCE = """
 #include "share_rules.hpp"
 extern "C" uint32_t next_own_granule(uint32_t g, uint32_t ks) { return atlas::next_own_granule(g, ks); }
+extern "C" void mma_shrink_grid(uint32_t slots, uint32_t granules, uint32_t chunks, uint32_t rows, uint32_t sms, int beside, uint32_t* out) {
+    const atlas::MmaShrinkGrid g = atlas::mma_shrink_grid(slots, granules, chunks, rows, sms, atlas::MachineBeside(beside));
+    out[0] = g.ksplit; out[1] = g.row_parts_log2; out[2] = g.prefetch_ctas;
+}
 """
 
 
@@ -36,3 +40,38 @@ def test_granules_of_a_k_split(rules, ks, n_gran):
             taken[g] = kz
             before, g = g, rules.next_own_granule(g, ks)
     assert taken == {g: (g // 4) % ks for g in range(n_gran)}
+
+
+NONE, PART, ALL = 0, 1, 2       # of the machine wanted by a dependent beside the grid
+
+
+def _grid(rules, slots, granules, chunks, rows, beside, sms=148):
+    out = (C.c_uint32 * 3)()
+    rules.mma_shrink_grid(slots, granules, chunks, rows, sms, beside, out)
+    return tuple(out)
+
+
+@pytest.mark.parametrize("slots,granules,chunks", [(1, 1, 1), (1, 8, 4), (2, 1, 4), (8, 1, 2), (8, 4, 2), (16, 1, 4), (37, 2, 1), (64, 4, 1), (4096, 8, 4)])
+@pytest.mark.parametrize("rows", [1, 32, 33, 130, 256])
+@pytest.mark.parametrize("beside", [NONE, PART, ALL])
+def test_grid_of_the_mma_shrink(rules, slots, granules, chunks, rows, beside):
+    """Row parts stay within what can be resident, and beside a kernel that wants the machine within half of it where more would mostly
+    be CTAs without rows."""
+    items, resident = slots * granules * chunks, 148 * 8
+    ksplit, log2, first = _grid(rules, slots, granules, chunks, rows, beside)
+    assert first == resident and ksplit in ((2, 4, 8) if beside == PART else (8,))
+    if ksplit < 8:
+        assert items * 2 * ksplit > resident // 2
+    if log2:
+        ctas = items * ksplit << log2
+        assert 32 << (log2 - 1) < rows and ctas <= resident
+        assert ctas <= resident // 2 or beside != ALL or rows >= slots * 32 << (log2 - 1) or chunks == 1 or (log2 == 1 and chunks == 2)
+
+
+def test_clusters_without_rows_do_not_fill_the_machine(rules):
+    assert _grid(rules, 8, 1, 2, 256, ALL)[:2] == (8, 2)       # 512 tokens of 8 adapters of rank 16: 512 CTAs, not 1024
+    assert _grid(rules, 8, 1, 4, 256, ALL)[:2] == (8, 1)       # 1000 tokens of them
+    assert _grid(rules, 16, 1, 4, 256, ALL)[:2] == (8, 0)      # ... of 16
+    assert _grid(rules, 8, 4, 2, 256, ALL)[:2] == (8, 1)       # rank 64, two chunks: two clusters
+    assert _grid(rules, 1, 8, 4, 256, ALL)[:2] == (8, 2)       # one adapter for all rows: 1024 CTAs with rows
+    assert _grid(rules, 8, 1, 4, 256, NONE)[:2] == (8, 2)
