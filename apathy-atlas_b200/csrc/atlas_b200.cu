@@ -1176,10 +1176,15 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
     // Base linear — a dense BF16 weight on the tensor cores where the shape allows, everything else on CUDA cores —
     // then the reference's two-stage LoRA in place
     const bool dense_tc = !(d.flags & ATLAS_B200_FLAG_FORCE_SIMT) && !staged && dense_tc_eligible(d);
-    // The shrink goes first where the base can run beside it (a batch whose shrink leaves it room): it waits for what is before the
-    // call, and the base then starts at once.  (Behind the base, with that
-    // kernel's former reduction: 16 tokens x 4096 x 4096, 4 adapters of rank 16 23.9 instead of 14.0 us.)
-    const bool shrink_first = dense_tc && d.seq_slot && d.m <= 1024;
+    // The shrink goes first where the base can run beside it: it waits for what is before the call, and the base then starts at once.
+    // That is where its grid is resident at once, and for few tokens and features.  Base first / shrink first (us), adapters x rank:
+    // 4096 x 4096, 16 tokens 4 x 16 19.6 / 14.2, 64 x 64 23.2 / 20.7, 100 tokens 128 x 16 35.8 / 30.3, 64 x 64 45.6 / 48.0, 300 tokens
+    // 128 x 16 50.6 / 54.2, 8 x 64 46.4 / 45.9, 1000 tokens 4 x 16 65.1 / 65.5, 8 x 64 89.7 / 95.6; 14336 x 4096, 64 tokens 4 x 16 42.7 /
+    // 40.8, 64 x 64 71.9 / 81.8; 1024 x 8192, 512 tokens 8 x 64 49.1 / 43.3, 64 x 64 78.7 / 87.1, 1000 tokens 4 x 16 51.0 / 41.1, 1500
+    // tokens 59.8 / 66.9.
+    const uint64_t shrink_ctas = uint64_t(d.max_loras) * ((d.max_rank + 15) / 16) * ((d.m + SHM_CHUNK - 1) / SHM_CHUNK) * SHM_KSPLIT;
+    const bool shrink_first = dense_tc && d.seq_slot && d.m <= 1024 &&
+                              (shrink_ctas <= uint64_t(rt_sm_count()) * MMA_SHRINK_CTAS_PER_SM || (d.m <= 64 && d.n <= 4096));
     auto base = [&]() { return dense_tc ? launch_dense_tc(d, shrink_first, st) : launch_simt_linear(d, st); };
     if (!shrink_first) {
         rc = base();
