@@ -338,7 +338,12 @@ static int launch_expand(const ExpandParams& p, cudaStream_t st) {
         while (splits * 2 <= most && uint64_t(cols) * chunks * splits * 2 <= uint64_t(rt_sm_count()) * 8) splits *= 2;
         const dim3 grid(cols, chunks * splits);
         if (grid.y > 65535) return ATLAS_B200_ERR_LIMIT;
-        if (p.max_rank <= 16) return launch_chained(lora_expand_mma_kernel<1>, grid, EXM_THREADS, st, p, chunk, splits);
+        // One granule: six CTAs on an SM, with two registers too few, where five of them would not be resident at once.  Five / six (us):
+        // dense base and 1000 tokens of 128 adapters of rank 16 x 14336 x 4096 (896 CTAs) 301 / 290; 256 tokens of 4 x 4096 x 4096 (512)
+        // 30.7 / 32.1.
+        if (p.max_rank <= 16)
+            return uint64_t(grid.x) * grid.y > uint64_t(rt_sm_count()) * 5 ? launch_chained(lora_expand_mma_kernel<1, 6>, grid, EXM_THREADS, st, p, chunk, splits)
+                                                                           : launch_chained(lora_expand_mma_kernel<1>, grid, EXM_THREADS, st, p, chunk, splits);
         if (p.max_rank <= 32) return launch_chained(lora_expand_mma_kernel<2>, grid, EXM_THREADS, st, p, chunk, splits);
         if (p.max_rank <= 64) return launch_chained(lora_expand_mma_kernel<4>, grid, EXM_THREADS, st, p, chunk, splits);
         return launch_chained(lora_expand_mma_kernel<8>, grid, EXM_THREADS, st, p, chunk, splits);

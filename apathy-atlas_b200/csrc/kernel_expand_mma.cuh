@@ -6,10 +6,10 @@
 //
 // A CTA owns 128 features (32 per warp) and up to 128 rows.  It sorts its rows by slot, so that sixteen consecutive rows
 // (the M of mma.sync.m16n8k16) hold few runs of one slot, and takes the runs in turn: B_s fragments stay in registers for as
-// long as the slot does not change, the next run's rows are on their way, the product of a run starts from zero and is folded into the run's rows alone.  (Rows of
-// other slots in the same sixteen are computed and dropped, not masked with zeros: an infinity in one adapter's B must not
-// reach another adapter's rows.)  A decode batch has few rows and as many runs as adapters, each waiting for its B_s:
-// `splits` CTAs share the runs of a chunk.
+// long as the slot does not change, the next run's rows are on their way, the product of a run starts from zero and is folded
+// into the run's rows alone.  (Rows of other slots in the same sixteen are computed and dropped, not masked with zeros: an
+// infinity in one adapter's B must not reach another adapter's rows.)  A decode batch has few rows and as many runs as
+// adapters, each waiting for its B_s: `splits` CTAs share the runs of a chunk.
 //
 // Fragments: in every 16-wide K step the thread of quad lane t holds ranks 4t..4t+3 of xa rows g, g+8 and of its B row (64-bit
 // loads; both operands use the same assignment, so each rank meets its partner).  The four n-tiles of a warp interleave
@@ -26,9 +26,9 @@ constexpr int EXM_ROWS = 128;        // rows of a chunk: one per thread while th
 constexpr int EXM_OUTS = 128;        // features per CTA
 constexpr int EXM_MAX_RANK = 128;    // B_s fragments of 32 features are held in registers: 64 at this rank
 
-// KS: 16-wide K steps held in registers, >= ceil(max_rank / 16)
-template <int KS>
-__global__ void __launch_bounds__(EXM_THREADS, KS >= 8 ? 3 : (KS >= 4 ? 4 : 5))
+// KS: 16-wide K steps held in registers, >= ceil(max_rank / 16); CTAS on an SM
+template <int KS, int CTAS = KS >= 8 ? 3 : (KS >= 4 ? 4 : 5)>
+__global__ void __launch_bounds__(EXM_THREADS, CTAS)
 lora_expand_mma_kernel(ExpandParams p, uint32_t chunk, uint32_t splits) {
     constexpr bool AHEAD = KS <= 4;                          // xa too (more of it does not fit beside B_s)
     __shared__ __align__(16) uint32_t slot_in[EXM_ROWS];     // slot, ~0 for a row without a term
