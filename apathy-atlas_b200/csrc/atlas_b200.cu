@@ -863,13 +863,18 @@ static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* sh
     // to 18944 features, and beyond, CTAs at different points of their lives fill each other's gaps.  Eight / four warps, 1 and 8
     // tokens, 8 adapters of rank 16 (us): 11008 x 4096 15.9 / 14.0, 21.4 / 16.7; 14336 x 4096 17.9 / 16.3, 22.1 / 19.5; 28672 x 8192
     // 48.1 / 45.4, 56.8 / 52.3; but 8192 x 8192 (256 CTAs) 17.1 / 18.6, 19.7 / 25.9.
-    // Granules are shared by half as many warps then.  8 tokens, 8 adapters of rank 64: 14336 x 4096 30.8 / 29.7, x 5120 35.4 / 36.2, 14848 x
-    // 6912 44.0 / 49.8; of rank 128: 37.5 / 41.5, 43.6 / 49.8, 52.5 / 61.7.  (By what the pool may hold, not by the batch: a token's sums are
-    // the same in any batch of up to eight.)
-    const uint32_t granules = d.seq_slot ? std::min(d.max_loras, uint32_t(DCM_MAX_TOKENS)) * ((d.max_rank + 15) / 16) : 0u;
-    const bool four = granules <= (d.k <= 4096 ? 32u : 8u);
-    const uint32_t slots = 2u * uint32_t(rt_sm_count());
+    // The batch's granules are shared by half as many warps then, which the longer loop pays for less and less as K grows.  Eight /
+    // four warps (us) by granules: 14336 x 4096, 16 23.6 / 21.1, 32 28.7 / 27.9, 64 33.4 / 37.1; x 5120, 16 28.5 / 26.1, 32 33.4 / 34.2;
+    // x 6912, 8 29.2 / 28.0, 16 32.9 / 36.8; x 2048, 32 20.8 / 18.8.  Beyond eight tokens, 8 and 16: 14336 x 4096 25.4 / 24.3, 28.2 /
+    // 28.3, x 5120 29.4 / 29.0, 31.5 / 37.1, x 6912 36.0 / 39.0, 39.5 / 48.2, but 11008 x 4096, hardly more than a wave of eight-warp
+    // CTAs, 25.1 / 20.7, 28.1 / 24.4.  Beyond one wave of four-warp CTAs, 8 and 16 whatever K: 28672 x 4096 34.5 / 34.0, 42.9 / 45.2, x
+    // 8192 55.0 / 54.7, 60.9 / 64.1, 16 tokens 71.1 / 69.7, 78.9 / 89.5; 8 of one adapter x 4096 31.2 / 32.5.
+    // (Both forms give the same bits.)
     const bool few = d.m <= 8;
+    const uint32_t slots = 2u * uint32_t(rt_sm_count());
+    const uint64_t granules = d.seq_slot ? std::min(d.max_loras, d.m) * ((d.max_rank + 15) / 16) : 0u, k = few ? std::max(d.k, 4096u) : d.k;
+    const bool four = d.n > 64u * slots ? granules <= 8u && d.max_rank <= 64u
+                                        : granules * k * k * k * (few ? 1u : (d.n <= 40u * slots ? 2u : 4u)) <= 32ull * 4096 * 4096 * 4096;
     if (d.n <= 16u * slots) return few ? launch_decode_as<1, 1, 8>(d, shrink, st) : launch_decode_as<1, 2, 8>(d, shrink, st);
     if (d.n <= 32u * slots || !four) return few ? launch_decode_as<2, 1, 8>(d, shrink, st) : launch_decode_as<2, 2, 8>(d, shrink, st);
     return few ? launch_decode_as<2, 1, 4>(d, shrink, st) : launch_decode_as<2, 2, 4>(d, shrink, st);

@@ -146,11 +146,11 @@ def test_small_batches_of_four_and_eight_warps(cuda, atlas, oracle, M, K, N):
     assert atlas.device_status() == 0
 
 
-@pytest.mark.parametrize("M", [1, 7, 8, 13, 16])
-def test_small_batches_have_the_bits_of_any_pool(cuda, atlas, oracle, M):
-    """Four warps to a CTA (a pool of two slots, no pool at all) and eight (one of twenty): the same partial sums."""
+@pytest.mark.parametrize("M,max_rank", [(1, 16), (7, 64), (8, 64), (13, 32), (16, 16)])
+def test_small_batches_have_the_bits_of_any_pool(cuda, atlas, oracle, M, max_rank):
+    """Four warps to a CTA (a pool of two slots, no pool at all) and, from seven tokens on, eight (one of twenty): the same partial sums."""
     from atlas_b200 import synth
-    case = synth.make_case("pools", M=M, K=4352, N=9488, ranks=[16, 8], max_rank=16, none_frac=0.3, scale2=0.02, b_std=0.1, seed=M)
+    case = synth.make_case("pools", M=M, K=4352, N=9488, ranks=[max_rank, 8], max_rank=max_rank, none_frac=0.3, scale2=0.02, b_std=0.1, seed=M)
     if M > 2:
         case.seq_slot[:3] = (0, 1, -1)
     small, _ = DeviceCase(cuda, atlas, case).run()
