@@ -339,7 +339,7 @@ static int launch_expand(const ExpandParams& p, cudaStream_t st) {
         const dim3 grid(cols, chunks * splits);
         if (grid.y > 65535) return ATLAS_B200_ERR_LIMIT;
         // One granule: six CTAs on an SM, with two registers too few, where five of them would not be resident at once.  Five / six (us):
-        // dense base and 1000 tokens of 128 adapters of rank 16 x 14336 x 4096 (896 CTAs) 301 / 290; 256 tokens of 4 x 4096 x 4096 (512)
+        // dense base and 1000 tokens of 128 adapters of rank 16 x 14336 x 4096 (896 CTAs) 302 / 293; 256 tokens of 4 x 4096 x 4096 (512)
         // 30.7 / 32.1.
         if (p.max_rank <= 16)
             return uint64_t(grid.x) * grid.y > uint64_t(rt_sm_count()) * 5 ? launch_chained(lora_expand_mma_kernel<1, 6>, grid, EXM_THREADS, st, p, chunk, splits)
@@ -657,8 +657,9 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = 0u; t_last_shape[5] = 0u;
     if (shrink) {
-        // A small batch: let this kernel start under the shrink.  A large one: the shrink is a sizeable grid that
-        // should have the whole machine first; this kernel then follows it.
+        // A small batch: the mma.sync shrink releases this kernel as soon as it is resident, which then runs beside it.  A large one:
+        // the tcgen05 shrink fills its SMs and releases this kernel at the same point, whose CTAs then take SMs that are free or
+        // become so; the mma.sync shrink, where it has to stand in, keeps the machine to itself.
         const uint32_t main_ctas = grid.x * grid.y * grid.z;
         const int rc = launch_shrink(*shrink, d.max_loras, st, d.m <= 1024, main_ctas * 3 <= uint32_t(rt_sm_count()) * 2);
         if (rc) return rc;
@@ -666,8 +667,8 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     p.profile = (g_profile_buf && size_t(grid.x) * grid.y * tc::PROFILE_WORDS <= g_profile_words) ? g_profile_buf : nullptr;
     if (grid.y > 65535) return ATLAS_B200_ERR_LIMIT;
     // Launched as a programmatic dependent of the shrink that precedes it in the stream: its CTAs
-    // may start while the shrink still runs (the shrink releases them as soon as it is resident) and
-    // wait for the shrink's completion only where they first read t, after the base K loop.
+    // may start while the shrink still runs (see above) and wait for the shrink's completion only
+    // where they first read t, after the base K loop.
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(tc::NUM_THREADS);
@@ -835,18 +836,18 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):
-//   no adapters          1 token     1024 x 4096 5/9    4096 x 4096 7/12   14336 x 4096 17/28   4096 x 14336 17/26   28672 x 8192 51/95
-//                        16 tokens   1024 x 4096 6/10   4096 x 4096 9/12   14336 x 4096 21/28   4096 x 14336 24/27   28672 x 8192 63/96
-//   8 of rank 16         1 token     1024 x 4096 6/11   4096 x 4096 8/14   14336 x 4096 20/30   4096 x 14336 18/29   28672 x 8192 55/101
-//                        8 tokens    1024 x 4096 7/12   4096 x 4096 10/15  14336 x 4096 23/31   8192 x 8192 21/32    28672 x 8192 64/102
-//                        16 tokens                                         14336 x 4096 27/31                        28672 x 8192 73/103
-//   8 of rank 64         8 tokens    1024 x 4096 11/13  4096 x 4096 16/17  14336 x 4096 29/33   8192 x 8192 30/34    28672 x 8192 80/107
+//   no adapters          1 token     1024 x 4096 4/9    4096 x 4096 6/12   14336 x 4096 15/26   4096 x 14336 15/25   28672 x 8192 45/90
+//                        16 tokens   1024 x 4096 5/9    4096 x 4096 9/12   14336 x 4096 19/26   4096 x 14336 23/25   28672 x 8192 59/91
+//   8 of rank 16         1 token     1024 x 4096 6/10   4096 x 4096 7/14   14336 x 4096 17/28   4096 x 14336 16/27   28672 x 8192 48/94
+//                        8 tokens    1024 x 4096 7/11   4096 x 4096 9/14   14336 x 4096 20/29   8192 x 8192 20/30    28672 x 8192 55/95
+//                        16 tokens                                         14336 x 4096 25/29                        28672 x 8192 70/96
+//   8 of rank 64         8 tokens    1024 x 4096 9/12   4096 x 4096 16/15  14336 x 4096 28/32   8192 x 8192 30/31    28672 x 8192 72/101
 // With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does: up
 // to eight tokens there unless the weights (N >= 2 K) outweigh it, and a long K only as long as the shrink is short (4096 x 14336,
-// 7 tokens: eight of rank 32 25/30, of rank 64 37/32; 6 tokens of rank 64 32/31).
+// 7 tokens: eight of rank 32 24/28, of rank 64 35/29; 6 tokens: eight of rank 64 32/29, sixteen 32/36).
 // Beyond eight tokens a granule (16 ranks of a slot) costs it some 0.3 us more than the tcgen05 form, against what it gains on the
-// weights: most where those are more than one wave of tiles there.  N >= 2 K, 16 adapters, 16 tokens: 32 granules 14336 x 4096 38/36,
-// 16384 x 6144 53/47, 28672 x 8192 100/110; 64 granules 47/43, 74/59, 122/122; 96 granules (12 tokens) 28672 x 8192 135/140.
+// weights: most where those are more than one wave of tiles there.  N >= 2 K, 16 adapters, 16 tokens: 32 granules 14336 x 4096 32/31,
+// 16384 x 6144 47/42, 28672 x 8192 88/101; 64 granules 37/35, 60/48, 103/107.
 static bool decode_pays(const atlas_b200_linear_desc& d) {
     if (d.m > uint32_t(DCM_MAX_TOKENS)) return false;
     if (!d.seq_slot) return true;
@@ -1047,9 +1048,11 @@ static TcPlan plan_tc(const atlas_b200_linear_desc& d, uint32_t flags, bool shri
     p.two_tiles = p.persistent && !act_fp4 && !(flags & ATLAS_B200_FLAG_ONE_TILE_PASS) && d.m >= 768;
     if (p.two_tiles) {
         // ... unless whole waves say otherwise: the last wave costs a full pass however few CTA pairs it holds, and a pass of two
-        // 192-token tiles takes about 1.4 times as long as one of a 256-token tile.  One-tile / two-tile calls by waves (us,
-        // K = 4096; K = 14336): 2 : 2 83 / 109; 209 / 303   5 : 4 158 / 172; 495 / 544   4 : 3 129 / 140; 374 / 414   7 : 5 206 / 207;
-        // 686 / 683   3 : 2 110 / 108; 291 / 286   6 : 4 178 / 171; 579 / 552.  The line lies between 4 : 3 and 7 : 5.
+        // 192-token tiles takes 1.2 (K = 4096) to 1.4 times as long as one of a 256-token tile.  One-tile / two-tile calls by waves, calls
+        // with pauses between them (us, K = 4096; K = 14336): 2 : 2 82 / 101; 227 / 310   4 : 3 122 / 131; 364 / 396   5 : 4 133 / 144;
+        // 412 / 464   7 : 5 202 / 210; 645 / 675   3 : 2 98 / 98; 276 / 283   25 : 17 658 / 645   2 : 1 60 / 61; 159 / 156.  Call upon
+        // call the power limit sets the clock, and two tiles, which expand a weight once for both, need less of it: with 7 : 5 on the
+        // other side of the line a layer of 8192 tokens took 2.73 instead of 2.69 ms.  The line lies between 4 : 3 and 7 : 5.
         const int c2 = persist_resident_clusters<192, 2, false>(2), c1 = persist_resident_clusters<256, 1, false>(0);
         if (c1 > 0 && c2 > 0) {
             const uint64_t w2 = (persist_tiles<192, 2>(d) + uint32_t(c2) - 1) / uint32_t(c2);

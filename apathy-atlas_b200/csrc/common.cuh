@@ -36,9 +36,12 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 //                              main kernel or of the dense linear
 //   neither                    a main kernel without adapters releases but is launched in order; the NVFP4 decode, the maximum, the
 //                              CUDA-core linear and expand do neither
-// A dependent begins with the wait.  Only the main kernel and the dense linear behind their shrink read anything ahead of it (x, weights,
-// routing), and that shrink has waited before releasing them; they wait before they read t, or before they end, on every path, so that
-// nothing behind them overtakes the shrink.
+// A dependent begins with the wait, with two exceptions:
+//   the main kernel and the dense linear behind their shrink read x, weights and routing ahead of it: that shrink has waited before
+//   releasing them; they wait before they read t, or before they end, on every path, so that nothing behind them overtakes the shrink;
+//   lora_shrink_mma_kernel looks at seq_slot, a_table and rank_table while the kernel ahead may still be writing them.  Those values
+//   only choose lines of A to prefetch, out of the declared pool alone; they are read past the first-level cache, and everything is
+//   read again behind the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The pointer as a value that does not exist before this point: keeps read-only loads through it behind pdl_wait().

@@ -4,11 +4,11 @@
 //
 // A decode batch is bound by streaming the weights once.  The tcgen05 form cannot keep up with that stream: its weight operand
 // goes through tensor memory, which fixes the order of the K elements (four byte permutes per eight codes), and its
-// eight expansion warps need 585 cycles per 128 x 64 block whatever the batch: one token x 14336 features x 4096 took 30 us
-// for 33 MB.  Here every warp of the SM expands, the operand stays in the registers the codes were expanded in, and since
-// BOTH operands of mma.sync come from registers the K elements may take any order as long as they meet their partners:
-// the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired the same way (four permutes
-// per eight elements of x, shared by all features of the warp).
+// eight expansion warps are busy for 540 cycles per 128 x 64 block whatever the batch, 650 with their waits: one token x 14336
+// features x 4096 takes 26 us for 33 MB, 15 here.  Here every warp of the SM expands, the operand stays in the registers the
+// codes were expanded in, and since BOTH operands of mma.sync come from registers the K elements may take any order as long as
+// they meet their partners: the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired
+// the same way (four permutes per eight elements of x, shared by all features of the warp).
 //
 // A CTA owns 16 * TILES features and all of K.  Interleaved 128-wide K steps make eight partial sums, one to each of eight warps or
 // two to each of four (with as many more CTAs on an SM): the same bits, so that either form may be taken for any batch and pool, and

@@ -139,8 +139,9 @@ dense_bf16_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __g
         tcgen05_fence_before();
         __syncwarp();
         cluster_sync_all();                              // every CTA's partial tile is in its shared memory
-        // Tokens kz, kz + ks, ... by this CTA, four at a time, all their loads in flight before the first sum.  (All of them by
-        // the first CTA, sum by sum, were a chain of remote latencies: this kernel 11.5 -> 7.7 us for 16 tokens x 4096 x 4096.)
+        // Tokens kz, kz + ks, ... by this CTA, two at a time (four from tiles of 64 tokens on), all their loads in flight before the
+        // first sum.  (All of them by the first CTA, sum by sum, were a chain of remote latencies: this kernel 11.5 -> 7.7 us for
+        // 16 tokens x 4096 x 4096.)
         if (warp >= 2 && acc_ready) {
             const uint32_t te = tid - 64;                // 0..127 = feature within the tile
             const uint32_t f = f0 + te;

@@ -39,7 +39,7 @@ def test_values_far_below_the_maximum(cuda, atlas, oracle, scale2):
 
 @pytest.mark.parametrize("total,offset", [(1, 0), (7, 0), (8, 0), (4097, 0), (16 * 148 * 256 * 8 * 4 + 8, 0), (1000001, 0), (4096, 1)])
 def test_maximum(cuda, atlas, oracle, total, offset):
-    """Fewer values than a load, remainders of the unrolled loop, an address that allows no vector loads; NaN gives way."""
+    """Fewer values than a load, a remainder behind several turns of the whole grid, an address that allows no vector loads; NaN gives way."""
     g = np.random.default_rng(total)
     w = (g.integers(0, 0x4000, total + offset).astype(np.uint16)) | (g.integers(0, 2, total + offset).astype(np.uint16) << 15)
     w[offset + total - 1] = 0xC123
