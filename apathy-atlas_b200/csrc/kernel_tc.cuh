@@ -57,12 +57,9 @@ constexpr int KB = 64;               // K elements per MMA stage (one 128-byte s
 constexpr int KRAW = 256;            // K elements per raw weight stage
 constexpr int RAW_PACKED_BYTES = FT * (KRAW / 2);    // 16 KiB
 constexpr int RAW_SCALE_BYTES = FT * (KRAW / 16);    // 2 KiB
-// Expansion warps come in groups of eight (one warp per TMEM quadrant and K half).  With G groups, group
-// i expands K blocks i, i+G, ... of each raw stage.  One group measured best: a second group does not
-// shorten the K loop (which is bound by shared-memory bandwidth at 256 tokens and by the MMA thread's
-// issue rate below) and takes issue slots from the MMA thread.
-constexpr int DEQ_GROUPS = 1;
-constexpr int DEQ_WARP0 = 6, DEQ_GROUP_WARPS = 8, DEQ_WARPS = 8 * DEQ_GROUPS, DEQ_THREADS = 32 * DEQ_WARPS;
+// Eight expansion warps: one per TMEM quadrant and K half.  (A second eight shorten the K loop by a tenth, but then the shrink finds no
+// registers beside this kernel: 256 tokens x 17408 x 5120 46 -> 56 us.)
+constexpr int DEQ_WARP0 = 6, DEQ_WARPS = 8, DEQ_THREADS = 32 * DEQ_WARPS;
 constexpr int RAW_WARP = DEQ_WARP0 + DEQ_WARPS;      // TMA producer of the raw weight stages
 constexpr int NUM_THREADS = 32 * (RAW_WARP + 1);
 constexpr int EPI_WARP0 = 2, EPI_THREADS = 128;
@@ -92,6 +89,9 @@ constexpr int MAX_DEST = 8;            // tensor-parallel ranks whose output buf
 template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int XROWS = PAIR ? MT / 2 : MT;                       // token rows of the tile this CTA stages
     static constexpr int X_TILE_BYTES = XROWS * KB * 2;
+    // A16: a stage of activations is two K blocks: a round of the MMA thread (wait, MMAs, commit) takes some 340 cycles and 9 for every
+    // MMA of 16 columns, whatever it covers; with a round to a K block and a wait for either operand it was what the loop waited for
+    static constexpr int X_STAGE_BYTES = 2 * X_TILE_BYTES;
     // A4: one stage = packed W [128 x 128 B] | packed x [MT x 128 B] | W scale bytes [128 x 16] | x scale bytes [MT x 16]
     static constexpr int S4_W = 0;
     static constexpr int S4_X = S4_W + RAW_PACKED_BYTES;
@@ -99,11 +99,17 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int S4_XS = S4_WS + RAW_SCALE_BYTES;
     static constexpr int S4_BYTES = ((S4_XS + MT * 16) + 1023) / 1024 * 1024;
     static constexpr int S4_STAGES = (200 * 1024) / S4_BYTES > 8 ? 8 : (200 * 1024) / S4_BYTES;
-    static constexpr int STAGES = A4 ? S4_STAGES : (XROWS >= 256 ? 5 : 8);
+    static constexpr int STAGES = A4 ? S4_STAGES : (XROWS >= 256 ? 2 : 4);
     // raw weight stages in flight: small token tiles leave shared memory free, and they are the
     // HBM-bound shapes that need many bytes in flight per SM
     static constexpr int RAW_STAGES = A4 ? STAGES : (XROWS >= 256 ? 2 : (XROWS >= 128 ? 4 : 6));
-    static constexpr int A_COLS = KB / 2;                                  // TMEM columns of one weight-operand stage
+    // A16: the weight operand's ring in TMEM, two groups of the four K blocks of a raw stage.  A group changes hands as one: tcgen05.wait::st
+    // takes some 250 cycles whatever it waits for, a wait for the MMAs 80, and the arithmetic of four K blocks 760.  One token x 14336
+    // features x 4096: an expansion warp was busy for 546 cycles a K block with a hand-over per pair of them, 349 of them without its
+    // arithmetic; 344 now, and with stages of two K blocks of activations the base loop went from 41.7 to 24.8 thousand cycles, the
+    // call from 26 to 19 us (17 tokens, 8 adapters of rank 16 29.1 -> 22.2).
+    static constexpr int A_COLS = KB / 2;                                  // TMEM columns of one K block
+    static constexpr int A_GROUP = KRAW / KB;
     static constexpr int TMEM_A_BASE = MT < 32 ? 32 : MT;                  // accumulator occupies [0, MT)
     // A4: scale factors in TMEM.  One instruction reads, per operand, 4 scale bytes (one 32-bit column
     // entry) for each of its rows; lane l of every 32-lane quadrant holds rows l, l+32, l+64, l+96 of a
@@ -111,12 +117,12 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     // instructions x (4 columns per 128 tokens).
     static constexpr int XSF_BLOCKS = MT > 128 ? MT / 128 : 1;
     static constexpr int SF_COLS = 16 + 16 * XSF_BLOCKS;
-    static constexpr int TMEM_NEEDED = TMEM_A_BASE + (A4 ? STAGES * SF_COLS : STAGES * A_COLS);
+    static constexpr int TMEM_NEEDED = TMEM_A_BASE + (A4 ? STAGES * SF_COLS : 2 * A_GROUP * A_COLS);
     static constexpr int TMEM_COLS = TMEM_NEEDED <= 64 ? 64 : TMEM_NEEDED <= 128 ? 128 : TMEM_NEEDED <= 256 ? 256 : 512;
     static constexpr int MAX_GRANULES = MT * (MAX_RANK_TC / 16);
     // shared memory map (offsets from a 1024-byte aligned base)
     static constexpr int OFF_X = 0;
-    static constexpr int OFF_RAWP = OFF_X + STAGES * X_TILE_BYTES;
+    static constexpr int OFF_RAWP = OFF_X + STAGES * X_STAGE_BYTES;
     static constexpr int OFF_RAWS = OFF_RAWP + RAW_STAGES * RAW_PACKED_BYTES;
     static constexpr int STAGING_BASE = A4 ? STAGES * S4_BYTES : OFF_RAWS + RAW_STAGES * RAW_SCALE_BYTES;
     // After the base K loop the whole staging area is re-used for the LoRA K blocks: each block holds up
@@ -131,7 +137,7 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int OFF_GRAN = OFF_KEY + MT * 4;                            // uint16[MAX_GRANULES]
     static constexpr int OFF_BITMAP = OFF_GRAN + MAX_GRANULES * 2;               // uint32[128]
     static constexpr int OFF_BAR = OFF_BITMAP + (MAX_LORAS_TC / 32) * 4;         // mbarriers
-    static constexpr int NUM_BARS = 2 * STAGES + 2 * RAW_STAGES + 4 + 2 * L_STAGES;
+    static constexpr int NUM_BARS = 2 * STAGES + 2 * RAW_STAGES + 4 + 2 * L_STAGES + 4;
     static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;                      // tmem ptr, n_gran, abort
     static constexpr int SMEM_BYTES = OFF_MISC + 32 + 1024;                      // + alignment slack
     static_assert(!PAIR || MT >= 128, "pairs are built for token tiles of 128 and 256");
@@ -731,9 +737,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     uint16_t* gran = reinterpret_cast<uint16_t*>(smem_gen + C::OFF_GRAN);
     uint32_t* bitmap = reinterpret_cast<uint32_t*>(smem_gen + C::OFF_BITMAP);
     const uint32_t bar0 = smem_base + C::OFF_BAR;
-    // FULL[s]: both operands of stage s are in place.  DEQ_GROUP_WARPS + 1 arrivals per phase: the eight
-    // expansion warps, plus the TMA producer (with the tile's byte count) for a base K block or one
-    // extra arrival by an expansion thread for a LoRA K block, whose activation tile they build.
+    // FULL[s]: what TMA brings for stage s is in place (A4: its block scales in tensor memory too); AFULL[g]: group g of the weight operand.
     const uint32_t BAR_FULL = bar0;                                    // [STAGES] operands -> MMA
     const uint32_t BAR_EMPTY = bar0 + 8 * C::STAGES;                   // [STAGES] MMA -> producers
     const uint32_t BAR_FULL_RAW = bar0 + 16 * C::STAGES;               // [C::RAW_STAGES]
@@ -744,6 +748,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     const uint32_t BAR_LEMPTY = BAR_LFULL + 8 * C::L_STAGES;           // [L_STAGES] MMA -> LoRA operand build
     const uint32_t BAR_DRAINED = BAR_LEMPTY + 8 * C::L_STAGES;         // every expansion warp is done with the staging area
     const uint32_t BAR_EPI = BAR_DRAINED + 8;                          // every epilogue warp has put its part of the tile into shared memory
+    const uint32_t BAR_AFULL = BAR_EPI + 8, BAR_AEMPTY = BAR_AFULL + 16;   // [2] each, A16: groups of the weight operand
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + C::OFF_MISC);
     // misc[0] = TMEM base address, misc[1] = granule count, misc[2] = abort flag, misc[3] = slots that occur in the tile
     volatile uint32_t* abort_flag = misc + 2;
@@ -776,8 +781,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 
     if (tid == 0) {
         for (int i = 0; i < C::STAGES; ++i) {
-            // A16: every expansion warp of the pair writes part of a stage; A4: the four warps of one half do
-            mbar_init(BAR_FULL + 8 * i, CTAS * (A4 ? DEQ_GROUP_WARPS / 2 : DEQ_GROUP_WARPS) + 1);     // used in the pair's first CTA only
+            // (used in the pair's first CTA only)  A4: the four warps of one half carry a stage's scales
+            mbar_init(BAR_FULL + 8 * i, (A4 ? CTAS * (DEQ_WARPS / 2) : 0u) + 1u);
             mbar_init(BAR_EMPTY + 8 * i, 1);
         }
         for (int i = 0; i < C::RAW_STAGES; ++i) {
@@ -788,6 +793,10 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         mbar_init(BAR_LIST, 1);
         mbar_init(BAR_DRAINED, DEQ_WARPS);
         mbar_init(BAR_EPI, EPI_WARPS);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(BAR_AFULL + 8 * i, CTAS * DEQ_WARPS);
+            mbar_init(BAR_AEMPTY + 8 * i, 1);
+        }
         for (int i = 0; i < C::L_STAGES; ++i) {
             mbar_init(BAR_LFULL + 8 * i, p.t_tile_cap ? 1u : CTAS * DEQ_WARPS + 1);
             mbar_init(BAR_LEMPTY + 8 * i, 1);
@@ -816,13 +825,14 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     tcgen05_fence_after();
     // barriers the MMA thread waits on live in the pair's first CTA; everyone else arrives there
     const uint32_t full_at_leader = PAIR ? map_to_cta(BAR_FULL, leader_rank) : BAR_FULL;
+    const uint32_t afull_at_leader = PAIR ? map_to_cta(BAR_AFULL, leader_rank) : BAR_AFULL;
     const uint32_t lfull_at_leader = PAIR ? map_to_cta(BAR_LFULL, leader_rank) : BAR_LFULL;
     auto arrive_at_leader = [&](uint32_t bar_at_leader) {
         if constexpr (PAIR) mbar_arrive_cluster(bar_at_leader); else mbar_arrive(bar_at_leader);
     };
     pdl_release();
     const uint32_t tmem_acc = misc[0];
-    const uint32_t tmem_a0 = tmem_acc + C::TMEM_A_BASE;   // A16: weight-operand stages [tmem_a0 + s * A_COLS, + A_COLS);
+    const uint32_t tmem_a0 = tmem_acc + C::TMEM_A_BASE;   // A16: K block j of group g of the weight operand [tmem_a0 + (A_GROUP g + j) * A_COLS, + A_COLS);
                                                           // A4: scale-factor stages [tmem_a0 + s * SF_COLS, + SF_COLS)
 
     if (warp == 0) {
@@ -855,12 +865,15 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             // CTAs start their K loop at different K offsets (a rotation in units of one raw stage),
             // so concurrently running CTAs do not all pull the same activation lines at one moment.
             uint32_t s = 0, ph = 0;
-            for (uint32_t it = 0; it < num_kb; ++it) {
+            for (uint32_t it = 0; it < num_kb; it += 2) {
                 if (!mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
-                if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, CTAS * C::X_TILE_BYTES);
-                const uint32_t kb = kb_lo + (it + 4u * rot_raw) % num_kb;
-                if constexpr (PAIR) tma_load_2d_pair(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(mx0), full_at_leader + 8 * s);
-                else tma_load_2d(x_tile0 + s * C::X_TILE_BYTES, &map_x, int32_t(kb * KB), int32_t(m0), BAR_FULL + 8 * s);
+                const uint32_t n = SROWS && it + 1u == num_kb ? 1u : 2u;
+                if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, CTAS * n * C::X_TILE_BYTES);
+                for (uint32_t u = 0; u < n; ++u) {
+                    const uint32_t kb = kb_lo + (it + u + 4u * rot_raw) % num_kb, dst = x_tile0 + s * C::X_STAGE_BYTES + u * C::X_TILE_BYTES;
+                    if constexpr (PAIR) tma_load_2d_pair(dst, &map_x, int32_t(kb * KB), int32_t(mx0), full_at_leader + 8 * s);
+                    else tma_load_2d(dst, &map_x, int32_t(kb * KB), int32_t(m0), BAR_FULL + 8 * s);
+                }
                 if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
             }
         }
@@ -930,26 +943,30 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; bar_full = BAR_FULL; bar_empty = BAR_EMPTY; st = smem_base; sf = tmem_a0; }
                 }
             } else {
-                uint32_t a_tmem = tmem_a0;
-                uint64_t b_desc = make_kmajor_sw128_desc(x_tile0);
-                constexpr uint64_t b_desc_step = uint64_t(C::X_TILE_BYTES >> 4);
-                for (uint32_t it = 0; it < num_kb; ++it) {
-                    ok = mbar_wait_warp_timed(bar_full, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
+                static_assert(C::A_GROUP == 4, "two stages of activations to a group of the weight operand");
+                for (uint32_t it = 0; it < num_kb; it += 2) {
+                    const uint32_t j = it % 4u, g = (it / 4u) & 1u, a_tmem = tmem_a0 + (g * C::A_GROUP + j) * C::A_COLS;
+                    // one wait for both operands: half of the lanes poll the group's barrier
+                    const bool on_a = j == 0u && lane >= 16u;
+                    ok = mbar_wait_warp_timed(on_a ? BAR_AFULL + 8 * g : bar_full, on_a ? (it / 8u) & 1u : ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
                     tcgen05_fence_after();
+                    const uint64_t b_desc = make_kmajor_sw128_desc(x_tile0 + s * C::X_STAGE_BYTES);
                     if (elect_one()) {
                         // 16 k per instruction: 8 TMEM columns of A, 32 bytes along the swizzled row of B
 #pragma unroll
                         for (uint32_t i = 0; i < 4; ++i) umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 8 * i, b_desc + 2 * i, idesc, acc | i);
+                        if (!SROWS || it + 1u < num_kb)
+#pragma unroll
+                            for (uint32_t i = 0; i < 4; ++i)
+                                umma_bf16_ts<PAIR>(tmem_acc, a_tmem + C::A_COLS + 8 * i, b_desc + uint64_t(C::X_TILE_BYTES >> 4) + 2 * i, idesc, 1u);
                         umma_commit<PAIR>(bar_empty, pair_mask);
+                        if (j || it + 2u >= num_kb) umma_commit<PAIR>(BAR_AEMPTY + 8 * g, pair_mask);
                     }
                     __syncwarp();
                     acc = 1u;
-                    bar_full += 8; bar_empty += 8; a_tmem += C::A_COLS; b_desc += b_desc_step;
-                    if (++s == uint32_t(C::STAGES)) {
-                        s = 0; ph ^= 1u;
-                        bar_full = BAR_FULL; bar_empty = BAR_EMPTY; a_tmem = tmem_a0; b_desc -= b_desc_step * C::STAGES;
-                    }
+                    bar_full += 8; bar_empty += 8;
+                    if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; bar_full = BAR_FULL; bar_empty = BAR_EMPTY; }
                 }
             }
             if (prof && lane == 0) { prof_row[14] = (unsigned long long)(clock64() - t_begin); prof_row[15] = w_full; }
@@ -1082,10 +1099,9 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         // ========================== NVFP4 -> BF16 weight operand, into TMEM ======================
         // warp w may touch TMEM lanes [32 (w % 4), +32): it owns those 32 features; the two warps
         // of a quadrant split each K block in halves of 32.  K blocks are expanded two at a time so
-        // that each warp has two independent dependency chains in flight.
+        // that each warp has two independent dependency chains in flight, and handed over four at a time (Cfg::A_GROUP).
         const uint32_t q = warp & 3u;
         const uint32_t half = ((warp - DEQ_WARP0) >> 2) & 1u;
-        const uint32_t grp = (warp - DEQ_WARP0) >> 3;       // expansion group of this warp
         const uint32_t row = q * 32 + lane;
         const uint32_t td = tid - DEQ_WARP0 * 32;
         const uint32_t lane_base = (q * 32u) << 16;
@@ -1093,7 +1109,6 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         unsigned long long w_raw = 0, w_empty = 0;
         const long long t_begin = clock64();
         const uint32_t num_raw = (num_kb + 3u) / 4u;
-        uint32_t s = grp, ph = 0;                            // stage / phase of this group's next K block
         uint32_t rs = 0, rph = 0;
         if constexpr (A4) {
             // Block scales, shared memory -> registers -> TMEM.  The warp of quadrant q writes lanes
@@ -1101,7 +1116,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             // rows l, l+32, l+64, l+96 of the 128-row block), so the four warps of a half write the same
             // values.  The halves take alternate stages (both operands' scales), so that one stage's
             // load -> store -> wait chain runs under the other's.
-            s = 0;
+            uint32_t s = 0, ph = 0;
             for (uint32_t it = 0; ok && it < num_kb; ++it) {
                 if ((it & 1u) != half) {
                     if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
@@ -1190,20 +1205,19 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             }
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j) scw[j] = e4m3x4_clear_nan(scw[j]);
+            const uint32_t g = ri & 1u, a_group = tmem_a0 + lane_base + g * (C::A_GROUP * C::A_COLS) + 16 * half;
 #pragma unroll
-            for (uint32_t jr = 0; jr < 4; jr += 2 * DEQ_GROUPS) {
-                if (ri * 4 + jr + grp >= num_kb) break;
-                const bool two = ri * 4 + jr + grp + DEQ_GROUPS < num_kb;
+            for (uint32_t jr = 0; jr < 4; jr += 2) {
+                if (SROWS && ri * 4 + jr >= num_kb) break;           // (otherwise raw stages are whole)
                 uint32_t o[2][16];
 #pragma unroll
                 for (uint32_t u = 0; u < 2; ++u) {
-                    const uint32_t j = jr + grp + DEQ_GROUPS * u;       // K block of the raw stage (0..3)
+                    const uint32_t j = jr + u;                          // K block of the raw stage (0..3)
                     // 32 codes of this row: logical chunk 2j + half of the swizzled 128-byte raw row
                     const uint4 pk = lds128(rawp0 + rs * RAW_PACKED_BYTES + sw128_off(row, 2 * j + half));
                     const uint32_t pw[4] = {pk.x, pk.y, pk.z, pk.w};
-                    const uint32_t scj = j == 0 ? scw[0] : (j == 1 ? scw[1] : (j == 2 ? scw[2] : scw[3]));
                     uint32_t mul0, mul1;                                        // of scale bytes 2 * half, 2 * half + 1 of word j
-                    e4m3x2_to_bf16x2_shifted(scj, half ? 0x4342u : 0x4140u, mul0, mul1);
+                    e4m3x2_to_bf16x2_shifted(scw[j], half ? 0x4342u : 0x4140u, mul0, mul1);
 #pragma unroll
                     for (uint32_t qd = 0; qd < 4; ++qd) {
                         uint32_t o4[4];
@@ -1211,33 +1225,23 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                         o[u][4 * qd] = o4[0]; o[u][4 * qd + 1] = o4[1]; o[u][4 * qd + 2] = o4[2]; o[u][4 * qd + 3] = o4[3];
                     }
                 }
-                const uint32_t s0 = s, ph0 = ph;
-                uint32_t s1 = s0 + DEQ_GROUPS, ph1 = ph0;
-                if (s1 >= uint32_t(C::STAGES)) { s1 -= C::STAGES; ph1 ^= 1u; }
-                ok = mbar_wait_timed(BAR_EMPTY + 8 * s0, ph0 ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
-                if (!ok) break;
-                tcgen05_fence_after();
-                // this thread's 32 k of its feature row: 16 columns at 16 * half of the stage
-                tmem_st16(tmem_a0 + lane_base + s0 * C::A_COLS + 16 * half, o[0]);
-                if (two) {
-                    ok = mbar_wait_timed(BAR_EMPTY + 8 * s1, ph1 ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
+                if (jr == 0u) {
+                    ok = mbar_wait_timed(BAR_AEMPTY + 8 * g, ((ri >> 1) & 1u) ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
                     if (!ok) break;
                     tcgen05_fence_after();
-                    tmem_st16(tmem_a0 + lane_base + s1 * C::A_COLS + 16 * half, o[1]);
                 }
-                tmem_st_wait();
-                tcgen05_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    arrive_at_leader(full_at_leader + 8 * s0);
-                    if (two) arrive_at_leader(full_at_leader + 8 * s1);
-                }
-                s = s1 + DEQ_GROUPS; ph = ph1;
-                if (s >= uint32_t(C::STAGES)) { s -= C::STAGES; ph ^= 1u; }
+                // this thread's 32 k of its feature row: 16 columns of a K block's 32
+#pragma unroll
+                for (uint32_t u = 0; u < 2; ++u) tmem_st16(a_group + (jr + u) * C::A_COLS, o[u]);
             }
             if (!ok) break;
+            tmem_st_wait();
+            tcgen05_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(BAR_EMPTY_RAW + 8 * rs);
+            if (lane == 0) {
+                arrive_at_leader(afull_at_leader + 8 * g);
+                mbar_arrive(BAR_EMPTY_RAW + 8 * rs);
+            }
             if (++rs == uint32_t(C::RAW_STAGES)) { rs = 0; rph ^= 1u; }
         }
         }
@@ -1258,17 +1262,18 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         if (p.wait_for_shrink) pdl_wait();
         const uint32_t n_gran = ok ? misc[1] : 0u;
         const uint32_t n_lb = (n_gran + 3u) / 4u;
-        s = num_kb % uint32_t(C::STAGES);                    // stage / phase the K block after the last one would take
-        ph = (num_kb / uint32_t(C::STAGES)) & 1u;
         if (ok && n_lb > 0) {
             // the staging area is about to be overwritten: every base MMA must have read its x tile,
             // and every expansion warp must be done with the raw weight stages
-            {
-                uint32_t ss = s, pp = ph;
+            if constexpr (A4) {
+                uint32_t ss = num_kb % uint32_t(C::STAGES), pp = (num_kb / uint32_t(C::STAGES)) & 1u;      // where the stage after the last would go
                 for (int i = 0; ok && i < C::STAGES; ++i) {
                     ok = mbar_wait(BAR_EMPTY + 8 * ss, pp ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT);
                     if (++ss == uint32_t(C::STAGES)) { ss = 0; pp ^= 1u; }
                 }
+            } else {
+                // (the last group's; of the stages of x this warp has not waited for any, and several uses of one may be open)
+                ok = mbar_wait(BAR_AEMPTY + 8 * ((num_raw - 1u) & 1u), ((num_raw - 1u) >> 1) & 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT);
             }
             // (an mbarrier rather than bar.sync, so that this wait is bounded like every other one)
             __syncwarp();

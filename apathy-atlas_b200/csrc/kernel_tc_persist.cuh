@@ -169,7 +169,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
 
     if (tid == 0) {
         for (int i = 0; i < C::STAGES; ++i) {
-            mbar_init(BAR_FULL + 8 * i, 2 * (A4 ? DEQ_GROUP_WARPS / 2 : DEQ_GROUP_WARPS) + 1);
+            mbar_init(BAR_FULL + 8 * i, 2 * (A4 ? DEQ_WARPS / 2 : DEQ_WARPS) + 1);
             mbar_init(BAR_EMPTY + 8 * i, 1);
         }
         for (int i = 0; i < C::RAW_STAGES; ++i) {

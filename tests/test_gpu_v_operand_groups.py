@@ -1,0 +1,49 @@
+"""Operands handed over in groups: four K blocks of the expanded weights, two of the activations.  Lengths that leave part of a group and
+rings that wrap, on scratch that holds garbage: within the path's tolerance of the oracle, and the same bits call for call."""
+import numpy as np
+import pytest
+
+from gpu_util import DeviceCase, assert_close, ideal
+
+pytestmark = pytest.mark.gpu
+
+MIXED = [16, 64, 8, 48, 32, 64, 16, 24, 56, 64, 40, 16]
+
+
+def _sample(case, seed):
+    rng = np.random.default_rng(seed)
+    pick = lambda n, k: np.sort(rng.choice(n, min(n, k), replace=False)).astype(np.uint32)
+    return pick(case.M, 48), pick(case.N, 96)
+
+
+# K blocks of 64: 4, 8, 12, 20, 36 of them, and 5, 7, 8 (the last half full), 12 (half full), 45
+@pytest.mark.parametrize("form", ["", "single", "unsplit"])
+@pytest.mark.parametrize("K", [256, 512, 768, 1280, 2304, 288, 416, 480, 736, 2880])
+@pytest.mark.parametrize("M", [20, 60, 130, 250])
+def test_every_length_of_the_base_loop(cuda, atlas, oracle, M, K, form):
+    from atlas_b200 import synth
+    case = synth.make_case("groups", M=M, K=K, N=376, ranks=MIXED, max_rank=64, max_loras=13, none_frac=0.15, scale2=0.02, b_std=0.1, seed=M + K)
+    dc = DeviceCase(cuda, atlas, case)
+    flags = {"": 0, "single": atlas.FLAG_NO_CTA_PAIR, "unsplit": atlas.FLAG_NO_K_SPLIT}[form]
+    y, variant = dc.run(flags=flags, lora_ws=True)
+    assert variant == atlas.VARIANT_TCGEN05
+    rows, cols = _sample(case, K)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), form)
+    for _ in range(3):                                   # fresh scratch every time
+        assert np.array_equal(dc.run(flags=flags, lora_ws=True)[0], y)
+    assert atlas.device_status() == 0
+
+
+# two K blocks of 256-token tiles on their own hold two stages: a ring that wraps before the expansion has waited for it
+@pytest.mark.parametrize("K", [1280, 2560, 4096])
+def test_a_ring_of_two_stages(cuda, atlas, oracle, K):
+    from atlas_b200 import synth
+    case = synth.make_case("two_stages", M=256, K=K, N=8704, ranks=[32] * 16, max_rank=32, none_frac=0.1, scale2=0.02, b_std=0.1, seed=K)
+    dc = DeviceCase(cuda, atlas, case)
+    y, _ = dc.run(flags=atlas.FLAG_NO_CTA_PAIR, lora_ws=True)
+    assert not atlas.last_launch_shape()["cta_pair"]
+    rows, cols = _sample(case, K)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "single")
+    for _ in range(5):
+        assert np.array_equal(dc.run(flags=atlas.FLAG_NO_CTA_PAIR, lora_ws=True)[0], y)
+    assert atlas.device_status() == 0
