@@ -64,13 +64,17 @@ template <int MT, int G, bool A4> struct PCfg {
     static_assert(!A4 || G == 1, "FP4 activations: one token tile per pass");
     static constexpr int XROWS = MT / 2;                                   // token rows of a tile this CTA stages
     static constexpr int X_TILE_BYTES = XROWS * KB * 2;
-    static constexpr int X_STAGE_BYTES = G * X_TILE_BYTES;
+    // K blocks of a stage of both operands of the base loop: two where shared memory allows it, for fewer waits, arrivals and commits
+    // (tc::Cfg).  8192 tokens x 14336 x 4096 by one-tile passes 949 -> 875 thousand cycles a CTA.  (Groups of four K blocks of the weight operand,
+    // as in the one-tile kernel, need a barrier and a commit of their own here: 1049; passes of two tiles 930 -> 937.)
+    static constexpr int XB = G == 1 && !A4 ? 2 : 1;
+    static constexpr int X_STAGE_BYTES = XB * G * X_TILE_BYTES;
     static constexpr int S4_W = 0;
     static constexpr int S4_X = S4_W + RAW_PACKED_BYTES;
     static constexpr int S4_BYTES = S4_X + XROWS * 128;
     // A4: the block scales of two K blocks at a time, rows of 32 bytes (SWIZZLE_32B): W [128 x 32 B] | x [MT x 32 B]
     static constexpr int S4_SCALES = (FT + MT) * A4_SCALE_ROW;
-    static constexpr int A_COLS = KB / 2;
+    static constexpr int A_COLS = KB / 2, A_STAGE_COLS = XB * A_COLS;
     static constexpr int XSF_BLOCKS = MT > 128 ? MT / 128 : 1;
     static constexpr int SF_COLS = 16 + 16 * XSF_BLOCKS;
     static constexpr int ACC_COLS = G * MT;
@@ -81,10 +85,10 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int L_STAGE = L_GRAN_A + L_GRAN_T;
     static constexpr int L_STAGES = EPI_BYTES / L_STAGE > 16 ? 16 : EPI_BYTES / L_STAGE;
     // ring depths: what the 227 KB of shared memory and the 512 columns of tensor memory leave
-    static constexpr int STAGES = A4 ? 4 : (G == 1 ? 6 : 3);
+    static constexpr int STAGES = A4 ? 4 : 3;
     static constexpr int RAW_STAGES = G == 1 && !A4 ? 3 : 2;             // (A4: of block scales)
     static constexpr int TMEM_A_BASE = ACC_COLS;
-    static constexpr int TMEM_NEEDED = TMEM_A_BASE + (A4 ? STAGES * SF_COLS : STAGES * A_COLS);
+    static constexpr int TMEM_NEEDED = TMEM_A_BASE + (A4 ? STAGES * SF_COLS : STAGES * A_STAGE_COLS);
     static constexpr int TMEM_COLS = 512;
     static constexpr int MAX_GRANULES = MT * (MAX_RANK_TC / 16);
     static constexpr int OFF_X = 0;
@@ -252,15 +256,17 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             for (uint32_t i = 0; ok && i < my_tiles; ++i) {
                 const uint32_t m0 = tile_pass(i) * (MT * G);
                 const uint32_t rot_raw = tile_fpair(i) % num_raw;
-                for (uint32_t it = 0; it < num_kb; ++it) {
+                for (uint32_t it = 0; it < num_kb; it += C::XB) {
                     ok = mbar_wait(BAR_EMPTY + 8 * xs, xph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER);
                     if (!ok) break;
                     if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * xs, 2 * C::X_STAGE_BYTES);
                     const uint32_t kb = (it + 4u * rot_raw) % num_kb;
 #pragma unroll
-                    for (uint32_t g = 0; g < uint32_t(G); ++g)
-                        tma_load_2d_pair(x_tile0 + xs * C::X_STAGE_BYTES + g * C::X_TILE_BYTES, &map_x, int32_t(kb * KB),
-                                         int32_t(m0 + g * MT + cta_rank * C::XROWS), full_at_leader + 8 * xs);
+                    for (uint32_t u = 0; u < uint32_t(C::XB); ++u)
+#pragma unroll
+                        for (uint32_t g = 0; g < uint32_t(G); ++g)
+                            tma_load_2d_pair(x_tile0 + xs * C::X_STAGE_BYTES + (u * G + g) * C::X_TILE_BYTES, &map_x, int32_t((kb + u) * KB),
+                                             int32_t(m0 + g * MT + cta_rank * C::XROWS), full_at_leader + 8 * xs);
                     if (++xs == uint32_t(C::STAGES)) { xs = 0; xph ^= 1u; }
                 }
             }
@@ -387,19 +393,21 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                     }
                 } else {
-                    for (uint32_t it = 0; it < num_kb; ++it) {
+                    for (uint32_t it = 0; it < num_kb; it += C::XB) {
                         if (prof && it == 4) w_head += w_full - w_full_at_pass;
                         ok = mbar_wait_warp_timed(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        const uint32_t a_tmem = tmem_a0 + s * C::A_COLS;
+                        const uint32_t a_tmem = tmem_a0 + s * C::A_STAGE_COLS;
                         const uint64_t b_desc = make_kmajor_sw128_desc(x_tile0 + s * C::X_STAGE_BYTES);
                         if (elect_one()) {
 #pragma unroll
-                            for (uint32_t g = 0; g < uint32_t(G); ++g)
+                            for (uint32_t u = 0; u < uint32_t(C::XB); ++u)
 #pragma unroll
-                                for (uint32_t j = 0; j < 4; ++j)
-                                    umma_bf16_ts<true>(tmem_acc + g * MT, a_tmem + 8 * j, b_desc + g * uint64_t(C::X_TILE_BYTES >> 4) + 2 * j, idesc, acc | j);
+                                for (uint32_t g = 0; g < uint32_t(G); ++g)
+#pragma unroll
+                                    for (uint32_t j = 0; j < 4; ++j)
+                                        umma_bf16_ts<true>(tmem_acc + g * MT, a_tmem + u * C::A_COLS + 8 * j, b_desc + (u * G + g) * uint64_t(C::X_TILE_BYTES >> 4) + 2 * j, idesc, acc | u | j);
                             umma_commit<true>(BAR_EMPTY + 8 * s, pair_mask);
                         }
                         __syncwarp();
@@ -711,26 +719,29 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                                 o[u][4 * qd] = o4[0]; o[u][4 * qd + 1] = o4[1]; o[u][4 * qd + 2] = o4[2]; o[u][4 * qd + 3] = o4[3];
                             }
                         }
-                        const uint32_t s0 = s, ph0 = ph;
-                        uint32_t s1 = s0 + 1, ph1 = ph0;
-                        if (s1 >= uint32_t(C::STAGES)) { s1 -= C::STAGES; ph1 ^= 1u; }
-                        ok = mbar_wait_timed(BAR_EMPTY + 8 * s0, ph0 ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
+                        // the two K blocks: one stage, or one each
+                        uint32_t s1 = s, ph1 = ph;
+                        if (C::XB == 1 && ++s1 == uint32_t(C::STAGES)) { s1 = 0; ph1 ^= 1u; }
+                        const uint32_t a_tmem = tmem_a0 + lane_base + 16 * half;
+                        ok = mbar_wait_timed(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        tmem_st16(tmem_a0 + lane_base + s0 * C::A_COLS + 16 * half, o[0]);
-                        ok = mbar_wait_timed(BAR_EMPTY + 8 * s1, ph1 ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
-                        if (!ok) break;
-                        tcgen05_fence_after();
-                        tmem_st16(tmem_a0 + lane_base + s1 * C::A_COLS + 16 * half, o[1]);
+                        tmem_st16(a_tmem + s * C::A_STAGE_COLS, o[0]);
+                        if (C::XB == 1) {
+                            ok = mbar_wait_timed(BAR_EMPTY + 8 * s1, ph1 ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_empty);
+                            if (!ok) break;
+                            tcgen05_fence_after();
+                        }
+                        tmem_st16(a_tmem + s1 * C::A_STAGE_COLS + (C::XB - 1) * C::A_COLS, o[1]);
                         tmem_st_wait();
                         tcgen05_fence_before();
                         __syncwarp();
                         if (lane == 0) {
-                            mbar_arrive_cluster(full_at_leader + 8 * s0);
-                            mbar_arrive_cluster(full_at_leader + 8 * s1);
+                            mbar_arrive_cluster(full_at_leader + 8 * s);
+                            if (C::XB == 1) mbar_arrive_cluster(full_at_leader + 8 * s1);
                         }
-                        s = s1 + 1; ph = ph1;
-                        if (s >= uint32_t(C::STAGES)) { s -= C::STAGES; ph ^= 1u; }
+                        s = s1; ph = ph1;
+                        if (++s == uint32_t(C::STAGES)) { s = 0; ph ^= 1u; }
                     }
                     if (!ok) break;
                     __syncwarp();
