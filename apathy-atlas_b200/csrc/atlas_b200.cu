@@ -467,6 +467,12 @@ static bool b_pool_is_strided(const atlas_b200_linear_desc& d) {
            d.max_rank % 8 == 0;
 }
 
+// Granules of B_s that one copy may bring: a copy of 128 rows takes as long for one of 16 ranks as for four of a slot.  With it, and one copy
+// of masked t for a K block (us, by granules / so): 64 tokens of 64 adapters of rank 64 x 14336 x 4096 82.9 / 75.4 on the one-tile kernel.
+static uint32_t granules_per_copy(const atlas_b200_linear_desc& d) {
+    return !b_pool_is_strided(d) ? 1u : (d.max_rank % 64 == 0 ? 4u : (d.max_rank % 32 == 0 ? 2u : 1u));
+}
+
 // Where the shrink's masked-t tiles live in `ws` (tiles == nullptr: the fused kernel builds them itself from lora_t)
 struct TTiles {
     uint16_t* tiles = nullptr;
@@ -474,13 +480,13 @@ struct TTiles {
     uint32_t part_rows = 0;    // rows of a block: the token tile, or half of it for CTA pairs
 };
 
-// The six tensor maps of a tcgen05 launch.  `xrows` = token rows of an activation tile one CTA stages, `mt` = token
+// The tensor maps of a tcgen05 launch (`b`: one granule of B_s, `bw`: `lora_wide` of them).  `xrows` = token rows of an activation tile one CTA stages, `mt` = token
 // tile, `l_gran_t` = bytes of one masked-t block as the shrink writes it ([part_rows x 16] BF16).
-struct TcMaps { CUtensorMap x, w, s, b, xs, t; };
+struct TcMaps { CUtensorMap x, w, s, b, bw, xs, t; };
 
-// `a4_scale_row` = scale bytes per row of a stage (FP4 activations), `lora_wide` = granules of B_s per copy.
+// `t_blocks` = masked-t blocks per copy, `a4_scale_row` = scale bytes per row of a stage (FP4 activations).
 static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xrows, uint32_t mt, uint32_t l_gran_t,
-                          const TTiles& tt, TcMaps& m, uint32_t a4_scale_row = tc::KRAW / 16, uint32_t lora_wide = 1) {
+                          const TTiles& tt, TcMaps& m, uint32_t t_blocks, uint32_t a4_scale_row = tc::KRAW / 16, uint32_t lora_wide = 1) {
     const CUtensorMapSwizzle scale_swizzle = a4_scale_row == 32 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE;
     if (a4) {
         // the quantised activations in `ws`, in the weights' own layout
@@ -506,19 +512,23 @@ static int encode_tc_maps(const atlas_b200_linear_desc& d, bool a4, uint32_t xro
     if (b_pool_is_strided(d)) {
         const uint64_t dims[3] = {d.max_rank, d.n, d.max_loras};
         const uint64_t strides[2] = {uint64_t(d.max_rank) * 2, uint64_t(d.b_slot_stride)};
-        const uint32_t box[3] = {16 * lora_wide, tc::FT, 1};
-        if (!encode_tiled(&m.b, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d.b_pool_base, dims, strides, box,
-                          lora_wide == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : (lora_wide == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B)))
-            return ATLAS_B200_ERR_DIMS;
+        auto encode_b = [&](CUtensorMap& map, uint32_t granules) {
+            const uint32_t box[3] = {16 * granules, tc::FT, 1};
+            return encode_tiled(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, d.b_pool_base, dims, strides, box,
+                                granules == 4 ? CU_TENSOR_MAP_SWIZZLE_128B : (granules == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B));
+        };
+        if (!encode_b(m.bw, lora_wide)) return ATLAS_B200_ERR_DIMS;
+        m.b = m.bw;
+        if (lora_wide > 1 && !encode_b(m.b, 1)) return ATLAS_B200_ERR_DIMS;
     } else {
-        m.b = m.s;   // never dereferenced
+        m.b = m.bw = m.s;   // never dereferenced
     }
     if (!a4) m.xs = m.s;   // never dereferenced
     if (tt.tiles) {
-        // the masked-t blocks are shared-memory images already: plain bytes, 256 to a row, one block per copy
+        // the masked-t blocks are shared-memory images already: plain bytes, 256 to a row, `t_blocks` blocks per copy
         const uint64_t rows = uint64_t((d.m + mt - 1) / mt) * tt.cap * mt * 32 / 256;
         if (l_gran_t % 256 != 0 ||
-            !encode_2d(&m.t, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, tt.tiles, 256, rows, 256, 256, l_gran_t / 256, CU_TENSOR_MAP_SWIZZLE_NONE))
+            !encode_2d(&m.t, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, tt.tiles, 256, rows, 256, 256, t_blocks * l_gran_t / 256, CU_TENSOR_MAP_SWIZZLE_NONE))
             return ATLAS_B200_ERR_DIMS;
     } else {
         m.t = m.s;         // never dereferenced
@@ -634,17 +644,19 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     }
     TcMaps maps;
     const bool b_strided = b_pool_is_strided(d);
+    const uint32_t lora_wide = granules_per_copy(d);
     {
-        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps);
+        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, 4, tc::KRAW / 16, lora_wide);
         if (rc) return rc;
     }
-    const CUtensorMap &map_x = maps.x, &map_w = maps.w, &map_s = maps.s, &map_b = maps.b, &map_xs = maps.xs, &map_t = maps.t;
+    const CUtensorMap &map_x = maps.x, &map_w = maps.w, &map_s = maps.s, &map_b = maps.b, &map_bw = maps.bw, &map_xs = maps.xs, &map_t = maps.t;
 
     tc::Params p{};
     {
         const int rc = fill_tc_params(d, A4, b_strided, tt, p);
         if (rc) return rc;
     }
+    p.lora_wide = lora_wide;
     dim3 grid((d.n + tc::FT - 1) / tc::FT, (d.m + MT - 1) / MT);
     if (PAIR) grid.x = (grid.x + 1u) & ~1u;      // whole pairs: a CTA past the last feature loads zeros and stores nothing
     // split K: k_split CTAs along z form a cluster (times two for pairs), share one tile and exchange partial sums;
@@ -691,7 +703,7 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     p.wait_for_shrink = after_shrink ? 1u : 0u;
-    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS, ISO>, map_x, map_w, map_s, map_b, map_xs, map_t, p));
+    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_kernel<MT, A4, PAIR, SROWS, ISO>, map_x, map_w, map_s, map_b, map_bw, map_xs, map_t, p));
 }
 
 template <int MT, bool A4, bool PAIR>
@@ -753,13 +765,10 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     using C = tc::PCfg<MT, G, A4>;
     const int clusters = persist_resident_clusters<MT, G, A4, ISO>(idx);
     if (clusters <= 0) return ATLAS_B200_ERR_DIMS;
-    // Granules of B_s per copy: a copy of 128 rows takes as long for one granule as for four.  Two in the ring of a one-tile BF16
-    // pass, which holds only two stages of four, and slots of lower rank leave part of a stage unused (thousand cycles, two / four:
-    // ranks 8 to 64, 1237 tokens x 14336 x 4096 162.8 / 165.1; FP4, rank 64, 8192 tokens 376 / 362).
-    const uint32_t lora_wide = d.max_rank % 64 == 0 && (A4 || G == 2) ? 4u : (d.max_rank % 32 == 0 ? 2u : 1u);
+    const uint32_t lora_wide = std::min(granules_per_copy(d), uint32_t(C::LB));
     TcMaps maps;
     {
-        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, tc::A4_SCALE_ROW, lora_wide);
+        const int rc = encode_tc_maps(d, A4, C::XROWS, MT, C::L_GRAN_T, tt, maps, C::LB, tc::A4_SCALE_ROW, lora_wide);
         if (rc) return rc;
     }
     tc::Params p{};
@@ -772,7 +781,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     pp.n_fpairs = ((d.n + tc::FT - 1) / tc::FT + 1) / 2;
     pp.n_passes = (d.m + MT * G - 1) / (MT * G);
     pp.n_tiles = pp.n_fpairs * pp.n_passes;
-    pp.lora_wide = d.seq_slot ? lora_wide : 1u;
+    p.lora_wide = lora_wide;
     const uint32_t pairs = std::min<uint32_t>(uint32_t(clusters), pp.n_tiles);
     t_last_shape[0] = MT; t_last_shape[1] = 1u; t_last_shape[2] = 1u; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs;
@@ -801,7 +810,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     cfg.attrs = attr;
     cfg.numAttrs = n_attr;
     p.wait_for_shrink = shrink ? 1u : 0u;
-    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4, ISO>, maps.x, maps.w, maps.s, maps.b,
+    return cuda_status(cudaLaunchKernelEx(&cfg, tc::nvfp4_lora_linear_tc_persistent_kernel<MT, G, A4, ISO>, maps.x, maps.w, maps.s, maps.b, maps.bw,
                                           maps.xs, maps.t, p, pp));
 }
 

@@ -67,8 +67,9 @@ constexpr int EPI_WARPS = 4 + DEQ_WARPS;   // warps that take part in the epilog
 constexpr int MAX_LORAS_TC = 4096;
 constexpr int MAX_RANK_TC = 128;
 // a granule list entry: slot << GRAN_SHIFT | which 16 ranks of the slot (4096 slots of up to eight granules in 16 bits)
-constexpr uint32_t GRAN_SHIFT = 3, GRAN_MASK = 7;
-static_assert(MAX_RANK_TC / 16 <= int(GRAN_MASK) + 1 && (MAX_LORAS_TC << GRAN_SHIFT) <= 65536, "granule list entries are 16 bits");
+// GRAN_WIDE (one-tile kernel): it and the next Params::lora_wide - 1 come in one copy
+constexpr uint32_t GRAN_SHIFT = 3, GRAN_MASK = 7, GRAN_WIDE = 0x8000u;
+static_assert(MAX_RANK_TC / 16 <= int(GRAN_MASK) + 1 && (MAX_LORAS_TC << GRAN_SHIFT) <= int(GRAN_WIDE), "granule list entries are 16 bits");
 constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;    // 1 s
 constexpr int PROFILE_WORDS = 16;
 constexpr int MAX_DEST = 8;            // tensor-parallel ranks whose output buffers one launch can store into
@@ -166,6 +167,7 @@ struct Params {
     uint32_t t_tile_cap;           // != 0: the shrink wrote masked-t tiles (ShrinkParams::tile_out) with this many blocks
                                    //       reserved per token tile; they are fetched by TMA (map_t) and `t` is not read
     uint32_t b_pool_strided;       // B_s tiles can be fetched by TMA from a [max_loras][N][max_rank] strided pool ...
+    uint32_t lora_wide;            // granules of B_s that may come in one copy: 1, 2 or 4
     unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
@@ -557,6 +559,33 @@ template <int N> __device__ __forceinline__ void cp_async_wait_group() { asm vol
 // byte offset of logical 16-byte chunk `c` (0..7) of row `r` in a SWIZZLE_128B tile of 128-byte rows
 __device__ __forceinline__ uint32_t sw128_off(uint32_t r, uint32_t c) { return r * 128u + ((c ^ (r & 7u)) << 4); }
 
+// Whether granule `g` of a slot's `n`, at place `pos` of a list, starts a copy of `lora_wide` granules of B_s that lies within a block of four.
+__device__ __forceinline__ uint32_t granule_wide(uint32_t pos, uint32_t g, uint32_t n, uint32_t lora_wide) {
+    return lora_wide > 1u && pos % lora_wide == 0u && g + lora_wide <= n ? GRAN_WIDE : 0u;
+}
+// The MMAs of a LoRA K block by the converged warp of the MMA thread: one 16-wide K step for each of the `n` <= LB granules whose list
+// entries stand at `e` (2 LB-byte aligned), B_s at `base`, the masked-t blocks `t_off` bytes behind; granules of a wide copy lie side by side in its rows.
+template <bool PAIR, int LB = 4>
+__device__ __forceinline__ void lora_block_mmas(uint32_t d_tmem, uint32_t base, uint32_t t_off, uint32_t a_bytes, uint32_t t_bytes, const uint16_t* e,
+                                                uint32_t n, uint32_t lora_wide, uint32_t idesc, uint32_t bar_empty, uint32_t pair_mask) {
+    const uint64_t narrow = make_kmajor_sw32_desc(base), wide = make_kmajor_desc(base, lora_wide), t = make_kmajor_sw32_desc(base + t_off);
+    uint32_t in_wide[4] = {0u, 0u, 0u, 0u};
+    if (lora_wide > 1u) {
+        in_wide[0] = in_wide[1] = in_wide[2] = in_wide[3] = e[0] & GRAN_WIDE;
+        if (LB == 4 && lora_wide == 2u) in_wide[2] = in_wide[3] = e[2] & GRAN_WIDE;
+    }
+    if (elect_one()) {
+#pragma unroll
+        for (uint32_t k = 0; k < uint32_t(LB); ++k) {
+            const uint32_t in_copy = k & (lora_wide - 1u);
+            const uint64_t a = in_wide[k] ? wide + (k - in_copy) * (a_bytes >> 4) + 2 * in_copy : narrow + k * (a_bytes >> 4);
+            if (k < n) umma_bf16_ss<PAIR>(d_tmem, a, t + k * (t_bytes >> 4), idesc, 1u);
+        }
+        umma_commit<PAIR>(bar_empty, pair_mask);
+    }
+    __syncwarp();
+}
+
 // FP4 activations: the K block with which a pair of feature tiles starts, so that pairs running at one moment do not all pull the
 // same activation lines.  In units of four; two share a stage of scales in the persistent kernel.
 __device__ __forceinline__ uint32_t a4_rotation(uint32_t fpair, uint32_t num_kb) { return num_kb % 4u == 0u && num_kb ? 4u * (fpair % (num_kb / 4u)) : 0u; }
@@ -722,6 +751,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                             const __grid_constant__ CUtensorMap map_w,
                             const __grid_constant__ CUtensorMap map_s,
                             const __grid_constant__ CUtensorMap map_b,
+                            const __grid_constant__ CUtensorMap map_bw,
                             const __grid_constant__ CUtensorMap map_xs,
                             const __grid_constant__ CUtensorMap map_t,
                             const Params p) {
@@ -815,6 +845,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         tma_prefetch_desc(&map_w);
         tma_prefetch_desc(&map_s);
         if (p.b_pool_strided) tma_prefetch_desc(&map_b);
+        if (p.lora_wide > 1u) tma_prefetch_desc(&map_bw);
         if (A4) tma_prefetch_desc(&map_xs);
         if (p.t_tile_cap) tma_prefetch_desc(&map_t);
     }
@@ -878,8 +909,9 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             }
         }
         if (lane == 0) {
-            // LoRA K blocks: when the adapter pool is strided, this thread also fetches the B_s tiles
-            // (one 3-D TMA per granule), running ahead of the warps that build the masked-t tiles.
+            // LoRA K blocks: when the adapter pool is strided, this thread also fetches the B_s tiles (3-D boxes of a granule, or of
+            // several of a slot), running ahead of the warps that build the masked-t tiles, and the blocks of those that the shrink
+            // has written: one copy for all of a K block, since they are consecutive (what it brings beyond the last is not read).
             if (p.seq_slot && p.b_pool_strided && !*abort_flag &&
                 mbar_wait(BAR_LIST, 0, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 64)) {
                 const uint32_t n_gran = misc[1];
@@ -894,16 +926,18 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                         if (!mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
                         const uint32_t ng = min(4u, n_gran - g0);
                         const uint32_t base = x_tile0 + ls * C::L_BLOCK;
-                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, CTAS * ng * (C::L_GRAN_A + (p.t_tile_cap ? C::L_GRAN_T : 0)));
-                        for (uint32_t g = 0; g < ng; ++g) {
-                            const uint32_t e = gran[g0 + g];
-                            if constexpr (PAIR) tma_load_3d_pair(base + g * C::L_GRAN_A, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
-                            else tma_load_3d(base + g * C::L_GRAN_A, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), BAR_LFULL + 8 * ls);
-                            if (p.t_tile_cap) {
-                                const int32_t row = int32_t(t_row0 + (g0 + g) * uint32_t(C::L_GRAN_T / 256));
-                                if constexpr (PAIR) tma_load_2d_pair(base + C::L_TILE_A + g * C::L_GRAN_T, &map_t, 0, row, lfull_at_leader + 8 * ls);
-                                else tma_load_2d(base + C::L_TILE_A + g * C::L_GRAN_T, &map_t, 0, row, BAR_LFULL + 8 * ls);
-                            }
+                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, CTAS * (ng * C::L_GRAN_A + (p.t_tile_cap ? 4 * C::L_GRAN_T : 0)));
+                        if (p.t_tile_cap) {
+                            const int32_t row = int32_t(t_row0 + g0 * uint32_t(C::L_GRAN_T / 256));
+                            if constexpr (PAIR) tma_load_2d_pair(base + C::L_TILE_A, &map_t, 0, row, lfull_at_leader + 8 * ls);
+                            else tma_load_2d(base + C::L_TILE_A, &map_t, 0, row, BAR_LFULL + 8 * ls);
+                        }
+                        for (uint32_t g = 0; g < ng;) {
+                            const uint32_t e = gran[g0 + g], at = base + g * C::L_GRAN_A;
+                            const CUtensorMap* map = e & GRAN_WIDE ? &map_bw : &map_b;
+                            if constexpr (PAIR) tma_load_3d_pair(at, map, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t((e & ~GRAN_WIDE) >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
+                            else tma_load_3d(at, map, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t((e & ~GRAN_WIDE) >> GRAN_SHIFT), BAR_LFULL + 8 * ls);
+                            g += e & GRAN_WIDE ? p.lora_wide : 1u;
                         }
                         if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
                     }
@@ -980,15 +1014,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
                     tcgen05_fence_after();
-                    const uint32_t ksteps = min(4u, n_gran - g0);
-                    const uint64_t la = make_kmajor_sw32_desc(x_tile0 + ls * C::L_BLOCK);
-                    const uint64_t lb_ = make_kmajor_sw32_desc(x_tile0 + ls * C::L_BLOCK + C::L_TILE_A);
-                    if (elect_one()) {
-                        for (uint32_t k = 0; k < ksteps; ++k)   // one granule = one 16-wide K step with its own pair of tiles
-                            umma_bf16_ss<PAIR>(tmem_acc, la + k * (C::L_GRAN_A >> 4), lb_ + k * (C::L_GRAN_T >> 4), idesc, 1u);
-                        umma_commit<PAIR>(BAR_LEMPTY + 8 * ls, pair_mask);
-                    }
-                    __syncwarp();
+                    lora_block_mmas<PAIR>(tmem_acc, x_tile0 + ls * C::L_BLOCK, C::L_TILE_A, C::L_GRAN_A, C::L_GRAN_T, gran + g0, min(4u, n_gran - g0),
+                                          p.lora_wide, idesc, BAR_LEMPTY + 8 * ls, pair_mask);
                     if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
                 }
             }
@@ -1050,7 +1077,9 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 if (r >= uint32_t(MT)) continue;
                 row_pg[r] = mine[u] == ~0u ? uint16_t(0xFFFFu) : uint16_t(pos[u] << 4 | n);
                 if (!(mine[u] >> 31))
-                    for (uint32_t g = 0; g < n; ++g) gran[pos[u] + g] = uint16_t(((mine[u] >> 4) << GRAN_SHIFT) | g);
+                    for (uint32_t g = 0; g < n; ++g) {
+                        gran[pos[u] + g] = uint16_t(((mine[u] >> 4) << GRAN_SHIFT) | g | granule_wide(pos[u] + g, g, n, p.lora_wide));
+                    }
             }
             if (te == 0) misc[1] = n_gran;
             named_bar_sync(1, EPI_THREADS);
@@ -1062,7 +1091,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             const uint32_t f = f0 + te;
             if (f < p.N) {
                 for (uint32_t g = 4 * kz; g < n_gran; g = next_own_granule(g, ks)) {
-                    const uint32_t e = gran[g];
+                    const uint32_t e = gran[g] & ~GRAN_WIDE;
                     // (a strided pool's addresses are arithmetic: a table read per granule made this loop a chain of loads)
                     const unsigned long long b_s = p.b_pool_strided ? p.b_pool_base + (e >> GRAN_SHIFT) * p.b_slot_stride : p.b_table[e >> GRAN_SHIFT];
                     const unsigned long long src = b_s + (size_t(f) * p.max_rank + (e & GRAN_MASK) * 16u) * 2u;

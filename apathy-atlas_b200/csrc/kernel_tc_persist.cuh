@@ -10,8 +10,8 @@
 //     run straight across tile boundaries: while tile i's last K blocks are multiplied, tile i+1's first
 //     stages are already fetched and expanded;
 //   * the LoRA K-steps have their own ring of (B_s tile, masked-t tiles) stages, fetched by their own producer
-//     thread while the base K loop runs, so they are issued back to back after the last base block.  B_s comes up to
-//     four granules of a slot at a time: a TMA copy costs cycles per row of its box, 128 here, however short the rows;
+//     thread while the base K loop runs, so they are issued back to back after the last base block, some granules at a time.
+//     B_s comes up to four granules of a slot at a time: a TMA copy costs cycles per row of its box, 128 here, however short the rows;
 //   * the epilogue is split: four warps first move the accumulator out of tensor memory into a shared-memory
 //     tile (BF16, [token][128 features]) and hand the accumulator back to the MMA thread, and only then write
 //     the rows to global memory (to every destination buffer), under the next tile's K loop.  The tensor pipe
@@ -82,8 +82,12 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int EPI_BYTES = G * MT * 256;
     static constexpr int L_GRAN_A = FT * 32;                               // B_s granule [128 x 16] BF16, SWIZZLE_32B
     static constexpr int L_GRAN_T = XROWS * 32;                            // masked-t granule [XROWS x 16] BF16
-    static constexpr int L_STAGE = L_GRAN_A + L_GRAN_T;
-    static constexpr int L_STAGES = EPI_BYTES / L_STAGE > 16 ? 16 : EPI_BYTES / L_STAGE;
+    // A LoRA K block of LB granules, for one round of the MMA thread (some 340 cycles beside its MMAs): four, or two where the ring would hold
+    // only two blocks of four.  Granule by granule / in blocks (us): 2048 tokens x 14336 x 4096, 128 adapters of rank 16 304 / 280, 64 of
+    // rank 32 425 / 389; one-tile BF16 passes, blocks of two / four: 512 x 14336 x 4096, 64 of rank 32 111 / 116, of rank 64 172 / 180.
+    static constexpr int LB = EPI_BYTES / (4 * (L_GRAN_A + L_GRAN_T)) > 2 || A4 ? 4 : 2;
+    static constexpr int L_TILE_A = LB * L_GRAN_A, L_STAGE = L_TILE_A + LB * L_GRAN_T;
+    static constexpr int L_STAGES = EPI_BYTES / L_STAGE;
     // ring depths: what the 227 KB of shared memory and the 512 columns of tensor memory leave
     static constexpr int STAGES = A4 ? 4 : 3;
     static constexpr int RAW_STAGES = G == 1 && !A4 ? 3 : 2;             // (A4: of block scales)
@@ -106,7 +110,8 @@ template <int MT, int G, bool A4> struct PCfg {
     static constexpr int OFF_MISC = OFF_BAR + NUM_BARS * 8;                       // tmem ptr, abort, n_gran[G]
     static constexpr int SMEM_BYTES = OFF_MISC + 64 + 1024;
     static_assert(OFF_EPI % 1024 == 0, "drain tile / LoRA ring alignment");
-    static_assert(L_STAGE % 256 == 0, "LoRA ring stages keep the swizzle atoms aligned: 256 bytes for one granule wide, 512 for two, 1024 for four");
+    static_assert(L_STAGE % 1024 == 0, "LoRA ring stages keep the swizzle atoms aligned: 256 bytes for one granule wide, 512 for two, 1024 for four");
+    static_assert(L_STAGES >= 2, "LoRA ring");
     static_assert(TMEM_NEEDED <= 512, "tensor memory budget");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
@@ -116,7 +121,6 @@ struct PParams {
     uint32_t n_fpairs;       // pairs of feature tiles along N
     uint32_t n_passes;       // token passes (G tiles of MT tokens each) along M
     uint32_t n_tiles;        // n_fpairs * n_passes
-    uint32_t lora_wide;      // granules of B_s in one fetch: 1, 2 or 4
 };
 
 template <int MT, int G, bool A4, bool ISO = false>
@@ -125,6 +129,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                                        const __grid_constant__ CUtensorMap map_w,
                                        const __grid_constant__ CUtensorMap map_s,
                                        const __grid_constant__ CUtensorMap map_b,
+                                       const __grid_constant__ CUtensorMap map_bw,
                                        const __grid_constant__ CUtensorMap map_xs,
                                        const __grid_constant__ CUtensorMap map_t,
                                        const Params p, const PParams pp) {
@@ -166,7 +171,6 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     const uint32_t num_raw = A4 ? num_kb : num_kb / 4u;
     const uint32_t my_tiles = pp.n_tiles > pair ? (pp.n_tiles - pair + n_pairs - 1u) / n_pairs : 0u;
     const bool prof = p.profile != nullptr;
-    const uint32_t lw = pp.lora_wide, n_ls = uint32_t(C::L_STAGES) / lw;      // stages of the LoRA ring: lw granules of B_s, as many of t
     uint32_t nan_seen = 0;                                              // (kNanBits) this thread stored a NaN
     const long long t_entry = clock64();
     unsigned long long* prof_row = prof ? p.profile + size_t(blockIdx.x) * PROFILE_WORDS : nullptr;
@@ -203,6 +207,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     }
     if (warp == P_LORA_WARP && lane == 0 && p.seq_slot) {
         tma_prefetch_desc(&map_b);
+        if (p.lora_wide > 1u) tma_prefetch_desc(&map_bw);
         tma_prefetch_desc(&map_t);
     }
     if (p.seq_slot) {
@@ -328,28 +333,19 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                         waited_for_shrink = true;
                     }
                     const uint32_t t_row0 = ((tile_pass(i) * G + g) * 2u + cta_rank) * p.t_tile_cap * uint32_t(C::L_GRAN_T / 256);
-                    // (granule by granule in a loop of its own: with many adapters of one granule the LoRA steps take as long as this thread
-                    //  and the MMA thread need to get round; 1000 tokens of 128 adapters of rank 16 x 14336 x 4096, this kernel alone, 138 us,
-                    //  153 in the loop below)
-                    for (uint32_t q = 0; lw == 1u && q < n_gran; ++q) {
+                    for (uint32_t g0 = 0; g0 < n_gran; g0 += C::LB) {
                         ok = mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
                         if (!ok) break;
-                        const uint32_t base = epi0 + ls * C::L_STAGE, e = gran[g * C::MAX_GRANULES + q];
-                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * C::L_STAGE);
-                        tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
-                        tma_load_2d_pair(base + C::L_GRAN_A, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
+                        const uint32_t base = epi0 + ls * C::L_STAGE, ng = min(uint32_t(C::LB), n_gran - g0);
+                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * (ng * C::L_GRAN_A + C::LB * C::L_GRAN_T));
+                        tma_load_2d_pair(base + C::L_TILE_A, &map_t, 0, int32_t(t_row0 + g0 * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
+                        for (uint32_t k = 0; k < ng;) {
+                            const uint32_t e = gran[g * C::MAX_GRANULES + g0 + k];
+                            tma_load_3d_pair(base + k * C::L_GRAN_A, e & GRAN_WIDE ? &map_bw : &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0),
+                                             int32_t((e & ~GRAN_WIDE) >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
+                            k += e & GRAN_WIDE ? p.lora_wide : 1u;
+                        }
                         if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
-                    }
-                    for (uint32_t q = 0; lw > 1u && q < n_gran;) {
-                        ok = mbar_wait(BAR_LEMPTY + 8 * ls, lph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER, 32);
-                        if (!ok) break;
-                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE), e = gran[g * C::MAX_GRANULES + q];
-                        const uint32_t n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);      // of this slot, from this granule on
-                        if (leader) mbar_arrive_expect_tx(BAR_LFULL + 8 * ls, 2 * (lw * C::L_GRAN_A + n * C::L_GRAN_T));
-                        tma_load_3d_pair(base, &map_b, int32_t((e & GRAN_MASK) * 16u), int32_t(f0), int32_t(e >> GRAN_SHIFT), lfull_at_leader + 8 * ls);
-                        for (uint32_t k = 0; k < n; ++k, ++q)
-                            tma_load_2d_pair(base + lw * C::L_GRAN_A + k * C::L_GRAN_T, &map_t, 0, int32_t(t_row0 + q * uint32_t(C::L_GRAN_T / 256)), lfull_at_leader + 8 * ls);
-                        if (++ls == n_ls) { ls = 0; lph ^= 1u; }
                     }
                 }
             }
@@ -423,35 +419,13 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                 }
                 for (uint32_t g = 0; ok && g < uint32_t(G); ++g) {
                     const uint32_t n_gran = p.seq_slot ? misc[4 + g] : 0u;
-                    for (uint32_t q = 0; lw == 1u && q < n_gran; ++q) {
+                    for (uint32_t g0 = 0; g0 < n_gran; g0 += C::LB) {
                         ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
                         if (!ok) break;
                         tcgen05_fence_after();
-                        const uint64_t la = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE);
-                        const uint64_t lb = make_kmajor_sw32_desc(epi0 + ls * C::L_STAGE + C::L_GRAN_A);
-                        if (elect_one()) {
-                            umma_bf16_ss<true>(tmem_acc + g * MT, la, lb, idesc, 1u);
-                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
-                        }
-                        __syncwarp();
+                        lora_block_mmas<true, C::LB>(tmem_acc + g * MT, epi0 + ls * C::L_STAGE, C::L_TILE_A, C::L_GRAN_A, C::L_GRAN_T, gran + g * C::MAX_GRANULES + g0,
+                                                     min(uint32_t(C::LB), n_gran - g0), p.lora_wide, idesc, BAR_LEMPTY + 8 * ls, pair_mask);
                         if (++ls == uint32_t(C::L_STAGES)) { ls = 0; lph ^= 1u; }
-                    }
-                    for (uint32_t q = 0; lw > 1u && q < n_gran;) {
-                        ok = mbar_wait_warp_timed(BAR_LFULL + 8 * ls, lph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_lora, MMA_BACKOFF_NS);
-                        if (!ok) break;
-                        tcgen05_fence_after();
-                        const uint32_t base = epi0 + ls * (lw * C::L_STAGE), e = gran[g * C::MAX_GRANULES + q];
-                        const uint32_t n = min(gcount[e >> GRAN_SHIFT] - (e & GRAN_MASK), lw);
-                        const uint64_t la = make_kmajor_desc(base, lw), lb = make_kmajor_sw32_desc(base + lw * C::L_GRAN_A);
-                        if (elect_one()) {
-#pragma unroll
-                            for (uint32_t k = 0; k < 4; ++k)         // 16 ranks = 32 bytes along the swizzled row of B_s; a block of masked t each
-                                if (k < n) umma_bf16_ss<true>(tmem_acc + g * MT, la + 2 * k, lb + k * uint64_t(C::L_GRAN_T >> 4), idesc, 1u);
-                            umma_commit<true>(BAR_LEMPTY + 8 * ls, pair_mask);
-                        }
-                        __syncwarp();
-                        q += n;
-                        if (++ls == n_ls) { ls = 0; lph ^= 1u; }
                     }
                     if (ok && elect_one()) umma_commit<true>(BAR_ACC_FULL + 8 * g, pair_mask);
                     __syncwarp();
@@ -519,7 +493,8 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
                     uint32_t pos = base + incl - cnt;
                     for (uint32_t w = word; w; w &= w - 1) {
                         const uint32_t s2 = te * 32 + (__ffs(w) - 1);
-                        for (uint32_t k = 0; k < gcount[s2]; ++k) gran[g * C::MAX_GRANULES + pos++] = uint16_t((s2 << GRAN_SHIFT) | k);
+                        const uint32_t n = gcount[s2];
+                        for (uint32_t k = 0; k < n; ++k, ++pos) gran[g * C::MAX_GRANULES + pos] = uint16_t((s2 << GRAN_SHIFT) | k | granule_wide(pos, k, n, p.lora_wide));
                     }
                     if (te == 0) misc[4 + g] = scan[0] + scan[1] + scan[2] + scan[3];
                 }

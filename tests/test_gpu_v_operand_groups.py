@@ -1,5 +1,6 @@
-"""Operands handed over in groups: four K blocks of the expanded weights, two of the activations.  Lengths that leave part of a group and
-rings that wrap, on scratch that holds garbage: within the path's tolerance of the oracle, and the same bits call for call."""
+"""Operands handed over in groups: four K blocks of the expanded weights, two of the activations, blocks of two or four LoRA granules with one,
+two or four of B_s in a copy.  Lengths that leave part of a group, rings that wrap and lists whose slots straddle a block, on scratch
+that holds garbage: within the path's tolerance of the oracle, and the same bits call for call and form for form."""
 import numpy as np
 import pytest
 
@@ -46,4 +47,28 @@ def test_a_ring_of_two_stages(cuda, atlas, oracle, K):
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "single")
     for _ in range(5):
         assert np.array_equal(dc.run(flags=atlas.FLAG_NO_CTA_PAIR, lora_ws=True)[0], y)
+    assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("fp4", [False, True])
+@pytest.mark.parametrize("ranks,max_rank,ids", [
+    ([16] * 45, 16, "uniform"),                          # one granule a slot, the last block part full
+    ([32, 16, 32, 32, 16] * 7, 32, "uniform"),           # copies of two, some slots off their boundary
+    (MIXED * 3, 64, "uniform"),                          # copies of four (two in one-tile BF16 passes)
+    ([64] * 3, 64, "segments"),
+])
+def test_lora_blocks_of_the_persistent_kernel(cuda, atlas, oracle, ranks, max_rank, ids, fp4):
+    from atlas_b200 import synth
+    case = synth.make_case("blocks", M=2085, K=512, N=4864, ranks=ranks, max_rank=max_rank, max_loras=len(ranks) + 2, ids=ids, segments=24,
+                           none_frac=0.15, scale2=0.02, b_std=0.1, seed=len(ranks) + max_rank)
+    dc = DeviceCase(cuda, atlas, case)
+    mode = atlas.FLAG_ACT_FP4 if fp4 else 0
+    y, _ = dc.run(flags=mode, lora_ws=True)
+    assert atlas.last_launch_shape()["persistent_tiles_per_pass"] == (1 if fp4 else 2)
+    one, _ = dc.run(flags=mode | atlas.FLAG_ONE_TILE_PASS, lora_ws=True)
+    assert atlas.last_launch_shape()["persistent_tiles_per_pass"] == 1
+    tile, _ = dc.run(flags=mode | atlas.FLAG_NO_PERSISTENT, lora_ws=True)
+    assert np.array_equal(y, one) and np.array_equal(y, tile)
+    rows, cols = _sample(case, max_rank)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols, act_fp4=fp4), "blocks")
     assert atlas.device_status() == 0
