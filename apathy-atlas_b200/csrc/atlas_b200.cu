@@ -695,7 +695,8 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
         attr[n_attr].val.clusterDim.z = k_split;
         ++n_attr;
     }
-    if (after_shrink) {
+    p.chained = d.seq_slot ? 0u : 1u;
+    if (after_shrink || p.chained) {
         attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
         ++n_attr;
@@ -802,7 +803,8 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     attr[n_attr].val.clusterDim.y = 1;
     attr[n_attr].val.clusterDim.z = 1;
     ++n_attr;
-    if (shrink) {
+    p.chained = d.seq_slot ? 0u : 1u;
+    if (shrink || p.chained) {
         attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[n_attr].val.programmaticStreamSerializationAllowed = 1;
         ++n_attr;
@@ -840,8 +842,9 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = shrink ? 1 : 0;
-    return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS>, w, p));
+    cfg.numAttrs = shrink || !d.seq_slot ? 1 : 0;             // (t made ready by another call: in order)
+    return cuda_status(d.seq_slot ? cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, false>, w, p)
+                                  : cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, true>, w, p));
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):

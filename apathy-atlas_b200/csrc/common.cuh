@@ -30,12 +30,12 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 // A decode step is a chain of short kernels, and between two of them an ordinary launch leaves the machine idle for a few
 // microseconds.  A kernel may (a) release the next launch once all its own CTAs run, and (b) be launched as a dependent, which may
 // then start early and has to wait until everything before it in the stream has completed and is visible.
-//   launched as dependents     both tensor-core shrinks, the main kernel behind a shrink, the tensor-core expand, the dense linear,
-//                              the QKV consumers, SwiGLU in both forms, the quantiser
+//   launched as dependents     both tensor-core shrinks, the main kernel behind a shrink and without adapters, the tensor-core expand, the
+//                              dense linear, the QKV consumers, SwiGLU in both forms, the quantiser
 //   releasing                  all of these but lora_shrink_mma_kernel and lora_shrink_grouped_kernel, which do so only in front of a
 //                              main kernel or of the dense linear
-//   neither                    a main kernel without adapters releases but is launched in order; the NVFP4 decode, the maximum, the
-//                              CUDA-core linear and expand do neither
+//   neither                    a main kernel over a t that an earlier call left releases but is launched in order; the NVFP4 decode, the
+//                              maximum, the CUDA-core linear and expand do neither
 // A dependent begins with the wait, with two exceptions:
 //   the main kernel and the dense linear behind their shrink read x, weights and routing ahead of it: that shrink has waited before
 //   releasing them; they wait before they read t, or before they end, on every path, so that nothing behind them overtakes the shrink;

@@ -38,7 +38,9 @@ struct DecodeParams {
     uint32_t x_row_stride;
 };
 
-template <int TILES, int NT, int WARPS>
+// BASE: no adapters, launched as a dependent of whatever is before it (an instance of its own: the wait in all of them cost calls with
+// adapters 1 to 2 %).
+template <int TILES, int NT, int WARPS, bool BASE>
 __global__ void __launch_bounds__(32 * WARPS, 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     constexpr int SETS = DCM_SUMS / WARPS;                             // partial sums of a warp
@@ -50,10 +52,16 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t f0 = blockIdx.x * (TILES * 16);
     pdl_release();
+    const uint8_t *w_packed = w.w_packed, *w_scale = w.w_scale;
+    const uint16_t* x = w.x;
+    if constexpr (BASE) {
+        pdl_wait();
+        w_packed = pdl_after(w_packed); w_scale = pdl_after(w_scale); x = pdl_after(x);
+    }
 
-    if (tid < DCM_MAX_TOKENS) {
+    if (!BASE && tid < DCM_MAX_TOKENS) {
         int32_t s = -1;
-        if (p.seq_slot && tid < p.M) {
+        if (tid < p.M) {
             s = p.seq_slot[tid];
             if (s >= 0) {
                 if (uint32_t(s) >= p.max_loras) { record_status(STATUS_SLOT_OUT_OF_RANGE); s = -1; }
@@ -76,12 +84,12 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t f = min(f0 + 16 * i + 8 * h + g, p.N - 1u);          // (rows past N repeat the last one and are not stored)
-            code_row[i][h] = w.w_packed + size_t(f) * (p.K / 2u) + 16 * t;
-            scale_row[i][h] = w.w_scale + size_t(f) * (p.K / 16u) + 2 * t;
+            code_row[i][h] = w_packed + size_t(f) * (p.K / 2u) + 16 * t;
+            scale_row[i][h] = w_scale + size_t(f) * (p.K / 16u) + 2 * t;
         }
     const uint16_t* x_row[NT];
 #pragma unroll
-    for (int n = 0; n < NT; ++n) x_row[n] = w.x + size_t(min(8 * n + g, p.M - 1u)) * w.x_row_stride + 32 * t;
+    for (int n = 0; n < NT; ++n) x_row[n] = x + size_t(min(8 * n + g, p.M - 1u)) * w.x_row_stride + 32 * t;
 
     float acc[SETS][TILES][NT][4] = {};                                // sums `warp`, `warp` + WARPS
     // (one n-tile: x travels with the codes; more of them would not fit in registers and are read where they are used)
@@ -147,7 +155,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     }
 
     // ---- LoRA granules of this warp ----
-    if (p.seq_slot) {
+    if constexpr (!BASE) {
         __syncthreads();                                                        // slot_s, rank_s, b_s
         // this CTA's rows of B into L2 while the shrink may still run
         for (uint32_t m = warp; m < p.M; m += WARPS) {

@@ -170,6 +170,7 @@ struct Params {
     uint32_t lora_wide;            // granules of B_s that may come in one copy: 1, 2 or 4
     unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
+    uint32_t chained;              // launched as a programmatic dependent of whatever is before it (no adapters): wait before reading anything
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
     // isolate != 0 (ISO instances only): outputs that another adapter's infinity or NaN has made a NaN are computed again (isolate.cuh), from:
@@ -868,6 +869,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
 
     if (warp == 0) {
         // ===================================== TMA producer =====================================
+        if (p.chained) pdl_wait();
         if (lane == 0 && A4) {
             // One ring: a stage's two packed operand tiles complete FULL[s] (which the MMA thread waits
             // on), its two scale-byte tiles FULL_RAW[s] (which the warps that move them to TMEM wait on).
@@ -1113,6 +1115,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         // ===================================== TMA producer, raw weight stages ===================
         // A thread of its own: try_wait may suspend its caller for a while, so one thread polling both rings' barriers in
         // turn keeps a free slot of one ring waiting behind the other's.
+        if (p.chained) pdl_wait();
         if (lane == 0 && !A4) {
             uint32_t rs = 0, rph = 0;
             for (uint32_t ri = 0; ri < num_raw_kb; ++ri) {
@@ -1219,7 +1222,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 dst[j] = sc_row && ri < num_raw && at < p.K / 16u ? uint32_t(__ldg(reinterpret_cast<const uint16_t*>(sc_row + at))) << (16u * half) : 0u;
             }
         };
-        if constexpr (SROWS) { fetch_scales(0, sc_next[0]); fetch_scales(1, sc_next[1]); }
+        if constexpr (SROWS) {
+            if (p.chained) pdl_wait();
+            sc_row = pdl_after(sc_row);
+            fetch_scales(0, sc_next[0]);
+            fetch_scales(1, sc_next[1]);
+        }
         for (uint32_t ri = 0; ok && ri < num_raw; ++ri) {
             ok = mbar_wait_timed(BAR_FULL_RAW + 8 * rs, rph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT, prof, w_raw);
             if (!ok) break;

@@ -235,6 +235,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
 
     if (warp == 0) {
         // ===================================== TMA producer, base K loop =====================================
+        if (p.chained) pdl_wait();
         if (lane == 0 && A4) {
             uint32_t s = 0, ph = 0;
             for (uint32_t i = 0; i < my_tiles; ++i) {
@@ -279,6 +280,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
     } else if (warp == P_RAW_WARP) {
         // ===================================== TMA producer, raw weight stages ===============================
         // (one per four K blocks; a thread of its own, see nvfp4_lora_linear_tc_kernel)
+        if (p.chained) pdl_wait();
         if (lane == 0 && A4) {
             // block scales of both operands, two K blocks to a stage (zero-filled past K)
             const uint32_t n_ss = (num_kb + A4_SCALE_BLOCKS - 1u) / A4_SCALE_BLOCKS;
