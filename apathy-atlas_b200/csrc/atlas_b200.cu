@@ -225,8 +225,9 @@ static int shrink_tc_clusters(DeviceState& dst, uint32_t ksplit) {
     return dst.shrink_tc_clusters[ksplit];
 }
 
-static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool release_dependents = false,
-                         bool dependent_leaves_sms_free = false) {
+// `beside`: what of the machine the kernel behind it wants, which is then released as soon as this one's CTAs run (none: not released)
+static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, MachineBeside beside = MachineBeside::none) {
+    const bool release_dependents = beside != MachineBeside::none;
     p.release_dependents = release_dependents ? 1u : 0u;
     p.profile = nullptr;
     if (p.M == 0 || p.max_rank == 0) return ATLAS_B200_OK;
@@ -297,8 +298,7 @@ static int launch_shrink(ShrinkParams p, uint32_t n_slots, cudaStream_t st, bool
     if (mma_ok) {
         const uint32_t chunk = p.chunk ? p.chunk : uint32_t(SHM_CHUNK);
         const MmaShrinkGrid rule = mma_shrink_grid(n_slots, (p.max_rank + SHM_RANKS - 1) / SHM_RANKS, (p.M + chunk - 1) / chunk, std::min(p.M, chunk),
-                                                   uint32_t(rt_sm_count()), !release_dependents ? MachineBeside::none
-                                                   : dependent_leaves_sms_free ? MachineBeside::part : MachineBeside::all);
+                                                   uint32_t(rt_sm_count()), beside);
         const uint32_t ksplit = p.ksplit = rule.ksplit;
         p.row_parts_log2 = rule.row_parts_log2;
         p.prefetch_ctas = rule.prefetch_ctas;
@@ -673,7 +673,8 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
         // the tcgen05 shrink fills its SMs and releases this kernel at the same point, whose CTAs then take SMs that are free or
         // become so; the mma.sync shrink, where it has to stand in, keeps the machine to itself.
         const uint32_t main_ctas = grid.x * grid.y * grid.z;
-        const int rc = launch_shrink(*shrink, d.max_loras, st, d.m <= 1024, main_ctas * 3 <= uint32_t(rt_sm_count()) * 2);
+        const int rc = launch_shrink(*shrink, d.max_loras, st, d.m > 1024 ? MachineBeside::none
+                                     : (main_ctas * 3 <= uint32_t(rt_sm_count()) * 2 ? MachineBeside::part : MachineBeside::tiles));
         if (rc) return rc;
     }
     p.profile = (g_profile_buf && size_t(grid.x) * grid.y * tc::PROFILE_WORDS <= g_profile_words) ? g_profile_buf : nullptr;
@@ -787,7 +788,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     t_last_shape[0] = MT; t_last_shape[1] = 1u; t_last_shape[2] = 1u; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs;
     if (shrink) {
-        const int rc = launch_shrink(*shrink, d.max_loras, st, d.m <= 1024, false);
+        const int rc = launch_shrink(*shrink, d.max_loras, st, d.m > 1024 ? MachineBeside::none : MachineBeside::all);
         if (rc) return rc;
     }
     p.profile = (g_profile_buf && size_t(pairs) * 2 * tc::PROFILE_WORDS <= g_profile_words) ? g_profile_buf : nullptr;
@@ -830,7 +831,7 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
     const uint32_t ctas = (d.n + 16 * TILES - 1) / (16 * TILES);
     t_last_shape[0] = 8u; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
     if (shrink) {
-        rc = launch_shrink(*shrink, d.max_loras, st, true, ctas * 3 <= uint32_t(rt_sm_count()) * 2);
+        rc = launch_shrink(*shrink, d.max_loras, st, ctas * 3 <= uint32_t(rt_sm_count()) * 2 ? MachineBeside::part : MachineBeside::all);
         if (rc) return rc;
     }
     p.wait_for_shrink = shrink ? 1u : 0u;
@@ -1225,7 +1226,7 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         sp.out = static_cast<uint16_t*>(d.lora_t);
         sp.M = d.m; sp.k_in = d.k; sp.max_rank = d.max_rank; sp.x_row_stride = d.x_row_stride; sp.max_loras = d.max_loras;
         sp.post = 0.0f;
-        rc = launch_shrink(sp, d.max_loras, st, shrink_first);
+        rc = launch_shrink(sp, d.max_loras, st, shrink_first ? MachineBeside::all : MachineBeside::none);
         if (rc) return rc;
         if (shrink_first) {
             rc = base();

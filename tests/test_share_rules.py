@@ -75,3 +75,16 @@ def test_clusters_without_rows_do_not_fill_the_machine(rules):
     assert _grid(rules, 8, 4, 2, 256, ALL)[:2] == (8, 1)       # rank 64, two chunks: two clusters
     assert _grid(rules, 1, 8, 4, 256, ALL)[:2] == (8, 2)       # one adapter for all rows: 1024 CTAs with rows
     assert _grid(rules, 8, 1, 4, 256, NONE)[:2] == (8, 2)
+
+
+@pytest.mark.parametrize("slots,granules,chunks", [(1, 1, 1), (1, 8, 4), (8, 4, 2), (8, 4, 4), (8, 8, 2), (16, 1, 4), (64, 4, 1), (128, 1, 1), (4096, 8, 4)])
+@pytest.mark.parametrize("rows", [1, 32, 33, 130, 256])
+def test_one_more_cluster_beside_a_kernel_of_one_tile_a_cta(rules, slots, granules, chunks, rows):
+    TILES = 3
+    ksplit, log2, first = _grid(rules, slots, granules, chunks, rows, TILES)
+    assert (ksplit, first) == (8, 148 * 8)
+    if log2 != _grid(rules, slots, granules, chunks, rows, ALL)[1]:
+        assert log2 == 1 and rows > 32 and slots * granules * chunks * 16 <= 2 * 148 * 8
+        assert chunks <= 2 or rows >= slots * 32
+    if (slots, granules, chunks, rows) == (8, 4, 4, 256):      # 1000 tokens of 8 adapters of rank 64
+        assert log2 == 1
