@@ -86,6 +86,7 @@ struct DeviceState {
     int shrink_tc_clusters[SHT_MAX_KSPLIT + 1] = {};   // resident clusters of that many CTAs of the prefill shrink; 0 = not asked yet
     bool push_attr_set = false;
     bool dense_attr_set[5] = {};      // token tiles 16, 32, 64, 128, 256 of the dense-BF16 kernel
+    bool decode_attr_set[8] = {};     // TMA form of the small-batch kernel: features of a CTA x {four, eight warps} x {adapters, none}
 };
 static DeviceState g_dev[kMaxDevices];
 static std::mutex g_dev_mutex;
@@ -818,8 +819,8 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
 }
 
 // ---- the smallest batches (kernel_decode_mma.cuh) ----
-template <int TILES, int NT, int WARPS>
-static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+template <int TILES, int NT, int WARPS, bool TMA, bool BASE>
+static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
     tc::Params p{};
     int rc = fill_tc_params(d, false, false, TTiles{}, p);
     if (rc) return rc;
@@ -835,17 +836,55 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
         if (rc) return rc;
     }
     p.wait_for_shrink = shrink ? 1u : 0u;
+    using R = DcmRing<TILES, WARPS>;
+    const auto kernel = nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, TMA, BASE>;
+    CUtensorMap map_w, map_s;
+    if constexpr (TMA) {
+        DeviceState* dst = device_state();
+        if (!dst) return ATLAS_B200_ERR_ARCH;
+        bool& set = dst->decode_attr_set[(TILES - 1) * 4 + (WARPS == 8 ? 2 : 0) + (BASE ? 1 : 0)];
+        if (!set) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM_BYTES);
+            if (e != cudaSuccess) return cuda_status(e);
+            set = true;
+        }
+        if (!encode_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_packed, d.k / 2, d.n, d.k / 2, 128, R::ROWS, CU_TENSOR_MAP_SWIZZLE_128B) ||
+            !encode_2d(&map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, 8 * WARPS, R::ROWS,
+                       WARPS == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B))
+            return ATLAS_B200_ERR_DIMS;
+    } else {
+        std::memset(&map_w, 0, sizeof(map_w));                // never dereferenced
+        std::memset(&map_s, 0, sizeof(map_s));
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(32 * WARPS);
+    cfg.blockDim = dim3(32 * (WARPS + (TMA ? 1 : 0)));
+    cfg.dynamicSmemBytes = TMA ? R::SMEM_BYTES : 0;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = shrink || !d.seq_slot ? 1 : 0;             // (t made ready by another call: in order)
-    return cuda_status(d.seq_slot ? cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, false>, w, p)
-                                  : cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, true>, w, p));
+    cfg.numAttrs = shrink || BASE ? 1 : 0;                    // (t made ready by another call: in order)
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, w, p, map_w, map_s));
+}
+
+// Weights by TMA (one n-tile; K of whole boxes): the warps' loads then are those of x, t and B alone, which is what the shrink beside this
+// kernel and the granules behind it gain from; a small layer pays for the barriers and the longer way of its first bytes.  By the warps'
+// loads / TMA (us), granules of the batch: 4096 x 4096 8 9.2 / 10.1, 12 10.0 / 10.8, 16 12.2 / 11.0, 32 16.2 / 12.9; 5120 x 5120 8 13.4 /
+// 13.5, 16 14.8 / 14.2, 32 18.7 / 15.7; 14336 x 4096 8 17.8 / 18.3, 16 22.9 / 20.4, 32 28.5 / 23.7; 4096 x 14336 8 18.5 / 18.1, 16 26.1 /
+// 18.6, 24 32.4 / 19.9; but 11008 x 4096 16 18.7 / 19.1, 2560 x 2560 16 8.2 / 9.0, 64 13.7 / 13.6.  Large layers whatever the batch: 8192 x
+// 8192 one token, no adapters 15.7 / 15.3, 28672 x 8192 44.8 / 42.8, 8192 x 28672 48.1 / 43.3, 8 tokens of 8 x 64 x 28672 x 8192 73 / 59.
+static bool decode_by_tma(const atlas_b200_linear_desc& d) {
+    const uint64_t weights = uint64_t(d.n) * d.k, granules = d.seq_slot ? std::min(d.max_loras, d.m) * ((d.max_rank + 15) / 16) : 0u;
+    return d.k % tc::KRAW == 0 && (weights >= 1u << 26 || (weights >= 1u << 24 && granules >= 16));
+}
+template <int TILES, int NT, int WARPS>
+static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+    if constexpr (NT == 1)
+        if (decode_by_tma(d))
+            return d.seq_slot ? launch_decode_form<TILES, NT, WARPS, true, false>(d, shrink, st) : launch_decode_form<TILES, NT, WARPS, true, true>(d, shrink, st);
+    return d.seq_slot ? launch_decode_form<TILES, NT, WARPS, false, false>(d, shrink, st) : launch_decode_form<TILES, NT, WARPS, false, true>(d, shrink, st);
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):

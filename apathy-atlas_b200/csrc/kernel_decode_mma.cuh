@@ -38,11 +38,21 @@ struct DecodeParams {
     uint32_t x_row_stride;
 };
 
-// BASE: no adapters, launched as a dependent of whatever is before it (an instance of its own: the wait in all of them cost calls with
-// adapters 1 to 2 %).
-template <int TILES, int NT, int WARPS, bool BASE>
-__global__ void __launch_bounds__(32 * WARPS, 16 / WARPS)
-nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
+// TMA form: the ring of a CTA, filled by a warp of its own.  A stage is a step of every warp: [16 TILES rows x 128 B] of codes for every two
+// of them, swizzled, then their scale bytes [16 TILES rows x 8 WARPS B], swizzled over their own width.
+template <int TILES, int WARPS> struct DcmRing {
+    static constexpr int ROWS = 16 * TILES, BOXES = WARPS / 2;
+    static constexpr int CODES = BOXES * ROWS * 128, SCALES = ROWS * 8 * WARPS;
+    static constexpr int STAGE = (CODES + SCALES + 1023) / 1024 * 1024, STAGES = 4;
+    static constexpr int SMEM_BYTES = STAGES * STAGE + 1024;
+};
+
+// TMA: codes and scales come through shared memory (decode_by_tma); the same bits.  BASE: no adapters, launched as a dependent of whatever
+// is before it (an instance of its own: the wait in all of them cost calls with adapters 1 to 2 %).
+template <int TILES, int NT, int WARPS, bool TMA, bool BASE>
+__global__ void __launch_bounds__(32 * (WARPS + (TMA ? 1 : 0)), 16 / WARPS)
+nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {
+    using R = DcmRing<TILES, WARPS>;
     constexpr int SETS = DCM_SUMS / WARPS;                             // partial sums of a warp
     static_assert(SETS * WARPS == DCM_SUMS && SETS <= 2, "two steps to a turn of the base loop, one for either sum");
     __shared__ float part[DCM_SUMS][NT * 8][TILES * 16 + 1];           // [partial sum][token][feature]
@@ -51,12 +61,41 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     __shared__ uint64_t b_s[DCM_MAX_TOKENS];                           // and its B (read once, not granule by granule behind the shrink)
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t f0 = blockIdx.x * (TILES * 16);
+    const uint32_t n_steps = (p.K + DCM_KSTEP - 1) / DCM_KSTEP;
+    extern __shared__ uint8_t dcm_dyn[];
+    __shared__ uint64_t bars[TMA ? 2 * R::STAGES : 1];
+    __shared__ uint32_t abort_s;
+    const uint32_t ring = (tc::smem_u32(dcm_dyn) + 1023u) & ~1023u, BAR_FULL = tc::smem_u32(bars), BAR_EMPTY = BAR_FULL + 8 * R::STAGES;
+    volatile uint32_t* abort_flag = &abort_s;
+    if constexpr (TMA) {
+        if (tid == 0) {
+            for (int i = 0; i < R::STAGES; ++i) { tc::mbar_init(BAR_FULL + 8 * i, 1); tc::mbar_init(BAR_EMPTY + 8 * i, WARPS); }
+            abort_s = 0u;
+            tc::fence_barrier_init();
+        }
+        __syncthreads();
+    }
     pdl_release();
     const uint8_t *w_packed = w.w_packed, *w_scale = w.w_scale;
     const uint16_t* x = w.x;
     if constexpr (BASE) {
         pdl_wait();
         w_packed = pdl_after(w_packed); w_scale = pdl_after(w_scale); x = pdl_after(x);
+    }
+    if (TMA && warp == WARPS) {
+        if (lane == 0) {
+            uint32_t s = 0, ph = 0;
+            for (uint32_t k0 = 0; k0 < p.K; k0 += DCM_KSTEP * WARPS) {          // (zero-filled past K and N)
+                if (!tc::mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
+                const uint32_t st = ring + s * R::STAGE;
+                tc::mbar_arrive_expect_tx(BAR_FULL + 8 * s, R::CODES + R::SCALES);
+                for (uint32_t b = 0; b < uint32_t(R::BOXES); ++b)
+                    tc::tma_load_2d(st + b * (R::ROWS * 128), &map_w, int32_t(k0 / 2 + 128 * b), int32_t(f0), BAR_FULL + 8 * s);
+                tc::tma_load_2d(st + R::CODES, &map_s, int32_t(k0 / 16), int32_t(f0), BAR_FULL + 8 * s);
+                if (++s == uint32_t(R::STAGES)) { s = 0; ph ^= 1u; }
+            }
+        }
+        __syncwarp();
     }
 
     if (!BASE && tid < DCM_MAX_TOKENS) {
@@ -76,7 +115,6 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     }
 
     // ---- base: this thread's 32 codes per step of feature rows g and g + 8 of every tile, and of x rows g (+ 8 per n-tile) ----
-    const uint32_t n_steps = (p.K + DCM_KSTEP - 1) / DCM_KSTEP;
     const uint8_t* code_row[TILES][2];
     const uint8_t* scale_row[TILES][2];
 #pragma unroll
@@ -146,19 +184,61 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             }
         }
     };
-    load(warp, code[0], sc[0], xv[0]);
-    for (uint32_t step = warp; step < n_steps; step += 2 * WARPS) {
-        load(step + WARPS, code[1], sc[1], xv[1]);
-        multiply(step, code[0], sc[0], xv[0], acc[0]);
-        load(step + 2 * WARPS, code[0], sc[0], xv[0]);
-        if (step + WARPS < n_steps) multiply(step + WARPS, code[1], sc[1], xv[1], acc[SETS - 1]);
+    if constexpr (TMA) {
+        auto load_x = [&](uint32_t step, uint4 (&xs)[X_AHEAD ? 4 : 1]) {
+            if constexpr (X_AHEAD) {
+                const bool in = step < n_steps && g < p.M;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) xs[u] = in ? __ldg(reinterpret_cast<const uint4*>(x_row[0] + step * DCM_KSTEP + 8 * u)) : make_uint4(0u, 0u, 0u, 0u);
+            }
+        };
+        // a stage's chunk 4 (warp % 2) + t of box warp / 2, and bytes 8 warp + 2 t of its scale rows
+        const uint32_t code_at = (warp >> 1) * (R::ROWS * 128) + g * 128 + (((4 * (warp & 1u) + t) ^ g) << 4);
+        const uint32_t swz = WARPS == 8 ? (g >> 1) & 3u : (g >> 2) & 1u;
+        const uint32_t scale_at = R::CODES + g * (8 * WARPS) + (((warp >> 1) ^ swz) << 4) + (warp & 1u) * 8 + 2 * t;
+        uint32_t s = 0, ph = 0;
+        auto turn = [&](uint32_t step, const uint4 (&xs)[X_AHEAD ? 4 : 1], float (&sum)[TILES][NT][4]) -> bool {
+            if (!tc::mbar_wait(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT)) return false;
+            const uint32_t st = ring + s * R::STAGE;
+#pragma unroll
+            for (int i = 0; i < TILES; ++i)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    code[0][i][h] = tc::lds128(st + code_at + (16 * i + 8 * h) * 128);
+                    uint16_t v;
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(st + scale_at + (16 * i + 8 * h) * (8 * WARPS)));
+                    sc[0][i][h] = v;
+                }
+            if (step < n_steps) multiply(step, code[0], sc[0], xs, sum);
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(BAR_EMPTY + 8 * s);
+            if (++s == uint32_t(R::STAGES)) { s = 0; ph ^= 1u; }
+            return true;
+        };
+        if (warp < WARPS) {
+            load_x(warp, xv[0]);
+            for (uint32_t step = warp; step - warp < n_steps; step += 2 * WARPS) {      // (all warps go through all stages)
+                load_x(step + WARPS, xv[1]);
+                if (!turn(step, xv[0], acc[0]) || step + WARPS - warp >= n_steps) break;
+                load_x(step + 2 * WARPS, xv[0]);
+                if (!turn(step + WARPS, xv[1], acc[SETS - 1])) break;
+            }
+        }
+    } else {
+        load(warp, code[0], sc[0], xv[0]);
+        for (uint32_t step = warp; step < n_steps; step += 2 * WARPS) {
+            load(step + WARPS, code[1], sc[1], xv[1]);
+            multiply(step, code[0], sc[0], xv[0], acc[0]);
+            load(step + 2 * WARPS, code[0], sc[0], xv[0]);
+            if (step + WARPS < n_steps) multiply(step + WARPS, code[1], sc[1], xv[1], acc[SETS - 1]);
+        }
     }
 
     // ---- LoRA granules of this warp ----
     if constexpr (!BASE) {
         __syncthreads();                                                        // slot_s, rank_s, b_s
         // this CTA's rows of B into L2 while the shrink may still run
-        for (uint32_t m = warp; m < p.M; m += WARPS) {
+        for (uint32_t m = warp; (!TMA || warp < WARPS) && m < p.M; m += WARPS) {
             if (slot_s[m] < 0 || lane >= TILES * 16u || f0 + lane >= p.N) continue;
             const uint64_t row = b_s[m] + size_t(f0 + lane) * p.max_rank * 2u;
             for (uint32_t j = 0; j < rank_s[m]; j += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"((row + 2u * j) & ~15ull));
@@ -218,6 +298,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
     }
 
     // ---- the partial sums, added in their order ----
+    if (!TMA || warp < WARPS)
 #pragma unroll
     for (int h = 0; h < SETS; ++h)
 #pragma unroll
@@ -227,7 +308,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
 #pragma unroll
                 for (int e = 0; e < 4; ++e) part[warp + h * WARPS][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[h][i][n][e];
     __syncthreads();
-    for (uint32_t i = tid; i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
+    for (uint32_t i = tid; (!TMA || warp < WARPS) && i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
         const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
         float sum = part[0][m][fi];
 #pragma unroll
@@ -250,6 +331,12 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p) {
             else if (lane % 8u == 0) *reinterpret_cast<uint4*>(p.y_dest[r] + at) = make_uint4(w0, w1, w2, w3);
         }
     }
+    if constexpr (TMA)
+        if (*abort_flag) {
+            // give copies that may still be in flight time to land before shared memory is released
+            const uint64_t t0 = tc::global_timer_ns();
+            while (tc::global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        }
 }
 
 }  // namespace atlas
