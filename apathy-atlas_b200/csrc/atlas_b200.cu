@@ -819,8 +819,8 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
 }
 
 // ---- the smallest batches (kernel_decode_mma.cuh) ----
-template <int TILES, int NT, int WARPS, bool TMA, bool BASE>
-static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+template <int TILES, int NT, int WARPS, bool BASE>
+static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, bool tma, cudaStream_t st) {
     tc::Params p{};
     int rc = fill_tc_params(d, false, false, TTiles{}, p);
     if (rc) return rc;
@@ -836,37 +836,39 @@ static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParam
         if (rc) return rc;
     }
     p.wait_for_shrink = shrink ? 1u : 0u;
-    using R = DcmRing<TILES, WARPS>;
-    const auto kernel = nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, TMA, BASE>;
-    CUtensorMap map_w, map_s;
-    if constexpr (TMA) {
-        DeviceState* dst = device_state();
-        if (!dst) return ATLAS_B200_ERR_ARCH;
-        bool& set = dst->decode_attr_set[(TILES - 1) * 4 + (WARPS == 8 ? 2 : 0) + (BASE ? 1 : 0)];
-        if (!set) {
-            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM_BYTES);
-            if (e != cudaSuccess) return cuda_status(e);
-            set = true;
-        }
-        if (!encode_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_packed, d.k / 2, d.n, d.k / 2, 128, R::ROWS, CU_TENSOR_MAP_SWIZZLE_128B) ||
-            !encode_2d(&map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, 8 * WARPS, R::ROWS,
-                       WARPS == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B))
-            return ATLAS_B200_ERR_DIMS;
-    } else {
-        std::memset(&map_w, 0, sizeof(map_w));                // never dereferenced
-        std::memset(&map_s, 0, sizeof(map_s));
-    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(ctas);
-    cfg.blockDim = dim3(32 * (WARPS + (TMA ? 1 : 0)));
-    cfg.dynamicSmemBytes = TMA ? R::SMEM_BYTES : 0;
+    cfg.blockDim = dim3(32 * WARPS);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = shrink || BASE ? 1 : 0;                    // (t made ready by another call: in order)
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, w, p, map_w, map_s));
+    cfg.numAttrs = shrink || BASE ? 1 : 0;
+    if constexpr (NT == 1)
+        if (tma) {
+            using R = DcmRing<TILES, WARPS>;
+            const auto kernel = nvfp4_lora_decode_mma_kernel<TILES, 1, WARPS, true, BASE>;
+            DeviceState* dst = device_state();
+            if (!dst) return ATLAS_B200_ERR_ARCH;
+            bool& set = dst->decode_attr_set[(TILES - 1) * 4 + (WARPS == 8 ? 2 : 0) + (BASE ? 1 : 0)];
+            if (!set) {
+                const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM_BYTES);
+                if (e != cudaSuccess) return cuda_status(e);
+                set = true;
+            }
+            CUtensorMap map_w, map_s;
+            if (!encode_2d(&map_w, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_packed, d.k / 2, d.n, d.k / 2, 128, R::ROWS, CU_TENSOR_MAP_SWIZZLE_128B) ||
+                !encode_2d(&map_s, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, d.w_scale, d.k / 16, d.n, d.k / 16, 8 * WARPS, R::ROWS,
+                           WARPS == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B))
+                return ATLAS_B200_ERR_DIMS;
+            cfg.blockDim = dim3(32 * (WARPS + 1));
+            cfg.dynamicSmemBytes = R::SMEM_BYTES;
+            return cuda_status(cudaLaunchKernelEx(&cfg, kernel, w, p, map_w, map_s));
+        }
+    CUtensorMap none;
+    std::memset(&none, 0, sizeof(none));                      // never dereferenced
+    return cuda_status(cudaLaunchKernelEx(&cfg, nvfp4_lora_decode_mma_kernel<TILES, NT, WARPS, false, BASE>, w, p, none, none));
 }
 
 // Weights by TMA (one n-tile; K of whole boxes): the warps' loads then are those of x, t and B alone, which is what the shrink beside this
@@ -881,10 +883,10 @@ static bool decode_by_tma(const atlas_b200_linear_desc& d) {
 }
 template <int TILES, int NT, int WARPS>
 static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
+    const bool tma = NT == 1 && decode_by_tma(d);
     if constexpr (NT == 1)
-        if (decode_by_tma(d))
-            return d.seq_slot ? launch_decode_form<TILES, NT, WARPS, true, false>(d, shrink, st) : launch_decode_form<TILES, NT, WARPS, true, true>(d, shrink, st);
-    return d.seq_slot ? launch_decode_form<TILES, NT, WARPS, false, false>(d, shrink, st) : launch_decode_form<TILES, NT, WARPS, false, true>(d, shrink, st);
+        if (!d.seq_slot) return launch_decode_form<TILES, NT, WARPS, true>(d, shrink, tma, st);
+    return launch_decode_form<TILES, NT, WARPS, false>(d, shrink, tma, st);
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):

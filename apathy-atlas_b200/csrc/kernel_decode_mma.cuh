@@ -4,8 +4,8 @@
 //
 // A decode batch is bound by streaming the weights once.  The tcgen05 form cannot keep up with that stream: its weight operand
 // goes through tensor memory, which fixes the order of the K elements (four byte permutes per eight codes), and its
-// eight expansion warps are busy for 540 cycles per 128 x 64 block whatever the batch, 650 with their waits: one token x 14336
-// features x 4096 takes 26 us for 33 MB, 15 here.  Here every warp of the SM expands, the operand stays in the registers the
+// eight expansion warps are busy for 344 cycles per 128 x 64 block whatever the batch: one token x 14336 features x 4096
+// takes 17.7 us for 33 MB, 14.8 here.  Here every warp of the SM expands, the operand stays in the registers the
 // codes were expanded in, and since BOTH operands of mma.sync come from registers the K elements may take any order as long as
 // they meet their partners: the pairs (i, i + 4) that fall out of a word of eight codes are used as they are, and x is paired
 // the same way (four permutes per eight elements of x, shared by all features of the warp).
@@ -48,7 +48,10 @@ template <int TILES, int WARPS> struct DcmRing {
 };
 
 // TMA: codes and scales come through shared memory (decode_by_tma); the same bits.  BASE: no adapters, launched as a dependent of whatever
-// is before it (an instance of its own: the wait in all of them cost calls with adapters 1 to 2 %).
+// is before it (instances of their own: the wait in all of them cost calls with adapters 1 to 2 %).  Those release late: a next grid
+// that comes while this one's CTAs are all at work takes the places they happen to leave, and its SMs get unequal numbers of CTAs.  One
+// token behind one another, launched in order / released at the start / behind the loop (us): 11008 x 4096 12.8 / 14.4 / 11.9, 2048 x
+// 2048 2.8 / - / 2.4; 12 tokens x 1280 x 17408 14.1 / 20.4 / 15.2.
 template <int TILES, int NT, int WARPS, bool TMA, bool BASE>
 __global__ void __launch_bounds__(32 * (WARPS + (TMA ? 1 : 0)), 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {
@@ -61,7 +64,6 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
     __shared__ uint64_t b_s[DCM_MAX_TOKENS];                           // and its B (read once, not granule by granule behind the shrink)
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t f0 = blockIdx.x * (TILES * 16);
-    const uint32_t n_steps = (p.K + DCM_KSTEP - 1) / DCM_KSTEP;
     extern __shared__ uint8_t dcm_dyn[];
     __shared__ uint64_t bars[TMA ? 2 * R::STAGES : 1];
     __shared__ uint32_t abort_s;
@@ -75,7 +77,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
         }
         __syncthreads();
     }
-    pdl_release();
+    if constexpr (!BASE) pdl_release();
     const uint8_t *w_packed = w.w_packed, *w_scale = w.w_scale;
     const uint16_t* x = w.x;
     if constexpr (BASE) {
@@ -100,7 +102,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
 
     if (!BASE && tid < DCM_MAX_TOKENS) {
         int32_t s = -1;
-        if (tid < p.M) {
+        if (p.seq_slot && tid < p.M) {
             s = p.seq_slot[tid];
             if (s >= 0) {
                 if (uint32_t(s) >= p.max_loras) { record_status(STATUS_SLOT_OUT_OF_RANGE); s = -1; }
@@ -115,6 +117,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
     }
 
     // ---- base: this thread's 32 codes per step of feature rows g and g + 8 of every tile, and of x rows g (+ 8 per n-tile) ----
+    const uint32_t n_steps = (p.K + DCM_KSTEP - 1) / DCM_KSTEP;
     const uint8_t* code_row[TILES][2];
     const uint8_t* scale_row[TILES][2];
 #pragma unroll
@@ -234,8 +237,9 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
         }
     }
 
+    if constexpr (BASE) pdl_release();
     // ---- LoRA granules of this warp ----
-    if constexpr (!BASE) {
+    if (!BASE && p.seq_slot) {
         __syncthreads();                                                        // slot_s, rank_s, b_s
         // this CTA's rows of B into L2 while the shrink may still run
         for (uint32_t m = warp; (!TMA || warp < WARPS) && m < p.M; m += WARPS) {

@@ -108,7 +108,7 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     // takes some 250 cycles whatever it waits for, a wait for the MMAs 80, and the arithmetic of four K blocks 760.  One token x 14336
     // features x 4096: an expansion warp was busy for 546 cycles a K block with a hand-over per pair of them, 349 of them without its
     // arithmetic; 344 now, and with stages of two K blocks of activations the base loop went from 41.7 to 24.8 thousand cycles, the
-    // call from 26 to 19 us (17 tokens, 8 adapters of rank 16 29.1 -> 22.2).
+    // call from 28.1 to 20.9 us (17 tokens, 8 adapters of rank 16 29.1 -> 22.2).
     static constexpr int A_COLS = KB / 2;                                  // TMEM columns of one K block
     static constexpr int A_GROUP = KRAW / KB;
     static constexpr int TMEM_A_BASE = MT < 32 ? 32 : MT;                  // accumulator occupies [0, MT)
