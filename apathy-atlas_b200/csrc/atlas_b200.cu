@@ -890,26 +890,32 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
 }
 
 // Where it is the faster one, both sides measured at cold L2 (us, this kernel / tcgen05):
-//   no adapters          1 token     1024 x 4096 4/9    4096 x 4096 6/12   14336 x 4096 15/26   4096 x 14336 15/25   28672 x 8192 45/90
-//                        16 tokens   1024 x 4096 5/9    4096 x 4096 9/12   14336 x 4096 19/26   4096 x 14336 23/25   28672 x 8192 59/91
-//   8 of rank 16         1 token     1024 x 4096 6/10   4096 x 4096 7/14   14336 x 4096 17/28   4096 x 14336 16/27   28672 x 8192 48/94
-//                        8 tokens    1024 x 4096 7/11   4096 x 4096 9/14   14336 x 4096 20/29   8192 x 8192 20/30    28672 x 8192 55/95
-//                        16 tokens                                         14336 x 4096 25/29                        28672 x 8192 70/96
-//   8 of rank 64         8 tokens    1024 x 4096 9/12   4096 x 4096 16/15  14336 x 4096 28/32   8192 x 8192 30/31    28672 x 8192 72/101
-// With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does: up
-// to eight tokens there unless the weights (N >= 2 K) outweigh it, and a long K only as long as the shrink is short (4096 x 14336,
-// 7 tokens: eight of rank 32 24/28, of rank 64 35/29; 6 tokens: eight of rank 64 32/29, sixteen 32/36).
-// Beyond eight tokens a granule (16 ranks of a slot) costs it some 0.3 us more than the tcgen05 form, against what it gains on the
-// weights: most where those are more than one wave of tiles there.  N >= 2 K, 16 adapters, 16 tokens: 32 granules 14336 x 4096 32/31,
-// 16384 x 6144 47/42, 28672 x 8192 88/101; 64 granules 37/35, 60/48, 103/107.
+//   no adapters          2 tokens    1024 x 4096 4.2/6.2   4096 x 4096 5.8/8.8    14336 x 4096 14.8/17.7  4096 x 14336 14.5/17.6  28672 x 8192 42/61
+//                        16 tokens   1024 x 4096 5.9/6.6   4096 x 4096 8.2/9.0    14336 x 4096 19.3/17.8  4096 x 14336 22.9/18.1  28672 x 8192 60/61
+//   8 of rank 16         2 tokens    1024 x 4096 6.1/9.4   4096 x 4096 7.6/12.1   14336 x 4096 17.3/21.1  4096 x 14336 16.1/20.7  28672 x 8192 47/65
+//                        16 tokens   1024 x 4096 7.7/10.5  4096 x 4096 11.6/12.8  14336 x 4096 24.6/22.1  4096 x 14336 28.8/21.9  28672 x 8192 69/67
+//   32 of rank 64        8 tokens    1024 x 4096 13.5/13.5 4096 x 4096 16.2/17.6  14336 x 4096 29.5/26.5  4096 x 14336 29.6/31.4  28672 x 8192 66/73
+// With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does.
+// N >= 2 K: up to eight tokens whatever the batch; beyond, a granule (16 ranks of a slot) costs it some 0.3 us more than the other, against
+// what it gains on the weights, most where those are more than one wave of tiles there.  The pool's size moves no call across that line
+// below 32 granules: a token's bits there do not depend on the adapters that are loaded.
+// N < 2 K, up to eight tokens: it loses only to many granules and where a long K meets so few features that the other splits it (8 tokens
+// of 32 of rank 16 x 4096 x 14336 24.3/21.7, 2 of rank 64 22.0/21.2; but of 32 of rank 64 29.6/31.4, 4 of rank 32 x 13824 x 14336 43/56).
+// Beyond eight (two n-tiles, no weights by TMA) both are estimated, in us: this kernel by its weights, the length of a CTA's loop and its
+// granules, the other by the K blocks a CTA takes one behind the other; measured from K = 1024 on.  12 tokens, 8 of rank 16 x 1024 x 4096
+// 7.3/10.3, x 4096 x 4096 10.9/12.7, x 8192 x 8192 21.9/22.5, but x 5120 x 5120 15.0/14.1 and 32 of rank 64 x 4096 x 4096 20.6/18.7.
 static bool decode_pays(const atlas_b200_linear_desc& d) {
     if (d.m > uint32_t(DCM_MAX_TOKENS)) return false;
     if (!d.seq_slot) return true;
-    if (uint64_t(d.n) >= 2ull * d.k) {
-        const uint32_t granules = std::min(d.m, d.max_loras) * ((d.max_rank + 15) / 16), waves = (d.n + tc::FT - 1) / tc::FT > uint32_t(rt_sm_count()) ? 2 : 1;
-        return d.m <= 8 || granules <= std::max(32u, d.k / (waves > 1 ? 80u : 128u));
-    }
-    return d.m <= 8 && uint64_t(d.m) * d.k <= (d.max_rank > 32 ? 86400u : 112000u);
+    const uint32_t granules = std::min(d.m, d.max_loras) * ((d.max_rank + 15) / 16), tiles = (d.n + tc::FT - 1) / tc::FT, sms = uint32_t(rt_sm_count());
+    if (uint64_t(d.n) >= 2ull * d.k) return d.m <= 8 || granules <= std::max(32u, d.k / (tiles > sms ? 80u : 128u));
+    if (d.m <= 8) return granules < 64 && (uint64_t(d.m) * d.k <= (d.max_rank > 32 ? 86400u : 112000u) || d.n > 5120 || granules > 8);
+    if (d.k < 1024) return false;
+    const uint32_t split = std::max(1u, std::min(std::min(sms / tiles, 8u), d.k / uint32_t(tc::KRAW))), waves = (tiles * split + sms - 1) / sms;
+    const float k = float(d.k) / 1024.0f, g = float(granules);
+    const float here = 4.7f + 0.26f * k * float(d.n) / 1024.0f + 0.27f * k + g * (0.08f * std::max(float(d.n) / 4096.0f, 1.0f) + 0.017f * k);
+    const float there = 8.1f + 3.4f * k * float(waves) / float(split) + 0.04f * g * float(waves);
+    return here < 0.93f * there;                 // (a batch may use fewer adapters than it could, which the other gains on)
 }
 
 static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {
