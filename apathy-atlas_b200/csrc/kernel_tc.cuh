@@ -91,8 +91,10 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int XROWS = PAIR ? MT / 2 : MT;                       // token rows of the tile this CTA stages
     static constexpr int X_TILE_BYTES = XROWS * KB * 2;
     // A16: a stage of activations is two K blocks: a round of the MMA thread (wait, MMAs, commit) takes some 340 cycles and 9 for every
-    // MMA of 16 columns, whatever it covers; with a round to a K block and a wait for either operand it was what the loop waited for
-    static constexpr int X_STAGE_BYTES = 2 * X_TILE_BYTES;
+    // MMA of 16 columns, whatever it covers; with a round to a K block and a wait for either operand it was what the loop waited for.
+    // One where 256 rows of it are staged: its MMAs hide the round, and there is room for two such stages only.
+    static constexpr int X_BLOCKS = XROWS >= 256 ? 1 : 2;
+    static constexpr int X_STAGE_BYTES = X_BLOCKS * X_TILE_BYTES;
     // A4: one stage = packed W [128 x 128 B] | packed x [MT x 128 B] | W scale bytes [128 x 16] | x scale bytes [MT x 16]
     static constexpr int S4_W = 0;
     static constexpr int S4_X = S4_W + RAW_PACKED_BYTES;
@@ -100,7 +102,7 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int S4_XS = S4_WS + RAW_SCALE_BYTES;
     static constexpr int S4_BYTES = ((S4_XS + MT * 16) + 1023) / 1024 * 1024;
     static constexpr int S4_STAGES = (200 * 1024) / S4_BYTES > 8 ? 8 : (200 * 1024) / S4_BYTES;
-    static constexpr int STAGES = A4 ? S4_STAGES : (XROWS >= 256 ? 2 : 4);
+    static constexpr int STAGES = A4 ? S4_STAGES : 4;
     // raw weight stages in flight: small token tiles leave shared memory free, and they are the
     // HBM-bound shapes that need many bytes in flight per SM
     static constexpr int RAW_STAGES = A4 ? STAGES : (XROWS >= 256 ? 2 : (XROWS >= 128 ? 4 : 6));
@@ -898,9 +900,9 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             // CTAs start their K loop at different K offsets (a rotation in units of one raw stage),
             // so concurrently running CTAs do not all pull the same activation lines at one moment.
             uint32_t s = 0, ph = 0;
-            for (uint32_t it = 0; it < num_kb; it += 2) {
+            for (uint32_t it = 0; it < num_kb; it += C::X_BLOCKS) {
                 if (!mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
-                const uint32_t n = SROWS && it + 1u == num_kb ? 1u : 2u;
+                const uint32_t n = SROWS && it + 1u == num_kb ? 1u : uint32_t(C::X_BLOCKS);
                 if (leader) mbar_arrive_expect_tx(BAR_FULL + 8 * s, CTAS * n * C::X_TILE_BYTES);
                 for (uint32_t u = 0; u < n; ++u) {
                     const uint32_t kb = kb_lo + (it + u + 4u * rot_raw) % num_kb, dst = x_tile0 + s * C::X_STAGE_BYTES + u * C::X_TILE_BYTES;
@@ -980,7 +982,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 }
             } else {
                 static_assert(C::A_GROUP == 4, "two stages of activations to a group of the weight operand");
-                for (uint32_t it = 0; it < num_kb; it += 2) {
+                for (uint32_t it = 0; it < num_kb; it += C::X_BLOCKS) {
                     const uint32_t j = it % 4u, g = (it / 4u) & 1u, a_tmem = tmem_a0 + (g * C::A_GROUP + j) * C::A_COLS;
                     // one wait for both operands: half of the lanes poll the group's barrier
                     const bool on_a = j == 0u && lane >= 16u;
@@ -992,12 +994,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                         // 16 k per instruction: 8 TMEM columns of A, 32 bytes along the swizzled row of B
 #pragma unroll
                         for (uint32_t i = 0; i < 4; ++i) umma_bf16_ts<PAIR>(tmem_acc, a_tmem + 8 * i, b_desc + 2 * i, idesc, acc | i);
-                        if (!SROWS || it + 1u < num_kb)
+                        if (C::X_BLOCKS > 1 && (!SROWS || it + 1u < num_kb))
 #pragma unroll
                             for (uint32_t i = 0; i < 4; ++i)
                                 umma_bf16_ts<PAIR>(tmem_acc, a_tmem + C::A_COLS + 8 * i, b_desc + uint64_t(C::X_TILE_BYTES >> 4) + 2 * i, idesc, 1u);
                         umma_commit<PAIR>(bar_empty, pair_mask);
-                        if (j || it + 2u >= num_kb) umma_commit<PAIR>(BAR_AEMPTY + 8 * g, pair_mask);
+                        if (j + C::X_BLOCKS == 4u || it + C::X_BLOCKS >= num_kb) umma_commit<PAIR>(BAR_AEMPTY + 8 * g, pair_mask);
                     }
                     __syncwarp();
                     acc = 1u;
