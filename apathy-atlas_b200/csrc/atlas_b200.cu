@@ -670,6 +670,12 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = 0u; t_last_shape[5] = 0u;
     if (shrink) {
+        // Gaps for the shrink where the two are about as long: two or three CTAs to a long K and up to 64 granules.  Without / with (us):
+        // 512 tokens x 4096 x 14336 8 of rank 16 60.8 / 57.9, 16 of rank 32 90.6 / 79.1, 700 x 2560 x 6912 59.6 / 52.4; but 64 of rank 64
+        // (several rounds of the shrink) 158.7 / 167.0, four CTAs (400 x 2048 x 14336) 37.0 / 39.7, one (1000 x 4096 x 14336, 8 of
+        // rank 64) 132 / 141, and 2048 of K to a CTA (512 x 4096 x 4096, 8 of rank 16) 25.2 / 27.3.
+        p.leave_gaps = MT >= 256 && (k_split == 2 || k_split == 3) && d.k > 2048 * k_split && d.m <= 1024 &&
+                               uint64_t(d.max_loras) * ((d.max_rank + 15) / 16) <= 64 ? 1u : 0u;
         // A small batch: the mma.sync shrink releases this kernel as soon as it is resident, which then runs beside it.  A large one:
         // the tcgen05 shrink fills its SMs and releases this kernel at the same point, whose CTAs then take SMs that are free or
         // become so; the mma.sync shrink, where it has to stand in, keeps the machine to itself.

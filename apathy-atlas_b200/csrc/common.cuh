@@ -34,8 +34,9 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 //                              dense linear, the QKV consumers, SwiGLU in both forms, the quantiser
 //   releasing                  all of these but lora_shrink_mma_kernel and lora_shrink_grouped_kernel, which do so only in front of a
 //                              main kernel or of the dense linear
-//   neither                    a main kernel over a t that an earlier call left releases but is launched in order; the NVFP4 decode, the
-//                              maximum, the CUDA-core linear and expand do neither
+//   neither                    a main kernel over a t that an earlier call left, and the small-batch kernel for more than eight tokens without
+//                              adapters, release but are launched in order; the NVFP4 decode, the maximum, the CUDA-core linear and
+//                              expand do neither
 // A dependent begins with the wait, with two exceptions:
 //   the main kernel and the dense linear behind their shrink read x, weights and routing ahead of it: that shrink has waited before
 //   releasing them; they wait before they read t, or before they end, on every path, so that nothing behind them overtakes the shrink;

@@ -172,6 +172,7 @@ struct Params {
     uint32_t lora_wide;            // granules of B_s that may come in one copy: 1, 2 or 4
     unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
+    uint32_t leave_gaps;           // 256-token tiles: the MMA thread lets the tensor cores run dry between stages, for the shrink beside
     uint32_t chained;              // launched as a programmatic dependent of whatever is before it (no adapters): wait before reading anything
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
@@ -988,6 +989,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     const bool on_a = j == 0u && lane >= 16u;
                     ok = mbar_wait_warp_timed(on_a ? BAR_AFULL + 8 * g : bar_full, on_a ? (it / 8u) & 1u : ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
+                    // MMAs of 256 columns queued behind one another leave the mma.sync of the shrink beside this kernel next to nothing: the
+                    // stage before has to be done (every EMPTY of it is committed), which is a gap of some 100 in 1024 cycles
+                    if (MT >= 256 && p.leave_gaps && it) {
+                        ok = mbar_wait_warp(s ? bar_empty - 8 : BAR_EMPTY + 8 * (C::STAGES - 1), s ? ph : ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, 32);
+                        if (!ok) break;
+                    }
                     tcgen05_fence_after();
                     const uint64_t b_desc = make_kmajor_sw128_desc(x_tile0 + s * C::X_STAGE_BYTES);
                     if (elect_one()) {

@@ -72,3 +72,21 @@ def test_lora_blocks_of_the_persistent_kernel(cuda, atlas, oracle, ranks, max_ra
     rows, cols = _sample(case, max_rank)
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols, act_fp4=fp4), "blocks")
     assert atlas.device_status() == 0
+
+
+# two and three CTAs to a tile's K beside the shrink, pairs and single CTAs: rings that wrap with the stage before waited for
+@pytest.mark.parametrize("form", ["", "single"])
+@pytest.mark.parametrize("M,K,N", [(400, 4608, 4096), (512, 6400, 2560), (300, 4352, 4090)])
+def test_gaps_for_the_shrink(cuda, atlas, oracle, M, K, N, form):
+    from atlas_b200 import synth
+    case = synth.make_case("gaps", M=M, K=K, N=N, ranks=[32, 16, 8, 24], max_rank=32, none_frac=0.15, scale2=0.02, b_std=0.1, seed=M + K)
+    dc = DeviceCase(cuda, atlas, case)
+    flags = atlas.FLAG_NO_CTA_PAIR if form else 0
+    y, _ = dc.run(flags=flags, lora_ws=True)
+    shape = atlas.last_launch_shape()
+    assert shape["token_tile"] == 256 and shape["k_split"] in (2, 3), shape
+    rows, cols = _sample(case, K)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), form)
+    for _ in range(3):
+        assert np.array_equal(dc.run(flags=flags, lora_ws=True)[0], y)
+    assert atlas.device_status() == 0
