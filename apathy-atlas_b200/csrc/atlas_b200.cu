@@ -919,9 +919,9 @@ static bool decode_pays(const atlas_b200_linear_desc& d) {
     if (d.k < 1024) return false;
     const uint32_t split = std::max(1u, std::min(std::min(sms / tiles, 8u), d.k / uint32_t(tc::KRAW))), waves = (tiles * split + sms - 1) / sms;
     const float k = float(d.k) / 1024.0f, g = float(granules);
-    const float here = 4.7f + 0.26f * k * float(d.n) / 1024.0f + 0.27f * k + g * (0.08f * std::max(float(d.n) / 4096.0f, 1.0f) + 0.017f * k);
+    const float here = 4.7f + 0.26f * k * float(d.n) / 1024.0f + 0.27f * k + g * (0.07f * std::max(float(d.n) / 4096.0f, 1.0f) + 0.017f * k);
     const float there = 8.1f + 3.4f * k * float(waves) / float(split) + 0.04f * g * float(waves);
-    return here < 0.93f * there;                 // (a batch may use fewer adapters than it could, which the other gains on)
+    return here < 0.95f * there;                 // (a batch may use fewer adapters than it could, which the other gains on)
 }
 
 static int launch_decode(const atlas_b200_linear_desc& d, const ShrinkParams* shrink, cudaStream_t st) {

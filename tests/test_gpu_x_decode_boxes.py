@@ -41,3 +41,21 @@ def test_rows_of_a_large_layer(cuda, atlas, m, n, k, loras, rank):
     for _ in range(3):
         assert torch.equal(call(0, n), want)
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,ads,max_rank,small", [
+    (12, 1024, 1024, 2, 16, True), (16, 1056, 1100, 3, 8, True), (9, 992, 1024, 2, 16, False),       # N < 2 K from K = 1024 on
+    (12, 4096, 4096, 8, 16, True), (12, 4096, 4096, 32, 64, False), (12, 5120, 1280, 2, 16, True),  # few granules, many
+    (8, 1024, 1024, 8, 112, True), (8, 1024, 1024, 8, 128, False),                                  # up to eight tokens: 56 granules, 64
+    (8, 14336, 6144, 2, 32, True), (8, 14336, 136, 2, 32, False), (8, 14336, 136, 8, 32, True),     # features, granules over a long K
+])
+def test_which_batches_below_twice_k_are_small(cuda, atlas, oracle, M, K, N, ads, max_rank, small):
+    import numpy as np
+    from atlas_b200 import synth
+    from gpu_util import DeviceCase, assert_close, ideal
+    case = synth.make_case("line", M=M, K=K, N=N, ranks=[max_rank] * ads, max_rank=max_rank, scale2=0.02, b_std=0.1, seed=M + N)
+    y, variant = DeviceCase(cuda, atlas, case).run(lora_ws=True)
+    assert variant == atlas.VARIANT_TCGEN05 and (atlas.last_launch_shape()["token_tile"] == 8) == small
+    rows, cols = np.arange(M, dtype=np.uint32), np.sort(np.random.default_rng(N).choice(N, min(N, 96), replace=False)).astype(np.uint32)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), "line")
+    assert atlas.device_status() == 0
