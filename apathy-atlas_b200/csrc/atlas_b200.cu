@@ -660,11 +660,9 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     p.lora_wide = lora_wide;
     dim3 grid((d.n + tc::FT - 1) / tc::FT, (d.m + MT - 1) / MT);
     if (PAIR) grid.x = (grid.x + 1u) & ~1u;      // whole pairs: a CTA past the last feature loads zeros and stores nothing
-    // split K: k_split CTAs along z form a cluster (times two for pairs), share one tile and exchange partial sums;
-    // the receive area is ceil(chunks / k_split) 8 KB blocks from each of them
-    if (k_split > 1 && (k_split * (PAIR ? 2u : 1u) > 8u ||
-                        size_t(k_split) * ((MT / 16 + k_split - 1) / k_split) * 8192 > size_t(C::STAGING_BYTES)))
-        return ATLAS_B200_ERR_LIMIT;
+    // split K: k_split CTAs along z form a cluster (times two for pairs), share one tile and exchange partial sums
+    // (the staging area holds those of every split up to this one)
+    if (k_split > uint32_t(C::MAX_SPLIT)) return ATLAS_B200_ERR_LIMIT;
     grid.z = k_split;
     p.k_split = k_split;
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;

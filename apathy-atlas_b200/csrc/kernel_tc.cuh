@@ -135,7 +135,15 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static constexpr int L_TILE_A = 4 * L_GRAN_A;
     static constexpr int L_BLOCK = L_TILE_A + 4 * L_GRAN_T;
     static constexpr int L_STAGES = (STAGING_BASE / L_BLOCK) >= 4 ? 4 : ((STAGING_BASE / L_BLOCK) >= 3 ? 3 : 4);
-    static constexpr int STAGING_BYTES = STAGING_BASE > L_STAGES * L_BLOCK ? STAGING_BASE : L_STAGES * L_BLOCK;
+    // ... and then for the partial tiles of a split K, of which each CTA receives ceil(chunks / k_split) chunks of 16 tokens from each.  (Not
+    // every split wants the same: of 16 chunks seven CTAs exchange 168 KB, eight 128 KB.)
+    static constexpr int MAX_SPLIT = PAIR ? 4 : 8;                               // (clusters of eight CTAs)
+    static constexpr int split_bytes(int k_split) { return k_split * ((MT / 16 + k_split - 1) / k_split) * (16 * FT * 4); }
+    static constexpr int most_split_bytes(int k_split = MAX_SPLIT) {
+        return k_split < 2 ? 0 : (split_bytes(k_split) > most_split_bytes(k_split - 1) ? split_bytes(k_split) : most_split_bytes(k_split - 1));
+    }
+    static constexpr int STAGING_RINGS = STAGING_BASE > L_STAGES * L_BLOCK ? STAGING_BASE : L_STAGES * L_BLOCK;
+    static constexpr int STAGING_BYTES = STAGING_RINGS > most_split_bytes() ? STAGING_RINGS : most_split_bytes();
     static constexpr int OFF_KEY = STAGING_BYTES;                                // uint32[MT]  (scratch of the list build)
     static constexpr int OFF_GRAN = OFF_KEY + MT * 4;                            // uint16[MAX_GRANULES]
     static constexpr int OFF_BITMAP = OFF_GRAN + MAX_GRANULES * 2;               // uint32[128]

@@ -42,3 +42,31 @@ def test_split_matches_unsplit_and_oracle(cuda, atlas, oracle, M, K, N, ranks, m
     none = case.seq_slot < 0
     assert none.any() and np.array_equal(y_split[none], yb[none])
     assert atlas.device_status() == 0
+
+
+# every number of CTAs that may share a tile's K, tiles of 256 tokens by single CTAs and by pairs: their partial tiles fit
+@pytest.mark.parametrize("mode", ["", "fp4", "single", "base"])
+@pytest.mark.parametrize("M,K,N", [(200, 1792, 1024), (256, 1792, 256), (140, 2304, 128)] + [(250, 256 * s, 376) for s in range(2, 9)] + [(130, 1920, 520), (256, 2016, 264)])
+def test_every_split_of_256_token_tiles(cuda, atlas, oracle, M, K, N, mode):
+    from atlas_b200 import synth
+    fp4 = mode == "fp4"
+    if fp4 and K % 256:
+        pytest.skip("FP4 activations take whole stages of 256")
+    case = synth.make_case("splits", M=M, K=K, N=N, ranks=[8, 16, 32], max_rank=32, none_frac=0.1, scale2=0.02, b_std=0.1, seed=M + K + N)
+    dc = DeviceCase(cuda, atlas, case)
+    flags = (atlas.FLAG_ACT_FP4 if fp4 else 0) | (atlas.FLAG_NO_CTA_PAIR if mode == "single" else 0)
+    y, variant = dc.run(flags=flags, lora_ws=True, lora=mode != "base")
+    assert variant == atlas.VARIANT_TCGEN05
+    shape = atlas.last_launch_shape()
+    assert shape["token_tile"] == 256
+    if mode == "single" and K // 256 <= 8:               # (residency may take the paired form to fewer)
+        assert shape["k_split"] == K // 256, shape
+    rng = np.random.default_rng(K)
+    rows, cols = (np.sort(rng.choice(n, min(n, k), replace=False)).astype(np.uint32) for n, k in ((M, 48), (N, 96)))
+    if mode != "base":
+        assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols, act_fp4=fp4), mode)
+    else:
+        one, _ = dc.run(flags=atlas.FLAG_NO_K_SPLIT, lora=False)
+        a, b = oracle.bf16_to_f32(y), oracle.bf16_to_f32(one)      # (they differ only in the order of FP32 additions)
+        assert np.abs(a - b).max() <= 2e-2 * np.abs(b).max()
+    assert atlas.device_status() == 0
