@@ -1640,6 +1640,35 @@ int atlas_b200_selftest_bounded_wait(uint64_t limit_ns, uint32_t out_host[3]) {
     return cuda_status(e);
 }
 
+int atlas_b200_selftest_ring_wait(uint32_t* out_written) {
+    if (!out_written) return ATLAS_B200_ERR_NULL;
+    constexpr uint32_t K = 1024, N = 16;
+    using R = DcmRing<1, 8>;
+    const auto kernel = nvfp4_lora_decode_mma_kernel<1, 1, 8, true, true, true>;
+    uint16_t* buf = nullptr;                                  // x [K], then y [N]
+    uint16_t y[N];
+    CUtensorMap none;
+    std::memset(&none, 0, sizeof(none));                      // never dereferenced: nothing is fetched
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaMalloc(&buf, (K + N) * sizeof(uint16_t));
+    if (e != cudaSuccess) return cuda_status(e);
+    e = cudaMemset(buf, 0x5A, (K + N) * sizeof(uint16_t));
+    tc::Params p{};
+    DecodeParams w{};
+    w.x = buf; w.x_row_stride = K;
+    p.y = p.y_dest[0] = buf + K; p.n_dest = 1;
+    p.M = 1; p.N = N; p.K = K; p.out_row_stride = N; p.out_scale = 1.0f; p.k_split = 1;
+    if (e == cudaSuccess) {
+        kernel<<<1, 32 * 9, R::SMEM_BYTES>>>(w, p, none, none);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(y, buf + K, sizeof(y), cudaMemcpyDeviceToHost);
+    cudaFree(buf);
+    *out_written = 0;
+    for (const uint16_t v : y) *out_written += v != 0x5A5A;
+    return cuda_status(e);
+}
+
 int atlas_b200_last_variant(void) { return t_last_variant; }
 
 int atlas_b200_last_launch_shape(uint32_t out[4]) {

@@ -51,8 +51,8 @@ template <int TILES, int WARPS> struct DcmRing {
 // is before it (instances of their own: the wait in all of them cost calls with adapters 1 to 2 %).  Those release late: a next grid
 // that comes while this one's CTAs are all at work takes the places they happen to leave, and its SMs get unequal numbers of CTAs.  One
 // token behind one another, launched in order / released at the start / behind the loop (us): 11008 x 4096 12.8 / 14.4 / 11.9, 2048 x
-// 2048 2.8 / - / 2.4; 12 tokens x 1280 x 17408 14.1 / 20.4 / 15.2.
-template <int TILES, int NT, int WARPS, bool TMA, bool BASE>
+// 2048 2.8 / - / 2.4; 12 tokens x 1280 x 17408 14.1 / 20.4 / 15.2.  SELFTEST: nothing fills the ring, and every wait on it runs out.
+template <int TILES, int NT, int WARPS, bool TMA, bool BASE, bool SELFTEST = false>
 __global__ void __launch_bounds__(32 * (WARPS + (TMA ? 1 : 0)), 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {
     using R = DcmRing<TILES, WARPS>;
@@ -85,7 +85,7 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
         w_packed = pdl_after(w_packed); w_scale = pdl_after(w_scale); x = pdl_after(x);
     }
     if (TMA && warp == WARPS) {
-        if (lane == 0) {
+        if (lane == 0 && !SELFTEST) {
             uint32_t s = 0, ph = 0;
             for (uint32_t k0 = 0; k0 < p.K; k0 += DCM_KSTEP * WARPS) {          // (zero-filled past K and N)
                 if (!tc::mbar_wait(BAR_EMPTY + 8 * s, ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_PRODUCER)) break;
@@ -201,7 +201,8 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
         const uint32_t scale_at = R::CODES + g * (8 * WARPS) + (((warp >> 1) ^ swz) << 4) + (warp & 1u) * 8 + 2 * t;
         uint32_t s = 0, ph = 0;
         auto turn = [&](uint32_t step, const uint4 (&xs)[X_AHEAD ? 4 : 1], float (&sum)[TILES][NT][4]) -> bool {
-            if (!tc::mbar_wait(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT)) return false;
+            // (a vote: lanes that gave up one by one would leave the others in warp-wide instructions, waiting for them)
+            if (!tc::mbar_wait_warp(BAR_FULL + 8 * s, ph, abort_flag, STATUS_WAIT_EXPIRED_DEQUANT)) return false;
             const uint32_t st = ring + s * R::STAGE;
 #pragma unroll
             for (int i = 0; i < TILES; ++i)

@@ -481,6 +481,10 @@ ATLAS_B200_API int atlas_b200_device_status(uint32_t* out_word, int clear);
  * raise the CTA's abort flag, through which a second waiter leaves; the kernel returns normally.
  * out[0], out[1] = 1 if the first / second waiter gave up, out[2] = nanoseconds the first one waited. */
 ATLAS_B200_API int atlas_b200_selftest_bounded_wait(uint64_t limit_ns, uint32_t out[3]);
+/* The same for a ring of the kernel for the smallest batches, whose waiters are whole warps in front of warp-wide instructions: one CTA of
+ * it, with nothing that fills the ring, must give up after its limit (1 s), record status 0x101 and return.
+ * *out_written = how many of its 16 outputs it wrote all the same. */
+ATLAS_B200_API int atlas_b200_selftest_ring_wait(uint32_t* out_written);
 ATLAS_B200_API int atlas_b200_last_variant(void);
 /* Launch shape of the most recent tcgen05 call on this thread (launcher audit, no counterpart in the reference):
  * out[0] = token tile (8: the mma.sync form of the smallest batches; 16 and more otherwise), out[1] = 1 if CTAs were paired for two-CTA MMAs, out[2] = CTAs per output tile (K split),

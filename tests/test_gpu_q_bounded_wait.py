@@ -28,3 +28,11 @@ def test_wait_gives_up_records_the_status_and_the_context_survives(cuda, atlas, 
 def test_selftest_refuses_long_limits(atlas, cuda):
     with pytest.raises(atlas.AtlasError):
         atlas.selftest_bounded_wait(10_000_000_000)
+
+
+def test_a_ring_that_nothing_fills(atlas, cuda):
+    """The small-batch kernel's warps wait in front of warp-wide instructions: they give up together, and the kernel returns."""
+    assert atlas.device_status() == 0
+    atlas.selftest_ring_wait()
+    assert atlas.device_status() == 0x101          # STATUS_WAIT_EXPIRED_DEQUANT
+    assert (cuda.ones(64, device="cuda") * 2).sum().item() == 128 and atlas.device_status() == 0
