@@ -313,7 +313,9 @@ nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __g
 #pragma unroll
                 for (int e = 0; e < 4; ++e) part[warp + h * WARPS][8 * n + 2 * t + (e & 1)][16 * i + g + 8 * (e >> 1)] = acc[h][i][n][e];
     __syncthreads();
-    for (uint32_t i = tid; (!TMA || warp < WARPS) && i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
+    // (a tile whose weights did not all arrive stays unwritten)
+    const bool whole_sums = !TMA || (warp < WARPS && !*abort_flag);
+    for (uint32_t i = tid; whole_sums && i < NT * 8 * TILES * 16; i += (32 * WARPS)) {          // (whole warps: a multiple of 128)
         const uint32_t m = i / (TILES * 16), fi = i % (TILES * 16), f = f0 + fi;
         float sum = part[0][m][fi];
 #pragma unroll

@@ -31,8 +31,9 @@ def test_selftest_refuses_long_limits(atlas, cuda):
 
 
 def test_a_ring_that_nothing_fills(atlas, cuda):
-    """The small-batch kernel's warps wait in front of warp-wide instructions: they give up together, and the kernel returns."""
+    """The small-batch kernel's warps wait in front of warp-wide instructions: they give up together, and the kernel returns, its outputs
+    unwritten."""
     assert atlas.device_status() == 0
-    atlas.selftest_ring_wait()
+    assert atlas.selftest_ring_wait() == 0
     assert atlas.device_status() == 0x101          # STATUS_WAIT_EXPIRED_DEQUANT
     assert (cuda.ones(64, device="cuda") * 2).sum().item() == 128 and atlas.device_status() == 0
