@@ -993,10 +993,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                 static_assert(C::A_GROUP == 4, "two stages of activations to a group of the weight operand");
                 for (uint32_t it = 0; it < num_kb; it += C::X_BLOCKS) {
                     const uint32_t j = it % 4u, g = (it / 4u) & 1u, a_tmem = tmem_a0 + (g * C::A_GROUP + j) * C::A_COLS;
-                    // one wait for both operands: half of the lanes poll the group's barrier
+                    // one wait for both operands: half of the lanes poll the group's barrier, and the __syncwarp orders the lane that
+                    // issues behind what the others have seen (a vote does not)
                     const bool on_a = j == 0u && lane >= 16u;
                     ok = mbar_wait_warp_timed(on_a ? BAR_AFULL + 8 * g : bar_full, on_a ? (it / 8u) & 1u : ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
+                    __syncwarp();
                     // MMAs of 256 columns queued behind one another leave the mma.sync of the shrink beside this kernel next to nothing: the
                     // stage before has to be done (every EMPTY of it is committed), which is a gap of some 100 in 1024 cycles
                     if (MT >= 256 && p.leave_gaps && it) {
