@@ -47,7 +47,7 @@ EXPORTS = (
     "atlas_b200_build_seq_slot", "atlas_b200_routed_prefill_slot_of", "atlas_b200_peft_scaling",
     "atlas_b200_module_dims", "atlas_b200_pool_slot_bytes", "atlas_b200_slot_base_offset",
     "atlas_b200_module_slot_offsets", "atlas_b200_pack_module", "atlas_b200_build_route_tables", "atlas_b200_select_victim_slot",
-    "atlas_b200_device_status", "atlas_b200_last_variant", "atlas_b200_last_launch_shape", "atlas_b200_last_persistent_shape",
+    "atlas_b200_device_status", "atlas_b200_last_variant", "atlas_b200_last_launch_shape", "atlas_b200_last_persistent_shape", "atlas_b200_last_launch_details",
     "atlas_b200_set_profile_buffer", "atlas_b200_peft_parse", "atlas_b200_peft_config_scaling", "atlas_b200_classify_key",
     "atlas_b200_adapter_id_hash", "atlas_b200_convert_to_bf16", "atlas_b200_registry_create", "atlas_b200_registry_destroy",
     "atlas_b200_registry_slot_bytes", "atlas_b200_registry_pool_bytes", "atlas_b200_registry_load_adapter",
@@ -477,8 +477,10 @@ def last_launch_shape() -> dict:
     _check("atlas_b200_last_launch_shape", lib().atlas_b200_last_launch_shape(out))
     per = (C.c_uint32 * 2)()
     _check("atlas_b200_last_persistent_shape", lib().atlas_b200_last_persistent_shape(per))
+    more = (C.c_uint32 * 1)()
+    _check("atlas_b200_last_launch_details", lib().atlas_b200_last_launch_details(more))
     return {"token_tile": out[0], "cta_pair": bool(out[1]), "k_split": out[2], "lora_tiles_from_shrink": bool(out[3]),
-            "persistent_tiles_per_pass": per[0], "persistent_cta_pairs": per[1]}
+            "persistent_tiles_per_pass": per[0], "persistent_cta_pairs": per[1], "gaps_for_shrink": bool(more[0])}
 
 
 def device_status(clear: bool = True) -> int:

@@ -38,7 +38,7 @@
 namespace atlas {
 
 static thread_local int t_last_variant = ATLAS_B200_VARIANT_NONE;
-static thread_local uint32_t t_last_shape[6] = {0, 0, 0, 0, 0, 0};
+static thread_local uint32_t t_last_shape[7] = {0, 0, 0, 0, 0, 0, 0};
 static unsigned long long* g_profile_buf = nullptr;   // device buffer for per-CTA cycle counters (diagnostics)
 static size_t g_profile_words = 0;
 
@@ -666,14 +666,18 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     grid.z = k_split;
     p.k_split = k_split;
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;
-    t_last_shape[4] = 0u; t_last_shape[5] = 0u;
+    t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
     if (shrink) {
-        // Gaps for the shrink where the two are about as long: two or three CTAs to a long K and up to 64 granules.  Without / with (us):
-        // 512 tokens x 4096 x 14336 8 of rank 16 60.8 / 57.9, 16 of rank 32 90.6 / 79.1, 700 x 2560 x 6912 59.6 / 52.4; but 64 of rank 64
-        // (several rounds of the shrink) 158.7 / 167.0, four CTAs (400 x 2048 x 14336) 37.0 / 39.7, one (1000 x 4096 x 14336, 8 of
-        // rank 64) 132 / 141, and 2048 of K to a CTA (512 x 4096 x 4096, 8 of rank 16) 25.2 / 27.3.
-        p.leave_gaps = MT >= 256 && (k_split == 2 || k_split == 3) && d.k > 2048 * k_split && d.m <= 1024 &&
+        // Gaps while the shrink runs, for pairs whose CTAs contract more than it takes (their MMAs leave no idle cycles): up to three CTAs
+        // to a long K, and up to 64 granules.  Without / before every other stage / before every stage / before every stage of the whole
+        // loop (us): 512 tokens x 4096 x 14336 8 of rank 16 59.3 / 52.3 / 53.4 / 57.9, 16 of rank 32 in sequences 87.5 / 74.4 / 73.2 /
+        // 79.2, 400 x 2560 x 6912 31.1 / 27.8 / 28.4 / 29.5, 1000 x 4096 x 14336 8 of rank 32 in sequences 123.9 / 111.1 / 112.7 / -; but
+        // 64 of rank 64 (several rounds of the shrink) 512 x 4096 x 14336 157.8 / 159.2, 512 x 2560 x 6912 79.1 / 80.6, four CTAs (130
+        // x 4096 x 14336) 34.7 / 36.5, 2048 of K to one of two (512 x 4096 x 4096) 25.2 / 25.8, K = 4096 (256 x 14336) 35.3 / 35.8, and
+        // single CTAs, which wait for shared memory (700 x 3072 x 9216) 38.7 / 41.6.
+        p.leave_gaps = PAIR && MT >= 256 && !A4 && k_split <= 3 && d.k > std::max(4096u, 2048u * k_split) && d.m <= 1024 &&
                                uint64_t(d.max_loras) * ((d.max_rank + 15) / 16) <= 64 ? 1u : 0u;
+        t_last_shape[6] = p.leave_gaps;
         // A small batch: the mma.sync shrink releases this kernel as soon as it is resident, which then runs beside it.  A large one:
         // the tcgen05 shrink fills its SMs and releases this kernel at the same point, whose CTAs then take SMs that are free or
         // become so; the mma.sync shrink, where it has to stand in, keeps the machine to itself.
@@ -791,7 +795,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     p.lora_wide = lora_wide;
     const uint32_t pairs = std::min<uint32_t>(uint32_t(clusters), pp.n_tiles);
     t_last_shape[0] = MT; t_last_shape[1] = 1u; t_last_shape[2] = 1u; t_last_shape[3] = tt.tiles ? 1u : 0u;
-    t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs;
+    t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs; t_last_shape[6] = 0u;
     if (shrink) {
         const int rc = launch_shrink(*shrink, d.max_loras, st, d.m > 1024 ? MachineBeside::none : MachineBeside::all);
         if (rc) return rc;
@@ -834,7 +838,7 @@ static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParam
     w.w_scale = static_cast<const uint8_t*>(d.w_scale);
     w.x_row_stride = d.x_row_stride;
     const uint32_t ctas = (d.n + 16 * TILES - 1) / (16 * TILES);
-    t_last_shape[0] = 8u; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
+    t_last_shape[0] = 8u; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
     if (shrink) {
         rc = launch_shrink(*shrink, d.max_loras, st, ctas * 3 <= uint32_t(rt_sm_count()) * 2 ? MachineBeside::part : MachineBeside::all);
         if (rc) return rc;
@@ -997,7 +1001,7 @@ static int launch_dense_tc(const atlas_b200_linear_desc& d, bool after_shrink, c
     const uint32_t tiles = ((d.n + tc::FT - 1) / tc::FT) * ((d.m + mt - 1) / mt);
     uint32_t k_split = std::max(1u, std::min(std::min(uint32_t(rt_sm_count()) / std::max(tiles, 1u), 8u), d.k / uint32_t(tc::KB)));
     while (k_split & (k_split - 1)) --k_split;           // a power of two: clusters of 1, 2, 4 or 8
-    t_last_shape[0] = mt; t_last_shape[1] = 0u; t_last_shape[2] = k_split; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u;
+    t_last_shape[0] = mt; t_last_shape[1] = 0u; t_last_shape[2] = k_split; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
     if (mt == 16) return launch_dense_tc_mt<16>(d, 0, k_split, after_shrink, st);
     if (mt == 32) return launch_dense_tc_mt<32>(d, 1, k_split, after_shrink, st);
     if (mt == 64) return launch_dense_tc_mt<64>(d, 2, k_split, after_shrink, st);
@@ -1681,6 +1685,12 @@ int atlas_b200_last_persistent_shape(uint32_t out[2]) {
     if (!out) return ATLAS_B200_ERR_NULL;
     out[0] = t_last_shape[4];
     out[1] = t_last_shape[5];
+    return ATLAS_B200_OK;
+}
+
+int atlas_b200_last_launch_details(uint32_t out[1]) {
+    if (!out) return ATLAS_B200_ERR_NULL;
+    out[0] = t_last_shape[6];
     return ATLAS_B200_OK;
 }
 

@@ -180,7 +180,8 @@ struct Params {
     uint32_t lora_wide;            // granules of B_s that may come in one copy: 1, 2 or 4
     unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
-    uint32_t leave_gaps;           // 256-token tiles: the MMA thread lets the tensor cores run dry between stages, for the shrink beside
+    uint32_t leave_gaps;           // pairs, 256-token tiles: while the shrink runs beside this kernel the MMA thread lets the tensor cores
+                                   //       run dry before every other stage
     uint32_t chained;              // launched as a programmatic dependent of whatever is before it (no adapters): wait before reading anything
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
@@ -792,7 +793,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
     const uint32_t BAR_EPI = BAR_DRAINED + 8;                          // every epilogue warp has put its part of the tile into shared memory
     const uint32_t BAR_AFULL = BAR_EPI + 8, BAR_AEMPTY = BAR_AFULL + 16;   // [2] each, A16: groups of the weight operand
     volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(smem_gen + C::OFF_MISC);
-    // misc[0] = TMEM base address, misc[1] = granule count, misc[2] = abort flag, misc[3] = slots that occur in the tile
+    // misc[0] = TMEM base address, misc[1] = granule count, misc[2] = abort flag, misc[3] = slots that occur in the tile, misc[4] = the
+    // shrink is done (leave_gaps)
     volatile uint32_t* abort_flag = misc + 2;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -846,6 +848,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
         misc[1] = 0;
         misc[2] = 0;
         misc[3] = 0;
+        misc[4] = 0;
         fence_barrier_init();
     }
     if (warp == 1) {
@@ -967,6 +970,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             bool ok = true;
             uint32_t s = 0, ph = 0, acc = 0;
             uint32_t bar_full = BAR_FULL, bar_empty = BAR_EMPTY;
+            // (single CTAs never leave gaps, but keep the test: without it 512 tokens x 2048 x 8192, 8 of rank 16, take 28.5 instead of 27.9 us)
+            bool gaps = MT >= 256 && p.leave_gaps;
             if constexpr (A4) {
                 // four K=64 block-scaled instructions per stage; both operands are the packed tiles, the
                 // scales sit in this stage's TMEM columns
@@ -999,9 +1004,11 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     ok = mbar_wait_warp_timed(on_a ? BAR_AFULL + 8 * g : bar_full, on_a ? (it / 8u) & 1u : ph, abort_flag, STATUS_WAIT_EXPIRED_MMA, prof, w_full, MMA_BACKOFF_NS);
                     if (!ok) break;
                     __syncwarp();
-                    // MMAs of 256 columns queued behind one another leave the mma.sync of the shrink beside this kernel next to nothing: the
-                    // stage before has to be done (every EMPTY of it is committed), which is a gap of some 100 in 1024 cycles
-                    if (MT >= 256 && p.leave_gaps && it) {
+                    // MMAs of 256 columns queued behind one another leave the mma.sync of the shrink beside this kernel next to nothing: before
+                    // every other stage the one before has to be done (every EMPTY of it is committed), a gap of some 100 in 2048 cycles,
+                    // until the list warps have seen the shrink end
+                    gaps = gaps && !__any_sync(0xFFFFFFFFu, misc[4]);
+                    if (gaps && (it & 2u)) {
                         ok = mbar_wait_warp(s ? bar_empty - 8 : BAR_EMPTY + 8 * (C::STAGES - 1), s ? ph : ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, 32);
                         if (!ok) break;
                     }
@@ -1119,6 +1126,12 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(src & ~15ull));
                 }
             }
+        }
+
+        // (these warps have nothing to do until the accumulator is complete, which wants the shrink's t anyway)
+        if (PAIR && MT >= 256 && !A4 && p.leave_gaps) {
+            pdl_wait();
+            if (te == 0) misc[4] = 1;
         }
 
         // ---- epilogue, shared with the expansion warps: TMEM lane = feature, column = token ----

@@ -74,7 +74,7 @@ def test_lora_blocks_of_the_persistent_kernel(cuda, atlas, oracle, ranks, max_ra
     assert atlas.device_status() == 0
 
 
-# two and three CTAs to a tile's K beside the shrink, pairs and single CTAs: rings that wrap with the stage before waited for
+# two and three CTAs to a tile's K beside the shrink, pairs (with gaps) and single CTAs: rings that wrap with the stage before waited for
 @pytest.mark.parametrize("form", ["", "single"])
 @pytest.mark.parametrize("M,K,N", [(400, 4608, 4096), (512, 6400, 2560), (300, 4352, 4090)])
 def test_gaps_for_the_shrink(cuda, atlas, oracle, M, K, N, form):
@@ -85,8 +85,25 @@ def test_gaps_for_the_shrink(cuda, atlas, oracle, M, K, N, form):
     y, _ = dc.run(flags=flags, lora_ws=True)
     shape = atlas.last_launch_shape()
     assert shape["token_tile"] == 256 and shape["k_split"] in (2, 3), shape
+    assert shape["gaps_for_shrink"] == shape["cta_pair"] and shape["cta_pair"] == (form == ""), shape
     rows, cols = _sample(case, K)
     assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols), form)
     for _ in range(3):
         assert np.array_equal(dc.run(flags=flags, lora_ws=True)[0], y)
+    assert atlas.device_status() == 0
+
+
+# either side of the lines: K, CTAs to a tile's K, granules, tokens, pairs, a shrink to run beside
+@pytest.mark.parametrize("M,K,N,ads,max_rank,flags,gaps", [
+    (1000, 4352, 4096, 4, 32, 0, True), (1000, 4096, 4096, 4, 32, 0, False), (512, 4352, 2560, 4, 32, 0, False), (512, 6400, 1024, 4, 32, 0, False),
+    (400, 4608, 4096, 16, 64, 0, True), (400, 4608, 4096, 65, 16, 0, False), (400, 4608, 4096, 1, 8, 0, True), (300, 4608, 4096, 2, 16, "single", False),
+    (400, 4608, 4096, 2, 16, "base", False), (1030, 4352, 1000, 2, 16, 0, False)])
+def test_which_calls_leave_gaps(cuda, atlas, oracle, M, K, N, ads, max_rank, flags, gaps):
+    from atlas_b200 import synth
+    case = synth.make_case("gap_lines", M=M, K=K, N=N, ranks=[max_rank] * ads, max_rank=max_rank, none_frac=0.15, scale2=0.02, b_std=0.1, seed=M + ads)
+    dc = DeviceCase(cuda, atlas, case)
+    y, _ = dc.run(flags=atlas.FLAG_NO_CTA_PAIR if flags == "single" else 0, lora_ws=True, lora=flags != "base")
+    assert atlas.last_launch_shape()["gaps_for_shrink"] == gaps, atlas.last_launch_shape()
+    rows, cols = _sample(case, K)
+    assert_close(oracle, y[np.ix_(rows, cols)], ideal(oracle, case, rows=rows, cols=cols, lora=flags != "base"), "gaps")
     assert atlas.device_status() == 0
