@@ -1198,8 +1198,11 @@ int nvfp4_lora_linear(const atlas_b200_linear_desc& d, cudaStream_t st, const Sh
         // (the shrink alone writes tiles, which the decode form does not read: it is planned as a call of the tcgen05 form)
         const TcPlan plan = plan_tc(d, shrink_only ? d.flags | ATLAS_B200_FLAG_FORCE_TCGEN05 : d.flags, shrink_takes_mma_path(sp));
         if (plan.decode) {
-            // (t rows in lora_t are written by every call: the tiles a tcgen05 call leaves in `ws` are not what this kernel reads)
-            rc = launch_decode(d, d.seq_slot ? &sp : nullptr, st);
+            // t rows are written to lora_t by every call of up to eight tokens, and of up to sixteen where N >= 2 K.  Beyond, where calls
+            // of the same shape once left tiles in `ws` and were reused, they are read again as the call before has left them.  (Computed
+            // again / read, 8 of rank 16: 12 tokens x 4096 x 4096 10.9 / 9.5 us, 16 x 2048 x 4096 10.8 / 7.7.)
+            reuse_shrink = reuse_shrink && d.m > 8 && uint64_t(d.n) < 2ull * d.k;
+            rc = launch_decode(d, d.seq_slot && !reuse_shrink ? &sp : nullptr, st);
             if (rc == ATLAS_B200_OK) t_last_variant = ATLAS_B200_VARIANT_TCGEN05;
             return rc;
         }

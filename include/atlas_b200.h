@@ -61,9 +61,9 @@ extern "C" {
 #define ATLAS_B200_FLAG_REUSE_SHRINK   8u   /* tcgen05 path only: lora_t and ws still hold this call's shrink result (same x,
                                                seq_slot, tables, scale2, scratch and ACT_FP4 as the call that wrote it, which had
                                                none of the flags for comparison runs); skip the shrink launch.  Computed all the
-                                               same where that call left it in another form than this one reads: for the smallest
-                                               batches, K not a multiple of 256, ranks above 64, and calls with a comparison
-                                               flag that lay their LoRA activations out differently */
+                                               same where that call left it in another form than this one reads: for up to eight
+                                               tokens (sixteen where n >= 2 k), K not a multiple of 256, ranks above
+                                               64, and calls with a comparison flag that lay their LoRA activations out differently */
 #define ATLAS_B200_FLAG_ACT_FP4       16u   /* W4A4: the base product sees x quantised to NVFP4 (group of 16, E4M3 scale =
                                                group max / 6, tensor scale 1) and runs as a block-scaled FP4 x FP4 MMA; the
                                                LoRA term still sees exact x.  The opt-in W4A4 arm of the reference:

@@ -77,3 +77,18 @@ def test_reuse_after_a_plain_call(cuda, atlas, oracle, M, K, N, strided_ws):
         y, _ = dc.run(flags=flag | atlas.FLAG_REUSE_SHRINK, ws=left.clone() if strided_ws else None)
         assert np.array_equal(y, want), f"flag {flag}"
     assert atlas.device_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,max_rank", [(9, 1024, 1024, 16), (16, 4096, 4096, 32), (12, 5120, 1280, 48)])
+def test_reuse_beyond_eight_tokens(cuda, atlas, oracle, M, K, N, max_rank):
+    """FLAG_REUSE_SHRINK on the small-batch kernel, N < 2 K: the rows of t that the plain call left are read, not computed again."""
+    from atlas_b200 import synth
+    case = synth.make_case("reuse", M=M, K=K, N=N, ranks=[max_rank, 8], max_rank=max_rank, none_frac=0.1, scale2=0.02, b_std=0.1, seed=M)
+    dc = DeviceCase(cuda, atlas, case)
+    plain, _ = dc.run(lora_ws=True)
+    assert atlas.last_launch_shape()["token_tile"] == 8
+    assert np.array_equal(dc.run(lora_ws=True, flags=atlas.FLAG_REUSE_SHRINK)[0], plain)
+    dc.lora_t.zero_()
+    reused, _ = dc.run(lora_ws=True, flags=atlas.FLAG_REUSE_SHRINK)
+    assert np.array_equal(reused, dc.run(lora=False)[0]) and not np.array_equal(reused, plain)
+    assert atlas.device_status() == 0
