@@ -668,16 +668,25 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;
     t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
     if (shrink) {
-        // Gaps while the shrink runs, for pairs whose CTAs contract more than it takes (their MMAs leave no idle cycles): up to three CTAs
-        // to a long K, and up to 64 granules.  Without / before every other stage / before every stage / before every stage of the whole
-        // loop (us): 512 tokens x 4096 x 14336 8 of rank 16 59.3 / 52.3 / 53.4 / 57.9, 16 of rank 32 in sequences 87.5 / 74.4 / 73.2 /
-        // 79.2, 400 x 2560 x 6912 31.1 / 27.8 / 28.4 / 29.5, 1000 x 4096 x 14336 8 of rank 32 in sequences 123.9 / 111.1 / 112.7 / -; but
-        // 64 of rank 64 (several rounds of the shrink) 512 x 4096 x 14336 157.8 / 159.2, 512 x 2560 x 6912 79.1 / 80.6, four CTAs (130
-        // x 4096 x 14336) 34.7 / 36.5, 2048 of K to one of two (512 x 4096 x 4096) 25.2 / 25.8, K = 4096 (256 x 14336) 35.3 / 35.8, and
-        // single CTAs, which wait for shared memory (700 x 3072 x 9216) 38.7 / 41.6.
-        p.leave_gaps = PAIR && MT >= 256 && !A4 && k_split <= 3 && d.k > std::max(4096u, 2048u * k_split) && d.m <= 1024 &&
-                               uint64_t(d.max_loras) * ((d.max_rank + 15) / 16) <= 64 ? 1u : 0u;
-        t_last_shape[6] = p.leave_gaps;
+        // Gaps while the shrink runs, for pairs whose CTAs contract more than it takes (their MMAs leave no idle cycles).  Two or three CTAs
+        // to a long K, up to 64 granules: before every stage, up to rank 16 before every other.  Without / before every other / before every
+        // stage / before every stage of the whole loop (us): 512 tokens x 4096 x 14336 8 of rank 16 59.3 / 52.3 / 53.4 / 57.9, 16 of rank
+        // 32 in sequences 87.5 / 74.4 / 73.2 / 79.2, 280 tokens 8 of rank 32 in sequences 70.4 / 61.7 / 58.7 / 59.7, 400 x 2560 x 6912 8 of
+        // rank 16 31.1 / 27.8 / 28.4 / 29.5; but 64 of rank 64 (several rounds of the shrink) 512 x 4096 x 14336 157.8 /
+        // 159.2, four CTAs (130 x 4096 x 14336) 34.7 / 36.5, 2048 of K to one of two (512 x 4096 x 4096) 25.2 / 25.8, and single CTAs,
+        // which wait for shared memory (700 x 3072 x 9216) 38.7 / 41.6.
+        // One CTA: before every fourth, and only for more tokens than a tile, whose shrink is the longer one, of few granules.  Without /
+        // so / before every other stage: 1000 x 4096 x 14336 8 of rank 32 in sequences 125.5 / 114.8 / 112.7, of rank 16 95.2 / 90.7 / 90.9,
+        // 512 x 8192 x 6144 8 of rank 32 in sequences 52.1 / 47.5 / 47.1, of rank 16 (the dearest, a per cent) 42.9 / 43.3 / 43.5; but 256
+        // x 17408 x 5120 16 of rank 32 42.5 / 42.6 / 43.1, one of rank 16 (1000 x 4096 x 6144) 42.6 / 43.4 / 43.5, 32 of rank 32 (512 x
+        // 8192 x 8192) 72.6 / 73.4 / 73.7, K = 4096 (1000 x 4096, 16 of rank 32) 45.7 / - / 46.1.
+        const uint64_t granules = uint64_t(d.max_loras) * ((d.max_rank + 15) / 16);
+        p.leave_gaps = 0u;
+        if (PAIR && MT >= 256 && !A4 && d.k > 4096 && d.m <= 1024) {
+            if (k_split == 1) p.leave_gaps = d.m > uint32_t(MT) && granules > 1 && granules <= 32 ? 4u : 0u;
+            else p.leave_gaps = k_split <= 3 && d.k > 2048 * k_split && granules <= 64 ? (d.max_rank > 16 ? 1u : 2u) : 0u;
+        }
+        t_last_shape[6] = p.leave_gaps ? 1u : 0u;
         // A small batch: the mma.sync shrink releases this kernel as soon as it is resident, which then runs beside it.  A large one:
         // the tcgen05 shrink fills its SMs and releases this kernel at the same point, whose CTAs then take SMs that are free or
         // become so; the mma.sync shrink, where it has to stand in, keeps the machine to itself.

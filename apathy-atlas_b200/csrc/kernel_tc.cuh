@@ -181,7 +181,7 @@ struct Params {
     unsigned long long b_pool_base, b_slot_stride;   // ... of this address and slot stride (bytes)
     uint32_t wait_for_shrink;      // launched as a programmatic dependent of the shrink: wait before reading t
     uint32_t leave_gaps;           // pairs, 256-token tiles: while the shrink runs beside this kernel the MMA thread lets the tensor cores
-                                   //       run dry before every other stage
+                                   //       run dry before every stage of two K blocks (1), every second (2) or fourth (4), or never (0)
     uint32_t chained;              // launched as a programmatic dependent of whatever is before it (no adapters): wait before reading anything
     const uint8_t* w_scale_rows;   // non-null (A16, K not a multiple of 256): the scale rows [N][K/16] are read from here by the
                                    //       expansion warps, because TMA wants row strides of whole 16 bytes
@@ -971,7 +971,8 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             uint32_t s = 0, ph = 0, acc = 0;
             uint32_t bar_full = BAR_FULL, bar_empty = BAR_EMPTY;
             // (single CTAs never leave gaps, but keep the test: without it 512 tokens x 2048 x 8192, 8 of rank 16, take 28.5 instead of 27.9 us)
-            bool gaps = MT >= 256 && p.leave_gaps;
+            bool gaps = MT >= 256 && p.leave_gaps != 0u;
+            const uint32_t gap_mask = 2u * p.leave_gaps - 2u;
             if constexpr (A4) {
                 // four K=64 block-scaled instructions per stage; both operands are the packed tiles, the
                 // scales sit in this stage's TMEM columns
@@ -1005,10 +1006,10 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
                     if (!ok) break;
                     __syncwarp();
                     // MMAs of 256 columns queued behind one another leave the mma.sync of the shrink beside this kernel next to nothing: before
-                    // every other stage the one before has to be done (every EMPTY of it is committed), a gap of some 100 in 2048 cycles,
-                    // until the list warps have seen the shrink end
+                    // some stages the one before has to be done (every EMPTY of it is committed), a gap of some 100 cycles in the 1024 of
+                    // each stage since the last, until the list warps have seen the shrink end
                     gaps = gaps && !__any_sync(0xFFFFFFFFu, misc[4]);
-                    if (gaps && (it & 2u)) {
+                    if (gaps && it && (it & gap_mask) == gap_mask) {
                         ok = mbar_wait_warp(s ? bar_empty - 8 : BAR_EMPTY + 8 * (C::STAGES - 1), s ? ph : ph ^ 1u, abort_flag, STATUS_WAIT_EXPIRED_MMA, 32);
                         if (!ok) break;
                     }

@@ -95,7 +95,8 @@ def test_gaps_for_the_shrink(cuda, atlas, oracle, M, K, N, form):
 
 # either side of the lines: K, CTAs to a tile's K, granules, tokens, pairs, a shrink to run beside
 @pytest.mark.parametrize("M,K,N,ads,max_rank,flags,gaps", [
-    (1000, 4352, 4096, 4, 32, 0, True), (1000, 4096, 4096, 4, 32, 0, False), (512, 4352, 2560, 4, 32, 0, False), (512, 6400, 1024, 4, 32, 0, False),
+    (1000, 4352, 4096, 4, 32, 0, True), (1000, 4096, 4096, 4, 32, 0, False), (1000, 4352, 4096, 1, 16, 0, False),
+    (1000, 4352, 4096, 17, 32, 0, False), (256, 4352, 14336, 4, 32, 0, False), (260, 4352, 8192, 4, 32, 0, True), (512, 4352, 2560, 4, 32, 0, False), (512, 6400, 1024, 4, 32, 0, False),
     (400, 4608, 4096, 16, 64, 0, True), (400, 4608, 4096, 65, 16, 0, False), (400, 4608, 4096, 1, 8, 0, True), (300, 4608, 4096, 2, 16, "single", False),
     (400, 4608, 4096, 2, 16, "base", False), (1030, 4352, 1000, 2, 16, 0, False)])
 def test_which_calls_leave_gaps(cuda, atlas, oracle, M, K, N, ads, max_rank, flags, gaps):
