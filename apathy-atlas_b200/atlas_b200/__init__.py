@@ -477,10 +477,11 @@ def last_launch_shape() -> dict:
     _check("atlas_b200_last_launch_shape", lib().atlas_b200_last_launch_shape(out))
     per = (C.c_uint32 * 2)()
     _check("atlas_b200_last_persistent_shape", lib().atlas_b200_last_persistent_shape(per))
-    more = (C.c_uint32 * 1)()
+    more = (C.c_uint32 * 2)()
     _check("atlas_b200_last_launch_details", lib().atlas_b200_last_launch_details(more))
     return {"token_tile": out[0], "cta_pair": bool(out[1]), "k_split": out[2], "lora_tiles_from_shrink": bool(out[3]),
-            "persistent_tiles_per_pass": per[0], "persistent_cta_pairs": per[1], "gaps_for_shrink": bool(more[0])}
+            "persistent_tiles_per_pass": per[0], "persistent_cta_pairs": per[1], "gaps_for_shrink": bool(more[0]),
+            "weights_by_tma": bool(more[1])}
 
 
 def device_status(clear: bool = True) -> int:

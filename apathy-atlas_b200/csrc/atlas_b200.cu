@@ -38,7 +38,7 @@
 namespace atlas {
 
 static thread_local int t_last_variant = ATLAS_B200_VARIANT_NONE;
-static thread_local uint32_t t_last_shape[7] = {0, 0, 0, 0, 0, 0, 0};
+static thread_local uint32_t t_last_shape[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 static unsigned long long* g_profile_buf = nullptr;   // device buffer for per-CTA cycle counters (diagnostics)
 static size_t g_profile_words = 0;
 
@@ -666,7 +666,7 @@ static int launch_tc_as(const atlas_b200_linear_desc& d, int slot_idx, const Shr
     grid.z = k_split;
     p.k_split = k_split;
     t_last_shape[0] = MT; t_last_shape[1] = PAIR ? 1u : 0u; t_last_shape[2] = k_split; t_last_shape[3] = tt.tiles ? 1u : 0u;
-    t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
+    t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u; t_last_shape[7] = 0u;
     if (shrink) {
         // Gaps while the shrink runs, for pairs whose CTAs contract more than it takes (their MMAs leave no idle cycles).  Two or three CTAs
         // to a long K, up to 64 granules: before every stage, up to rank 16 before every other.  Without / before every other / before every
@@ -804,7 +804,7 @@ static int launch_tc_persist(const atlas_b200_linear_desc& d, int idx, const Shr
     p.lora_wide = lora_wide;
     const uint32_t pairs = std::min<uint32_t>(uint32_t(clusters), pp.n_tiles);
     t_last_shape[0] = MT; t_last_shape[1] = 1u; t_last_shape[2] = 1u; t_last_shape[3] = tt.tiles ? 1u : 0u;
-    t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs; t_last_shape[6] = 0u;
+    t_last_shape[4] = uint32_t(G); t_last_shape[5] = pairs; t_last_shape[6] = 0u; t_last_shape[7] = 0u;
     if (shrink) {
         const int rc = launch_shrink(*shrink, d.max_loras, st, d.m > 1024 ? MachineBeside::none : MachineBeside::all);
         if (rc) return rc;
@@ -848,6 +848,7 @@ static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParam
     w.x_row_stride = d.x_row_stride;
     const uint32_t ctas = (d.n + 16 * TILES - 1) / (16 * TILES);
     t_last_shape[0] = 8u; t_last_shape[1] = 0u; t_last_shape[2] = 1u; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
+    t_last_shape[7] = tma ? 1u : 0u;
     if (shrink) {
         rc = launch_shrink(*shrink, d.max_loras, st, ctas * 3 <= uint32_t(rt_sm_count()) * 2 ? MachineBeside::part : MachineBeside::all);
         if (rc) return rc;
@@ -1011,6 +1012,7 @@ static int launch_dense_tc(const atlas_b200_linear_desc& d, bool after_shrink, c
     uint32_t k_split = std::max(1u, std::min(std::min(uint32_t(rt_sm_count()) / std::max(tiles, 1u), 8u), d.k / uint32_t(tc::KB)));
     while (k_split & (k_split - 1)) --k_split;           // a power of two: clusters of 1, 2, 4 or 8
     t_last_shape[0] = mt; t_last_shape[1] = 0u; t_last_shape[2] = k_split; t_last_shape[3] = 0u; t_last_shape[4] = 0u; t_last_shape[5] = 0u; t_last_shape[6] = 0u;
+    t_last_shape[7] = 0u;
     if (mt == 16) return launch_dense_tc_mt<16>(d, 0, k_split, after_shrink, st);
     if (mt == 32) return launch_dense_tc_mt<32>(d, 1, k_split, after_shrink, st);
     if (mt == 64) return launch_dense_tc_mt<64>(d, 2, k_split, after_shrink, st);
@@ -1700,9 +1702,10 @@ int atlas_b200_last_persistent_shape(uint32_t out[2]) {
     return ATLAS_B200_OK;
 }
 
-int atlas_b200_last_launch_details(uint32_t out[1]) {
+int atlas_b200_last_launch_details(uint32_t out[2]) {
     if (!out) return ATLAS_B200_ERR_NULL;
     out[0] = t_last_shape[6];
+    out[1] = t_last_shape[7];
     return ATLAS_B200_OK;
 }
 

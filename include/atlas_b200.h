@@ -493,8 +493,9 @@ ATLAS_B200_API int atlas_b200_last_launch_shape(uint32_t out[4]);
 /* The persistent form of the most recent tcgen05 call on this thread: out[0] = token tiles per pass (0: the call ran one
  * output tile per CTA), out[1] = CTA pairs in the grid. */
 ATLAS_B200_API int atlas_b200_last_persistent_shape(uint32_t out[2]);
-/* More of it: out[0] = 1 if the call's MMAs left gaps for the shrink that ran beside it. */
-ATLAS_B200_API int atlas_b200_last_launch_details(uint32_t out[1]);
+/* More of it: out[0] = 1 if the call's MMAs left gaps for the shrink that ran beside it, out[1] = 1 if the kernel for the smallest
+ * batches had its weights brought by TMA. */
+ATLAS_B200_API int atlas_b200_last_launch_details(uint32_t out[2]);
 /* Per-CTA cycle counters of the tcgen05 kernel, the counterpart of the reference's per-phase timers
  * (crates/spark-model/src/layers/qwen3_attention/trait_impl/multi_seq/mod.rs:125-141).  While a device
  * buffer of `n_words` u64 is set (16 words per CTA, CTA index = blockIdx.y * gridDim.x + blockIdx.x) each

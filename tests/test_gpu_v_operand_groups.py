@@ -35,11 +35,11 @@ def test_every_length_of_the_base_loop(cuda, atlas, oracle, M, K, form):
     assert atlas.device_status() == 0
 
 
-# two K blocks of 256-token tiles on their own hold two stages: a ring that wraps before the expansion has waited for it
+# 256-token tiles by single CTAs: a ring of four stages of one K block, beside groups of four, that wraps before the expansion has waited for it
 @pytest.mark.parametrize("K", [1280, 2560, 4096])
-def test_a_ring_of_two_stages(cuda, atlas, oracle, K):
+def test_a_ring_of_single_blocks(cuda, atlas, oracle, K):
     from atlas_b200 import synth
-    case = synth.make_case("two_stages", M=256, K=K, N=8704, ranks=[32] * 16, max_rank=32, none_frac=0.1, scale2=0.02, b_std=0.1, seed=K)
+    case = synth.make_case("single_blocks", M=256, K=K, N=8704, ranks=[32] * 16, max_rank=32, none_frac=0.1, scale2=0.02, b_std=0.1, seed=K)
     dc = DeviceCase(cuda, atlas, case)
     y, _ = dc.run(flags=atlas.FLAG_NO_CTA_PAIR, lora_ws=True)
     assert not atlas.last_launch_shape()["cta_pair"]

@@ -5,11 +5,12 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-# small-batch kernel; one-tile kernel, its scales by TMA, from rows, and with a split K; pairs; persistent kernel (the last; FP4 too)
-@pytest.mark.parametrize("m,k,fp4", [(1, 1024, False), (8, 2080, False), (16, 736, False), (20, 1024, False), (60, 736, False), (60, 4096, False),
+# small-batch kernel, weights by the warps' loads and by TMA; one-tile kernel, its scales by TMA, from rows, and with a split K; pairs; persistent kernel (the last; FP4 too)
+@pytest.mark.parametrize("m,k,fp4", [(1, 1024, False), (8, 2080, False), (16, 736, False), (1, 8192, False), (8, 8192, False), (20, 1024, False), (60, 736, False), (60, 4096, False),
                                      (250, 2048, False), (250, 2048, True), (2048, 2560, False), (2048, 2560, True)])
 def test_a_chain_without_adapters(cuda, atlas, m, k, fp4):
     torch = cuda
+    tma = m <= 8 and k * k >= 1 << 26
     g = torch.Generator(device="cuda")
     g.manual_seed(m + k)
     passes = 12
@@ -25,6 +26,7 @@ def test_a_chain_without_adapters(cuda, atlas, m, k, fp4):
         for i in range(passes):
             atlas.nvfp4_lora_linear(atlas.make_linear_desc(x=xs[i], m=m, k=k, n=k, y=xs[i + 1], w_packed=weights[i % 2], w_scale=scales,
                                                            scale2=0.3 * k ** -0.5, ws=ws, ws_bytes=ws.numel(), flags=flags))
+            assert atlas.last_launch_shape()["weights_by_tma"] == tma
             if sync:
                 torch.cuda.synchronize()
         torch.cuda.synchronize()

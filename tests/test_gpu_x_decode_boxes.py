@@ -34,8 +34,12 @@ def test_rows_of_a_large_layer(cuda, atlas, m, n, k, loras, rank):
                                    ws=ws, ws_bytes=ws.numel(), **kw)
         atlas.nvfp4_lora_linear(d)
         torch.cuda.synchronize()
+        shape = atlas.last_launch_shape()
+        assert shape["token_tile"] == 8 and shape["weights_by_tma"] == (b - a == n and tma)
         return y.view(torch.int16)
 
+    # (the slices have less than 2^26 weights, or fewer than 2^24; where the batch has too few granules both sides are the warps' loads)
+    tma = n * k >= 1 << 26 or min(loras, m) * ((rank + 15) // 16) >= 16
     want = torch.cat([call(a, min(a + 2048, n)) for a in range(0, n, 2048)], dim=1)
     assert torch.isfinite(want.view(torch.bfloat16)).all()
     for _ in range(3):
