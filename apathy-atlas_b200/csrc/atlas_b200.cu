@@ -121,7 +121,8 @@ static int rt_sm_count() { DeviceState* st = device_state(); return st ? st->sm_
 
 // Encoded tensor maps are a pure function of (address, shape, strides, box, type, swizzle): a serving loop calls with the
 // same tensors step after step, so recent encodings are kept per host thread and a repeated call costs a compare instead of a
-// driver call per map.  A 32-layer model has some 1300 maps per batch shape: 4096 are held, in sets of four of which the least
+// driver call per map.  A 32-layer model has some 1300 maps per batch shape (some 1500 with adapters of rank 32 or 64, whose B
+// is fetched in boxes of two widths; 450 where the smallest batches have their weights by TMA): 4096 are held, in sets of four of which the least
 // recently used one is replaced (1 MiB per calling thread, allocated at its first call and given back when the thread ends; with
 // no memory for it every map is encoded anew).  With 64 entries a decode step of one layer evicted its own maps and spent about
 // half of its host time (145 us) in the driver's encoder.
@@ -895,6 +896,9 @@ static int launch_decode_form(const atlas_b200_linear_desc& d, const ShrinkParam
 // 13.5, 16 14.8 / 14.2, 32 18.7 / 15.7; 14336 x 4096 8 17.8 / 18.3, 16 22.9 / 20.4, 32 28.5 / 23.7; 4096 x 14336 8 18.5 / 18.1, 16 26.1 /
 // 18.6, 24 32.4 / 19.9; but 11008 x 4096 16 18.7 / 19.1, 2560 x 2560 16 8.2 / 9.0, 64 13.7 / 13.6.  Large layers whatever the batch: 8192 x
 // 8192 one token, no adapters 15.7 / 15.3, 28672 x 8192 44.8 / 42.8, 8192 x 28672 48.1 / 43.3, 8 tokens of 8 x 64 x 28672 x 8192 73 / 59.
+// What a batch uses of the granules that it could is not known on the host.  8 tokens of 32 x 32, all different / most without an adapter:
+// 4096 x 4096 15.2 / 12.6, 10.0 / 10.8; 5120 x 5120 17.3 / 15.8, 13.9 / 13.6; 8192 x 4096 18.8 / 18.7, 13.3 / 13.7; 14336 x 4096 27.8 /
+// 22.7, 19.1 / 19.4; 4096 x 14336 33.2 / 20.9, 25.7 / 19.1; 4 tokens of one among 32 x 128, 3072 x 14336 18.6 / 19.9.
 static bool decode_by_tma(const atlas_b200_linear_desc& d) {
     const uint64_t weights = uint64_t(d.n) * d.k, granules = d.seq_slot ? std::min(d.max_loras, d.m) * ((d.max_rank + 15) / 16) : 0u;
     return d.k % tc::KRAW == 0 && (weights >= 1u << 26 || (weights >= 1u << 24 && granules >= 16));
@@ -914,14 +918,20 @@ static int launch_decode_as(const atlas_b200_linear_desc& d, const ShrinkParams*
 //                        16 tokens   1024 x 4096 7.7/10.5  4096 x 4096 11.6/12.8  14336 x 4096 24.6/22.1  4096 x 14336 28.8/21.9  28672 x 8192 69/67
 //   32 of rank 64        8 tokens    1024 x 4096 13.5/13.5 4096 x 4096 16.2/17.6  14336 x 4096 29.5/26.5  4096 x 14336 29.6/31.4  28672 x 8192 66/73
 // With adapters the shrink runs beside it, and this kernel leaves that less of the memory system than the tcgen05 form does.
-// N >= 2 K: up to eight tokens whatever the batch; beyond, a granule (16 ranks of a slot) costs it some 0.3 us more than the other, against
-// what it gains on the weights, most where those are more than one wave of tiles there.  The pool's size moves no call across that line
-// below 32 granules: a token's bits there do not depend on the adapters that are loaded.
+// Without adapters, and for N >= 2 K up to eight tokens and beyond them up to 32 granules, it is taken whatever the sizes, although the
+// other is ahead at both tables' ends (16 tokens, no adapters, x 4096 x 14336; 8 of 32 x 64 x 14336 x 4096): a row without an adapter has
+// the bits of the call without adapters, and a token's do not depend on the adapters that are loaded, only where all of these run here.
+// N >= 2 K, beyond that: a granule (16 ranks of a slot) costs it some 0.3 us more than the other, against what it gains on the weights, most
+// where those are more than one wave of tiles there.
 // N < 2 K, up to eight tokens: it loses only to many granules and where a long K meets so few features that the other splits it (8 tokens
 // of 32 of rank 16 x 4096 x 14336 24.3/21.7, 2 of rank 64 22.0/21.2; but of 32 of rank 64 29.6/31.4, 4 of rank 32 x 13824 x 14336 43/56).
-// Beyond eight (two n-tiles, no weights by TMA) both are estimated, in us: this kernel by its weights, the length of a CTA's loop and its
-// granules, the other by the K blocks a CTA takes one behind the other; measured from K = 1024 on.  12 tokens, 8 of rank 16 x 1024 x 4096
-// 7.3/10.3, x 4096 x 4096 10.9/12.7, x 8192 x 8192 21.9/22.5, but x 5120 x 5120 15.0/14.1 and 32 of rank 64 x 4096 x 4096 20.6/18.7.
+// Beyond eight granules it is ahead or even there again, its weights coming by TMA from 2^24 of them on, the other's granules a chain of
+// their own behind the loop: 8 tokens, 16 granules of rank 32 / 32 of rank 64, x 136 x 14336 14.4/17.2, 16.3/17.7, x 1024 x 14336 14.9/16.2,
+// 19.1/18.7, x 2048 x 14336 16.5/17.8, 20.3/19.5, x 4096 x 14336 19.9/21.7, 22.8/22.6; 12 granules (6 tokens of 8 of rank 32), still by
+// the warps' loads, x 136 x 14336 13.2/16.7, but x 3072 x 14336 20.8/18.7.
+// Beyond eight tokens (two n-tiles, no weights by TMA) both are estimated, in us: this kernel by its weights, the length of a CTA's loop and
+// its granules, the other by the K blocks a CTA takes one behind the other; measured from K = 1024 on.  12 tokens, 8 of rank 16 x 1024 x
+// 4096 7.3/10.3, x 4096 x 4096 10.9/12.7, x 8192 x 8192 21.9/22.5, but x 5120 x 5120 15.0/14.1 and 32 of rank 64 x 4096 x 4096 20.6/18.7.
 static bool decode_pays(const atlas_b200_linear_desc& d) {
     if (d.m > uint32_t(DCM_MAX_TOKENS)) return false;
     if (!d.seq_slot) return true;

@@ -37,9 +37,11 @@ __device__ __forceinline__ void record_status(uint32_t code) { atomicCAS(&g_stat
 //   neither                    a main kernel over a t that an earlier call left, and the small-batch kernel for more than eight tokens without
 //                              adapters, release but are launched in order; the NVFP4 decode, the maximum, the CUDA-core linear and
 //                              expand do neither
-// A dependent begins with the wait, with two exceptions:
+// A dependent begins with the wait, with three exceptions:
 //   the main kernel and the dense linear behind their shrink read x, weights and routing ahead of it: that shrink has waited before
 //   releasing them; they wait before they read t, or before they end, on every path, so that nothing behind them overtakes the shrink;
+//   the main kernel without adapters, its scales by TMA or from rows: only the warps that read memory begin with the wait, and the others
+//   work on what those bring;
 //   lora_shrink_mma_kernel looks at seq_slot, a_table and rank_table while the kernel ahead may still be writing them.  Those values
 //   only choose lines of A to prefetch, out of the declared pool alone; they are read past the first-level cache, and everything is
 //   read again behind the wait.

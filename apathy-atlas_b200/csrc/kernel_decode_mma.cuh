@@ -13,8 +13,9 @@
 // A CTA owns 16 * TILES features and all of K.  Interleaved 128-wide K steps make eight partial sums, one to each of eight warps or
 // two to each of four (with as many more CTAs on an SM): the same bits, so that either form may be taken for any batch and pool, and
 // a row without an adapter is the base call's.  Per thread and feature row a step is one 128-bit load of 32 codes and their two scale
-// bytes, the next step's loads in flight while one is multiplied; the partial sums are added in their order through shared
-// memory.  No cluster, no tensor memory, no barriers but two.
+// bytes, from global memory with the next step's loads in flight while one is multiplied, or (TMA) from a ring in shared memory that
+// a warp of its own fills; the partial sums are added in their order through shared memory.  No cluster, no tensor memory; but for the
+// ring's barriers, two.
 // The MMA's M is 16 features, its N 8 tokens (NT of them side by side).
 //
 // LoRA: granule j (16 ranks) of slot s is one more K step of partial sum (s + 3 j) % 8, so that the order in which a token's terms
@@ -51,7 +52,7 @@ template <int TILES, int WARPS> struct DcmRing {
 // is before it (instances of their own: the wait in all of them cost calls with adapters 1 to 2 %).  Those release late: a next grid
 // that comes while this one's CTAs are all at work takes the places they happen to leave, and its SMs get unequal numbers of CTAs.  One
 // token behind one another, launched in order / released at the start / behind the loop (us): 11008 x 4096 12.8 / 14.4 / 11.9, 2048 x
-// 2048 2.8 / - / 2.4; 12 tokens x 1280 x 17408 14.1 / 20.4 / 15.2.  SELFTEST: nothing fills the ring, and every wait on it runs out.
+// 2048 2.8 / - / 2.4.  (Two n-tiles have no such instance: 12 tokens x 1280 x 17408 14.1 / 20.4 / 15.2.)  SELFTEST: nothing fills the ring, and every wait on it runs out.
 template <int TILES, int NT, int WARPS, bool TMA, bool BASE, bool SELFTEST = false>
 __global__ void __launch_bounds__(32 * (WARPS + (TMA ? 1 : 0)), 16 / WARPS)
 nvfp4_lora_decode_mma_kernel(const DecodeParams w, const tc::Params p, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_s) {

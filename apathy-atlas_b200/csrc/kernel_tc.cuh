@@ -67,7 +67,7 @@ constexpr int EPI_WARPS = 4 + DEQ_WARPS;   // warps that take part in the epilog
 constexpr int MAX_LORAS_TC = 4096;
 constexpr int MAX_RANK_TC = 128;
 // a granule list entry: slot << GRAN_SHIFT | which 16 ranks of the slot (4096 slots of up to eight granules in 16 bits)
-// GRAN_WIDE (one-tile kernel): it and the next Params::lora_wide - 1 come in one copy
+// GRAN_WIDE: it and the next Params::lora_wide - 1 come in one copy of B_s
 constexpr uint32_t GRAN_SHIFT = 3, GRAN_MASK = 7, GRAN_WIDE = 0x8000u;
 static_assert(MAX_RANK_TC / 16 <= int(GRAN_MASK) + 1 && (MAX_LORAS_TC << GRAN_SHIFT) <= int(GRAN_WIDE), "granule list entries are 16 bits");
 constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;    // 1 s
@@ -908,7 +908,7 @@ nvfp4_lora_linear_tc_kernel(const __grid_constant__ CUtensorMap map_x,
             }
         }
         if (lane == 0 && !A4) {
-            // Activation tiles, one per K block (the raw weight stages have a producer of their own).
+            // Activation tiles, X_BLOCKS K blocks to a stage (the raw weight stages have a producer of their own).
             // CTAs start their K loop at different K offsets (a rotation in units of one raw stage),
             // so concurrently running CTAs do not all pull the same activation lines at one moment.
             uint32_t s = 0, ph = 0;

@@ -256,7 +256,7 @@ nvfp4_lora_linear_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_x
             }
         }
         if (lane == 0 && !A4) {
-            // activation tiles: one stage per K block, G tiles each (the raw weight stages have a producer of their own)
+            // activation tiles: XB K blocks to a stage, G tiles each (the raw weight stages have a producer of their own)
             uint32_t xs = 0, xph = 0;
             bool ok = true;
             for (uint32_t i = 0; ok && i < my_tiles; ++i) {
