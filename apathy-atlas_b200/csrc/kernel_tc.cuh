@@ -143,7 +143,10 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
         return k_split < 2 ? 0 : (split_bytes(k_split) > most_split_bytes(k_split - 1) ? split_bytes(k_split) : most_split_bytes(k_split - 1));
     }
     static constexpr int STAGING_RINGS = STAGING_BASE > L_STAGES * L_BLOCK ? STAGING_BASE : L_STAGES * L_BLOCK;
-    static constexpr int STAGING_BYTES = STAGING_RINGS > most_split_bytes() ? STAGING_RINGS : most_split_bytes();
+    // (They run on into the lists behind the staging area, which are dead by then.  With an area of 168 KB of its own the shrink lost room
+    // beside 256-token tiles by single CTAs: 200 tokens x 4096 x 14336, 16 of rank 32 in sequences 40.4 -> 42.0 us.)
+    static constexpr int LIST_BYTES = MT * 4 + MAX_GRANULES * 2 + (MAX_LORAS_TC / 32) * 4;
+    static constexpr int STAGING_BYTES = STAGING_RINGS > most_split_bytes() - LIST_BYTES ? STAGING_RINGS : most_split_bytes() - LIST_BYTES;
     static constexpr int OFF_KEY = STAGING_BYTES;                                // uint32[MT]  (scratch of the list build)
     static constexpr int OFF_GRAN = OFF_KEY + MT * 4;                            // uint16[MAX_GRANULES]
     static constexpr int OFF_BITMAP = OFF_GRAN + MAX_GRANULES * 2;               // uint32[128]
@@ -154,6 +157,7 @@ template <int MT, bool A4 = false, bool PAIR = false> struct Cfg {
     static_assert(!PAIR || MT >= 128, "pairs are built for token tiles of 128 and 256");
     static_assert(TMEM_NEEDED <= 512, "tensor memory budget");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
+    static_assert(most_split_bytes() <= OFF_BAR && STAGING_BYTES % 16 == 0, "partial tiles end before the barriers");
 };
 
 struct Params {
